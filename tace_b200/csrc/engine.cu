@@ -597,6 +597,27 @@ struct Model : ModelBase {
     for (auto& e : weights) {
       if (e.name == name) {
         if (numel != e.numel) return TACE_ERR_INVALID_ARGUMENT;
+        std::vector<T> cubic;
+        if (e.name.size() > 5 && e.name.compare(e.name.size() - 5, 5, ".rtab") == 0) {
+          // the table arrives as (value, h slope) at both ends of every interval; the kernels evaluate the same cubic in its
+          // power basis (three multiply-adds for the weight, two more for its derivative, instead of four and four)
+          const T* in = static_cast<const T*>(host);
+          cubic.resize((size_t)numel);
+          for (int64_t k = 0; k + 3 < numel; k += 4) {
+            const double v0 = in[k], m0 = in[k + 1], v1 = in[k + 2], m1 = in[k + 3];
+            cubic[k] = in[k]; cubic[k + 1] = in[k + 1];
+            cubic[k + 2] = T(3.0 * (v1 - v0) - 2.0 * m0 - m1);
+            cubic[k + 3] = T(2.0 * (v0 - v1) + m0 + m1);
+          }
+          if constexpr (std::is_same<T, float>::value) {
+            if (tp_wide_channels(C)) {
+              std::vector<float> pairs(cubic.size());
+              tp_wide_table(cubic.data(), pairs.data(), numel / (4 * C), C);
+              cubic.swap(pairs);
+            }
+          }
+          host = cubic.data();
+        }
         if (cudaMemcpy(arena + e.offset, host, sizeof(T) * (size_t)numel, cudaMemcpyHostToDevice) != cudaSuccess)
           return TACE_ERR_CUDA;
         if (e.name == "bessel") memcpy(host_bessel, host, sizeof(T) * kNumBessel);
@@ -1260,8 +1281,8 @@ struct Model : ModelBase {
         TPArgs<T> ta;
         memset(&ta, 0, sizeof(ta));
         ta.L = L; ta.scalar_src = p.scalar_src; ta.Lin = Ln; ta.C = C; ta.n_seg = na; ta.rowptr = b.rowptr_dst + a0;
-        ta.e_src = b.e_src; ta.Y = b.Y; ta.W = lb.W; ta.x = x_src; ta.M = lb.M + (long long)a0 * p.tp.NM * C; ta.e_base = e0;
-        ta.env = b.env;
+        ta.e_src = b.e_src; ta.Y = b.Y; ta.W = lb.W; ta.x = x_src; ta.M = lb.M + (long long)a0 * p.tp.NM * C; ta.e_base = e0; ta.n_edges = Ec;
+        ta.split_sums = lb.xx == nullptr; ta.env = b.env;
         if (rt_K) { ta.rtab = w(pre + "rtab"); ta.rt_K = rt_K; ta.rt_inv_h = T(rt_K) / T(cfg.cutoff); ta.dlen = b.dlen; }
         if (split) {  // targets that read owned rows only (final in x itself); the others once the ghost rows have arrived
           ta.x = lb.x; ta.row_ids = b.row_ids; ta.row_split = b.row_split + 1; ta.row_part = 0;
@@ -1528,7 +1549,7 @@ struct Model : ModelBase {
         memset(&ta, 0, sizeof(ta));
         ta.L = L; ta.scalar_src = p.scalar_src; ta.Lin = Ln; ta.C = C; ta.e_src = b.e_src; ta.Y = b.Y;
         ta.W = lb.W; ta.x = lb.xx ? lb.xx : lb.x; ta.gM = lb.M + (long long)a0 * p.tp.NM * C; ta.n_seg = na;
-        ta.rowptr = b.rowptr_dst + a0; ta.dW = lb.W; ta.dY = b.dY; ta.e_base = e0;
+        ta.rowptr = b.rowptr_dst + a0; ta.dW = lb.W; ta.dY = b.dY; ta.e_base = e0; ta.n_edges = Ec;
         ta.accumulate_dY = (t != NL_ - 1); ta.dxe = p.scalar_src ? nullptr : b.dxe;
         ta.env = b.env; ta.denv = b.denv; ta.accumulate_denv = (t != NL_ - 1);
         if (rt_K) {

@@ -274,8 +274,197 @@ def gen_interaction(L, Lin, out):
                 o(f"    dY[{l2 * l2 + m2}] += w{p} * ({' + '.join(ts)});")
         o("  }")
     o("  }")
+    gen_interaction_wide(L, Lin, out, paths, lay, Ks, xoff)
     o("};")
     return dict(tag=tag, P=P, nm=lay.nm, ng=ng, nnz=nnz_total, groups=groups, gcnt=grp_gcnt, nmg=grp_nm)
+
+
+WIDE_MAX_OUT, WIDE_MAX_IN = 40, 7  # message / source components per forward group: what 128 registers hold for two channels
+
+
+def wide_groups(in1, outs_of):
+    """Source ranks in order, as few contiguous groups as the register limits allow."""
+    groups = []
+    for l1 in in1:
+        if groups and sum(outs_of[l] for l in groups[-1] + [l1]) <= WIDE_MAX_OUT and sum(2 * l + 1 for l in groups[-1] + [l1]) <= WIDE_MAX_IN:
+            groups[-1].append(l1)
+        else:
+            groups.append([l1])
+    return groups
+
+
+def gen_interaction_wide(L, Lin, out, paths, lay, Ks, xoff):
+    """The same contraction for kernels in which a thread owns 2 NV channels of an edge (NV pairs, ``F2`` arithmetic: one
+    packed fp32 instruction works on a pair, coupling entries are broadcast operands), fp32 only.  Paths are walked source
+    rank (l1) major, so only one rank block of the source features and of their gradient is live at a time, and the forward
+    groups (a warp's share each) are cut between source ranks: no source component, coupling entry or weight is read twice.
+
+    * ``v_order(i)``: path at position i of the walk, ``v_p0 / v_np``: positions of a group;
+    * ``build_v<g>``: coupling row of one edge for group g, entries in the order the code below reads them;
+    * ``fwd_v<g>``: acc[k] += w_p sum_m1 G[m1][m3] x[m1] for the components k of group g (``vmap<g>(k)``: message row);
+    * ``bwd_v``: as ``bwd_w``, for the thread's channels: dE/dY summed over them before the coupling is applied.
+
+    Weights come from an accessor: ``get<i>`` for the path at position i, ``put<i>`` for its gradient (backward)."""
+    scalar_src = Lin < 0
+    D = (L + 1) ** 2
+    o = out.append
+    order = sorted(range(len(paths)), key=lambda p: (paths[p][0], p))
+    nz = {p: [(m3, m1) for m3 in range(2 * paths[p][2] + 1) for m1 in range(2 * paths[p][0] + 1) if np.any(Ks[p][m1, :, m3] != 0.0)]
+          for p in order}
+    l1s = sorted({paths[p][0] for p in order})
+    rank_groups = wide_groups(l1s, {l: sum(2 * paths[p][2] + 1 for p in order if paths[p][0] == l) for l in l1s})
+    groups = [[p for p in order if paths[p][0] in ls] for ls in rank_groups]
+    gi, goff, gcnt = {}, [], []
+    n = 0
+    for ps in groups:
+        goff.append(n)
+        for p in ps:
+            for m3, m1 in nz[p]:
+                gi[(p, m1, m3)] = n
+                n += 1
+        n = (n + 3) // 4 * 4
+        gcnt.append(n - goff[-1])
+    # distance between the rows of two edges: an odd number of 16-byte pieces, so that the eight lanes of a store phase hit
+    # different banks
+    odd4 = lambda c: c if (c // 4) % 2 else c + 4
+    o(f"  static constexpr int NGV = {len(groups)}, GV = {n}, GVS = {odd4(n)}, GVMAX = {max(odd4(c) for c in gcnt)}, OUTMAX = "
+      f"{max(sum(2 * paths[p][2] + 1 for p in ps) for ps in groups)}, INMAX = {max(sum(2 * l + 1 for l in ls) for ls in rank_groups)};")
+    for name, arr in [("v_goff", goff), ("v_nout", [sum(2 * paths[p][2] + 1 for p in ps) for ps in groups]),
+                      ("v_x0", [xoff[ls[0]] for ls in rank_groups]), ("v_nx", [sum(2 * l + 1 for l in ls) for ls in rank_groups]),
+                      ("v_p0", [order.index(ps[0]) for ps in groups]), ("v_np", [len(ps) for ps in groups])]:
+        body = "".join(f"g == {g} ? {v} : " for g, v in enumerate(arr[:-1])) + str(arr[-1])
+        o(f"  static TACE_HD constexpr int {name}(int g) {{ return {body}; }}")
+    o(f"  template <int I> static TACE_HD constexpr int v_order() {{ constexpr int m[{len(order)}] = {{{', '.join(map(str, order))}}}; return m[I]; }}")
+    o("  template <int GRP> static TACE_HD TACE_INLINE int vmap(int k) {")
+    for g, ps in enumerate(groups):
+        rows = [lay.idx(p, m3) for p in ps for m3 in range(2 * paths[p][2] + 1)]
+        o(f"    if constexpr (GRP == {g}) {{ constexpr int m[{len(rows)}] = {{{', '.join(map(str, rows))}}}; return m[k]; }}")
+    o("  }")
+    # coupling rows
+    o("  template <int GRP> static TACE_HD TACE_INLINE void build_v(const float (&Y)[%d], float* __restrict__ G) {" % D)
+    for g, ps in enumerate(groups):
+        o(f"    if constexpr (GRP == {g}) {{")
+        exprs = []
+        for p in ps:
+            l1, l2, l3 = paths[p]
+            for m3, m1 in nz[p]:
+                exprs.append(" + ".join(f"float({float(Ks[p][m1, m2, m3])!r}) * Y[{l2 * l2 + m2}]" for m2 in range(2 * l2 + 1)
+                                        if Ks[p][m1, m2, m3] != 0.0))
+        while len(exprs) % 4:
+            exprs.append("0.0f")
+        for j in range(0, len(exprs), 4):
+            o(f"      st4(G + {j}, {', '.join(exprs[j:j + 4])});")
+        o("    }")
+    o("  }")
+
+    class Loader:
+        """128-bit reads of the coupling row, each where its first entry is needed."""
+
+        def __init__(self, base):
+            self.base, self.done = base, set()
+
+        def get(self, i):
+            j = (i - self.base) // 4
+            if j not in self.done:
+                self.done.add(j)
+                o(f"      float G_{4 * j}, G_{4 * j + 1}, G_{4 * j + 2}, G_{4 * j + 3}; "
+                  f"ld4(G + {4 * j}, G_{4 * j}, G_{4 * j + 1}, G_{4 * j + 2}, G_{4 * j + 3});")
+            return f"G_{i - self.base}"
+
+    V = "_Pragma(\"unroll\") for (int v = 0; v < NV; ++v)"
+    # forward: x[k]: source component v_x0 + k of this thread's channels
+    o("  template <int GRP, int NV, typename WF> static TACE_HD TACE_INLINE void fwd_v(const F2 (&x)[INMAX][NV], const float* __restrict__ G, "
+      "WF& wf, F2 (&acc)[OUTMAX][NV]) {")
+    for g, ps in enumerate(groups):
+        o(f"    if constexpr (GRP == {g}) {{")
+        ld = Loader(goff[g])
+        k0, x0 = 0, xoff[rank_groups[g][0]]
+        for p in ps:
+            l1, l2, l3 = paths[p]
+            o(f"      F2 w{p}[NV]; wf.template get<{order.index(p)}>(w{p});")
+            X = lambda m1: f"x[{xoff[l1] + m1 - x0}]"
+            if l1 <= l3:  # weight the source components (fewer than the outputs)
+                for m1 in range(2 * l1 + 1):
+                    o(f"      F2 y{p}_{m1}[NV]; {V} y{p}_{m1}[v] = mul2(w{p}[v], {X(m1)}[v]);")
+                for m3 in range(2 * l3 + 1):
+                    for m1 in range(2 * l1 + 1):
+                        if (p, m1, m3) in gi:
+                            e = ld.get(gi[(p, m1, m3)])
+                            o(f"      {V} acc[{k0 + m3}][v] = fma2s({e}, y{p}_{m1}[v], acc[{k0 + m3}][v]);")
+            else:  # contract first, weight the outputs
+                for m3 in range(2 * l3 + 1):
+                    first = True
+                    for m1 in range(2 * l1 + 1):
+                        if (p, m1, m3) in gi:
+                            e = ld.get(gi[(p, m1, m3)])
+                            if first:
+                                o(f"      F2 z{p}_{m3}[NV]; {V} z{p}_{m3}[v] = mul2s({e}, {X(m1)}[v]);")
+                            else:
+                                o(f"      {V} z{p}_{m3}[v] = fma2s({e}, {X(m1)}[v], z{p}_{m3}[v]);")
+                            first = False
+                    if not first:
+                        o(f"      {V} acc[{k0 + m3}][v] = fma2(w{p}[v], z{p}_{m3}[v], acc[{k0 + m3}][v]);")
+            k0 += 2 * l3 + 1
+        o("    }")
+    o("  }")
+    # backward: x through xs.load, dx through xs.store, message gradient through gm.load<row>, weights through wf
+    o(f"  template <int NV, typename XS, typename GM, typename WF> static TACE_HD TACE_INLINE void bwd_v(XS& xs, GM& gm, "
+      f"const float* __restrict__ G, WF& wf, float (&dY)[{D}]) {{")
+    flat = [p for ps in groups for p in ps]
+    have = None
+
+    def close(l1):
+        if not scalar_src:
+            for m1 in range(2 * l1 + 1):
+                o(f"      xs.template store<{xoff[l1] + m1}>(d{l1}_{m1});")
+        o("    }")
+
+    ld = Loader(0)
+    for ip, p in enumerate(flat):
+        l1, l2, l3 = paths[p]
+        K = Ks[p]
+        if have != l1:
+            if have is not None:
+                close(have)
+            have = l1
+            o("    {")
+            ld.done = set()  # reads cannot cross the scope
+            for m1 in range(2 * l1 + 1):
+                o(f"      F2 x{l1}_{m1}[NV]; xs.template load<{xoff[l1] + m1}>(x{l1}_{m1});")
+            if not scalar_src:
+                for m1 in range(2 * l1 + 1):
+                    o(f"      F2 d{l1}_{m1}[NV]; {V} d{l1}_{m1}[v] = F2{{0.0f, 0.0f}};")
+        o(f"      F2 w{p}[NV]; wf.template get<{ip}>(w{p});")
+        started = set()
+        for m3 in range(2 * l3 + 1):
+            used = [m1 for m1 in range(2 * l1 + 1) if (p, m1, m3) in gi]
+            if not used:
+                continue
+            o(f"      F2 g{p}_{m3}[NV]; gm.template load<{lay.idx(p, m3)}>(g{p}_{m3});")
+            for m1 in used:
+                e = ld.get(gi[(p, m1, m3)])
+                if m1 in started:
+                    o(f"      {V} u{p}_{m1}[v] = fma2s({e}, g{p}_{m3}[v], u{p}_{m1}[v]);")
+                else:
+                    started.add(m1)
+                    o(f"      F2 u{p}_{m1}[NV]; {V} u{p}_{m1}[v] = mul2s({e}, g{p}_{m3}[v]);")
+            o(f"      F2 h{p}_{m3}[NV]; {V} h{p}_{m3}[v] = mul2(w{p}[v], g{p}_{m3}[v]);")
+            for m1 in used:
+                o(f"      const float t{p}_{m1}_{m3} = dot2<NV>(x{l1}_{m1}, h{p}_{m3});")
+            for m2 in range(2 * l2 + 1):
+                for m1 in used:
+                    if K[m1, m2, m3] != 0.0:
+                        o(f"      dY[{l2 * l2 + m2}] += float({float(K[m1, m2, m3])!r}) * t{p}_{m1}_{m3};")
+        us = sorted(started)
+        o(f"      F2 q{p}[NV]; {V} q{p}[v] = mul2(x{l1}_{us[0]}[v], u{p}_{us[0]}[v]);")
+        for m1 in us[1:]:
+            o(f"      {V} q{p}[v] = fma2(x{l1}_{m1}[v], u{p}_{m1}[v], q{p}[v]);")
+        o(f"      wf.template put<{ip}>(q{p});")
+        if not scalar_src:
+            for m1 in us:
+                o(f"      {V} d{l1}_{m1}[v] = fma2(w{p}[v], u{p}_{m1}[v], d{l1}_{m1}[v]);")
+    close(have)
+    o("  }")
 
 
 # ------------------------------------------------------------- product basis code

@@ -42,10 +42,13 @@ struct TPArgs {
   const T* env;       // [E] or nullptr
   T* denv;            // [E] or nullptr
   int accumulate_denv;
+  long long n_edges;  // edges of the n_seg targets together (launch shapes)
+  int split_sums;     // the forward sum of one target may be cut into parts (off where partial passes must give the same bits)
   long long e_base;   // W, dW and dxe hold the rows of edges [e_base, ...) only (edge-chunked passes); Y, dY, e_src are whole
   // Tabulated path weights (models with the identity edge update, where the radial MLP's output is a function of the
-  // edge length alone): rtab [rt_K][NP*C][4] = (W, h dW/dd) at both ends of the interval [k h, (k + 1) h], read with cubic
-  // Hermite interpolation instead of W; the backward pass then writes no dW and adds sum_{p,c} dW * dW/dd into ddlen.
+  // edge length alone): rtab [rt_K][NP*C][4] = coefficients (a, b, c, d) of W = a + t (b + t (c + t d)) on the interval
+  // [k h, (k + 1) h], t = d / h - k, read instead of W; the backward pass then writes no dW and adds sum_{p,c} dW * dW/dd
+  // into ddlen.
   const T* rtab;      // nullptr: per-edge weights W / dW as above
   int rt_K;           // number of intervals
   T rt_inv_h;         // 1 / knot spacing
@@ -55,6 +58,12 @@ struct TPArgs {
 };
 template <typename T> cudaError_t launch_tp_fwd(const TPArgs<T>& a, cudaStream_t s);
 template <typename T> cudaError_t launch_tp_bwd(const TPArgs<T>& a, cudaStream_t s);
+// the fp32 kernels with several channels per thread (tp_wide_kernels.cu), taken by the two above where they apply
+inline bool tp_wide_channels(int C) { return C == 64 || C == 128; }
+void tp_wide_table(const float* in, float* out, long long rows, int C);  // table layout these kernels read
+bool tp_wide_supported(const TPArgs<float>& a);
+cudaError_t launch_tp_fwd_wide(const TPArgs<float>& a, cudaStream_t s);
+cudaError_t launch_tp_bwd_wide(const TPArgs<float>& a, cudaStream_t s);
 // gx[b] = sum of dxe over the edges whose source is b (edges listed by perm within rowptr_src segments)
 // for the source atoms [first_atom, first_atom + n_atoms)
 template <typename T> cudaError_t launch_segment_sum_rows(const T* dxe, const int* rowptr_src, const int* perm_src, T* gx,

@@ -12,6 +12,7 @@
 // the source features (one row per edge, summed per source atom by launch_segment_sum_rows).
 // Edge lists are sorted, so every sum is a segmented reduction: no atomics, bit-reproducible.
 #include <cstdint>
+#include <type_traits>
 #include "kernels.h"
 #include "tp_gen.cuh"
 
@@ -56,40 +57,38 @@ __device__ __forceinline__ int tp_row(const TPArgs<T>& a, int it) {
 
 // ENV: the path weights are multiplied by the per-edge envelope (radial_basis.apply_cutoff = False); a separate
 // instantiation so the default kernels carry none of its registers.
-// Cubic Hermite interpolation of the tabulated path weights: knot index and the four basis values of one edge
-// (and, for the backward pass, the basis derivatives with respect to the edge length).
+// Interpolation of the tabulated path weights: interval of one edge and the position inside it, 0 <= t < 1.
 template <typename T>
 struct RtEdge {
   int k;
-  T b[4];
-  T d[4];
+  T t;
 };
-template <typename T, bool DERIV>
+template <typename T>
 __device__ __forceinline__ void rt_prepare(const TPArgs<T>& a, T d, RtEdge<T>& r) {
   const T u = d * a.rt_inv_h;
   int k = (int)u;
   k = k < 0 ? 0 : (k > a.rt_K - 1 ? a.rt_K - 1 : k);
-  const T t = u - T(k), t2 = t * t, t3 = t2 * t;
   r.k = k;
-  r.b[0] = T(2) * t3 - T(3) * t2 + T(1);
-  r.b[1] = t3 - T(2) * t2 + t;
-  r.b[2] = T(3) * t2 - T(2) * t3;
-  r.b[3] = t3 - t2;
-  if (DERIV) {
-    r.d[0] = (T(6) * t2 - T(6) * t) * a.rt_inv_h;
-    r.d[1] = (T(3) * t2 - T(4) * t + T(1)) * a.rt_inv_h;
-    r.d[2] = (T(6) * t - T(6) * t2) * a.rt_inv_h;
-    r.d[3] = (T(3) * t2 - T(2) * t) * a.rt_inv_h;
-  }
+  r.t = u - T(k);
 }
-// One table entry = (W_k, h W'_k, W_{k+1}, h W'_{k+1}) of a (path, channel) pair for the interval [d_k, d_{k+1}]: the
-// four numbers the interpolation needs, in one 16-byte load.
+// One table entry = the coefficients of the cubic a + t (b + t (c + t d)) of a (path, channel) pair on one interval, in one
+// 16-byte load.
 template <typename T>
-__device__ __forceinline__ void rt_load(const T* p, T& v0, T& m0, T& v1, T& m1) { v0 = p[0]; m0 = p[1]; v1 = p[2]; m1 = p[3]; }
+struct RtCubic {
+  T a, b, c, d;
+  __device__ __forceinline__ T value(T t) const { return a + t * (b + t * (c + t * d)); }
+  __device__ __forceinline__ void value_slope(T t, T& w, T& dw) const {  // dw: derivative with respect to t
+    const T e = c + t * d, f = b + t * e;
+    w = a + t * f;
+    dw = f + t * (e + t * d);
+  }
+};
+template <typename T>
+__device__ __forceinline__ void rt_load(const T* p, RtCubic<T>& q) { q.a = p[0]; q.b = p[1]; q.c = p[2]; q.d = p[3]; }
 template <>
-__device__ __forceinline__ void rt_load<float>(const float* p, float& v0, float& m0, float& v1, float& m1) {
-  const float4 q = __ldg(reinterpret_cast<const float4*>(p));
-  v0 = q.x; m0 = q.y; v1 = q.z; m1 = q.w;
+__device__ __forceinline__ void rt_load<float>(const float* p, RtCubic<float>& q) {
+  const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+  q.a = v.x; q.b = v.y; q.c = v.z; q.d = v.w;
 }
 
 // RT: path weights interpolated from the table a.rtab instead of read from a.W.
@@ -109,7 +108,7 @@ __device__ __forceinline__ void tp_fwd_row(const TPArgs<T>& a, int i, T* Gs, int
     __syncthreads();
     if (threadIdx.x < nb) esrc[threadIdx.x] = a.e_src[e0 + threadIdx.x];
     if (RT && (int)threadIdx.x >= rt_first && (int)threadIdx.x < rt_first + nb)
-      rt_prepare<T, false>(a, a.dlen[e0 + threadIdx.x - rt_first], rts[threadIdx.x - rt_first]);
+      rt_prepare<T>(a, a.dlen[e0 + threadIdx.x - rt_first], rts[threadIdx.x - rt_first]);
     build_G_rows<T, TP>(a.Y, e0, nb, 2 * GRP, 2, Gs);
     __syncthreads();
     for (int e = 0; e < nb; ++e) {
@@ -119,12 +118,12 @@ __device__ __forceinline__ void tp_fwd_row(const TPArgs<T>& a, int i, T* Gs, int
       for (int k = 0; k < TP::NX; ++k) xv[k] = a.x[(s * TP::NX + k) * C + c];
       if constexpr (RT) {
         const T* r0 = a.rtab + ((long long)rts[e].k * TP::NP * C + (long long)P0 * C + c) * 4;
-        const T b0 = rts[e].b[0], b1 = rts[e].b[1], b2 = rts[e].b[2], b3 = rts[e].b[3];
+        const T t = rts[e].t;
 #pragma unroll
         for (int p = 0; p < NPG; ++p) {
-          T v0, m0, v1, m1;
-          rt_load<T>(r0 + (long long)p * C * 4, v0, m0, v1, m1);
-          wv[p] = b0 * v0 + b1 * m0 + b2 * v1 + b3 * m1;
+          RtCubic<T> q;
+          rt_load<T>(r0 + (long long)p * C * 4, q);
+          wv[p] = q.value(t);
         }
       } else {
         const T* We = a.W + ((long long)(e0 + e - a.e_base) * TP::NP + P0) * C;
@@ -170,18 +169,18 @@ template <typename T, typename TP, bool ENV>
 struct RtBwdWeights {
   const T* row;       // table entries of this edge's interval, this thread's channel: path p at row + p * stride
   long long stride;   // 4 * C
-  T b0, b1, b2, b3, d0, d1, d2, d3, u;
-  T v0, m0, v1, m1;   // entry of the next path
+  T t, inv_h, u;
+  RtCubic<T> q;       // entry of the next path
   T w_now, wd_now;    // weight and length derivative of the path in flight
   T dr, du;
   __device__ __forceinline__ void start() {
     dr = T(0); du = T(0);
-    rt_load<T>(row, v0, m0, v1, m1);
+    rt_load<T>(row, q);
   }
   template <int P> __device__ __forceinline__ T get() {
-    w_now = b0 * v0 + b1 * m0 + b2 * v1 + b3 * m1;
-    wd_now = d0 * v0 + d1 * m0 + d2 * v1 + d3 * m1;
-    if (P + 1 < TP::NP) rt_load<T>(row + (long long)(P + 1) * stride, v0, m0, v1, m1);
+    q.value_slope(t, w_now, wd_now);
+    wd_now *= inv_h;
+    if (P + 1 < TP::NP) rt_load<T>(row + (long long)(P + 1) * stride, q);
     return ENV ? w_now * u : w_now;
   }
   template <int P> __device__ __forceinline__ void put(T dwv) {
@@ -259,7 +258,7 @@ __device__ __forceinline__ void tp_bwd_row(const TPArgs<T>& a, int i, unsigned c
     __syncthreads();
     if (threadIdx.x < nb) esrc[threadIdx.x] = a.e_src[e0 + threadIdx.x];
     if (RT && (int)threadIdx.x >= rt_first && (int)threadIdx.x < rt_first + nb)
-      rt_prepare<T, true>(a, a.dlen[e0 + threadIdx.x - rt_first], rts[threadIdx.x - rt_first]);
+      rt_prepare<T>(a, a.dlen[e0 + threadIdx.x - rt_first], rts[threadIdx.x - rt_first]);
     build_G_rows<T, TP>(a.Y, e0, nb, 0, TP::NPART, Gs);
     __syncthreads();
     for (int e = 0; e < nb; ++e) {
@@ -277,8 +276,8 @@ __device__ __forceinline__ void tp_bwd_row(const TPArgs<T>& a, int i, unsigned c
         RtBwdWeights<T, TP, ENV> wf;
         wf.row = a.rtab + ((long long)rts[e].k * TP::NP * C + c) * 4;
         wf.stride = (long long)C * 4;
-        wf.b0 = rts[e].b[0]; wf.b1 = rts[e].b[1]; wf.b2 = rts[e].b[2]; wf.b3 = rts[e].b[3];
-        wf.d0 = rts[e].d[0]; wf.d1 = rts[e].d[1]; wf.d2 = rts[e].d[2]; wf.d3 = rts[e].d[3];
+        wf.t = rts[e].t;
+        wf.inv_h = a.rt_inv_h;
         wf.u = u;
         wf.start();
         TP::template bwd_w<T>(xv, gMs + c, C, Gs + e * TP::NG, wf, dYp, dx);
@@ -389,7 +388,7 @@ __global__ void tp_bwd_scalar_kernel(const TPArgs<T> a) {
     if (c < nb) {
       esrc[c] = a.e_src[e0 + c];
       if (ENV) env_s[c] = a.env[e0 + c];
-      if (RT) rt_prepare<T, true>(a, a.dlen[e0 + c], rts[c]);
+      if (RT) rt_prepare<T>(a, a.dlen[e0 + c], rts[c]);
     }
     for (int idx = c; idx < nb * D; idx += blockDim.x) Ys[idx] = a.Y[(long long)e0 * D + idx];
     __syncthreads();
@@ -406,10 +405,10 @@ __global__ void tp_bwd_scalar_kernel(const TPArgs<T> a) {
 #pragma unroll
         for (int l = 0; l < NP; ++l) {
           if constexpr (RT) {
-            T v0, m0, v1, m1;
-            rt_load<T>(a.rtab + ((long long)rts[e].k * NP * C + (long long)l * C + c) * 4, v0, m0, v1, m1);
-            w_[j][l] = rts[e].b[0] * v0 + rts[e].b[1] * m0 + rts[e].b[2] * v1 + rts[e].b[3] * m1;
-            wd_[j][l] = rts[e].d[0] * v0 + rts[e].d[1] * m0 + rts[e].d[2] * v1 + rts[e].d[3] * m1;
+            RtCubic<T> q;
+            rt_load<T>(a.rtab + ((long long)rts[e].k * NP * C + (long long)l * C + c) * 4, q);
+            q.value_slope(rts[e].t, w_[j][l], wd_[j][l]);
+            wd_[j][l] *= a.rt_inv_h;
           } else {
             w_[j][l] = a.W[wbase + l * C + c];
             wd_[j][l] = T(0);
@@ -628,8 +627,14 @@ cudaError_t launch_bwd_t(const TPArgs<T>& a, cudaStream_t s) {
   if (a.L == 3 && a.Lin == 3) return FN<T, TPX_L3_F>(a, s);               \
   return cudaErrorInvalidValue;
 
-template <typename T> cudaError_t launch_tp_fwd(const TPArgs<T>& a, cudaStream_t s) { TACE_TP_DISPATCH(launch_fwd_t) }
-template <typename T> cudaError_t launch_tp_bwd(const TPArgs<T>& a, cudaStream_t s) { TACE_TP_DISPATCH(launch_bwd_t) }
+template <typename T> cudaError_t launch_tp_fwd(const TPArgs<T>& a, cudaStream_t s) {
+  if constexpr (std::is_same<T, float>::value) { if (tp_wide_supported(a)) return launch_tp_fwd_wide(a, s); }
+  TACE_TP_DISPATCH(launch_fwd_t)
+}
+template <typename T> cudaError_t launch_tp_bwd(const TPArgs<T>& a, cudaStream_t s) {
+  if constexpr (std::is_same<T, float>::value) { if (tp_wide_supported(a)) return launch_tp_bwd_wide(a, s); }
+  TACE_TP_DISPATCH(launch_bwd_t)
+}
 
 template cudaError_t launch_tp_fwd<float>(const TPArgs<float>&, cudaStream_t);
 template cudaError_t launch_tp_fwd<double>(const TPArgs<double>&, cudaStream_t);
