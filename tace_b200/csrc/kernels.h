@@ -171,6 +171,16 @@ template <typename T> cudaError_t launch_graph_energy(const T* e_scaled, const T
                                                       const int* fidelity, int n_el, T* energy, int n_graphs, long long n_atoms,
                                                       T* partial, cudaStream_t s);
 template <typename T> cudaError_t launch_fill_zero(T* p, long long n, cudaStream_t s);
+// Several device-to-device copies (4-byte granules) in one launch; entries [pad_from, pad_to) of both rows of the [2][pad_to] edge
+// list `pad` are set to -1.
+struct CopySegments {
+  static constexpr int kMax = 10;
+  const void* src[kMax]; void* dst[kMax]; long long bytes[kMax];
+  int n = 0;
+  int64_t* pad = nullptr; long long pad_from = 0, pad_to = 0;
+  void add(void* d, const void* s, size_t b) { if (b) { src[n] = s; dst[n] = d; bytes[n] = (long long)b; ++n; } }
+};
+cudaError_t launch_copy_segments(const CopySegments& c, cudaStream_t s);
 // dst[i] = src[perm[i]] (gather) / dst[perm[i]] = src[i] (scatter), rows of row_len elements
 template <typename T> cudaError_t launch_gather_rows(const T* src, const int* perm, T* dst, long long n, int row_len, cudaStream_t s);
 template <typename T> cudaError_t launch_scatter_rows(const T* src, const int* perm, T* dst, long long n, int row_len, cudaStream_t s);
@@ -193,6 +203,7 @@ struct EdgeArgs {
   int L, n_layers;
   long long E;
   const int* e_src; const int* e_dst; const int* e_orig;  // target-sorted edges; e_orig = caller's edge id
+  const int* n_valid;    // device word: rows from here on are padding (they write no edge force)
   const T* positions;    // [N][3] or nullptr
   const T* lattice;      // [B][3][3]
   const int* atom_graph; // [N]
@@ -248,11 +259,11 @@ template <typename T> cudaError_t launch_graph_virial(const T* atom_virial, cons
 // ---- graph preparation (graph_kernels.cu) ------------------------------------------------------
 struct GraphPrepArgs {
   long long E; int n_atoms, n_local, n_graphs, n_elements;
-  const int64_t* edge_index;  // [2][E]
+  const int64_t* edge_index;  // [2][E]; entries with an index outside [0, n_atoms) are padding, in no view
   const int* species; const int* graph_ptr;
   // outputs
-  int* e_src; int* e_dst; int* e_orig;  // target-sorted
-  int* rowptr_dst;            // [n_local+1]
+  int* e_src; int* e_dst; int* e_orig;  // target-sorted; rows behind the last edge hold a valid dummy
+  int* rowptr_dst;            // [n_atoms+1]; its last entry is the number of edges in the views
   // split_rows: row_ids lists the owned targets none of whose sources is a ghost, then the others (each part in
   // ascending order); row_split[1] is the length of the first part
   int split_rows;
@@ -267,6 +278,7 @@ struct GraphPrepArgs {
 };
 size_t graph_prep_temp_bytes(long long E, int n_atoms);
 cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s);
+int graph_prep_launches(const GraphPrepArgs& a);  // kernels of this file it runs
 // Edge chunks for systems whose per-edge tensors do not fit: chunk c = target atoms [atom_ptr[c], atom_ptr[c+1]) with
 // atom_ptr[c] = first atom whose edge offset reaches c * target_edges; edge_ptr[c] = rowptr_dst[atom_ptr[c]].
 cudaError_t launch_chunk_bounds(const int* rowptr_dst, int n_local, long long target_edges, int n_chunks, int* atom_ptr,

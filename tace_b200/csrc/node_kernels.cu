@@ -22,6 +22,34 @@ cudaError_t launch_fill_zero(T* p, long long n, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+__global__ void copy_segments_kernel(const CopySegments c) {
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  for (int k = 0; k < c.n; ++k) {
+    if (((reinterpret_cast<uintptr_t>(c.src[k]) | reinterpret_cast<uintptr_t>(c.dst[k])) & 15) == 0) {
+      const uint4* src = static_cast<const uint4*>(c.src[k]);
+      uint4* dst = static_cast<uint4*>(c.dst[k]);
+      const long long n = c.bytes[k] >> 4;
+      for (long long i = first; i < n; i += step) dst[i] = src[i];
+      const int rest = (int)(c.bytes[k] & 15) >> 2;
+      if (first < rest) reinterpret_cast<uint32_t*>(dst + n)[first] = reinterpret_cast<const uint32_t*>(src + n)[first];
+    } else {
+      const uint32_t* src = static_cast<const uint32_t*>(c.src[k]);
+      uint32_t* dst = static_cast<uint32_t*>(c.dst[k]);
+      for (long long i = first; i < (c.bytes[k] >> 2); i += step) dst[i] = src[i];
+    }
+  }
+  if (c.pad)
+    for (long long i = c.pad_from + first; i < c.pad_to; i += step) { c.pad[i] = -1; c.pad[c.pad_to + i] = -1; }
+}
+cudaError_t launch_copy_segments(const CopySegments& c, cudaStream_t s) {
+  if (c.n == 0) return cudaSuccess;
+  long long most = 0;
+  for (int k = 0; k < c.n; ++k) most = c.bytes[k] > most ? c.bytes[k] : most;
+  const long long blocks = (most / 16 + 255) / 256;
+  copy_segments_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks > 148 * 8 ? 148 * 8 : blocks), 256, 0, s>>>(c);
+  return cudaGetLastError();
+}
+
 template <typename T>
 __global__ void add_inplace_kernel(T* dst, const T* src, long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) dst[i] += src[i];
