@@ -81,12 +81,6 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
   d |= (uint64_t)2 << 61;                          // SWIZZLE_128B
   return d;
 }
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -137,8 +131,7 @@ struct TcProblem {
   const int* atom_map;   // row of C for sorted atom a is atom_map[a]; nullptr: identity
   int accumulate;        // C += instead of C =
   int b_tiled;           // B maps are 4-D {32, N, K/32, groups} over K-tile-major weights
-  int c_tma;             // plain row-major result (q = 1, no map, no accumulate): written by TMA stores through tmC
-  CUtensorMap tmC;       // 2-D {N, rows}, box 32 x 32, 128-byte swizzle
+  int table;             // offset of its row pointers in the kernel's shared-memory tables, -1: read from global memory
 };
 constexpr int kTcMaxProblems = 4;
 struct TcBatch {
@@ -150,28 +143,28 @@ struct TcBatch {
   uint32_t extra_tx;     // test mode: bytes added to what the first load barrier expects, so that it never completes
 };
 
-// Warp roles (256 threads): warp 0 = TMA producer, warp 1 = MMA issuer, warps 2-3 = operand
-// splitters, warps 4-7 = epilogue (warp w owns the TMEM lanes 32 * (w % 4) .. + 31).
-constexpr int kSplitThreads = 64;  // without TS: warps 2 and 3
-
-// TS: the activation operand of the tensor-core instructions lives in tensor memory.  The splitters read the tile the TMA
+// Warp roles (448 threads): warp 0 = TMA producer, warp 1 = MMA issuer, warps 2, 3, 8, 9 = operand splitters (one per TMEM lane
+// quarter), warps 4..7 and 10..13 = epilogue (warp w owns the TMEM lanes 32 * (w % 4) .. + 31; the second four take the right
+// half of the columns, so that 64 running sums per thread fit its registers and a tile drains in half the time).
+//
+// The activation operand of the tensor-core instructions lives in tensor memory.  The splitters read the tile the TMA
 // unit wrote and store its high part and residual to TMEM (one thread per row = TMEM lane), so a stage needs no room for
-// them in shared memory: 48 KB instead of 64 KB at BN = 128, i.e. four K-steps in flight instead of three (six instead
-// of four at BN = 64), and the tensor core reads only the weight operand from shared memory.  The ring's round trip, not any
-// unit, is what bounds this kernel, so the number of stages in flight is its throughput.
-template <int BN, bool TS>
+// them in shared memory: 48 KB at BN = 128, i.e. four K-steps in flight (six at BN = 64), and the tensor core reads only the weight
+// operand from shared memory.
+template <int BN>
 struct TcSmem {
-  static constexpr int kStages = TS ? (BN == 128 ? 4 : 6) : (BN == 128 ? 3 : 4);
+  static constexpr int kStages = BN == 128 ? 4 : 6;
   static constexpr int kTileBBytes = BN * kBK * 4;
-  static constexpr int kStageBytes = (TS ? 1 : 2) * kTileABytes + 2 * kTileBBytes;
-  static constexpr int kThreads = TS ? 320 : 256;        // TS: four splitter warps (2, 3, 8, 9), one per TMEM lane quarter
-  static constexpr int kSplit = TS ? 128 : 64;           // splitter threads = arrivals on a `ready` barrier
-  static constexpr int kTmemCols = TS ? 512 : 2 * BN;    // accumulators [0, 2 BN) | TS: per stage 32 columns high part, 32 residual
-  static constexpr int kTmemA = 2 * BN;                  // first activation column (TS)
+  static constexpr int kStageBytes = kTileABytes + 2 * kTileBBytes;
+  static constexpr int kThreads = 448, kSplitWarps = 4, kEpilogueThreads = 256;
+  static constexpr int kTmemCols = 512;                  // accumulators [0, 2 BN) | per stage 32 columns high part, 32 residual
+  static constexpr int kTmemA = 2 * BN;                  // first activation column
   static constexpr int kBarrierBytes = 256;
-  // result staging for TMA stores: per epilogue warp two slabs of 32 rows x 32 columns (128-byte swizzled rows)
-  static constexpr int kStoreBytes = 4 * 2 * 32 * 128;
-  static constexpr int kTotal = kStages * kStageBytes + kStoreBytes + kBarrierBytes + 1024;  // + alignment slack
+  // result staging: per epilogue warp sixteen rows x 32 columns, and the addresses of its 32 rows
+  static constexpr int kStoreBytes = 8 * 16 * 128, kRowBytes = 8 * 32 * 8;
+  // row pointers of the species and tile tables of the grouped problems, copied in once (a tile is found by a search over them)
+  static constexpr int kTableInts = 1536;
+  static constexpr int kTotal = kStages * kStageBytes + kStoreBytes + kRowBytes + kBarrierBytes + 4 * kTableInts + 1024;  // + alignment slack
 };
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
@@ -191,18 +184,56 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(x), "r"(y) : "memory");
+// Result path of an epilogue warp: lane r holds 32 consecutive columns of row r.  Sixteen rows at a time go through shared
+// memory (16-byte chunk j of row r at chunk j ^ (r & 7)) and leave as whole 128-byte rows, eight lanes per row: stored straight
+// from the registers, every 16-byte store touched 32 rows, and that, not the tensor core, bounded the linears with few K steps.
+__device__ __forceinline__ void store_slab(unsigned char* slab, const uint32_t (&rr)[32], const float* bias, float* const* rows, int col,
+                                           bool accumulate, int lane) {
+  const int sub = lane & 7;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if ((lane >> 4) == h) {
+      float4* row = reinterpret_cast<float4*>(slab + (lane & 15) * 128);
+#pragma unroll
+      for (int q4 = 0; q4 < 8; ++q4)
+        row[q4 ^ (lane & 7)] = make_float4(__uint_as_float(rr[4 * q4]), __uint_as_float(rr[4 * q4 + 1]), __uint_as_float(rr[4 * q4 + 2]),
+                                           __uint_as_float(rr[4 * q4 + 3]));
+    }
+    __syncwarp();
+    float* dst[4];
+    float4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = 4 * i + (lane >> 3);
+      dst[i] = rows[16 * h + r];
+      v[i] = *reinterpret_cast<const float4*>(slab + r * 128 + ((sub ^ (r & 7)) << 4));
+    }
+    if (bias) {
+      const float4 b = *reinterpret_cast<const float4*>(bias + 4 * sub);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { v[i].x += b.x; v[i].y += b.y; v[i].z += b.z; v[i].w += b.w; }
+    }
+    if (accumulate) {  // every load before the first store: a load that follows a store to its line waits for it
+      float4 o[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[i] = dst[i] ? *reinterpret_cast<const float4*>(dst[i] + col + 4 * sub) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { v[i].x += o[i].x; v[i].y += o[i].y; v[i].z += o[i].z; v[i].w += o[i].w; }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (dst[i]) *reinterpret_cast<float4*>(dst[i] + col + 4 * sub) = v[i];
+    __syncwarp();
+  }
 }
 
 struct TileInfo {
   int prob, atom0, atom_end, group, n0, num_k;
 };
 // tile_start: prefix sums of the problems' tile counts (in shared memory: grouped problems only know
-// their tile count on the device)
+// their tile count on the device); tables: per grouped problem its tile_ptr, then group_ptr (P.table: offset, -1: not copied)
 template <int BN>
-__device__ __forceinline__ TileInfo decode_tile(const TcBatch& b, const int* tile_start, int tile) {
+__device__ __forceinline__ TileInfo decode_tile(const TcBatch& b, const int* tile_start, const int* tables, int tile) {
   int pi = 0;
   while (pi + 1 < b.n_problems && tile >= tile_start[pi + 1]) ++pi;
   const TcProblem& P = b.p[pi];
@@ -214,14 +245,16 @@ __device__ __forceinline__ TileInfo decode_tile(const TcBatch& b, const int* til
   t.n0 = (local - mt * tiles_n) * BN;
   t.num_k = P.K / kBK;
   if (P.n_groups > 0) {
+    const int* tile_ptr = P.table >= 0 ? tables + P.table : P.tile_ptr;
+    const int* group_ptr = P.table >= 0 ? tables + P.table + P.n_groups + 1 : P.group_ptr;
     int lo = 0, hi = P.n_groups;  // largest g with tile_ptr[g] <= mt
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if (P.tile_ptr[mid] <= mt) lo = mid; else hi = mid;
+      if (tile_ptr[mid] <= mt) lo = mid; else hi = mid;
     }
     t.group = lo;
-    t.atom0 = P.group_ptr[lo] + (mt - P.tile_ptr[lo]) * P.R;
-    t.atom_end = P.group_ptr[lo + 1];
+    t.atom0 = group_ptr[lo] + (mt - tile_ptr[lo]) * P.R;
+    t.atom_end = group_ptr[lo + 1];
   } else {
     t.group = 0;
     t.atom0 = mt * P.R;
@@ -232,16 +265,18 @@ __device__ __forceinline__ TileInfo decode_tile(const TcBatch& b, const int* til
 
 // ONE_CHUNK: every K loop of the launch fits one TMEM accumulation chunk, so the epilogue stores
 // straight from the drained registers and needs no running sums.
-template <int BN, bool ONE_CHUNK, bool TS>
-__global__ void __launch_bounds__(TcSmem<BN, TS>::kThreads, 1) tc_gemm_kernel(const __grid_constant__ TcBatch batch) {
-  using S = TcSmem<BN, TS>;
+template <int BN, bool ONE_CHUNK>
+__global__ void __launch_bounds__(TcSmem<BN>::kThreads, 1) tc_gemm_kernel(const __grid_constant__ TcBatch batch) {
+  using S = TcSmem<BN>;
   constexpr int kStages = S::kStages;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;  // 128-byte-swizzled tiles need 1024-byte alignment
   unsigned char* base_ptr = smem_raw + (base - raw);
   const uint32_t store_base = base + kStages * S::kStageBytes;  // 1024-byte aligned: stage sizes are multiples of 1024
-  const uint32_t bars = store_base + S::kStoreBytes;
+  const uint32_t bars = store_base + S::kStoreBytes + S::kRowBytes;
+  float** row_addr = reinterpret_cast<float**>(base_ptr + kStages * S::kStageBytes + S::kStoreBytes);  // [8 warps][32]
+  int* tables = reinterpret_cast<int*>(base_ptr + kStages * S::kStageBytes + S::kStoreBytes + S::kRowBytes + S::kBarrierBytes);
   // barriers: raw[s] TMA landed | ready[s] operands split | empty[s] MMAs done reading | acc_full[a] | acc_empty[a]
   auto raw_bar = [&](int s) { return bars + 8u * s; };
   auto ready_bar = [&](int s) { return bars + 8u * (kStages + s); };
@@ -249,15 +284,23 @@ __global__ void __launch_bounds__(TcSmem<BN, TS>::kThreads, 1) tc_gemm_kernel(co
   auto acc_full = [&](int a) { return bars + 8u * (3 * kStages + a); };
   auto acc_empty = [&](int a) { return bars + 8u * (3 * kStages + 2 + a); };
   const uint32_t drain_bar = bars + 8u * (3 * kStages + 4);  // abort path only: issued tensor-core work has retired
-  unsigned char* misc = base_ptr + kStages * S::kStageBytes + S::kStoreBytes + 8 * (3 * kStages + 5);
+  unsigned char* misc = base_ptr + kStages * S::kStageBytes + S::kStoreBytes + S::kRowBytes + 8 * (3 * kStages + 5);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(misc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(misc + 8);
   int* tile_start = reinterpret_cast<int*>(misc + 16);  // [n_problems + 1]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int i = 0; i < batch.n_problems; ++i) {
+    const TcProblem& P = batch.p[i];
+    if (P.n_groups > 0 && P.table >= 0)
+      for (int k = tid; k <= P.n_groups; k += S::kThreads) {
+        tables[P.table + k] = P.tile_ptr[k];
+        tables[P.table + P.n_groups + 1 + k] = P.group_ptr[k];
+      }
+  }
   if (tid == 0) {  // `ready` takes one arrival per splitter warp
-    for (int s = 0; s < kStages; ++s) { mbar_init(raw_bar(s), 1); mbar_init(ready_bar(s), S::kSplit / 32); mbar_init(empty_bar(s), 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), 128); }
+    for (int s = 0; s < kStages; ++s) { mbar_init(raw_bar(s), 1); mbar_init(ready_bar(s), S::kSplitWarps); mbar_init(empty_bar(s), 1); }
+    for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), S::kEpilogueThreads); }
     mbar_init(drain_bar, 1);
     *abort_flag = 0;
     int acc = 0;
@@ -283,8 +326,7 @@ __global__ void __launch_bounds__(TcSmem<BN, TS>::kThreads, 1) tc_gemm_kernel(co
   // instruction descriptor: D = F32, A = B = TF32, both K-major, N = BN, M = 128
   const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
   auto stage_a = [&](int s) { return base + s * S::kStageBytes; };
-  constexpr int kBOff = (TS ? 1 : 2) * kTileABytes;  // weights follow the activation tile (and, without TS, its residual)
-  auto stage_alo = [&](int s) { return base + s * S::kStageBytes + kTileABytes; };  // not TS
+  constexpr int kBOff = kTileABytes;  // weights follow the activation tile
   auto stage_bhi = [&](int s) { return base + s * S::kStageBytes + kBOff; };
   auto stage_blo = [&](int s) { return base + s * S::kStageBytes + kBOff + S::kTileBBytes; };
 
@@ -294,7 +336,7 @@ __global__ void __launch_bounds__(TcSmem<BN, TS>::kThreads, 1) tc_gemm_kernel(co
       int step = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const TileInfo t = decode_tile<BN>(batch, tile_start, tile);
+        const TileInfo t = decode_tile<BN>(batch, tile_start, tables, tile);
         const TcProblem& P = batch.p[t.prob];
         const uint32_t a_bytes = (uint32_t)P.R * P.q * kBK * 4;
         for (int ks = 0; ks < t.num_k; ++ks, ++step) {
@@ -328,11 +370,10 @@ __global__ void __launch_bounds__(TcSmem<BN, TS>::kThreads, 1) tc_gemm_kernel(co
       // the ring waits for: descriptors are built once (only their 14-bit start-address field, in 16-byte units, changes
       // from stage to stage and from one 8-wide K slice to the next, so the later ones are sums), and the stage index and
       // phase are counted instead of divided.
-      const uint64_t dA0 = umma_desc(stage_a(0)), dAl0 = umma_desc(stage_alo(0));
       const uint64_t dB0 = umma_desc(stage_bhi(0)), dBl0 = umma_desc(stage_blo(0));
       int s = 0, ph = 0;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const TileInfo t = decode_tile<BN>(batch, tile_start, tile);
+        const TileInfo t = decode_tile<BN>(batch, tile_start, tables, tile);
         for (int ks = 0; ks < t.num_k; ++ks, ph ^= (s == kStages - 1), s = (s == kStages - 1) ? 0 : s + 1) {
           const int a = chunk & 1;
           const bool chunk_begin = (ks % kChunk) == 0;
@@ -346,17 +387,11 @@ __global__ void __launch_bounds__(TcSmem<BN, TS>::kThreads, 1) tc_gemm_kernel(co
           for (int k8 = 0; k8 < kBK / 8; ++k8) {
             const uint64_t off = stage_off + (uint64_t)(k8 * 2);  // 8 fp32 = 32 bytes along K inside the swizzled row
             const uint64_t db = dB0 + off, dbl = dBl0 + off;
-            if constexpr (TS) {  // activations: 8 TMEM columns per slice, high part at +0, residual at +32 of the stage
-              const uint32_t ta = tmem_base + (uint32_t)(S::kTmemA + s * 64 + k8 * 8);
-              umma_tf32_ts(d, ta, db, idesc, (!chunk_begin || k8 > 0) ? 1u : 0u);
-              umma_tf32_ts(d, ta, dbl, idesc, 1u);
-              umma_tf32_ts(d, ta + 32, db, idesc, 1u);
-            } else {
-              const uint64_t da = dA0 + off, dal = dAl0 + off;
-              umma_tf32(d, da, db, idesc, (!chunk_begin || k8 > 0) ? 1u : 0u);
-              umma_tf32(d, da, dbl, idesc, 1u);
-              umma_tf32(d, dal, db, idesc, 1u);
-            }
+            // activations: 8 TMEM columns per slice, high part at +0, residual at +32 of the stage
+            const uint32_t ta = tmem_base + (uint32_t)(S::kTmemA + s * 64 + k8 * 8);
+            umma_tf32_ts(d, ta, db, idesc, (!chunk_begin || k8 > 0) ? 1u : 0u);
+            umma_tf32_ts(d, ta, dbl, idesc, 1u);
+            umma_tf32_ts(d, ta + 32, db, idesc, 1u);
           }
           umma_commit(empty_bar(s));  // ring slot reusable once these MMAs have read it
           if (chunk_end) { umma_commit(acc_full(a)); ++chunk; }  // partial sum of this chunk complete
@@ -368,63 +403,36 @@ __global__ void __launch_bounds__(TcSmem<BN, TS>::kThreads, 1) tc_gemm_kernel(co
           if (mbar_try_wait(drain_bar, 0)) break;
       }
     }
-  } else if (warp < 4 || (TS && warp >= 8)) {
+  } else if (warp < 4 || warp == 8 || warp == 9) {
     // ---- operand splitters: A = hi + lo with hi exact in TF32
-    const int t64 = tid - 64;
     int step = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-      const TileInfo t = decode_tile<BN>(batch, tile_start, tile);
+      const TileInfo t = decode_tile<BN>(batch, tile_start, tables, tile);
       for (int ks = 0; ks < t.num_k; ++ks, ++step) {
         const int s = step % kStages, ph = (step / kStages) & 1;
         if (!mbar_wait(raw_bar(s), ph, abort_flag, batch.error, 3, batch.spin_limit)) { ok = false; break; }
-        if constexpr (TS) {
-          // one thread per row (= TMEM lane): the row's eight 16-byte pieces sit at positions j ^ (row & 7) of its 128 bytes
-          // (the swizzle the TMA unit wrote); high parts go to 32 TMEM columns of the stage, residuals to the next 32
-          const int row = (warp & 3) * 32 + lane;
-          const float4* arow = reinterpret_cast<const float4*>(base_ptr + s * S::kStageBytes + row * 128);
-          uint32_t hi[32], lo[32];
+        // one thread per row (= TMEM lane): the row's eight 16-byte pieces sit at positions j ^ (row & 7) of its 128 bytes
+        // (the swizzle the TMA unit wrote); high parts go to 32 TMEM columns of the stage, residuals to the next 32
+        const int row = (warp & 3) * 32 + lane;
+        const float4* arow = reinterpret_cast<const float4*>(base_ptr + s * S::kStageBytes + row * 128);
+        uint32_t hi[32], lo[32];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float4 v = arow[j ^ (row & 7)];
-            const float x[4] = {v.x, v.y, v.z, v.w};
+        for (int j = 0; j < 8; ++j) {
+          const float4 v = arow[j ^ (row & 7)];
+          const float x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const uint32_t h = __float_as_uint(x[q]) & 0xFFFFE000u;
-              hi[4 * j + q] = h;
-              lo[4 * j + q] = __float_as_uint(x[q] - __uint_as_float(h));
-            }
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t h = __float_as_uint(x[q]) & 0xFFFFE000u;
+            hi[4 * j + q] = h;
+            lo[4 * j + q] = __float_as_uint(x[q] - __uint_as_float(h));
           }
-          const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(S::kTmemA + s * 64);
-          tmem_st32(ta, hi);
-          tmem_st32(ta + 32, lo);
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) mbar_arrive(ready_bar(s));
-          continue;
         }
-        float4* a = reinterpret_cast<float4*>(base_ptr + s * S::kStageBytes);
-        float4* alo = reinterpret_cast<float4*>(base_ptr + s * S::kStageBytes + kTileABytes);
-        // every load of the tile before its first store: the stores go to the buffer the loads come from, so the compiler
-        // must keep their order, and sixteen dependent load -> store rounds would put their latencies end to end on the
-        // critical path of the operand ring
-        constexpr int kPer = kTileABytes / 16 / kSplitThreads;
-        float4 v[kPer];
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) v[j] = a[t64 + j * kSplitThreads];
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-          const int idx = t64 + j * kSplitThreads;
-          float4 h, l;
-          h.x = __uint_as_float(__float_as_uint(v[j].x) & 0xFFFFE000u); l.x = v[j].x - h.x;
-          h.y = __uint_as_float(__float_as_uint(v[j].y) & 0xFFFFE000u); l.y = v[j].y - h.y;
-          h.z = __uint_as_float(__float_as_uint(v[j].z) & 0xFFFFE000u); l.z = v[j].z - h.z;
-          h.w = __uint_as_float(__float_as_uint(v[j].w) & 0xFFFFE000u); l.w = v[j].w - h.w;
-          a[idx] = h;
-          alo[idx] = l;
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> tensor-core reads
+        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(S::kTmemA + s * 64);
+        tmem_st32(ta, hi);
+        tmem_st32(ta + 32, lo);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(ready_bar(s));
       }
@@ -432,18 +440,26 @@ __global__ void __launch_bounds__(TcSmem<BN, TS>::kThreads, 1) tc_gemm_kernel(co
   } else {
     // ---- epilogue: drain each chunk's partial sum from TMEM, add in FP32 registers, store at tile end
     const int ew = warp & 3;  // a warp may only touch TMEM lanes 32 * (warp % 4) .. + 31
-    float accr[ONE_CHUNK ? 1 : BN];
-    int chunk = 0, slab = 0;
+    const int half = warp >= 10 ? 1 : 0;
+    constexpr int HN = BN / 2;  // columns of this warp: [half * HN, half * HN + HN)
+    unsigned char* slab = base_ptr + kStages * S::kStageBytes + (half * 4 + ew) * 16 * 128;
+    float** rows = row_addr + (half * 4 + ew) * 32;
+    float accr[ONE_CHUNK ? 1 : HN];
+    int chunk = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-      const TileInfo t = decode_tile<BN>(batch, tile_start, tile);
+      const TileInfo t = decode_tile<BN>(batch, tile_start, tables, tile);
       const TcProblem& P = batch.p[t.prob];
-      const int r = ew * 32 + lane;
-      const int al = r / P.q, m = r - al * P.q;
-      const bool valid = r < P.R * P.q && t.atom0 + al < t.atom_end;
-      long long atom = t.atom0 + al;
-      if (valid && P.atom_map) atom = P.atom_map[atom];
-      float* dst = P.C + atom * P.c_s1 + (long long)m * P.c_s2 + t.n0;
+      {  // addresses of this warp's 32 rows (every warp keeps its own: no barrier that a warp giving up could leave others at)
+        const int r = ew * 32 + lane;
+        const int al = r / P.q, m = r - al * P.q;
+        const bool valid = r < P.R * P.q && t.atom0 + al < t.atom_end;
+        long long atom = t.atom0 + al;
+        if (valid && P.atom_map) atom = P.atom_map[atom];
+        __syncwarp();
+        rows[lane] = valid ? P.C + atom * P.c_s1 + (long long)m * P.c_s2 + t.n0 : nullptr;
+        __syncwarp();
+      }
       const float* bias = P.bias ? P.bias + t.group * P.bias_group_stride + t.n0 : nullptr;
       const bool accumulate = P.accumulate != 0;
       const int n_chunks = (t.num_k + kChunk - 1) / kChunk;
@@ -452,61 +468,13 @@ __global__ void __launch_bounds__(TcSmem<BN, TS>::kThreads, 1) tc_gemm_kernel(co
         if (!mbar_wait(acc_full(a), (chunk >> 1) & 1, abort_flag, batch.error, 5, batch.spin_limit)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-        for (int c = 0; c < BN / 32; ++c) {
+        for (int c = 0; c < HN / 32; ++c) {
           uint32_t rr[32];
-          tmem_ld32(tmem_base + ((uint32_t)(ew * 32) << 16) + a * BN + c * 32, rr);
+          const int col = half * HN + c * 32;
+          tmem_ld32(tmem_base + ((uint32_t)(ew * 32) << 16) + a * BN + col, rr);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
           if constexpr (ONE_CHUNK) {
-            if (P.c_tma) {
-              // stage the warp's 32 x 32 slab in shared memory (16-byte chunk j of row r at chunk j ^ (r & 7), the
-              // 128-byte swizzle of the tensor map) and let the TMA unit write whole 128-byte rows; rows past the
-              // end of the tensor are clipped by the hardware
-              const uint32_t buf = store_base + (uint32_t)((ew * 2 + (slab & 1)) * 32 * 128);
-              if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // slab - 2 has left this buffer
-              __syncwarp();
-#pragma unroll
-              for (int q4 = 0; q4 < 8; ++q4) {
-                float4 v = make_float4(__uint_as_float(rr[4 * q4]), __uint_as_float(rr[4 * q4 + 1]), __uint_as_float(rr[4 * q4 + 2]),
-                                       __uint_as_float(rr[4 * q4 + 3]));
-                if (bias) {
-                  const float4 bv = *reinterpret_cast<const float4*>(bias + c * 32 + 4 * q4);
-                  v.x += bv.x; v.y += bv.y; v.z += bv.z; v.w += bv.w;
-                }
-                const uint32_t addr = buf + (uint32_t)(lane * 128 + ((q4 ^ (lane & 7)) << 4));
-                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-              }
-              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> TMA reads
-              __syncwarp();
-              if (lane == 0) {
-                tma_store_2d(&P.tmC, buf, t.n0 + c * 32, t.atom0 + ew * 32);
-                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-              }
-              ++slab;
-            } else if (valid) {
-              // all loads of a slab before its first store: a load that follows a store to the same 128-byte line
-              // waits for that store to be acknowledged by L2, which would serialise the row
-              float4 v[8];
-#pragma unroll
-              for (int q4 = 0; q4 < 8; ++q4)
-                v[q4] = make_float4(__uint_as_float(rr[4 * q4]), __uint_as_float(rr[4 * q4 + 1]), __uint_as_float(rr[4 * q4 + 2]),
-                                    __uint_as_float(rr[4 * q4 + 3]));
-              if (bias) {
-#pragma unroll
-                for (int q4 = 0; q4 < 8; ++q4) {
-                  const float4 bv = *reinterpret_cast<const float4*>(bias + c * 32 + 4 * q4);
-                  v[q4].x += bv.x; v[q4].y += bv.y; v[q4].z += bv.z; v[q4].w += bv.w;
-                }
-              }
-              if (accumulate) {
-                float4 ov[8];
-#pragma unroll
-                for (int q4 = 0; q4 < 8; ++q4) ov[q4] = *reinterpret_cast<const float4*>(dst + c * 32 + 4 * q4);
-#pragma unroll
-                for (int q4 = 0; q4 < 8; ++q4) { v[q4].x += ov[q4].x; v[q4].y += ov[q4].y; v[q4].z += ov[q4].z; v[q4].w += ov[q4].w; }
-              }
-#pragma unroll
-              for (int q4 = 0; q4 < 8; ++q4) *reinterpret_cast<float4*>(dst + c * 32 + 4 * q4) = v[q4];
-            }
+            store_slab(slab, rr, bias ? bias + col : nullptr, rows, col, accumulate, lane);
           } else {
 #pragma unroll
             for (int q = 0; q < 32; ++q) accr[c * 32 + q] = cin == 0 ? __uint_as_float(rr[q]) : accr[c * 32 + q] + __uint_as_float(rr[q]);
@@ -515,30 +483,20 @@ __global__ void __launch_bounds__(TcSmem<BN, TS>::kThreads, 1) tc_gemm_kernel(co
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         mbar_arrive(acc_empty(a));  // the issuer may overwrite this accumulator
         if constexpr (!ONE_CHUNK) {
-          if (cin == n_chunks - 1 && valid) {
-            if (accumulate) {  // every load of the row before its first store (see above)
+          if (cin == n_chunks - 1) {
 #pragma unroll
-              for (int q4 = 0; q4 < BN / 4; ++q4) {
-                const float4 ov = *reinterpret_cast<const float4*>(dst + 4 * q4);
-                accr[4 * q4] += ov.x; accr[4 * q4 + 1] += ov.y; accr[4 * q4 + 2] += ov.z; accr[4 * q4 + 3] += ov.w;
-              }
+            for (int c = 0; c < HN / 32; ++c) {
+              uint32_t rr[32];
+#pragma unroll
+              for (int q = 0; q < 32; ++q) rr[q] = __float_as_uint(accr[c * 32 + q]);
+              const int col = half * HN + c * 32;
+              store_slab(slab, rr, bias ? bias + col : nullptr, rows, col, accumulate, lane);
             }
-            if (bias) {
-#pragma unroll
-              for (int q4 = 0; q4 < BN / 4; ++q4) {
-                const float4 bv = *reinterpret_cast<const float4*>(bias + 4 * q4);
-                accr[4 * q4] += bv.x; accr[4 * q4 + 1] += bv.y; accr[4 * q4 + 2] += bv.z; accr[4 * q4 + 3] += bv.w;
-              }
-            }
-#pragma unroll
-            for (int q4 = 0; q4 < BN / 4; ++q4)
-              *reinterpret_cast<float4*>(dst + 4 * q4) = make_float4(accr[4 * q4], accr[4 * q4 + 1], accr[4 * q4 + 2], accr[4 * q4 + 3]);
           }
         }
       }
     }
   }
-  if (warp >= 4 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // TMA stores of this warp are complete
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S::kTmemCols));
@@ -600,40 +558,22 @@ bool make_map_3d(CUtensorMap* map, const float* ptr, long long atoms, int q, lon
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// 2-D fp32 result [rows][N] with row stride ldc; box = 32 rows x 32 columns, 128-byte swizzle.
-bool make_map_c(CUtensorMap* map, float* ptr, long long rows, long long N, long long ldc) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)ldc * sizeof(float)};
-  const cuuint32_t box[2] = {32, 32};
-  const cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // Function attributes and the SM count belong to a device, not to the process: one slot per device ordinal.
 constexpr int kMaxDevices = 64;
 
-template <int BN, bool ONE_CHUNK, bool TS>
-cudaError_t launch_tc_v(const TcBatch& b, int dev, int sms, cudaStream_t s) {
+template <int BN, bool ONE_CHUNK>
+cudaError_t launch_tc(const TcBatch& b, int dev, int sms, cudaStream_t s) {
   static bool configured[kMaxDevices] = {};
-  using S = TcSmem<BN, TS>;
+  using S = TcSmem<BN>;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_kernel<BN, ONE_CHUNK, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
+    cudaError_t e = cudaFuncSetAttribute(tc_gemm_kernel<BN, ONE_CHUNK>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
   const int tiles = b.tile_start[b.n_problems];  // upper bound for per-species problems
   const int grid = tiles < sms ? tiles : sms;
-  tc_gemm_kernel<BN, ONE_CHUNK, TS><<<grid, S::kThreads, S::kTotal, s>>>(b);
+  tc_gemm_kernel<BN, ONE_CHUNK><<<grid, S::kThreads, S::kTotal, s>>>(b);
   return cudaGetLastError();
-}
-template <int BN, bool ONE_CHUNK>
-cudaError_t launch_tc(const TcBatch& b, int dev, int sms, cudaStream_t s) {
-  // TACE_B200_GEMM_TMEM_OPERAND=0 selects the variant with both operands in shared memory (three / four stages)
-  static const bool ts = [] { const char* e = getenv("TACE_B200_GEMM_TMEM_OPERAND"); return !(e && e[0] == '0'); }();
-  return ts ? launch_tc_v<BN, ONE_CHUNK, true>(b, dev, sms, s) : launch_tc_v<BN, ONE_CHUNK, false>(b, dev, sms, s);
 }
 
 }  // namespace
@@ -670,15 +610,24 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
   b.error = error_flag;
   b.spin_limit = g_test_spin_limit ? g_test_spin_limit : kSpinLimit;
   b.extra_tx = g_test_extra_tx;
-  int tiles = 0;
+  // long K loops first: tiles are dealt round robin, and the short ones fill what the long ones leave of the last round
+  int order[kTcMaxProblems];
   for (int i = 0; i < n_problems; ++i) {
-    const TcLinearProblem& h = probs[i];
+    int j = i;
+    for (; j > 0 && probs[order[j - 1]].K < probs[i].K; --j) order[j] = order[j - 1];
+    order[j] = i;
+  }
+  int tiles = 0, table = 0;
+  for (int i = 0; i < n_problems; ++i) {
+    const TcLinearProblem& h = probs[order[i]];
     if (h.n_atoms <= 0) continue;
     TcProblem& P = b.p[b.n_problems];
     P.q = h.q; P.R = kBM / h.q; P.n_atoms = (int)h.n_atoms; P.N = h.N; P.K = h.K;
     P.C = h.C; P.bias = h.bias; P.c_s1 = h.c_s1; P.c_s2 = h.c_s2; P.bias_group_stride = h.bias_group_stride;
     P.n_groups = h.n_groups; P.group_ptr = h.group_ptr; P.tile_ptr = h.tile_ptr; P.atom_map = h.atom_map;
     P.accumulate = h.accumulate;
+    P.table = -1;
+    if (h.n_groups > 0 && table + 2 * (h.n_groups + 1) <= TcSmem<128>::kTableInts) { P.table = table; table += 2 * (h.n_groups + 1); }
     const int groups = h.n_groups > 0 ? h.n_groups : 1;
     if (h.n_groups > 0 && (!h.group_ptr || !h.tile_ptr)) return cudaErrorInvalidValue;
     P.b_tiled = h.b_tiled;
@@ -688,12 +637,6 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
                   : (!make_map_b(&P.tmBhi, h.Bhi, groups, h.N, h.K, h.b_group_stride, bn) ||
                      !make_map_b(&P.tmBlo, h.Blo, groups, h.N, h.K, h.b_group_stride, bn)))
       return cudaErrorInvalidValue;
-    // large plain results (the per-edge weights of the radial MLP) leave through TMA stores
-    P.c_tma = 0;
-    if (one && h.q == 1 && h.n_groups == 0 && !h.atom_map && !h.accumulate && (reinterpret_cast<uintptr_t>(h.C) & 15) == 0) {
-      if (!make_map_c(&P.tmC, h.C, h.n_atoms, h.N, h.c_s1)) return cudaErrorInvalidValue;
-      P.c_tma = 1;
-    }
     b.tile_start[b.n_problems] = tiles;
     tiles += (int)((h.n_atoms + P.R - 1) / P.R + h.n_groups) * (h.N / bn);
     ++b.n_problems;
