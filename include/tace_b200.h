@@ -277,6 +277,21 @@ int tace_nl_fill(const double* positions, const double* lattice, const uint8_t* 
                  int32_t n_graphs, int64_t n_atoms, double cutoff, const int64_t* row_ptr, int64_t n_edges,
                  int64_t* edge_index, int32_t* edge_shifts, void* workspace, size_t workspace_bytes, tace_stream_t stream);
 
+/* The same pair with the row pointers computed on the device and the preparation done once: tace_nl_rows fills counts and
+ * row_ptr[n_atoms + 1] (row_ptr[n_atoms] = number of edges) and leaves its bins in the workspace; tace_nl_fill_rows, called
+ * with the same structures and that workspace untouched, writes the edges.  n_targets >= 0: only the first n_targets atoms
+ * get rows (the others, ghost copies, act as sources only).  shift_type: TACE_F32 / TACE_F64 writes the shifts as reals of
+ * that type, anything else as int32.  Same edges, same order. */
+int tace_nl_rows(const double* positions, const double* lattice, const uint8_t* pbc, const int32_t* graph_ptr, int32_t n_graphs,
+                 int64_t n_atoms, int64_t n_targets, double cutoff, int32_t* counts, int64_t* row_ptr, void* workspace,
+                 size_t workspace_bytes, tace_stream_t stream);
+int tace_nl_fill_rows(const double* positions, const double* lattice, const uint8_t* pbc, const int32_t* graph_ptr, int32_t n_graphs,
+                      int64_t n_atoms, int64_t n_targets, double cutoff, const int64_t* row_ptr, int64_t n_edges, int64_t* edge_index,
+                      void* edge_shifts, int32_t shift_type, void* workspace, size_t workspace_bytes, tace_stream_t stream);
+
+/* out[i][:] = one-hot row of species[i] among n_elements, as reals of `dtype` (TACE_F32 / TACE_F64). */
+int tace_one_hot(const int32_t* species, int64_t n, int32_t n_elements, int32_t dtype, void* out, tace_stream_t stream);
+
 /* Neighbour list in one call that allocates nothing.  No counterpart in the reference.
  *
  * For hosts that must not allocate device memory while they run: an MD engine that has handed all of

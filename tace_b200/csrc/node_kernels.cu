@@ -2,6 +2,7 @@
 // Feature layout everywhere: [atom][component (l, m)][channel], channel fastest, so a warp
 // always touches 32 consecutive channels of one component.
 #include <cstdint>
+#include "../../include/tace_b200.h"
 #include "kernels.h"
 #include "tp_gen.cuh"
 
@@ -644,6 +645,14 @@ cudaError_t launch_graph_energy(const T* e_scaled, const T* e0, const int* speci
   return cudaGetLastError();
 }
 
+template <typename T>
+__global__ void one_hot_kernel(const int* __restrict__ species, long long n, int n_el, T* __restrict__ out) {
+  const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (k >= n * n_el) return;
+  const long long i = k / n_el;
+  out[k] = species[i] == (int)(k - i * n_el) ? T(1) : T(0);
+}
+
 #define INST(T)                                                                                               \
   template cudaError_t launch_fill_zero<T>(T*, long long, cudaStream_t);                                      \
   template cudaError_t launch_pb3_fwd<T>(const T*, const T*, T*, int, int, int, int, cudaStream_t);           \
@@ -669,3 +678,13 @@ INST(double)
 template cudaError_t launch_fill_zero<int>(int*, long long, cudaStream_t);
 
 }  // namespace tace
+
+extern "C" int tace_one_hot(const int32_t* species, int64_t n, int32_t n_elements, int32_t dtype, void* out, tace_stream_t stream) {
+  if (n < 0 || n_elements <= 0 || (n > 0 && (!species || !out)) || (dtype != TACE_F32 && dtype != TACE_F64)) return TACE_ERR_INVALID_ARGUMENT;
+  if (n == 0) return TACE_OK;
+  const unsigned grid = (unsigned)((n * n_elements + 255) / 256);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (dtype == TACE_F32) tace::one_hot_kernel<float><<<grid, 256, 0, s>>>(species, n, n_elements, static_cast<float*>(out));
+  else tace::one_hot_kernel<double><<<grid, 256, 0, s>>>(species, n, n_elements, static_cast<double*>(out));
+  return cudaGetLastError() == cudaSuccess ? TACE_OK : TACE_ERR_CUDA;
+}

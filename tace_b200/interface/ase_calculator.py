@@ -110,15 +110,22 @@ class TACEAseCalc(Calculator):
             "ptr": np.array([0, n], dtype=np.int64),
         }
         data = build_batch(host, self.atomic_numbers, self.cutoff, self.dtype, self.device)
-        outs = self.model(data)
+        with torch.no_grad():
+            outs, block = self.model._evaluate(data)
+        if block is not None:  # every result in one transfer
+            host, size = block.cpu().numpy(), block.element_size()
+            at = lambda x: (x.data_ptr() - block.data_ptr()) // size
+            fetch = lambda x: host[at(x):at(x) + x.numel()].reshape(x.shape)
+        else:
+            fetch = lambda x: x.cpu().numpy()
         self.results = {}
         for p in self.target_property:
             if outs.get(p) is None:
                 continue
             if p == "energy":
-                self.results["energy"] = float(outs[p].cpu().item())
+                self.results["energy"] = float(fetch(outs[p])[0])
                 self.results["free_energy"] = self.results["energy"]
             elif p in ("stress", "virials"):
-                self.results[p] = outs[p].cpu().numpy().squeeze(0)
+                self.results[p] = fetch(outs[p]).squeeze(0)
             else:
-                self.results[p] = outs[p].cpu().numpy()
+                self.results[p] = fetch(outs[p])

@@ -6,6 +6,7 @@ entry points the header declares, importing callers fail loudly here.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from ctypes import POINTER, c_char_p, c_double, c_int, c_int32, c_int64, c_size_t, c_uint8, c_void_p
@@ -21,7 +22,7 @@ EXPORTS = [
     "tace_launch_count", "tace_profile_enable", "tace_profile_count", "tace_profile_read", "tace_tc_gemm_f32", "tace_tc_gemm_set_test_mode",
     "tace_device_error", "tace_set_exchange", "tace_nl_build_noalloc", "tace_md_kick_drift", "tace_md_kinetic_energy",
     "tace_edge_vectors", "tace_edges_within", "tace_edges_scan_workspace_bytes", "tace_edges_scan", "tace_edges_compact", "tace_rows_gather", "tace_rows_scatter_add", "tace_set_graph_mode", "tace_graph_replays", "tace_set_exchange_sync", "tace_set_exchange_stream",
-    "tace_set_chunk_edges", "tace_md_langevin",
+    "tace_set_chunk_edges", "tace_md_langevin", "tace_nl_rows", "tace_nl_fill_rows", "tace_one_hot",
 ]
 
 
@@ -105,6 +106,11 @@ def load() -> ctypes.CDLL:
                                   ctypes.c_size_t, c_void_p]
     lib.tace_nl_fill.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int64, c_double, c_void_p, c_int64,
                                  c_void_p, c_void_p, c_void_p, ctypes.c_size_t, c_void_p]
+    lib.tace_nl_rows.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int64, c_int64, c_double, c_void_p, c_void_p, c_void_p,
+                                 ctypes.c_size_t, c_void_p]
+    lib.tace_nl_fill_rows.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int64, c_int64, c_double, c_void_p, c_int64,
+                                      c_void_p, c_void_p, c_int32, c_void_p, ctypes.c_size_t, c_void_p]
+    lib.tace_one_hot.argtypes = [c_void_p, c_int64, c_int32, c_int32, c_void_p, c_void_p]
     lib.tace_set_graph_mode.argtypes = [c_void_p, c_int]
     lib.tace_set_chunk_edges.argtypes = [c_void_p, c_int64]
     lib.tace_graph_replays.argtypes = [c_void_p]
@@ -122,6 +128,21 @@ def load() -> ctypes.CDLL:
     lib.tace_rows_scatter_add.argtypes = [c_void_p, c_void_p, c_int64, c_int32, c_int32, c_void_p, c_void_p]
     _lib = lib
     return lib
+
+
+_HERE = contextlib.nullcontext()
+
+
+def on_device(device):
+    """``torch.cuda.device(device)``, free of charge when that device is current already."""
+    import torch
+    return _HERE if device.index is None or device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+def stream_of(device) -> int:
+    """Handle of the current stream of ``device`` (no Stream object on the way)."""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 
 def dtype_code(dtype) -> int:

@@ -48,6 +48,8 @@ _DEFAULTS: Dict[str, Any] = {
     "dropout": {"use_first_dropout": False, "stochastic_depth": 0.0},
 }
 
+_ROW_STRIDES = {1: (1,), 2: (3, 1), 3: (9, 3, 1)}
+_RESULT_BLOCK = 1 << 16  # results of at most this many values share one allocation
 _SUPPORTED_TARGETS = {"energy", "forces", "stress", "virials", "edge_forces"}
 
 
@@ -479,6 +481,11 @@ class TensorModel(torch.nn.Module):
     # ---- forward -------------------------------------------------------------------------------------
     @torch.no_grad()
     def forward(self, data: Dict[str, torch.Tensor]) -> Dict[str, Optional[torch.Tensor]]:
+        return self._evaluate(data)[0]
+
+    def _evaluate(self, data: Dict[str, torch.Tensor]):
+        """(results, block): ``block`` is the one allocation the results are views of when they are small, so that a caller who
+        wants them on the host fetches them in one transfer; None when they are separate."""
         lib = _lib.load()
         dtype = self.get_model_dtype()
         node_attrs = data.get("node_attrs")
@@ -488,13 +495,14 @@ class TensorModel(torch.nn.Module):
         handle = self._native(device)
         flags = self.flags
         species = data["species"] if "species" in data else node_attrs.argmax(dim=-1)
-        species = species.to(torch.int32).contiguous()
-        edge_index = data["edge_index"].to(torch.int64).contiguous()
+        ready = lambda x, dt: x if x.dtype == dt and x.is_contiguous() else x.to(dt).contiguous()
+        species = ready(species, torch.int32)
+        edge_index = ready(data["edge_index"], torch.int64)
         E = int(edge_index.shape[1])
         keep = [species, edge_index]
 
         def real(x):
-            x = x.detach().to(dtype).contiguous()
+            x = ready(x, dtype)
             keep.append(x)
             return x
 
@@ -506,13 +514,13 @@ class TensorModel(torch.nn.Module):
             if n_atoms == 0:  # a rank of a domain decomposition that neither owns nor sees any atom
                 zeros = lambda *shape: torch.zeros(*shape, dtype=dtype, device=device)
                 return {"energy": zeros(1), "node_energy": zeros(0), "forces": zeros(0, 3) if flags.compute_forces else None,
-                        "virials": None, "stress": None, "edge_forces": zeros(0, 3)}
+                        "virials": None, "stress": None, "edge_forces": zeros(0, 3)}, None
             # an empty edge list (a rank that owns no atom) still has to say "edge-vector mode": never a NULL pointer
             vec = data["edge_vector"] if E > 0 else torch.zeros(1, 3, dtype=dtype, device=device)
             batch.edge_vector = real(vec).data_ptr()
         else:
             n_atoms = n_local = int(species.shape[0])
-            graph_ptr = data["ptr"].to(torch.int32).contiguous()
+            graph_ptr = ready(data["ptr"], torch.int32)
             n_graphs = int(graph_ptr.numel() - 1)
             batch.positions = real(data["positions"]).data_ptr()
             batch.lattice = real(data["lattice"]).reshape(-1, 3, 3).data_ptr()
@@ -533,19 +541,28 @@ class TensorModel(torch.nn.Module):
         out = _lib.TaceOutputs()
         res: Dict[str, Optional[torch.Tensor]] = {k: None for k in
                                                    ("energy", "node_energy", "forces", "virials", "stress", "edge_forces")}
-        res["energy"] = torch.empty(n_graphs, dtype=dtype, device=device)
-        res["node_energy"] = torch.empty(n_local, dtype=dtype, device=device)
-        out.energy, out.node_energy = res["energy"].data_ptr(), res["node_energy"].data_ptr()
+        shapes = {"energy": (n_graphs,), "node_energy": (n_local,)}
         if flags.compute_forces:  # edge-vector mode: rows of ghost atoms hold the force parts that belong to their owners
-            res["forces"] = torch.empty(n_atoms, 3, dtype=dtype, device=device)
-            out.forces = res["forces"].data_ptr()
+            shapes["forces"] = (n_atoms, 3)
         if (flags.compute_stress or flags.compute_virials) and not self.lmp:
-            res["virials"] = torch.empty(n_graphs, 3, 3, dtype=dtype, device=device)
-            res["stress"] = torch.empty(n_graphs, 3, 3, dtype=dtype, device=device)
-            out.virials, out.stress = res["virials"].data_ptr(), res["stress"].data_ptr()
+            shapes["virials"] = shapes["stress"] = (n_graphs, 3, 3)
         if flags.compute_edge_forces or self.lmp:
-            res["edge_forces"] = torch.empty(E, 3, dtype=dtype, device=device)
-            out.edge_forces = res["edge_forces"].data_ptr()
+            shapes["edge_forces"] = (E, 3)
+        sizes = {k: math.prod(s) for k, s in shapes.items()}
+        block = None
+        if sum(sizes.values()) <= _RESULT_BLOCK:
+            at, places = 0, {}
+            for k, size in sizes.items():
+                places[k] = at
+                at += (size + 3) & ~3  # every result starts at a multiple of 16 bytes
+            block = torch.empty(at, dtype=dtype, device=device)
+            for k, shape in shapes.items():
+                res[k] = block.as_strided(shape, _ROW_STRIDES[len(shape)], places[k])
+        else:
+            for k, shape in shapes.items():
+                res[k] = torch.empty(shape, dtype=dtype, device=device)
+        for k in shapes:
+            setattr(out, k, res[k].data_ptr())
 
         exchange_cb = None
         if self.lmp and n_atoms != n_local and self.readout_fn.num_layers > 1:
@@ -562,7 +579,7 @@ class TensorModel(torch.nn.Module):
             _lib.check(lib.tace_set_exchange(handle, exchange_cb, None), "tace_set_exchange")
             _lib.check(lib.tace_set_exchange_sync(handle, 0 if ordered else 1), "tace_set_exchange_sync")
             _lib.check(lib.tace_set_exchange_stream(handle, side.cuda_stream if side is not None else None), "tace_set_exchange_stream")
-        with torch.cuda.device(device):
+        with _lib.on_device(device):
             nbytes = ctypes.c_size_t()
 
             def needed() -> int:
@@ -605,20 +622,21 @@ class TensorModel(torch.nn.Module):
                 self._sized_for = shape_key
             ws = self._get_workspace(self._sized_bytes, device)
             ws_ptr = (ws.data_ptr() + 255) & ~255
-            stream = torch.cuda.current_stream(device).cuda_stream
-            self._exchange_error = None
+            stream = _lib.stream_of(device)
+            if exchange_cb is not None:
+                self._exchange_error = None
             try:
                 _lib.check(lib.tace_forward(handle, ctypes.byref(batch), ctypes.byref(out), ws_ptr,
                                             ws.numel() - (ws_ptr - ws.data_ptr()), stream), "tace_forward")
             except _lib.TaceError as exc:
-                if self._exchange_error is not None:  # the callback failed: show its exception, not the bare status
+                if exchange_cb is not None and self._exchange_error is not None:  # the callback failed: show its exception, not the bare status
                     raise self._exchange_error from exc
                 raise
             finally:
                 # the handle must never keep a pointer to a callback object that dies with this frame
                 if exchange_cb is not None:
                     lib.tace_set_exchange(handle, _lib.EXCHANGE_FN(0), None)
-        return res
+        return res, block
 
     def _make_exchange(self, lmp_data, dtype: torch.dtype, device: torch.device, sync: bool = True, stream=None):
         """ctypes callback handing the workspace rows to ``lmp_data.forward_exchange`` /
@@ -682,7 +700,7 @@ class TensorModel(torch.nn.Module):
         lib = _lib.load()
         device = self._workspace.device
         buf = torch.empty(numel, dtype=self.get_model_dtype(), device=device)
-        n = lib.tace_debug_read(self._handle, name.encode(), buf.data_ptr(), numel, torch.cuda.current_stream(device).cuda_stream)
+        n = lib.tace_debug_read(self._handle, name.encode(), buf.data_ptr(), numel, _lib.stream_of(device))
         if n < 0:
             raise _lib.TaceError(f"tace_debug_read({name}): status {n}")
         return buf[:n]

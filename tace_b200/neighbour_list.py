@@ -50,33 +50,38 @@ def neighbor_list_batch(positions: torch.Tensor, lattice: torch.Tensor, pbc: tor
     target) and ``edge_shifts int32[E,3]`` with edge vector = r[target] - r[source] + shift @ cell.
     ``n_targets``: keep only edges whose target is one of the first ``n_targets`` atoms (the owned
     atoms of a domain; the rest are ghost copies that only act as sources)."""
+    if positions.device.type != "cuda":
+        raise _lib.TaceError("tace_b200 neighbour lists run on CUDA devices only")
+    return _list_on_device(positions.to(torch.float64).contiguous(), lattice.to(torch.float64).reshape(-1, 3, 3).contiguous(),
+                           pbc.to(torch.uint8).reshape(-1, 3).contiguous(), graph_ptr.to(torch.int32).contiguous(), cutoff,
+                           -1 if n_targets is None else int(n_targets), torch.int32)
+
+
+_SHIFT_TYPES = {torch.int32: -1, torch.float32: _lib.TACE_F32, torch.float64: _lib.TACE_F64}
+
+
+def _list_on_device(positions: torch.Tensor, lattice: torch.Tensor, pbc: torch.Tensor, graph_ptr: torch.Tensor, cutoff: float,
+                    n_targets: int, shift_dtype: torch.dtype) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``neighbor_list_batch`` on arguments that have its types and layout already; shifts as ``shift_dtype``."""
     lib = _lib.load()
     dev = positions.device
-    if dev.type != "cuda":
-        raise _lib.TaceError("tace_b200 neighbour lists run on CUDA devices only")
-    positions = positions.to(torch.float64).contiguous()
-    lattice = lattice.to(torch.float64).reshape(-1, 3, 3).contiguous()
-    pbc = pbc.to(torch.uint8).reshape(-1, 3).contiguous()
-    graph_ptr = graph_ptr.to(torch.int32).contiguous()
     n, b = positions.shape[0], lattice.shape[0]
-    counts = torch.zeros(n, dtype=torch.int32, device=dev)
     need = ctypes.c_size_t()
     _lib.check(lib.tace_nl_workspace_bytes(n, b, ctypes.byref(need)), "tace_nl_workspace_bytes")
-    work = torch.empty(int(need.value), dtype=torch.uint8, device=dev)  # torch's caching allocator: no cudaMalloc once warm
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        _lib.check(lib.tace_nl_count(positions.data_ptr(), lattice.data_ptr(), pbc.data_ptr(), graph_ptr.data_ptr(), b, n,
-                                     float(cutoff), counts.data_ptr(), work.data_ptr(), work.numel(), stream), "tace_nl_count")
-        if n_targets is not None and n_targets < n:
-            counts[n_targets:] = 0  # rows without edges start at the end of the list and write nothing
-        row_ptr = torch.zeros(n + 1, dtype=torch.int64, device=dev)
-        torch.cumsum(counts, 0, out=row_ptr[1:])
-        n_edges = int(row_ptr[-1].item())
+    # one scratch from torch's caching allocator: row pointers | counts | the library's workspace
+    rows, counts = 8 * (n + 1), 4 * n
+    scratch = torch.empty(rows + counts + int(need.value) + 256, dtype=torch.uint8, device=dev)
+    row_ptr = scratch.data_ptr()
+    work = row_ptr + rows + counts
+    args = (positions.data_ptr(), lattice.data_ptr(), pbc.data_ptr(), graph_ptr.data_ptr(), b, n, n_targets, float(cutoff))
+    with _lib.on_device(dev):
+        stream = _lib.stream_of(dev)
+        _lib.check(lib.tace_nl_rows(*args, row_ptr + rows, row_ptr, work, int(need.value) + 256, stream), "tace_nl_rows")
+        n_edges = int(scratch[8 * n:8 * n + 8].view(torch.int64).item())
         edge_index = torch.empty(2, n_edges, dtype=torch.int64, device=dev)
-        shifts = torch.empty(n_edges, 3, dtype=torch.int32, device=dev)
-        _lib.check(lib.tace_nl_fill(positions.data_ptr(), lattice.data_ptr(), pbc.data_ptr(), graph_ptr.data_ptr(), b, n,
-                                    float(cutoff), row_ptr.data_ptr(), n_edges, edge_index.data_ptr(), shifts.data_ptr(),
-                                    work.data_ptr(), work.numel(), stream), "tace_nl_fill")
+        shifts = torch.empty(n_edges, 3, dtype=shift_dtype, device=dev)
+        _lib.check(lib.tace_nl_fill_rows(*args, row_ptr, n_edges, edge_index.data_ptr(), shifts.data_ptr(), _SHIFT_TYPES[shift_dtype],
+                                         work, int(need.value) + 256, stream), "tace_nl_fill_rows")
     return edge_index, shifts
 
 

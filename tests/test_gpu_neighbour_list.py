@@ -71,3 +71,35 @@ def test_batch_matches_per_structure():
     assert np.array_equal(gi, ref_i) and np.array_equal(gs, ref_s)
     # grouped by target: row 1 is non-decreasing
     assert (np.diff(ei[1].cpu().numpy()) >= 0).all()
+
+
+@pytest.mark.parametrize("n_mol,copies", [(1, 1), (5, 3), (900, 1), (2731, 1)])  # 3 atoms .. 8 193: one-block preparation and beyond it
+def test_rows_entry_equals_the_count_and_fill_pair(n_mol, copies):
+    """tace_nl_rows / tace_nl_fill_rows (device-side row pointers, reused preparation, real shifts) against tace_nl_count /
+    tace_nl_fill with host-side row pointers: the same edges in the same order."""
+    import ctypes
+    from tace_b200 import lib as _lib, synth
+    from tace_b200.neighbour_list import _list_on_device
+    lib, dev = _lib.load(), torch.device("cuda:0")
+    side = int(np.ceil(n_mol ** (1 / 3)))
+    structs = [synth.water_box(n_side=side, box=max(3.2 * side, 4.0), seed=k, n_mol=n_mol) for k in range(copies)]
+    b = synth.collate(structs)
+    pbc = torch.as_tensor(b["pbc"], device=dev)
+    pbc[0, 2] = 0  # one open axis
+    pos, lat = torch.as_tensor(b["positions"], device=dev), torch.as_tensor(b["lattice"], device=dev)
+    ptr = torch.as_tensor(b["ptr"], device=dev).to(torch.int32)
+    n, g, rc = pos.shape[0], lat.shape[0], 5.0
+    ei, es = _list_on_device(pos, lat, pbc, ptr, rc, -1, torch.float64)
+    need = ctypes.c_size_t()
+    assert lib.tace_nl_workspace_bytes(n, g, ctypes.byref(need)) == 0
+    work = torch.empty(need.value, dtype=torch.uint8, device=dev)
+    counts = torch.empty(n, dtype=torch.int32, device=dev)
+    args = (pos.data_ptr(), lat.data_ptr(), pbc.data_ptr(), ptr.data_ptr(), g, n, rc)
+    assert lib.tace_nl_count(*args, counts.data_ptr(), work.data_ptr(), work.numel(), 0) == 0
+    rows = torch.zeros(n + 1, dtype=torch.int64, device=dev)
+    rows[1:] = torch.cumsum(counts, 0)
+    E = int(rows[-1])
+    ei2, es2 = torch.empty(2, E, dtype=torch.int64, device=dev), torch.empty(E, 3, dtype=torch.int32, device=dev)
+    assert lib.tace_nl_fill(*args, rows.data_ptr(), E, ei2.data_ptr(), es2.data_ptr(), work.data_ptr(), work.numel(), 0) == 0
+    assert E > 0 or n_mol == 1
+    assert torch.equal(ei, ei2) and torch.equal(es, es2.double())
