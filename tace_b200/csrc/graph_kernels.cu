@@ -41,7 +41,7 @@ __global__ void lower_bound_kernel(const int* __restrict__ sorted_keys, long lon
   }
   rowptr[i] = (int)lo;
 }
-// tile_ptr: 64-row tiles of the CUDA-core GEMM; tc_tile_ptr: (128 / q)-atom tiles of the tensor-core GEMM; q = 1, 3, 5, 7.  One warp per
+// tile_ptr: 32-row tiles of gemm.cuh; tc_tile_ptr: (128 / q)-atom tiles of the tensor-core GEMM; q = 1, 3, 5, 7.  One warp per
 // table (`which` = 0..7), a warp scan over the species.
 __device__ __forceinline__ void tile_table(const int* species_ptr, int n_el, int which, int* tile_ptr, int* tc_tile_ptr) {
   const int qi = which & 3, lane = threadIdx.x & 31;
@@ -53,7 +53,7 @@ __device__ __forceinline__ void tile_table(const int* species_ptr, int n_el, int
     int tiles = 0;
     if (g < n_el) {
       const int cnt = species_ptr[g + 1] - species_ptr[g];
-      if (!tc) tiles = (cnt * (2 * qi + 1) + 63) >> 6;
+      if (!tc) tiles = (cnt * (2 * qi + 1) + 31) >> 5;
       else tiles = qi == 0 ? (cnt + 127) >> 7 : qi == 1 ? (cnt + 41) / 42 : qi == 2 ? (cnt + 24) / 25 : (cnt + 17) / 18;
     }
     int x = tiles;

@@ -272,7 +272,7 @@ struct GraphPrepArgs {
   int* perm_src; int* rowptr_src;       // [E], [n_atoms+1]
   int* atom_graph;            // [n_atoms]
   int* species_perm; int* species_ptr;  // [n_local], [n_elements+1]
-  int* tile_ptr;              // [4][n_elements+1] for q = 1,3,5,7: 64-row tiles per species
+  int* tile_ptr;              // [4][n_elements+1] for q = 1,3,5,7: 32-row tiles per species
   int* tc_tile_ptr;           // [4][n_elements+1]: (128 / q)-atom tiles per species
   void* temp; size_t temp_bytes;
 };
