@@ -394,8 +394,8 @@ struct Model : ModelBase {
   int rt_K = 0;               // > 0: path weights interpolated from per-layer tables with rt_K intervals (TaceConfig.radial_table)
   int t_NR = 0, t_NC = 0, t_NF = 0, t_G = 0, t_np = 0, t_WN = 0;  // rows (order-major / per weight / full), gates, paths, coefficients
   int t_k[4] = {1, 1, 1, 1}, t_base[4] = {0, 1, 4, 9};            // message layout of a TECE layer: one block of C per rank
-  int t_row_l[16], t_row_m[16], t_row_comp[16]; double t_row_scale[16];
-  int t_p_m1[12], t_p_m2[12], t_p_m3[12], t_p_sum[12]; double t_p_scale[12];
+  int t_wg = 0;  // packed Wigner entries per edge
+  double t_row_scale[16], t_p_scale[12];
   int m0 = 1;  // 1: every rank gated (gate_m0 = True); 0: e3nn Gate, scalars through SiLU (gate_m0 = False)
   std::vector<LayerPlan> layers;
   std::vector<WeightEntry> weights;
@@ -455,11 +455,7 @@ struct Model : ModelBase {
       t_NR = 0; t_NC = 0;
       for (int m = 0; m <= mmax; ++m) {
         for (int sign = 1; sign >= (m ? -1 : 1); sign -= 2)
-          for (int l = m; l <= L; ++l) {
-            t_row_l[t_NR] = l; t_row_m[t_NR] = sign * m; t_row_comp[t_NR] = t_NC + (l - m);
-            t_row_scale[t_NR] = l > mmax ? std::sqrt((2.0 * l + 1.0) / (2.0 * mmax + 1.0)) : 1.0;
-            ++t_NR;
-          }
+          for (int l = m; l <= L; ++l) t_row_scale[t_NR++] = l > mmax ? std::sqrt((2.0 * l + 1.0) / (2.0 * mmax + 1.0)) : 1.0;
         t_NC += L + 1 - m;
       }
       t_NF = n + 2 * n * mmax;
@@ -472,11 +468,12 @@ struct Model : ModelBase {
           for (int m2 = 0; m2 <= m1; ++m2) {
             const bool sum = (m1 + m2 == m3), diff = !sum && (m1 - m2 == m3);
             if (!sum && !diff) continue;
-            t_p_m1[t_np] = m1; t_p_m2[t_np] = m2; t_p_m3[t_np] = m3; t_p_sum[t_np] = sum ? 1 : 0; ++t_np;
+            ++t_np;
           }
         for (int q = first; q < t_np; ++q) t_p_scale[q] = 1.0 / std::sqrt((double)(t_np - first));
       }
       t_WN = t_np * n * Ca;
+      t_wg = tece_wigner_stride(L, mmax);
     }
     if (bilinear && c.correlation != 2) return TACE_ERR_UNSUPPORTED_CONFIG;
     if (zbl < 0 || zbl > 2 || density < 0 || density > 2 || (density && element2)) return TACE_ERR_UNSUPPORTED_CONFIG;
@@ -665,7 +662,7 @@ struct Model : ModelBase {
     T *XY, *gXY, *Zg, *gZg;     // gated bilinear product: both factors per (atom, component), gate pre-activations, gradients
     // TECE edge block (layouts at the top of tece_kernels.cu); gradients that may overwrite their forward buffer do
     T *tKs, *tQt, *tMw, *tKp, *tQp, *tlogit, *talpha, *tup, *tglu, *tcoef, *tU, *tdown;
-    T *tgdown, *tgalpha, *tglogit, *tgcut, *tgproj, *tproj, *tgQp, *tgKp, *tgKs, *tgQt, *tdxt, *tddlen;
+    T *tgdown, *tgalpha, *tglogit, *tgcut, *tgproj, *tproj, *tgQp, *tgKp, *tgKs, *tgQt, *tddlen;
   };
   struct Bufs {
     int *row_ids, *row_split;  // owned targets without / with a ghost source (passes split around the exchange)
@@ -675,7 +672,7 @@ struct Model : ModelBase {
     void* prep_temp; size_t prep_temp_bytes;
     T *energy_partial;  // slice sums of the per-graph energies (graph_energy_slices)
     T *vec, *Y, *dY, *g, *e_scaled, *atom_virial, *dxe, *dlen, *ddlen, *ro_factor, *env, *denv, *zbl_node;
-    T *tWg, *tgWg, *tgvec;  // TECE: Wigner rows of every edge (shared by the layers), their gradient, dE/d(edge vector) through them
+    T *tWg, *tgWg, *tgvec;  // TECE: Wigner rows of every edge (shared by the layers), their gradient (a share per 32 channels), dE/d(edge vector) through them
     std::vector<LayerBufs> lay;
   };
 
@@ -691,7 +688,7 @@ struct Model : ModelBase {
     b.energy_partial = ar.take<T>((size_t)B * graph_energy_slices(NL, B));
     b.e_scaled = ar.take<T>(NL); b.atom_virial = ar.take<T>(9 * NL); b.ro_factor = ar.take<T>(NL); b.zbl_node = zbl ? ar.take<T>(NL) : nullptr;
     b.tWg = b.tgWg = b.tgvec = nullptr;
-    if (tece_mask) { b.tWg = ar.take<T>((size_t)E * t_NR * D); b.tgWg = ar.take<T>((size_t)E * t_NR * D); b.tgvec = ar.take<T>(3 * (size_t)E); }
+    if (tece_mask) { b.tWg = ar.take<T>((size_t)E * t_wg); b.tgWg = ar.take<T>((size_t)E * t_wg * (C / 32)); b.tgvec = ar.take<T>(3 * (size_t)E); }
     b.dlen = ar.take<T>(E); b.ddlen = ar.take<T>(E);
     b.env = env_after ? ar.take<T>(E) : nullptr; b.denv = env_after ? ar.take<T>(E) : nullptr;
     const bool chunked = E > max_chunk_edges;
@@ -748,7 +745,7 @@ struct Model : ModelBase {
         lb.tgcut = ar.take<T>(Es * heads); lb.tgproj = ar.take<T>(Es * 2 * heads); lb.tproj = ar.take<T>(Es * 2 * heads);
         lb.tgQp = ar.take<T>(Es * t_NR * C); lb.tgKp = ar.take<T>(Es * t_NR * C);
         lb.tgKs = ar.take<T>(Es * t_NR * C); lb.tgQt = ar.take<T>(Es * t_NR * C);
-        lb.tdxt = ar.take<T>(Es * D * C); lb.tddlen = ar.take<T>(Es);
+        lb.tddlen = ar.take<T>(Es);
       }
       if (bilinear) {
         lb.XY = ar.take<T>((size_t)NL * D * 2 * C); lb.gXY = ar.take<T>((size_t)NL * D * 2 * C);
@@ -940,14 +937,14 @@ struct Model : ModelBase {
       off_out += (m == 0) ? sh.n_out[0] : 2 * sh.n_out[m];
     }
   }
-  TeceArgs<T> tece_args(const EdgeArgs<T>& ea, const Bufs& b, const LayerBufs& lb, const std::string& pre, const T* x_src, long long NL,
-                        long long E) const {
+  TeceArgs<T> tece_args(const EdgeArgs<T>& ea, const Bufs& b, const LayerBufs& lb, const std::string& pre, const T* x_src, long long N,
+                        long long NL, long long E) const {
     TeceArgs<T> a;
     memset(&a, 0, sizeof(a));
-    a.E = E; a.n_local = (int)NL; a.C = C; a.Ca = Ca; a.L = L; a.mmax = mmax; a.H = heads; a.NR = t_NR; a.NC = t_NC; a.G = t_G;
-    a.n_paths = t_np; a.gate_m0 = m0; a.act = edge_act;
-    for (int r = 0; r < t_NR; ++r) { a.row_l[r] = t_row_l[r]; a.row_m[r] = t_row_m[r]; a.row_comp[r] = t_row_comp[r]; a.row_scale[r] = T(t_row_scale[r]); }
-    for (int q = 0; q < t_np; ++q) { a.p_m1[q] = t_p_m1[q]; a.p_m2[q] = t_p_m2[q]; a.p_m3[q] = t_p_m3[q]; a.p_sum[q] = t_p_sum[q]; a.p_scale[q] = T(t_p_scale[q]); }
+    a.E = E; a.n_atoms = (int)N; a.n_local = (int)NL; a.C = C; a.Ca = Ca; a.L = L; a.mmax = mmax; a.H = heads; a.NR = t_NR;
+    a.gate_m0 = m0; a.act = edge_act;
+    for (int r = 0; r < t_NR; ++r) a.row_scale[r] = T(t_row_scale[r]);
+    for (int q = 0; q < t_np; ++q) a.p_scale[q] = T(t_p_scale[q]);
     a.rp = ea.rp; a.vec = b.vec; a.dlen = b.dlen; a.env = env_after ? b.env : nullptr;
     a.e_src = b.e_src; a.e_dst = b.e_dst; a.rowptr = b.rowptr_dst;
     a.x = x_src; a.W = lb.W; a.Wg = b.tWg; a.Ks = lb.tKs; a.Qt = lb.tQt; a.Mw = lb.tMw; a.Kp = lb.tKp; a.Qp = lb.tQp;
@@ -956,7 +953,7 @@ struct Model : ModelBase {
     a.gM = lb.M; a.gdown = lb.tgdown; a.galpha = lb.tgalpha; a.glogit = lb.tglogit; a.gcut = lb.tgcut; a.gproj = lb.tgproj; a.proj = lb.tproj;
     a.gQp = lb.tgQp; a.gKp = lb.tgKp; a.gKs = lb.tgKs; a.gQt = lb.tgQt; a.gMw = lb.tMw;
     a.gU = lb.tU; a.gup = lb.tup; a.gglu = lb.tglu; a.gcoefZ = lb.tcoef; a.gWg = b.tgWg; a.gvec = b.tgvec;
-    a.dxe = b.dxe; a.dxt = lb.tdxt; a.gx = lb.gx; a.ddlen_extra = lb.tddlen;
+    a.dxe = b.dxe; a.gx = lb.gx; a.ddlen_extra = lb.tddlen;
     return a;
   }
   // forward of the block for one layer: lb.W holds the radial weights, the result lands in lb.M
@@ -1005,9 +1002,7 @@ struct Model : ModelBase {
     so2_specs(sp, pre, 1, lb.tgQp, t_NR, lb.tgQt, t_NR, true, 0);
     CKL(run_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_ROTATE_IN_BWD, s));
-    CKL(launch_segment_sum_rows(b.dxe, b.rowptr_src, b.perm_src, lb.gx, 0, (int)N, D * C, s));
-    CKL(launch_tece(ta, TECE_TARGET_SUM, s));
-    CKL(launch_tece(ta, TECE_WIGNER_GRAD, s));
+    CKL(launch_segment_sum_rows(b.dxe, b.rowptr_src, b.perm_src, lb.gx, 0, (int)N, D * C, s, /*accumulate=*/1));
     ta.accumulate_gvec = first_tece ? 0 : 1;
     CKL(launch_tece(ta, TECE_WIGNER_BWD, s));
     return TACE_OK;
@@ -1302,7 +1297,7 @@ struct Model : ModelBase {
         PH(("t" + ts + ".fwd.tp").c_str());
         if (p.tece) {  // the edge block instead of the tensor product (whole batch only)
           if (chunked) return TACE_ERR_CAPACITY;
-          const TeceArgs<T> tc = tece_args(ea, b, lb, pre, x_src, NL, E);
+          const TeceArgs<T> tc = tece_args(ea, b, lb, pre, x_src, N, NL, E);
           if (!wigner_done) { CKL(launch_tece(tc, TECE_WIGNER, s)); wigner_done = true; }
           CKS(tece_forward(tc, lb, pre, E, s));
           continue;
@@ -1567,7 +1562,7 @@ struct Model : ModelBase {
             CKL(launch_fill_zero(b.dY, E * D, s));
             if (b.denv) CKL(launch_fill_zero(b.denv, E, s));
           }
-          const TeceArgs<T> tc = tece_args(ea, b, lb, pre, lb.xx ? lb.xx : lb.x, NL, E);
+          const TeceArgs<T> tc = tece_args(ea, b, lb, pre, lb.xx ? lb.xx : lb.x, N, NL, E);
           CKS(tece_backward(tc, b, lb, pre, N, E, !tece_seen, s));
           tece_seen = true;
           PH(("t" + ts + ".bwd.radial_gemm").c_str());

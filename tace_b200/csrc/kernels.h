@@ -67,7 +67,7 @@ cudaError_t launch_tp_bwd_wide(const TPArgs<float>& a, cudaStream_t s);
 // gx[b] = sum of dxe over the edges whose source is b (edges listed by perm within rowptr_src segments)
 // for the source atoms [first_atom, first_atom + n_atoms)
 template <typename T> cudaError_t launch_segment_sum_rows(const T* dxe, const int* rowptr_src, const int* perm_src, T* gx,
-                                                          int first_atom, int n_atoms, int row_len, cudaStream_t s);
+                                                          int first_atom, int n_atoms, int row_len, cudaStream_t s, int accumulate = 0);
 // Edge-chunked variant: positions [k0, k1) of the (chunk, source)-sorted edge list belong to one chunk whose dxe rows start
 // at edge k0; every run of equal keys is summed in list order and ADDED to gx[key - key_base] (runs of one chunk have
 // distinct sources, chunks are processed one after another, so the sum order is fixed).
@@ -299,14 +299,14 @@ namespace tace {
 enum TeceStage {
   TECE_WIGNER, TECE_ROTATE_IN, TECE_LOGIT, TECE_SOFTMAX, TECE_MIX, TECE_ROTATE_OUT,
   TECE_ROTATE_OUT_BWD, TECE_ALPHA_BWD, TECE_SOFTMAX_BWD, TECE_LOGIT_BWD, TECE_EDGE_SCALAR_BWD, TECE_MIX_BWD,
-  TECE_ROTATE_IN_BWD, TECE_TARGET_SUM, TECE_WIGNER_GRAD, TECE_WIGNER_BWD
+  TECE_ROTATE_IN_BWD, TECE_WIGNER_BWD
 };
 // One argument block for every kernel of the edge block (layouts are described at the top of tece_kernels.cu).
 template <typename T>
 struct TeceArgs {
-  long long E; int n_local, C, Ca, L, mmax, H, NR, NC, G, n_paths, gate_m0, act, accumulate_gvec;
-  int row_l[16], row_m[16], row_comp[16]; T row_scale[16];          // order-major rows: rank, signed order, weight component, inverse rescale
-  int p_m1[12], p_m2[12], p_m3[12], p_sum[12]; T p_scale[12];        // cluster-expansion paths
+  long long E; int n_atoms, n_local, C, Ca, L, mmax, H, NR, gate_m0, act, accumulate_gvec;
+  T row_scale[16];                                                   // inverse rescale of every order-major row
+  T p_scale[12];                                                     // scales of the cluster-expansion paths
   RadialParams<T> rp;
   const T* vec; const T* dlen; const T* env;                         // env == nullptr: no cutoff factor (apply_cutoff = True)
   const int* e_src; const int* e_dst; const int* rowptr;
@@ -314,8 +314,9 @@ struct TeceArgs {
   const T* temp; const T* rproj_w; const T* rproj_b;                 // per-head scale * temperature; radial projection [8][2H], [2H]
   T* up; T* glu; T* coefZ; T* U; T* down; T* M;
   const T* gM; T* gdown; T* galpha; T* glogit; T* gcut; T* gproj; T* proj; T* gQp; T* gKp; T* gKs; T* gQt; T* gMw;
-  const T* gU; T* gup; T* gglu; T* gcoefZ; T* gWg; T* gvec; T* dxe; T* dxt; T* gx; T* ddlen_extra;
+  const T* gU; T* gup; T* gglu; T* gcoefZ; T* gWg; T* gvec; T* dxe; T* gx; T* ddlen_extra;
 };
+int tece_wigner_stride(int L, int mmax);  // entries of one edge's packed Wigner rows (tece_kernels.cu)
 template <typename T> cudaError_t launch_tece(const TeceArgs<T>& a, int stage, cudaStream_t s);
 
 struct TcLinearProblem {

@@ -6,14 +6,16 @@
 // (y) axis is the edge, keep the orders |m| <= mmax, weight them with the radial MLP output, run SO(2) linears (GEMMs,
 // launched by the engine), gate + edge cluster expansion, attention-weighted inverse rotation and sum per target atom.
 //
-// Layouts (channel fastest): node features x [N][D][C], D = (L+1)^2; Wigner rows Wg [E][NR][D], NR rows in order-major
-// layout (m = 0: l = 0..L | +1: l = 1..L | -1 | +2 | -2); Ks / Qt / Kp / Qp / down [E][NR][C]; Mw [E][NR][2C];
+// Layouts (channel fastest): node features x [N][D][C], D = (L+1)^2; Wigner rows Wg [E][NEP], packed (see below); NR rows in
+// order-major layout (m = 0: l = 0..L | +1: l = 1..L | -1 | +2 | -2); Ks / Qt / Kp / Qp / down [E][NR][C]; Mw [E][NR][2C];
 // radial weights W [E][NC][2C]; up [E][G + NF][Ca]; glu, U [E][NF][Ca] with NF = n + 2 n mmax, n = L + 1 (every order
 // carries n rows there); coef [E][paths][n][Ca]; logit / alpha [E][H].  Edges are sorted by target (CSR rowptr).
 //
-// The derivative of the Wigner rows with respect to the edge vector is taken in forward mode (three directional
-// derivatives carried through the frame and the recursion), so no hand-derived adjoint of the quaternion blend exists.
+// The derivative of the Wigner rows with respect to the edge vector runs backwards through the recursion and in forward mode
+// (three directional derivatives) through the frame, so no hand-derived adjoint of the quaternion blend exists.
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "kernels.h"
 #include "tace_common.cuh"
@@ -100,42 +102,6 @@ TACE_D void edge_frame(S vx, S vy, S vz, S (&R)[9]) {
   R[6] = two * (a * c - w * b); R[7] = two * (b * c + w * a); R[8] = one - two * (a * a + b * b);
 }
 
-// blocks D^0..D^L of the rotation (wigner.py:316-357), D^l stored row-major at offset sum_{k<l} (2k+1)^2 of `blocks`
-// (1 + 9 + 25 + 49 = 84 entries for L = 3)
-template <typename T, typename S>
-TACE_D void wigner_blocks(const S (&R)[9], int L, S* blocks) {
-  blocks[0] = mkS(R[0], T(1));
-  if (L >= 1) for (int k = 0; k < 9; ++k) blocks[1 + k] = R[k];
-  int off_prev = 1, off = 10;
-  for (int l = 2; l <= L; ++l) {
-    const double* cg = (l == 2) ? w3j_1_1_2 : w3j_1_2_3;  // [3][2l-1][2l+1]
-    const int dp = 2 * l - 1, dl = 2 * l + 1;
-    // left[b][m][c] = sum_a cg[a][b][m] R[a][c]; then tmp[m][c][d] = sum_b left[b][m][c] Dprev[b][d]; D[m][n] = sum_cd tmp cg[c][d][n]
-    for (int m = 0; m < dl; ++m)
-      for (int n = 0; n < dl; ++n) {
-        S acc = mkS(R[0], T(0));
-        for (int c = 0; c < 3; ++c)
-          for (int d = 0; d < dp; ++d) {
-            const T cr = T(cg[(c * dp + d) * dl + n]);
-            if (cr == T(0)) continue;
-            S t = mkS(R[0], T(0));
-            for (int a = 0; a < 3; ++a)
-              for (int b = 0; b < dp; ++b) {
-                const T cl = T(cg[(a * dp + b) * dl + m]);
-                if (cl == T(0)) continue;
-                t = t + cl * (R[a * 3 + c] * blocks[off_prev + b * dp + d]);
-              }
-            acc = acc + cr * t;
-          }
-        blocks[off + m * dl + n] = T(dl) * acc;
-      }
-    off_prev = off;
-    off += dl * dl;
-  }
-}
-
-TACE_D TACE_INLINE int block_offset(int l) { return l == 0 ? 0 : l == 1 ? 1 : l == 2 ? 10 : 35; }
-
 template <typename T>
 TACE_D TACE_INLINE T act_eval(int kind, T x) { return kind == 0 ? T(1.8467055342154763) * sigmoid_(x) : T(1.6791767923989418) * silu_(x); }
 template <typename T>
@@ -144,271 +110,553 @@ TACE_D TACE_INLINE T act_grad(int kind, T x) {
   return T(1.6791767923989418) * silu_grad_(x);
 }
 
-// ---- K0: Wigner rows of every edge ---------------------------------------------------------------
-template <typename T>
-__global__ void tece_wigner_kernel(const TeceArgs<T> a) {
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (e >= a.E) return;
-  T R[9], blocks[84];
-  edge_frame<T, T>(a.vec[3 * e], a.vec[3 * e + 1], a.vec[3 * e + 2], R);
-  wigner_blocks<T, T>(R, a.L, blocks);
-  const int D = (a.L + 1) * (a.L + 1);
-  T* out = a.Wg + e * a.NR * D;
-  for (int r = 0; r < a.NR; ++r) {
-    const int l = a.row_l[r], m = a.row_m[r], dl = 2 * l + 1;
-    for (int j = 0; j < D; ++j) out[r * D + j] = T(0);
-    for (int j = 0; j < dl; ++j) out[r * D + l * l + j] = blocks[block_offset(l) + (l + m) * dl + j];
-  }
+// ---- compile-time geometry of the order-major rows --------------------------------------------------------------
+// Row r of the order-major layout belongs to order m, part (0: +m, 1: -m) and rank l.  The Wigner rows of one edge are kept
+// packed: only the 2l + 1 entries of the row's own rank block, in the order (m, l, part) in which for_rows visits the rows,
+// padded to a multiple of four entries (72 of them for L = 3, mmax = 2, where full rows would take 14 x 16).
+TACE_HD constexpr int row_index(int L, int m, int part, int l) { return (m == 0 ? 0 : m == 1 ? L + 1 : L + 1 + 2 * L) + part * (L + 1 - m) + (l - m); }
+TACE_HD constexpr int comp_base(int L, int m) { return m == 0 ? 0 : m == 1 ? L + 1 : 2 * L + 1; }
+TACE_HD constexpr int packed_offset(int L, int MM, int m, int part, int l) {
+  int k = 0;
+  for (int mm = 0; mm <= MM; ++mm)
+    for (int ll = mm; ll <= L; ++ll)
+      for (int pp = 0; pp < (mm ? 2 : 1); ++pp) {
+        if (mm == m && ll == l && pp == part) return k;
+        k += 2 * ll + 1;
+      }
+  return k;  // past the last row: the number of entries
 }
-// gvec[e][k] (+)= sum_{r, j} gWg[e][r][j] dWg[e][r][j] / dv_k
-template <typename T>
-__global__ void tece_wigner_bwd_kernel(const TeceArgs<T> a, int accumulate) {
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (e >= a.E) return;
-  typedef Dual3<T> S;
-  S R[9], blocks[84];
-  S vx = {a.vec[3 * e], {T(1), T(0), T(0)}}, vy = {a.vec[3 * e + 1], {T(0), T(1), T(0)}}, vz = {a.vec[3 * e + 2], {T(0), T(0), T(1)}};
-  edge_frame<T, S>(vx, vy, vz, R);
-  wigner_blocks<T, S>(R, a.L, blocks);
-  const int D = (a.L + 1) * (a.L + 1);
-  const T* g = a.gWg + e * a.NR * D;
-  T acc[3] = {T(0), T(0), T(0)};
-  for (int r = 0; r < a.NR; ++r) {
-    const int l = a.row_l[r], m = a.row_m[r], dl = 2 * l + 1;
-    for (int j = 0; j < dl; ++j) {
-      const S& d = blocks[block_offset(l) + (l + m) * dl + j];
-      const T gv = g[r * D + l * l + j];
-      acc[0] += gv * d.d[0]; acc[1] += gv * d.d[1]; acc[2] += gv * d.d[2];
-    }
-  }
-  for (int k = 0; k < 3; ++k) a.gvec[3 * e + k] = accumulate ? a.gvec[3 * e + k] + acc[k] : acc[k];
-}
-
-// ---- K1: rotate both ends into the edge frame, radial weighting ------------------------------------
-template <typename T>
-__global__ void tece_rotate_in_kernel(const TeceArgs<T> a) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= a.E * a.C) return;
-  const long long e = idx / a.C;
-  const int c = (int)(idx - e * a.C), C = a.C, D = (a.L + 1) * (a.L + 1);
-  const T* xs = a.x + (long long)a.e_src[e] * D * C + c;
-  const T* xt = a.x + (long long)a.e_dst[e] * D * C + c;
-  const T* Wg = a.Wg + e * a.NR * D;
-  const T* W = a.W + e * a.NC * 2 * C;
-  for (int r = 0; r < a.NR; ++r) {
-    const int l = a.row_l[r], dl = 2 * l + 1;
-    T ks = T(0), qt = T(0);
-    for (int j = 0; j < dl; ++j) {
-      const T wv = Wg[r * D + l * l + j];
-      ks += wv * xs[(long long)(l * l + j) * C];
-      qt += wv * xt[(long long)(l * l + j) * C];
-    }
-    a.Ks[(e * a.NR + r) * C + c] = ks;
-    a.Qt[(e * a.NR + r) * C + c] = qt;
-    const int comp = a.row_comp[r];
-    a.Mw[(e * a.NR + r) * 2 * C + c] = W[comp * 2 * C + c] * ks;
-    a.Mw[(e * a.NR + r) * 2 * C + C + c] = W[comp * 2 * C + C + c] * qt;
-  }
-}
-// backward of K1: gKs / gQt hold the gradients that came through the key / query projections; gMw the one through the
-// weighted features.  Writes dW (radial-weight gradient, over W), the per-edge source rows dxe [E][D][C] and the per-edge
-// target rows dxt [E][D][C] (summed per atom afterwards).
-template <typename T>
-__global__ void tece_rotate_in_bwd_kernel(const TeceArgs<T> a) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= a.E * a.C) return;
-  const long long e = idx / a.C;
-  const int c = (int)(idx - e * a.C), C = a.C, D = (a.L + 1) * (a.L + 1);
-  const T* Wg = a.Wg + e * a.NR * D;
-  T* W = a.W + e * a.NC * 2 * C;
-  T gs[16], gt[16], dws[9], dwt[9], ws[9], wt[9];
-  for (int j = 0; j < D; ++j) { gs[j] = T(0); gt[j] = T(0); }
-  for (int k = 0; k < a.NC; ++k) { dws[k] = T(0); dwt[k] = T(0); ws[k] = W[k * 2 * C + c]; wt[k] = W[k * 2 * C + C + c]; }
-  for (int r = 0; r < a.NR; ++r) {
-    const int l = a.row_l[r], dl = 2 * l + 1, comp = a.row_comp[r];
-    const long long at = (e * a.NR + r);
-    const T gms = a.gMw[at * 2 * C + c], gmt = a.gMw[at * 2 * C + C + c];
-    dws[comp] += gms * a.Ks[at * C + c];
-    dwt[comp] += gmt * a.Qt[at * C + c];
-    const T gks = a.gKs[at * C + c] + ws[comp] * gms;
-    const T gqt = a.gQt[at * C + c] + wt[comp] * gmt;
-    a.gKs[at * C + c] = gks;  // totals, read again by the Wigner-gradient kernel
-    a.gQt[at * C + c] = gqt;
-    for (int j = 0; j < dl; ++j) {
-      const T wv = Wg[r * D + l * l + j];
-      gs[l * l + j] += wv * gks;
-      gt[l * l + j] += wv * gqt;
-    }
-  }
-  for (int k = 0; k < a.NC; ++k) { W[k * 2 * C + c] = dws[k]; W[k * 2 * C + C + c] = dwt[k]; }
-  for (int j = 0; j < D; ++j) { a.dxe[(e * D + j) * C + c] = gs[j]; a.dxt[(e * D + j) * C + c] = gt[j]; }
-}
-// gx[i][j][c] += sum over the edges into i of dxt[e][j][c]
-template <typename T>
-__global__ void tece_target_sum_kernel(const TeceArgs<T> a) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const int D = (a.L + 1) * (a.L + 1);
-  if (idx >= (long long)a.n_local * D * a.C) return;
-  const long long i = idx / ((long long)D * a.C);
-  const long long jc = idx - i * D * a.C;
-  T acc = T(0);
-  for (int e = a.rowptr[i]; e < a.rowptr[i + 1]; ++e) acc += a.dxt[(long long)e * D * a.C + jc];
-  a.gx[idx] += acc;
-}
-
-// ---- the rotation kernels with rank and order limits known at compile time -------------------------------------
-// for_rows visits the order-major rows with constant (row, rank, weight component) after unrolling, so the per-thread
-// arrays of the kernels below are indexed statically and stay in registers.
+template <int L, int MM> struct Rows {
+  static constexpr int D = (L + 1) * (L + 1);
+  static constexpr int NR = row_index(L, MM, MM ? 1 : 0, L) + 1, NC = comp_base(L, MM) + L + 1 - MM;
+  static constexpr int NE = packed_offset(L, MM, MM + 1, 0, 0), NEP = (NE + 3) / 4 * 4;
+};
+// f(row, rank, weight component, packed offset), every argument a constant after unrolling, so that the per-thread arrays of
+// the kernels below are indexed statically and stay in registers
 template <int L, int MM, typename F>
 TACE_D TACE_INLINE void for_rows(F&& f) {
-  int r = 0, comp0 = 0;
 #pragma unroll
-  for (int m = 0; m <= MM; ++m) {
+  for (int m = 0; m <= MM; ++m)
 #pragma unroll
-    for (int part = 0; part < (m ? 2 : 1); ++part)
+    for (int l = m; l <= L; ++l)
 #pragma unroll
-      for (int l = m; l <= L; ++l) { f(r, l, comp0 + l - m); ++r; }
-    comp0 += L + 1 - m;
+      for (int part = 0; part < (m ? 2 : 1); ++part)
+        f(row_index(L, m, part, l), l, comp_base(L, m) + l - m, packed_offset(L, MM, m, part, l));
+}
+
+// ---- K0: Wigner rows of every edge ---------------------------------------------------------------
+// The recursion of wigner.py:316-357 with the coupling tables folded in at compile time (only the non-zero terms are left:
+// 11 of 45 and 23 of 105), one column of the block at a time: T[a][b] = sum_{c, d} cg[c][d][n] R[a][c] D[b][d], then
+// D'[m][n] = (2l + 1) sum_{a, b} cg[a][b][m] T[a][b].
+template <int LP, typename T>
+TACE_D TACE_INLINE T coupling(int a, int b, int m) { return T(LP == 1 ? w3j_1_1_2[(a * 3 + b) * 5 + m] : w3j_1_2_3[(a * 5 + b) * 7 + m]); }
+template <int LP, typename T>  // block of rank LP + 1 from the rotation and the block of rank LP
+TACE_D TACE_INLINE void wigner_up(const T (&R)[9], const T* Dp, T* Dn) {
+  constexpr int np = 2 * LP + 1, nn = 2 * LP + 3;
+#pragma unroll
+  for (int n = 0; n < nn; ++n) {
+    T t[3 * np];
+#pragma unroll
+    for (int k = 0; k < 3 * np; ++k) t[k] = T(0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int d = 0; d < np; ++d) {
+        const T w = coupling<LP, T>(c, d, n);
+        if (w != T(0)) {
+#pragma unroll
+          for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < np; ++b) t[a * np + b] += (w * R[a * 3 + c]) * Dp[b * np + d];
+        }
+      }
+#pragma unroll
+    for (int m = 0; m < nn; ++m) {
+      T v = T(0);
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < np; ++b) {
+          const T w = coupling<LP, T>(a, b, m);
+          if (w != T(0)) v += w * t[a * np + b];
+        }
+      Dn[m * nn + n] = T(nn) * v;
+    }
   }
 }
-template <int L, int MM> struct RowCount { static constexpr int NR = (L + 1) + (MM >= 1 ? 2 * L : 0) + (MM >= 2 ? 2 * (L - 1) : 0); };
+// adjoint of wigner_up: gDn -> += gR, gDp
+template <int LP, typename T>
+TACE_D TACE_INLINE void wigner_up_bwd(const T (&R)[9], const T* Dp, const T* gDn, T (&gR)[9], T* gDp) {
+  constexpr int np = 2 * LP + 1, nn = 2 * LP + 3;
+#pragma unroll
+  for (int n = 0; n < nn; ++n) {
+    T u[3 * np];  // d / d T[a][b]
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < np; ++b) {
+        T v = T(0);
+#pragma unroll
+        for (int m = 0; m < nn; ++m) {
+          const T w = coupling<LP, T>(a, b, m);
+          if (w != T(0)) v += w * gDn[m * nn + n];
+        }
+        u[a * np + b] = T(nn) * v;
+      }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int d = 0; d < np; ++d) {
+        const T w = coupling<LP, T>(c, d, n);
+        if (w != T(0)) {
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            T v = T(0);
+#pragma unroll
+            for (int b = 0; b < np; ++b) {
+              v += u[a * np + b] * Dp[b * np + d];
+              gDp[b * np + d] += (w * R[a * 3 + c]) * u[a * np + b];
+            }
+            gR[a * 3 + c] += w * v;
+          }
+        }
+      }
+  }
+}
 
+// One thread per edge; the packed rows leave through shared memory as whole lines.  526 k edges, L = 3, mmax = 2: 0.04 ms,
+// against 2.05 ms with run-time recursion loops over local arrays and rows stored entry by entry.
+constexpr int kFrameThreads = 64;
 template <typename T, int L, int MM>
-__global__ void __launch_bounds__(128) tece_rotate_in_t_kernel(const TeceArgs<T> a) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= a.E * a.C) return;
-  const long long e = idx / a.C;
-  constexpr int D = (L + 1) * (L + 1), NR = RowCount<L, MM>::NR;
-  const int c = (int)(idx - e * a.C), C = a.C;
-  const T* xs = a.x + (long long)a.e_src[e] * D * C + c;
-  const T* xt = a.x + (long long)a.e_dst[e] * D * C + c;
-  const T* __restrict__ Wg = a.Wg + e * NR * D;
-  const T* __restrict__ W = a.W + e * a.NC * 2 * C;
-  T vs[D], vt[D];
+__global__ void __launch_bounds__(kFrameThreads) tece_wigner_kernel(const TeceArgs<T> a) {
+  typedef Rows<L, MM> RW;
+  __shared__ T st[kFrameThreads * (RW::NEP + 1)];
+  const long long e0 = blockIdx.x * (long long)kFrameThreads, e = e0 + threadIdx.x;
+  if (e < a.E) {
+    T R[9], D2[25], D3[49];
+    edge_frame<T, T>(a.vec[3 * e], a.vec[3 * e + 1], a.vec[3 * e + 2], R);
+    if (L >= 2) wigner_up<1, T>(R, R, D2);
+    if (L >= 3) wigner_up<2, T>(R, D2, D3);
+    T* o = st + threadIdx.x * (RW::NEP + 1);
 #pragma unroll
-  for (int j = 0; j < D; ++j) { vs[j] = xs[(long long)j * C]; vt[j] = xt[(long long)j * C]; }
-  for_rows<L, MM>([&](int r, int l, int comp) {
-    T ks = T(0), qt = T(0);
+    for (int m = 0; m <= MM; ++m)
 #pragma unroll
-    for (int j = 0; j < 2 * l + 1; ++j) {
-      const T wv = Wg[r * D + l * l + j];
-      ks += wv * vs[l * l + j];
-      qt += wv * vt[l * l + j];
-    }
-    a.Ks[(e * NR + r) * C + c] = ks;
-    a.Qt[(e * NR + r) * C + c] = qt;
-    a.Mw[(e * NR + r) * 2 * C + c] = W[comp * 2 * C + c] * ks;
-    a.Mw[(e * NR + r) * 2 * C + C + c] = W[comp * 2 * C + C + c] * qt;
-  });
+      for (int l = m; l <= L; ++l)
+#pragma unroll
+        for (int part = 0; part < (m ? 2 : 1); ++part) {
+          const int k = packed_offset(L, MM, m, part, l), row = l + (part ? -m : m);
+#pragma unroll
+          for (int j = 0; j < 2 * l + 1; ++j)
+            o[k + j] = l == 0 ? T(1) : l == 1 ? R[(row * 3 + j) % 9] : l == 2 ? D2[(row * 5 + j) % 25] : D3[(row * 7 + j) % 49];
+        }
+#pragma unroll
+    for (int k = RW::NE; k < RW::NEP; ++k) o[k] = T(0);
+  }
+  __syncthreads();
+  const long long left = a.E - e0;
+  const int n = (int)(left < kFrameThreads ? left : kFrameThreads) * RW::NEP;
+  for (int k = threadIdx.x; k < n; k += kFrameThreads) a.Wg[e0 * RW::NEP + k] = st[k / RW::NEP * (RW::NEP + 1) + k % RW::NEP];
 }
+// gvec[e][k] (+)= sum over the packed entries of gWg dWg / dv_k: adjoint through the recursion down to the rotation matrix,
+// then the three directional derivatives of the frame in forward mode.  gWg comes as one share per group of 32 channels.
+// 526 k edges: 0.55 ms, against 1.76 ms with the whole recursion in forward mode.
 template <typename T, int L, int MM>
-__global__ void __launch_bounds__(128) tece_rotate_in_bwd_t_kernel(const TeceArgs<T> a) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= a.E * a.C) return;
-  const long long e = idx / a.C;
-  constexpr int D = (L + 1) * (L + 1), NR = RowCount<L, MM>::NR, NC = (L + 1) + (MM >= 1 ? L : 0) + (MM >= 2 ? L - 1 : 0);
-  const int c = (int)(idx - e * a.C), C = a.C;
-  const T* __restrict__ Wg = a.Wg + e * NR * D;
-  T* W = a.W + e * NC * 2 * C;
-  T gs[D], gt[D], dws[NC], dwt[NC], ws[NC], wt[NC];
+__global__ void __launch_bounds__(kFrameThreads) tece_wigner_bwd_kernel(const TeceArgs<T> a) {
+  typedef Rows<L, MM> RW;
+  __shared__ T st[kFrameThreads * (RW::NEP + 1)];
+  const long long e0 = blockIdx.x * (long long)kFrameThreads, e = e0 + threadIdx.x;
+  const long long left = a.E - e0;
+  const int n = (int)(left < kFrameThreads ? left : kFrameThreads) * RW::NEP, n_col = a.C / 32;
+  for (int k = threadIdx.x; k < n; k += kFrameThreads) {
+    T v = T(0);
+    for (int q = 0; q < n_col; ++q) v += a.gWg[((long long)q * a.E + e0) * RW::NEP + k];
+    st[k / RW::NEP * (RW::NEP + 1) + k % RW::NEP] = v;
+  }
+  __syncthreads();
+  if (e >= a.E) return;
+  typedef Dual3<T> S;
+  S RD[9];
+  const S vx = {a.vec[3 * e], {T(1), T(0), T(0)}}, vy = {a.vec[3 * e + 1], {T(0), T(1), T(0)}}, vz = {a.vec[3 * e + 2], {T(0), T(0), T(1)}};
+  edge_frame<T, S>(vx, vy, vz, RD);
+  T R[9], gR[9], D2[25], gD2[25], gD3[49];
 #pragma unroll
-  for (int j = 0; j < D; ++j) { gs[j] = T(0); gt[j] = T(0); }
+  for (int k = 0; k < 9; ++k) { R[k] = RD[k].v; gR[k] = T(0); }
 #pragma unroll
-  for (int k = 0; k < NC; ++k) { dws[k] = T(0); dwt[k] = T(0); ws[k] = W[k * 2 * C + c]; wt[k] = W[k * 2 * C + C + c]; }
-  // read-only inputs through restrict pointers: the stores of the totals below must not hold back the next rows' loads
-  const T* __restrict__ gMw = a.gMw;
-  const T* __restrict__ Ksp = a.Ks;
-  const T* __restrict__ Qtp = a.Qt;
-  for_rows<L, MM>([&](int r, int l, int comp) {
-    const long long at = (e * NR + r);
-    const T gms = gMw[at * 2 * C + c], gmt = gMw[at * 2 * C + C + c];
-    dws[comp] += gms * Ksp[at * C + c];
-    dwt[comp] += gmt * Qtp[at * C + c];
-    const T gks = a.gKs[at * C + c] + ws[comp] * gms;
-    const T gqt = a.gQt[at * C + c] + wt[comp] * gmt;
-    a.gKs[at * C + c] = gks;
-    a.gQt[at * C + c] = gqt;
+  for (int k = 0; k < 25; ++k) gD2[k] = T(0);
 #pragma unroll
-    for (int j = 0; j < 2 * l + 1; ++j) {
-      const T wv = Wg[r * D + l * l + j];
-      gs[l * l + j] += wv * gks;
-      gt[l * l + j] += wv * gqt;
-    }
-  });
+  for (int k = 0; k < 49; ++k) gD3[k] = T(0);
+  const T* g = st + threadIdx.x * (RW::NEP + 1);
 #pragma unroll
-  for (int k = 0; k < NC; ++k) { W[k * 2 * C + c] = dws[k]; W[k * 2 * C + C + c] = dwt[k]; }
+  for (int m = 0; m <= MM; ++m)
 #pragma unroll
-  for (int j = 0; j < D; ++j) { a.dxe[(e * D + j) * C + c] = gs[j]; a.dxt[(e * D + j) * C + c] = gt[j]; }
+    for (int l = m; l <= L; ++l)
+#pragma unroll
+      for (int part = 0; part < (m ? 2 : 1); ++part) {
+        const int k = packed_offset(L, MM, m, part, l), row = l + (part ? -m : m);
+#pragma unroll
+        for (int j = 0; j < 2 * l + 1; ++j) {
+          if (l == 1) gR[(row * 3 + j) % 9] = g[k + j];
+          if (l == 2) gD2[(row * 5 + j) % 25] = g[k + j];
+          if (l == 3) gD3[(row * 7 + j) % 49] = g[k + j];
+        }
+      }
+  if (L >= 3) {
+    wigner_up<1, T>(R, R, D2);
+    wigner_up_bwd<2, T>(R, D2, gD3, gR, gD2);
+  }
+  if (L >= 2) {
+    T gRp[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) gRp[k] = T(0);
+    wigner_up_bwd<1, T>(R, R, gD2, gR, gRp);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) gR[k] += gRp[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    T v = a.accumulate_gvec ? a.gvec[3 * e + k] : T(0);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) v += gR[q] * RD[q].d[k];
+    a.gvec[3 * e + k] = v;
+  }
 }
+
+// ---- rotations in and out of the edge frames ---------------------------------------------------------------------
+// All four kernels take one block of four warps per (target atom, 32 channels); lane = channel, and the warps share the
+// edges into the atom.  What belongs to the target - its features, the gradient of its message, the sums over its edges -
+// stays in registers over all of its edges, and the four partial sums meet in shared memory.  Each warp keeps the packed Wigner rows
+// of its edge in shared memory, read as broadcasts, while the next edge's are on their way in one coalesced load.
+// What bounds them is the memory traffic of the [E][rows][C] buffers.
+constexpr int kRotWarps = 4;
+
+template <typename T, int NEP>
+struct WigRows {
+  static constexpr int Q = NEP * (int)sizeof(T) / 16, PER = (Q + 31) / 32;
+  uint4 q[PER];
+  TACE_D TACE_INLINE void fetch(const T* __restrict__ Wg, long long e, int lane) {
+    const uint4* p = reinterpret_cast<const uint4*>(Wg + e * NEP);
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (i * 32 + lane < Q) q[i] = p[i * 32 + lane];
+  }
+  TACE_D TACE_INLINE void store(T* buf, int lane) const {
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (i * 32 + lane < Q) reinterpret_cast<uint4*>(buf)[i * 32 + lane] = q[i];
+  }
+};
+// where a block of the kernels below works (channel counts are multiples of 32)
+struct RotSlot {
+  int i, col, c, warp, lane;  // target, group of 32 channels, this lane's channel, warp = share of the edges
+  TACE_D TACE_INLINE RotSlot(int C) {
+    const int n_col = C / 32;
+    i = blockIdx.x / n_col; col = blockIdx.x - i * n_col;
+    warp = threadIdx.x >> 5; lane = threadIdx.x & 31;
+    c = col * 32 + lane;
+  }
+};
+// the D sums of the four warps added up and written (or added) to out[j * C]
+template <typename T, int D>
+TACE_D TACE_INLINE void reduce_warps(const T (&acc)[D], T (*red)[D][32], const RotSlot& s, T* out, int C) {
+  if (s.warp > 0)
+#pragma unroll
+    for (int j = 0; j < D; ++j) red[s.warp - 1][j][s.lane] = acc[j];
+  __syncthreads();
+  if (s.warp == 0)
+#pragma unroll
+    for (int j = 0; j < D; ++j) out[(long long)j * C] = ((acc[j] + red[0][j][s.lane]) + red[1][j][s.lane]) + red[2][j][s.lane];
+}
+
+// Rows of an edge on their way into shared memory: ROWS rows of 32 channels, C apart, 16 bytes per lane (with one element per
+// lane the copies fill the queue they share with the stores of the previous edge: 4.5 instead of 3.4 ms for tece_rotate_in_kernel,
+// 8.7 instead of 5.8 ms for its backward, at the size below)
+TACE_D TACE_INLINE void copy_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+template <int ROWS, typename T>
+TACE_D TACE_INLINE void copy_rows(T* dst, const T* src, int C, int lane) {
+  constexpr int V = 16 / (int)sizeof(T), LR = 32 / V, RI = 32 / LR;  // elements per lane, lanes per row, rows per instruction
+  const int r0 = lane / LR, v = lane % LR * V;
+#pragma unroll
+  for (int r = 0; r < ROWS; r += RI)
+    if (r + RI <= ROWS || r + r0 < ROWS) copy_async16(dst + (r + r0) * 32 + v, src + (long long)(r + r0) * C + v);
+}
+TACE_D TACE_INLINE void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+TACE_D TACE_INLINE void copy_wait_all_but_last() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+// K1: both ends into the frame, radial weighting.  The source's features and the radial weights of the next edge travel while
+// this edge's rows are formed: loads placed between the 56 stores of an edge would each wait out their latency.  526 k edges, 128 channels: 3.4 ms
+// (5.9 TB/s), against 4.5 ms with a thread per (edge, channel).
+template <typename T, int L, int MM> struct RotIn { static constexpr int kRows = 2 * Rows<L, MM>::NC + Rows<L, MM>::D; };
 template <typename T, int L, int MM>
-__global__ void __launch_bounds__(128) tece_rotate_out_t_kernel(const TeceArgs<T> a) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= (long long)a.n_local * a.C) return;
-  const long long i = idx / a.C;
-  constexpr int D = (L + 1) * (L + 1), NR = RowCount<L, MM>::NR;
-  const int c = (int)(idx - i * a.C), C = a.C, h = c / (C / a.H);
+__global__ void __launch_bounds__(kRotWarps * 32) tece_rotate_in_kernel(const TeceArgs<T> a) {
+  typedef Rows<L, MM> RW;
+  constexpr int D = RW::D, NR = RW::NR, NC = RW::NC, kRows = RotIn<T, L, MM>::kRows;
+  extern __shared__ __align__(16) unsigned char rot_smem[];
+  const RotSlot s(a.C);
+  const int C = a.C, c = s.c, e1 = a.rowptr[s.i + 1];
+  int e = a.rowptr[s.i] + s.warp;
+  if (e >= e1) return;
+  T* wbuf = reinterpret_cast<T*>(rot_smem) + s.warp * 2 * RW::NEP;
+  T* stage = reinterpret_cast<T*>(rot_smem) + kRotWarps * 2 * RW::NEP + s.warp * 2 * kRows * 32;
+  auto load = [&](int e, int src, T* st) {
+    copy_rows<2 * NC>(st, a.W + (long long)e * NC * 2 * C + s.col * 32, C, s.lane);
+    copy_rows<D>(st + 2 * NC * 32, a.x + (long long)src * D * C + s.col * 32, C, s.lane);
+  };
+  T vt[D], vs[D];
+#pragma unroll
+  for (int j = 0; j < D; ++j) vt[j] = a.x[((long long)s.i * D + j) * C + c];
+  WigRows<T, RW::NEP> wq;
+  load(e, a.e_src[e], stage);
+  copy_commit();
+  wq.fetch(a.Wg, e, s.lane);
+  int src = e + kRotWarps < e1 ? a.e_src[e + kRotWarps] : 0;
+  for (int b = 0; e < e1; e += kRotWarps, b ^= 1) {
+    T* w = wbuf + b * RW::NEP;
+    const T* st = stage + b * kRows * 32 + s.lane;
+    wq.store(w, s.lane);
+    __syncwarp();  // the other stage has been read by every lane
+    if (e + kRotWarps < e1) {
+      load(e + kRotWarps, src, stage + (b ^ 1) * kRows * 32);
+      wq.fetch(a.Wg, e + kRotWarps, s.lane);
+      if (e + 2 * kRotWarps < e1) src = a.e_src[e + 2 * kRotWarps];
+    }
+    copy_commit();
+    copy_wait_all_but_last();
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < D; ++j) vs[j] = st[(2 * NC + j) * 32];
+    for_rows<L, MM>([&](int r, int l, int comp, int k) {
+      T ks = T(0), qt = T(0);
+#pragma unroll
+      for (int j = 0; j < 2 * l + 1; ++j) {
+        ks += w[k + j] * vs[l * l + j];
+        qt += w[k + j] * vt[l * l + j];
+      }
+      const T ws = st[comp * 2 * 32], wt = st[(comp * 2 + 1) * 32];
+      const long long at = (long long)e * NR + r;
+      a.Ks[at * C + c] = ks;
+      a.Qt[at * C + c] = qt;
+      a.Mw[at * 2 * C + c] = ws * ks;
+      a.Mw[at * 2 * C + C + c] = wt * qt;
+    });
+  }
+}
+
+// Backward of K1.  gKs / gQt hold the gradients that came through the key / query projections, gMw the one through the weighted
+// features.  Writes dW (over W), the per-edge source rows dxe, the target's own gradient (to gx, before the source rows are
+// added) and the gradient of the packed Wigner rows, one share per group of 32 channels:
+//   gWg[row][j] = sum_c ( gKs_total x[source][j] + gQt_total x[target][j] + alpha scale gM[target][j] down[row] ).
+// Ks and Qt are rotated again from x rather than read, and neither the totals nor per-edge target rows go to memory: 122
+// rows of C per edge are left of the 238 that separate kernels for the rotation, the target sum and the Wigner gradient moved.
+// All rows of the next edge (104 for L = 3, mmax = 2: 13 KB per warp) travel while this one is worked on; two blocks per SM keep 100 KB in flight.
+// 526 k edges, L = 3, mmax = 2, 128 channels: 5.8 ms (6.5 TB/s), against 11.5 + 0.8 + 4.3 ms as those three kernels.
+template <typename T, int L, int MM> struct RotInBwd { static constexpr int kRows = 5 * Rows<L, MM>::NR + 2 * Rows<L, MM>::NC + Rows<L, MM>::D; };
+template <typename T, int L, int MM>
+__global__ void __launch_bounds__(kRotWarps * 32, sizeof(T) == 4 ? 2 : 1) tece_rotate_in_bwd_kernel(const TeceArgs<T> a) {
+  typedef Rows<L, MM> RW;
+  constexpr int D = RW::D, NR = RW::NR, NC = RW::NC, NE = RW::NE, NEP = RW::NEP, kRows = RotInBwd<T, L, MM>::kRows;
+  constexpr int kKs = 2 * NR, kQt = 3 * NR, kDn = 4 * NR, kW = 5 * NR, kX = 5 * NR + 2 * NC;  // first rows of a stage's parts (gMw first)
+  extern __shared__ __align__(16) unsigned char rot_smem[];
+  T* const smem = reinterpret_cast<T*>(rot_smem);
+  const RotSlot s(a.C);
+  const int C = a.C, c = s.c;
+  const bool owned = s.i < a.n_local;  // ghost atoms have no incoming edges: their gradient starts at zero
+  const int e1 = owned ? a.rowptr[s.i + 1] : 0;
+  int e = owned ? a.rowptr[s.i] + s.warp : 0;
+  T gt[D];
+#pragma unroll
+  for (int j = 0; j < D; ++j) gt[j] = T(0);
+  if (e < e1) {
+    const int h = c / (C / a.H);
+    T* wbuf = smem + s.warp * 2 * NEP;
+    T* stage = smem + kRotWarps * 2 * NEP + s.warp * 2 * kRows * 32;
+      auto load = [&](int e, int src, T* st) {
+      const long long at = (long long)e * NR * C + s.col * 32;
+      copy_rows<2 * NR>(st, a.gMw + (long long)e * NR * 2 * C + s.col * 32, C, s.lane);
+      copy_rows<NR>(st + kKs * 32, a.gKs + at, C, s.lane);
+      copy_rows<NR>(st + kQt * 32, a.gQt + at, C, s.lane);
+      copy_rows<NR>(st + kDn * 32, a.down + at, C, s.lane);
+      copy_rows<2 * NC>(st + kW * 32, a.W + (long long)e * NC * 2 * C + s.col * 32, C, s.lane);
+      copy_rows<D>(st + kX * 32, a.x + (long long)src * D * C + s.col * 32, C, s.lane);
+    };
+    T vt[D], vg[D], vs[D], gs[D];
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      vt[j] = a.x[((long long)s.i * D + j) * C + c];
+      vg[j] = a.gM[((long long)s.i * D + j) * C + c];
+    }
+    WigRows<T, NEP> wq;
+    load(e, a.e_src[e], stage);
+    copy_commit();
+    wq.fetch(a.Wg, e, s.lane);
+    int src = e + kRotWarps < e1 ? a.e_src[e + kRotWarps] : 0;
+    T al = a.alpha[(long long)e * a.H + h], al_next = al;
+    for (int b = 0; e < e1; e += kRotWarps, b ^= 1, al = al_next) {
+      T* w = wbuf + b * NEP;
+      const T* st = stage + b * kRows * 32 + s.lane;
+      wq.store(w, s.lane);
+      __syncwarp();  // the other stage has been read by every lane
+      if (e + kRotWarps < e1) {
+        load(e + kRotWarps, src, stage + (b ^ 1) * kRows * 32);
+        wq.fetch(a.Wg, e + kRotWarps, s.lane);
+        al_next = a.alpha[(long long)(e + kRotWarps) * a.H + h];
+        if (e + 2 * kRotWarps < e1) src = a.e_src[e + 2 * kRotWarps];
+      }
+      copy_commit();
+      copy_wait_all_but_last();
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < D; ++j) { vs[j] = st[(kX + j) * 32]; gs[j] = T(0); }
+      T* W = a.W + (long long)e * NC * 2 * C + c;
+      T* gw = a.gWg + ((long long)s.col * a.E + e) * NEP;
+      T buf[16];
+      T ws = T(0), wt = T(0), dws = T(0), dwt = T(0);
+      int comp_now = -1;
+      for_rows<L, MM>([&](int r, int l, int comp, int k) {
+        if (comp != comp_now) {
+          if (comp_now >= 0) { W[comp_now * 2 * C] = dws; W[comp_now * 2 * C + C] = dwt; }
+          comp_now = comp;
+          ws = st[(kW + comp * 2) * 32]; wt = st[(kW + comp * 2 + 1) * 32]; dws = T(0); dwt = T(0);
+        }
+        const T gms = st[2 * r * 32], gmt = st[(2 * r + 1) * 32];
+        const T gks = st[(kKs + r) * 32] + ws * gms, gqt = st[(kQt + r) * 32] + wt * gmt;
+        const T dn = al * a.row_scale[r] * st[(kDn + r) * 32];
+        T ks = T(0), qt = T(0);
+#pragma unroll
+        for (int j = 0; j < 2 * l + 1; ++j) {
+          const int q = l * l + j;
+          const T wv = w[k + j];
+          ks += wv * vs[q];
+          qt += wv * vt[q];
+          gs[q] += wv * gks;
+          gt[q] += wv * gqt;
+          // sum over the lanes of 16 entries at a time: every exchange halves the entries a lane still carries
+          buf[(k + j) & 15] = gks * vs[q] + gqt * vt[q] + dn * vg[q];
+          if (((k + j) & 15) == 15 || k + j == NE - 1) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (i > ((k + j) & 15)) buf[i] = T(0);
+#pragma unroll
+            for (int o = 16, n = 8; o >= 2; o >>= 1, n >>= 1)
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                if (i < n) {
+                  const bool up = s.lane & o;
+                  const T send = up ? buf[i] : buf[i + n];
+                  buf[i] = (up ? buf[i + n] : buf[i]) + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            buf[0] += __shfl_xor_sync(0xffffffffu, buf[0], 1);
+            const int at0 = ((k + j) & ~15) + (s.lane >> 1);
+            if (!(s.lane & 1) && at0 < NEP) gw[at0] = buf[0];
+          }
+        }
+        dws += gms * ks;
+        dwt += gmt * qt;
+      });
+      W[comp_now * 2 * C] = dws;
+      W[comp_now * 2 * C + C] = dwt;
+#pragma unroll
+      for (int j = 0; j < D; ++j) a.dxe[((long long)e * D + j) * C + c] = gs[j];
+    }
+  }
+  __syncthreads();  // every warp is done with its stages (no copy is in flight): the partial sums take their place
+  reduce_warps<T, D>(gt, reinterpret_cast<T(*)[D][32]>(smem), s, a.gx + (long long)s.i * D * C + c, C);
+}
+
+// K6: attention-weighted inverse rotation and sum per target atom.  526 k edges, 128 channels: 0.66 ms (5.7 TB/s), against 2.0 ms
+// with one thread walking all edges of its (target, channel); 8 k edges: 16 against 316 us.
+template <typename T, int L, int MM>
+__global__ void __launch_bounds__(kRotWarps * 32) tece_rotate_out_kernel(const TeceArgs<T> a) {
+  typedef Rows<L, MM> RW;
+  constexpr int D = RW::D, NR = RW::NR;
+  __shared__ __align__(16) T wbuf[kRotWarps][2][RW::NEP];
+  __shared__ T red[kRotWarps - 1][D][32];
+  const RotSlot s(a.C);
+  const int C = a.C, c = s.c, h = c / (C / a.H), e1 = a.rowptr[s.i + 1];
+  int e = a.rowptr[s.i] + s.warp;
+  const T* __restrict__ down = a.down;
   T acc[D];
 #pragma unroll
   for (int j = 0; j < D; ++j) acc[j] = T(0);
-  for (int e = a.rowptr[i]; e < a.rowptr[i + 1]; ++e) {
+  WigRows<T, RW::NEP> wq;
+  if (e < e1) wq.fetch(a.Wg, e, s.lane);
+  for (int b = 0; e < e1; e += kRotWarps, b ^= 1) {
+    T* w = wbuf[s.warp][b];
+    wq.store(w, s.lane);
     const T al = a.alpha[(long long)e * a.H + h];
-    const T* Wg = a.Wg + (long long)e * NR * D;
-    const T* dn = a.down + (long long)e * NR * C + c;
-    for_rows<L, MM>([&](int r, int l, int) {
-      const T v = al * a.row_scale[r] * dn[(long long)r * C];
+    const T* dn = down + (long long)e * NR * C + c;
+    T v[NR];
 #pragma unroll
-      for (int j = 0; j < 2 * l + 1; ++j) acc[l * l + j] += Wg[r * D + l * l + j] * v;
+    for (int r = 0; r < NR; ++r) v[r] = dn[(long long)r * C];
+    __syncwarp();
+    if (e + kRotWarps < e1) wq.fetch(a.Wg, e + kRotWarps, s.lane);
+    for_rows<L, MM>([&](int r, int l, int, int k) {
+      const T t = al * a.row_scale[r] * v[r];
+#pragma unroll
+      for (int j = 0; j < 2 * l + 1; ++j) acc[l * l + j] += w[k + j] * t;
     });
   }
-#pragma unroll
-  for (int j = 0; j < D; ++j) a.M[(i * D + j) * C + c] = acc[j];
+  reduce_warps<T, D>(acc, red, s, a.M + (long long)s.i * D * C + c, C);
 }
-// Wigner-row gradient, one warp per edge (see tece_wigner_grad_kernel below), with static shapes
-template <typename T, int L, int MM>
-__global__ void __launch_bounds__(128) tece_wigner_grad_t_kernel(const TeceArgs<T> a) {
-  const int lane = threadIdx.x & 31;
-  const long long e = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (e >= a.E) return;
-  constexpr int D = (L + 1) * (L + 1), NR = RowCount<L, MM>::NR;
-  constexpr int NE = D + (MM >= 1 ? 2 * (D - 1) : 0) + (MM >= 2 ? 2 * (D - 4) : 0);  // block entries of all rows
-  const int C = a.C, Ch = C / a.H;
-  T acc[NE];
+// gdown[e][r][c] = alpha scale_r sum_j Wg[r][j] gM[target][j][c] and galpha[e][h] = sum over the head's channels and the rows
+// of down scale_r t.  Heads whose channels are a power of two of neighbouring lanes finish galpha with shuffles (FUSE); other
+// heads leave it to tece_alpha_bwd_kernel, which gets the sums per channel in row 0 of the edge's gQp (written only later).  526 k edges, 128 channels:
+// 1.2 ms (6.2 TB/s), against 5.2 ms with the target's rows read again for every edge.
+template <typename T, int L, int MM, bool FUSE>
+__global__ void __launch_bounds__(kRotWarps * 32) tece_rotate_out_bwd_kernel(const TeceArgs<T> a) {
+  typedef Rows<L, MM> RW;
+  constexpr int D = RW::D, NR = RW::NR;
+  __shared__ __align__(16) T wbuf[kRotWarps][2][RW::NEP];
+  const RotSlot s(a.C);
+  const int C = a.C, c = s.c, Ch = C / a.H, h = c / Ch, e1 = a.rowptr[s.i + 1];
+  int e = a.rowptr[s.i] + s.warp;
+  if (e >= e1) return;
+  const T* __restrict__ down = a.down;
+  T vg[D];
 #pragma unroll
-  for (int k = 0; k < NE; ++k) acc[k] = T(0);
-  const T* xs = a.x + (long long)a.e_src[e] * D * C;
-  const T* xt = a.x + (long long)a.e_dst[e] * D * C;
-  const T* gM = a.gM + (long long)a.e_dst[e] * D * C;
-  for (int c = lane; c < C; c += 32) {
-    const T al = a.alpha[e * a.H + c / Ch];
-    T vs[D], vt[D], vg[D];
+  for (int j = 0; j < D; ++j) vg[j] = a.gM[((long long)s.i * D + j) * C + c];
+  WigRows<T, RW::NEP> wq;
+  wq.fetch(a.Wg, e, s.lane);
+  for (int b = 0; e < e1; e += kRotWarps, b ^= 1) {
+    T* w = wbuf[s.warp][b];
+    wq.store(w, s.lane);
+    const T al = a.alpha[(long long)e * a.H + h];
+    const T* dn = down + (long long)e * NR * C + c;
+    T v[NR];
 #pragma unroll
-    for (int j = 0; j < D; ++j) { vs[j] = xs[(long long)j * C + c]; vt[j] = xt[(long long)j * C + c]; vg[j] = al * gM[(long long)j * C + c]; }
-    int k = 0;
-    for_rows<L, MM>([&](int r, int l, int) {
-      const long long at = (e * NR + r) * C + c;
-      const T gk = a.gKs[at], gq = a.gQt[at], dn = a.row_scale[r] * a.down[at];
+    for (int r = 0; r < NR; ++r) v[r] = dn[(long long)r * C];
+    __syncwarp();
+    if (e + kRotWarps < e1) wq.fetch(a.Wg, e + kRotWarps, s.lane);
+    T part = T(0);
+    for_rows<L, MM>([&](int r, int l, int, int k) {
+      T t = T(0);
 #pragma unroll
-      for (int j = 0; j < 2 * l + 1; ++j, ++k) acc[k] += gk * vs[l * l + j] + gq * vt[l * l + j] + dn * vg[l * l + j];
+      for (int j = 0; j < 2 * l + 1; ++j) t += w[k + j] * vg[l * l + j];
+      t *= a.row_scale[r];
+      a.gdown[((long long)e * NR + r) * C + c] = al * t;
+      part += v[r] * t;
     });
-  }
-  T* out = a.gWg + e * NR * D;
-  int k = 0;
-  for_rows<L, MM>([&](int r, int l, int) {
-#pragma unroll
-    for (int j = 0; j < 2 * l + 1; ++j, ++k) {
-      T v = acc[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) out[r * D + l * l + j] = v;
+    if (FUSE) {
+      for (int o = Ch >> 1; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      if (s.lane % Ch == 0) a.galpha[(long long)e * a.H + h] = part;
+    } else {
+      a.gQp[(long long)e * NR * C + c] = part;
     }
-  });
+  }
 }
-#define TECE_LM_DISPATCH(KERNEL, GRID, BLOCK)                                              \
-  (a.L == 2 && a.mmax == 1   ? (KERNEL<T, 2, 1><<<GRID, BLOCK, 0, s>>>(a), true)          \
-   : a.L == 2 && a.mmax == 2 ? (KERNEL<T, 2, 2><<<GRID, BLOCK, 0, s>>>(a), true)          \
-   : a.L == 3 && a.mmax == 1 ? (KERNEL<T, 3, 1><<<GRID, BLOCK, 0, s>>>(a), true)          \
-   : a.L == 3 && a.mmax == 2 ? (KERNEL<T, 3, 2><<<GRID, BLOCK, 0, s>>>(a), true)          \
-                             : false)
+// galpha[e][h] from the per-channel sums that tece_rotate_out_bwd_kernel left in row 0 of the edge's gQp
+template <typename T>
+__global__ void tece_alpha_bwd_kernel(const TeceArgs<T> a) {
+  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (idx >= a.E * a.H) return;
+  const long long e = idx / a.H;
+  const int h = (int)(idx - e * a.H), Ch = a.C / a.H;
+  const T* p = a.gQp + e * a.NR * a.C + h * Ch;
+  T acc = T(0);
+  for (int u = 0; u < Ch; ++u) acc += p[u];
+  a.galpha[idx] = acc;
+}
 
 // ---- K3: attention logits ---------------------------------------------------------------------------
 template <typename T>
@@ -613,413 +861,206 @@ __global__ void tece_softmax_bwd_kernel(const TeceArgs<T> a) {
 }
 
 // ---- K5: gate + edge cluster expansion on the SO(2) features ------------------------------------------
-// rows of the full layout: order 0 rows [0, n); order m >= 1 real rows [n + (m-1) 2n, +n), imaginary rows the next n
-template <typename T>
-TACE_D TACE_INLINE int full_re(int n, int m) { return m == 0 ? 0 : n + (m - 1) * 2 * n; }
-
-template <typename T, bool BWD>
-__global__ void tece_mix_kernel(const TeceArgs<T> a) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= a.E * a.Ca) return;
-  const long long e = idx / a.Ca;
-  const int ca = (int)(idx - e * a.Ca), Ca = a.Ca, n = a.L + 1, NF = n + 2 * n * a.mmax, G = a.G;
-  constexpr int MAXF = 20, MAXG = 12, MAXW = 28;  // L <= 3, mmax <= 2
-  T x[MAXF], y[MAXF], gz[MAXG], cz[MAXW], out[MAXF];
-  const T* up = a.up + e * (long long)(G + NF) * Ca + ca;
-  const T* glu = a.glu + e * (long long)NF * Ca + ca;
-  const T* cf = a.coefZ + e * (long long)a.n_paths * n * Ca + ca;
-  for (int r = 0; r < G; ++r) gz[r] = up[(long long)r * Ca];
-  for (int r = 0; r < NF; ++r) { x[r] = up[(long long)(G + r) * Ca]; y[r] = glu[(long long)r * Ca]; out[r] = x[r]; }
-  for (int k = 0; k < a.n_paths * n; ++k) cz[k] = cf[(long long)k * Ca];
-  T gx[MAXF], gy[MAXF], gg[MAXG], gc[MAXW], go[MAXF];
-  if (BWD) {
-    const T* gU = a.gU + e * (long long)NF * Ca + ca;
-    for (int r = 0; r < NF; ++r) { go[r] = gU[(long long)r * Ca]; gx[r] = go[r]; gy[r] = T(0); }
-    for (int r = 0; r < G; ++r) gg[r] = T(0);
-    for (int k = 0; k < a.n_paths * n; ++k) gc[k] = T(0);
-  }
-  // gate (oam_2026_07_05.py:301-309, channel-wise layout): order m row i is scaled by act(gate[(m - start) n + i])
-  const int start = a.gate_m0 ? 0 : 1;
-  for (int m = 0; m <= a.mmax; ++m) {
-    for (int part = 0; part < (m == 0 ? 1 : 2); ++part)
-      for (int i = 0; i < n; ++i) {
-        const int r = full_re<T>(n, m) + part * n + i;
-        if (m == 0 && !a.gate_m0) {
-          out[r] += act_eval<T>(a.act, x[r]);
-          if (BWD) gx[r] += go[r] * act_grad<T>(a.act, x[r]);
-        } else {
-          const int g = (m - start) * n + i;
-          out[r] += act_eval<T>(a.act, gz[g]) * x[r];
-          if (BWD) { gx[r] += go[r] * act_eval<T>(a.act, gz[g]); gg[g] += go[r] * x[r] * act_grad<T>(a.act, gz[g]); }
-        }
-      }
-  }
-  // cluster expansion (oam_2026_07_05.py:417-488): channel-wise products of the complex order components
-  for (int p = 0; p < a.n_paths; ++p) {
-    const int m1 = a.p_m1[p], m2 = a.p_m2[p], m3 = a.p_m3[p], sum_mode = a.p_sum[p];
-    const T sc = a.p_scale[p];
-    const int x_re = full_re<T>(n, m1), y_re = full_re<T>(n, m2), o_re = full_re<T>(n, m3);
-    for (int i = 0; i < n; ++i) {
-      const T w = act_eval<T>(a.act, cz[p * n + i]) * sc;
-      const T xr = x[x_re + i], xi = m1 ? x[x_re + n + i] : T(0);
-      const T yr = y[y_re + i], yi = m2 ? y[y_re + n + i] : T(0);
-      T zr, zi;
-      if (sum_mode) { zr = xr * yr - xi * yi; zi = xr * yi + xi * yr; }
-      else { zr = xr * yr + xi * yi; zi = xi * yr - xr * yi; }
-      out[o_re + i] += w * zr;
-      if (m3) out[o_re + n + i] += w * zi;
-      if (BWD) {
-        const T gr = go[o_re + i], gi = m3 ? go[o_re + n + i] : T(0);
-        gc[p * n + i] += (gr * zr + gi * zi) * sc * act_grad<T>(a.act, cz[p * n + i]);
-        const T ar = w * gr, ai = w * gi;  // gradient of (zr, zi)
-        if (sum_mode) {
-          gx[x_re + i] += ar * yr + ai * yi;
-          if (m1) gx[x_re + n + i] += -ar * yi + ai * yr;
-          gy[y_re + i] += ar * xr + ai * xi;
-          if (m2) gy[y_re + n + i] += -ar * xi + ai * xr;
-        } else {
-          gx[x_re + i] += ar * yr - ai * yi;
-          if (m1) gx[x_re + n + i] += ar * yi + ai * yr;
-          gy[y_re + i] += ar * xr + ai * xi;
-          if (m2) gy[y_re + n + i] += ar * xi - ai * xr;
-        }
-      }
-    }
-  }
-  if (!BWD) {
-    T* U = a.U + e * (long long)NF * Ca + ca;
-    for (int r = 0; r < NF; ++r) U[(long long)r * Ca] = out[r];
-  } else {
-    T* gup = a.gup + e * (long long)(G + NF) * Ca + ca;
-    T* gglu = a.gglu + e * (long long)NF * Ca + ca;
-    T* gcf = a.gcoefZ + e * (long long)a.n_paths * n * Ca + ca;
-    for (int r = 0; r < G; ++r) gup[(long long)r * Ca] = gg[r];
-    for (int r = 0; r < NF; ++r) { gup[(long long)(G + r) * Ca] = gx[r]; gglu[(long long)r * Ca] = gy[r]; }
-    for (int k = 0; k < a.n_paths * n; ++k) gcf[(long long)k * Ca] = gc[k];
-  }
-}
-
-// The same kernel with rows per order, orders and gate layout known at compile time: every array index below is a constant
-// after unrolling, so the ~150 per-thread values live in registers instead of local memory.
-TACE_HD constexpr int mix_path_id(int mm, int m3, int m1, int m2) {  // position of path (m1, m2) -> m3 in the output-order-major list
+// Rows of the full layout: order 0 rows [0, N); order m >= 1 real rows [N + (m-1) 2N, +N), imaginary rows the next N.  Row i of
+// every order, its gate and its coefficients meet only one another (gate: oam_2026_07_05.py:301-309, channel-wise layout, order
+// m row i scaled by act(gate[(m - start) N + i]); cluster expansion: :417-488, channel-wise products of the complex order
+// components), so one thread takes (edge, i, channel): some 25 values in registers where a thread per (edge, channel) held
+// 150 and left the machine a third full.  526 k edges, 32 channels: 1.0 + 1.9 ms, against 1.3 + 4.2 ms.
+TACE_HD constexpr bool mix_path(int m3, int m1, int m2) { return m1 + m2 == m3 || m1 - m2 == m3; }
+TACE_HD constexpr int mix_path_id(int mm, int m3, int m1, int m2) {  // position in the output-order-major list; past the end: their number
   int p = 0;
   for (int q3 = 0; q3 <= mm; ++q3)
     for (int q1 = 0; q1 <= mm; ++q1)
       for (int q2 = 0; q2 <= q1; ++q2) {
-        if (!(q1 + q2 == q3 || q1 - q2 == q3)) continue;
+        if (!mix_path(q3, q1, q2)) continue;
         if (q3 == m3 && q1 == m1 && q2 == m2) return p;
         ++p;
       }
-  return -1;
-}
-TACE_HD constexpr int mix_path_count(int mm) {
-  int p = 0;
-  for (int q3 = 0; q3 <= mm; ++q3)
-    for (int q1 = 0; q1 <= mm; ++q1)
-      for (int q2 = 0; q2 <= q1; ++q2)
-        if (q1 + q2 == q3 || q1 - q2 == q3) ++p;
   return p;
 }
 template <typename T, int N, int MM, bool GATE_M0, bool BWD>
-__global__ void __launch_bounds__(64) tece_mix_t_kernel(const TeceArgs<T> a) {
+__global__ void __launch_bounds__(128) tece_mix_kernel(const TeceArgs<T> a) {
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= a.E * a.Ca) return;
-  const long long e = idx / a.Ca;
-  const int ca = (int)(idx - e * a.Ca), Ca = a.Ca;
-  constexpr int NF = N + 2 * N * MM, G = N * (MM + (GATE_M0 ? 1 : 0));
-  constexpr int START = GATE_M0 ? 0 : 1;
-  T x[NF], y[NF], gz[G > 0 ? G : 1], out[NF];
-  const T* up = a.up + e * (long long)(G + NF) * Ca + ca;
-  const T* glu = a.glu + e * (long long)NF * Ca + ca;
-  const T* cf = a.coefZ + e * (long long)a.n_paths * N * Ca + ca;
+  if (idx >= a.E * N * a.Ca) return;
+  const int Ca = a.Ca;
+  const long long ei = idx / Ca, e = ei / N;
+  const int ca = (int)(idx - ei * Ca), i = (int)(ei - e * N);
+  constexpr int NF = N + 2 * N * MM, G = N * (MM + (GATE_M0 ? 1 : 0)), M = 2 * MM + 1;
+  constexpr int START = GATE_M0 ? 0 : 1, NG = MM + 1 - START, NPATH = mix_path_id(MM, MM + 1, 0, 0);
+  // component q of the registers: order (q + 1) / 2, real (0, 1, 3) or imaginary (2, 4) part; its row is q N + i
+  T x[M], y[M], gz[NG > 0 ? NG : 1], cz[NPATH], out[M], go[M], gx[M], gy[M];
+  const long long up = e * (G + NF) * Ca + (long long)i * Ca + ca, full = e * NF * Ca + (long long)i * Ca + ca,
+                  path = e * NPATH * N * Ca + (long long)i * Ca + ca;
+  const int row = N * Ca;
+  // every input is in registers before the first store: the gradients overwrite their forward buffers
 #pragma unroll
-  for (int r = 0; r < G; ++r) gz[r] = up[(long long)r * Ca];
+  for (int q = 0; q < NG; ++q) gz[q] = a.up[up + q * row];
 #pragma unroll
-  for (int r = 0; r < NF; ++r) { x[r] = up[(long long)(G + r) * Ca]; y[r] = glu[(long long)r * Ca]; out[r] = x[r]; }
-  // every input is in registers before the first store: the gradients overwrite their forward buffers, so a load issued
-  // after a store would have to wait for it
-  constexpr int NW = mix_path_count(MM) * N;
-  T cz[NW];
-#pragma unroll
-  for (int k = 0; k < NW; ++k) cz[k] = cf[(long long)k * Ca];
-  T gx[NF], gy[NF], gg[G > 0 ? G : 1], go[NF];
-  T* gcf = nullptr;
-  if (BWD) {
-    const T* gU = a.gU + e * (long long)NF * Ca + ca;
-#pragma unroll
-    for (int r = 0; r < NF; ++r) { go[r] = gU[(long long)r * Ca]; gx[r] = go[r]; gy[r] = T(0); }
-#pragma unroll
-    for (int r = 0; r < G; ++r) gg[r] = T(0);
-    gcf = a.gcoefZ + e * (long long)a.n_paths * N * Ca + ca;
+  for (int q = 0; q < M; ++q) {
+    x[q] = a.up[up + G * Ca + q * row];
+    y[q] = a.glu[full + q * row];
+    if (BWD) { go[q] = a.gU[full + q * row]; gx[q] = go[q]; gy[q] = T(0); }
+    else out[q] = x[q];
   }
 #pragma unroll
+  for (int p = 0; p < NPATH; ++p) cz[p] = a.coefZ[path + p * row];
+#pragma unroll
   for (int m = 0; m <= MM; ++m) {
+    if (m < START) {
+      if (BWD) gx[0] += go[0] * act_grad<T>(a.act, x[0]);
+      else out[0] += act_eval<T>(a.act, x[0]);
+    } else {
+      const T ag = act_eval<T>(a.act, gz[m - START]);
+      T gg = T(0);
 #pragma unroll
-    for (int part = 0; part < (m == 0 ? 1 : 2); ++part)
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const int r = (m == 0 ? 0 : N + (m - 1) * 2 * N) + part * N + i;
-        if (m == 0 && !GATE_M0) {
-          out[r] += act_eval<T>(a.act, x[r]);
-          if (BWD) gx[r] += go[r] * act_grad<T>(a.act, x[r]);
-        } else {
-          const int g = (m - START) * N + i;
-          const T ag = act_eval<T>(a.act, gz[g]);
-          out[r] += ag * x[r];
-          if (BWD) { gx[r] += go[r] * ag; gg[g] += go[r] * x[r] * act_grad<T>(a.act, gz[g]); }
-        }
+      for (int q = (m ? 2 * m - 1 : 0); q <= 2 * m; ++q) {
+        if (BWD) { gx[q] += go[q] * ag; gg += go[q] * x[q]; }
+        else out[q] += ag * x[q];
       }
+      if (BWD) a.gup[up + (m - START) * row] = gg * act_grad<T>(a.act, gz[m - START]);
+    }
   }
 #pragma unroll
   for (int m3 = 0; m3 <= MM; ++m3)
 #pragma unroll
     for (int m1 = 0; m1 <= MM; ++m1)
 #pragma unroll
-      for (int m2 = 0; m2 <= m1; ++m2) {
-        const bool sum_mode = (m1 + m2 == m3);
-        if (!(sum_mode || m1 - m2 == m3)) continue;
-        const int p = mix_path_id(MM, m3, m1, m2);
-        const T sc = a.p_scale[p];
-        const int x_re = (m1 == 0 ? 0 : N + (m1 - 1) * 2 * N), y_re = (m2 == 0 ? 0 : N + (m2 - 1) * 2 * N),
-                  o_re = (m3 == 0 ? 0 : N + (m3 - 1) * 2 * N);
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-          const T czv = cz[p * N + i];
-          const T w = act_eval<T>(a.act, czv) * sc;
-          const T xr = x[x_re + i], xi = m1 ? x[x_re + (m1 ? N : 0) + i] : T(0);
-          const T yr = y[y_re + i], yi = m2 ? y[y_re + (m2 ? N : 0) + i] : T(0);
-          T zr, zi;
-          if (sum_mode) { zr = xr * yr - xi * yi; zi = xr * yi + xi * yr; }
-          else { zr = xr * yr + xi * yi; zi = xi * yr - xr * yi; }
-          out[o_re + i] += w * zr;
-          if (m3) out[o_re + (m3 ? N : 0) + i] += w * zi;
-          if (BWD) {
-            const T gr = go[o_re + i], gi = m3 ? go[o_re + (m3 ? N : 0) + i] : T(0);
-            gcf[(long long)(p * N + i) * Ca] = (gr * zr + gi * zi) * sc * act_grad<T>(a.act, czv);
+      for (int m2 = 0; m2 <= m1; ++m2)
+        if (mix_path(m3, m1, m2)) {
+          constexpr int kLast = M - 1;
+          const int p = mix_path_id(MM, m3, m1, m2);
+          const bool sum_mode = (m1 + m2 == m3);
+          const int xq = m1 ? 2 * m1 - 1 : 0, yq = m2 ? 2 * m2 - 1 : 0, oq = m3 ? 2 * m3 - 1 : 0;
+          const int xi_ = m1 ? 2 * m1 : kLast, yi_ = m2 ? 2 * m2 : kLast, oi_ = m3 ? 2 * m3 : kLast;
+          const T sc = a.p_scale[p], w = act_eval<T>(a.act, cz[p]) * sc;
+          const T xr = x[xq], xi = m1 ? x[xi_] : T(0), yr = y[yq], yi = m2 ? y[yi_] : T(0);
+          const T sg = sum_mode ? T(1) : T(-1);  // sum of the orders: product; difference: product with the conjugate of y
+          const T zr = xr * yr - sg * xi * yi, zi = sum_mode ? xr * yi + xi * yr : xi * yr - xr * yi;
+          if (!BWD) {
+            out[oq] += w * zr;
+            if (m3) out[oi_] += w * zi;
+          } else {
+            const T gr = go[oq], gi = m3 ? go[oi_] : T(0);
+            a.gcoefZ[path + p * row] = (gr * zr + gi * zi) * sc * act_grad<T>(a.act, cz[p]);
             const T ar = w * gr, ai = w * gi;
-            if (sum_mode) {
-              gx[x_re + i] += ar * yr + ai * yi;
-              if (m1) gx[x_re + (m1 ? N : 0) + i] += -ar * yi + ai * yr;
-              gy[y_re + i] += ar * xr + ai * xi;
-              if (m2) gy[y_re + (m2 ? N : 0) + i] += -ar * xi + ai * xr;
-            } else {
-              gx[x_re + i] += ar * yr - ai * yi;
-              if (m1) gx[x_re + (m1 ? N : 0) + i] += ar * yi + ai * yr;
-              gy[y_re + i] += ar * xr + ai * xi;
-              if (m2) gy[y_re + (m2 ? N : 0) + i] += ar * xi - ai * xr;
-            }
+            gx[xq] += ar * yr + sg * ai * yi;
+            if (m1) gx[xi_] += -sg * ar * yi + ai * yr;
+            gy[yq] += ar * xr + ai * xi;
+            if (m2) gy[yi_] += sum_mode ? -ar * xi + ai * xr : ar * xi - ai * xr;
           }
         }
-      }
-  if (!BWD) {
-    T* U = a.U + e * (long long)NF * Ca + ca;
 #pragma unroll
-    for (int r = 0; r < NF; ++r) U[(long long)r * Ca] = out[r];
-  } else {
-    T* gup = a.gup + e * (long long)(G + NF) * Ca + ca;
-    T* gglu = a.gglu + e * (long long)NF * Ca + ca;
-#pragma unroll
-    for (int r = 0; r < G; ++r) gup[(long long)r * Ca] = gg[r];
-#pragma unroll
-    for (int r = 0; r < NF; ++r) { gup[(long long)(G + r) * Ca] = gx[r]; gglu[(long long)r * Ca] = gy[r]; }
-  }
-}
-template <typename T, bool BWD>
-bool launch_mix_static(const TeceArgs<T>& a, cudaStream_t s) {
-  const unsigned grid = (unsigned)((a.E * a.Ca + 63) / 64);
-#define MIXCASE(N_, MM_)                                                                                        \
-  if (a.L + 1 == N_ && a.mmax == MM_) {                                                                         \
-    if (a.gate_m0) tece_mix_t_kernel<T, N_, MM_, true, BWD><<<grid, 64, 0, s>>>(a);                              \
-    else tece_mix_t_kernel<T, N_, MM_, false, BWD><<<grid, 64, 0, s>>>(a);                                       \
-    return true;                                                                                                \
-  }
-  MIXCASE(3, 1) MIXCASE(3, 2) MIXCASE(4, 1) MIXCASE(4, 2)
-#undef MIXCASE
-  return false;
-}
-
-// ---- K6: attention-weighted inverse rotation and sum per target atom --------------------------------------
-template <typename T>
-__global__ void tece_rotate_out_kernel(const TeceArgs<T> a) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= (long long)a.n_local * a.C) return;
-  const long long i = idx / a.C;
-  const int c = (int)(idx - i * a.C), C = a.C, D = (a.L + 1) * (a.L + 1), h = c / (C / a.H);
-  T acc[16];
-  for (int j = 0; j < D; ++j) acc[j] = T(0);
-  for (int e = a.rowptr[i]; e < a.rowptr[i + 1]; ++e) {
-    const T al = a.alpha[(long long)e * a.H + h];
-    const T* Wg = a.Wg + (long long)e * a.NR * D;
-    for (int r = 0; r < a.NR; ++r) {
-      const int l = a.row_l[r], dl = 2 * l + 1;
-      const T v = al * a.row_scale[r] * a.down[((long long)e * a.NR + r) * C + c];
-      for (int j = 0; j < dl; ++j) acc[l * l + j] += Wg[r * D + l * l + j] * v;
-    }
-  }
-  for (int j = 0; j < D; ++j) a.M[(i * D + j) * C + c] = acc[j];
-}
-// gdown[e][r][c] = alpha scale_r sum_j Wg[e][r][j] gM[target][j][c].  FUSE (channels per head a power of two <= 32, so one
-// head is a group of neighbouring lanes): also galpha[e][h] = sum over the head's channels and the rows of down * scale_r * t,
-// reduced with shuffles, which saves the separate pass of tece_alpha_bwd_kernel over the same data.
-template <typename T, bool FUSE>
-__global__ void tece_rotate_out_bwd_kernel(const TeceArgs<T> a) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= a.E * a.C) return;
-  const long long e = idx / a.C;
-  const int c = (int)(idx - e * a.C), C = a.C, D = (a.L + 1) * (a.L + 1), h = c / (C / a.H);
-  const T al = a.alpha[e * a.H + h];
-  const T* __restrict__ Wg = a.Wg + e * a.NR * D;
-  const T* __restrict__ gM = a.gM + (long long)a.e_dst[e] * D * C + c;
-  const T* __restrict__ down = a.down;
-  T part = T(0);
-  for (int r = 0; r < a.NR; ++r) {
-    const int l = a.row_l[r], dl = 2 * l + 1;
-    T t = T(0);
-    for (int j = 0; j < dl; ++j) t += Wg[r * D + l * l + j] * gM[(long long)(l * l + j) * C];
-    t *= a.row_scale[r];
-    a.gdown[(e * a.NR + r) * C + c] = al * t;
-    if (FUSE) part += down[(e * a.NR + r) * C + c] * t;
-  }
-  if (FUSE) {
-    const int Ch = C / a.H;
-    for (int o = Ch >> 1; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (c % Ch == 0) a.galpha[e * a.H + h] = part;
-  }
-}
-// galpha[e][h] = sum_{c in head} sum_r down[e][r][c] scale_r sum_j Wg[e][r][j] gM[target][j][c]
-template <typename T>
-__global__ void tece_alpha_bwd_kernel(const TeceArgs<T> a) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (idx >= a.E * a.H) return;
-  const long long e = idx / a.H;
-  const int h = (int)(idx - e * a.H), C = a.C, Ch = C / a.H, D = (a.L + 1) * (a.L + 1);
-  const T* Wg = a.Wg + e * a.NR * D;
-  T acc = T(0);
-  for (int u = 0; u < Ch; ++u) {
-    const int c = h * Ch + u;
-    const T* gM = a.gM + (long long)a.e_dst[e] * D * C + c;
-    for (int r = 0; r < a.NR; ++r) {
-      const int l = a.row_l[r], dl = 2 * l + 1;
-      T t = T(0);
-      for (int j = 0; j < dl; ++j) t += Wg[r * D + l * l + j] * gM[(long long)(l * l + j) * C];
-      acc += a.down[(e * a.NR + r) * C + c] * a.row_scale[r] * t;
-    }
-  }
-  a.galpha[idx] = acc;
-}
-// gWg[e][r][j] = sum_c ( gKs_total x[source][j] + gQt_total x[target][j] + alpha scale_r gM[target][j] down[e][r] )
-// One warp per edge: lane k owns the channels k, k + 32, ...; every lane accumulates all block entries of the edge (at most
-// 70 for L = 3, mmax = 2), then the warp reduces them.  All loads are contiguous in the channel index.
-template <typename T>
-__global__ void __launch_bounds__(128) tece_wigner_grad_kernel(const TeceArgs<T> a) {
-  const int lane = threadIdx.x & 31;
-  const long long e = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (e >= a.E) return;
-  const int D = (a.L + 1) * (a.L + 1), C = a.C, Ch = C / a.H;
-  constexpr int MAXE = 70;
-  T acc[MAXE];
-#pragma unroll
-  for (int k = 0; k < MAXE; ++k) acc[k] = T(0);
-  const T* xs = a.x + (long long)a.e_src[e] * D * C;
-  const T* xt = a.x + (long long)a.e_dst[e] * D * C;
-  const T* gM = a.gM + (long long)a.e_dst[e] * D * C;
-  for (int c = lane; c < C; c += 32) {
-    const T al = a.alpha[e * a.H + c / Ch];
-    T vs[16], vt[16], vg[16];
-    for (int j = 0; j < D; ++j) { vs[j] = xs[(long long)j * C + c]; vt[j] = xt[(long long)j * C + c]; vg[j] = al * gM[(long long)j * C + c]; }
-    int k = 0;
-    for (int r = 0; r < a.NR; ++r) {
-      const int l = a.row_l[r], dl = 2 * l + 1;
-      const long long at = (e * a.NR + r) * C + c;
-      const T gk = a.gKs[at], gq = a.gQt[at], dn = a.row_scale[r] * a.down[at];
-      for (int j = 0; j < dl; ++j, ++k) acc[k] += gk * vs[l * l + j] + gq * vt[l * l + j] + dn * vg[l * l + j];
-    }
-  }
-  T* out = a.gWg + e * a.NR * D;
-  int k = 0;
-  for (int r = 0; r < a.NR; ++r) {
-    const int l = a.row_l[r], dl = 2 * l + 1;
-    for (int j = 0; j < dl; ++j, ++k) {
-      T v = acc[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) out[r * D + l * l + j] = v;
-    }
+  for (int q = 0; q < M; ++q) {
+    if (BWD) { a.gup[up + G * Ca + q * row] = gx[q]; a.gglu[full + q * row] = gy[q]; }
+    else a.U[full + q * row] = out[q];
   }
 }
 
 }  // namespace
 
-#define TECE_LAUNCH(KERNEL, COUNT, ...)                                                   \
-  do {                                                                                    \
-    const long long cnt__ = (COUNT);                                                      \
-    if (cnt__ > 0) KERNEL<<<(unsigned)((cnt__ + 127) / 128), 128, 0, s>>>(__VA_ARGS__);    \
-    if (cudaGetLastError() != cudaSuccess) return cudaGetLastError();                      \
-  } while (0)
+// f<L, mmax>() for the ranks and orders a model can have (1 <= L <= 3, mmax <= min(L, 2))
+template <typename F>
+bool rank_dispatch(int L, int mmax, F&& f) {
+  switch (L * 4 + mmax) {
+    case 4: f(std::integral_constant<int, 1>(), std::integral_constant<int, 0>()); return true;
+    case 5: f(std::integral_constant<int, 1>(), std::integral_constant<int, 1>()); return true;
+    case 8: f(std::integral_constant<int, 2>(), std::integral_constant<int, 0>()); return true;
+    case 9: f(std::integral_constant<int, 2>(), std::integral_constant<int, 1>()); return true;
+    case 10: f(std::integral_constant<int, 2>(), std::integral_constant<int, 2>()); return true;
+    case 12: f(std::integral_constant<int, 3>(), std::integral_constant<int, 0>()); return true;
+    case 13: f(std::integral_constant<int, 3>(), std::integral_constant<int, 1>()); return true;
+    case 14: f(std::integral_constant<int, 3>(), std::integral_constant<int, 2>()); return true;
+  }
+  return false;
+}
+template <typename K>
+bool rot_smem_limit(K* kernel, int bytes) {  // a failure is left for the caller's cudaGetLastError
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+}
+int tece_wigner_stride(int L, int mmax) {
+  int n = 0;
+  rank_dispatch(L, mmax, [&](auto l, auto m) { n = Rows<decltype(l)::value, decltype(m)::value>::NEP; });
+  return n;
+}
 
 template <typename T>
 cudaError_t launch_tece(const TeceArgs<T>& a, int stage, cudaStream_t s) {
-  const int D = (a.L + 1) * (a.L + 1);
-  if (a.L > 3 || a.mmax > 2 || a.NR > 16 || a.NC > 9 || a.H > 16 || a.G > 12 || a.n_paths * (a.L + 1) > 28 || a.C % a.H != 0)
-    return cudaErrorInvalidValue;
-  cudaError_t err = cudaSuccess;
-  // nothing to launch: stages over atoms need local atoms, every other stage needs edges (an atom without edges still gets
-  // its zero message from TECE_ROTATE_OUT)
-  const bool per_atom = stage == TECE_SOFTMAX || stage == TECE_ROTATE_OUT || stage == TECE_SOFTMAX_BWD || stage == TECE_TARGET_SUM;
-  if (per_atom ? a.n_local <= 0 : a.E <= 0) return cudaSuccess;
-  const int ch = a.C / a.H;
-  const bool fuse_alpha = a.C % 32 == 0 && ch <= 32 && (ch & (ch - 1)) == 0;
+  if (a.H > 16 || a.C % a.H != 0 || a.C % 32 != 0) return cudaErrorInvalidValue;
+  // nothing to launch: stages over atoms need atoms (one without edges still gets its zero message and gradient), every other
+  // stage needs edges
+  const bool per_atom = stage == TECE_SOFTMAX || stage == TECE_ROTATE_OUT || stage == TECE_SOFTMAX_BWD;
+  if (stage == TECE_ROTATE_IN_BWD ? a.n_atoms <= 0 : per_atom ? a.n_local <= 0 : (a.E <= 0 || a.n_local <= 0)) return cudaSuccess;
+  const int ch = a.C / a.H, n_col = a.C / 32;
+  const bool fuse_alpha = ch <= 32 && (ch & (ch - 1)) == 0;
+  auto grid = [](long long count, int block) { return (unsigned)((count + block - 1) / block); };
+  const unsigned rot_grid = (unsigned)((long long)a.n_local * n_col);
+  constexpr int kRot = kRotWarps * 32;
+  bool known = true;
   switch (stage) {
-    case TECE_WIGNER: tece_wigner_kernel<T><<<(unsigned)((a.E + 63) / 64), 64, 0, s>>>(a); break;
+    case TECE_WIGNER:
+      known = rank_dispatch(a.L, a.mmax, [&](auto l, auto m) { tece_wigner_kernel<T, l(), m()><<<grid(a.E, kFrameThreads), kFrameThreads, 0, s>>>(a); });
+      break;
     case TECE_ROTATE_IN:
-      if (!TECE_LM_DISPATCH(tece_rotate_in_t_kernel, (unsigned)((a.E * a.C + 127) / 128), 128))
-        tece_rotate_in_kernel<T><<<(unsigned)((a.E * a.C + 127) / 128), 128, 0, s>>>(a);
+      known = rank_dispatch(a.L, a.mmax, [&](auto l, auto m) { constexpr int Lc = decltype(l)::value, Mc = decltype(m)::value;
+        constexpr int bytes = kRotWarps * 2 * (Rows<Lc, Mc>::NEP + RotIn<T, Lc, Mc>::kRows * 32) * (int)sizeof(T);
+        if (rot_smem_limit(tece_rotate_in_kernel<T, Lc, Mc>, bytes)) tece_rotate_in_kernel<T, Lc, Mc><<<rot_grid, kRot, bytes, s>>>(a);
+      });
       break;
     case TECE_LOGIT:
       if (fuse_alpha) {
-        tece_proj_kernel<T><<<(unsigned)((a.E + 127) / 128), 128, 0, s>>>(a);
-        tece_logit_lane_kernel<T, false><<<(unsigned)((a.E * a.C + 127) / 128), 128, 0, s>>>(a);
+        tece_proj_kernel<T><<<grid(a.E, 128), 128, 0, s>>>(a);
+        tece_logit_lane_kernel<T, false><<<grid(a.E * a.C, 128), 128, 0, s>>>(a);
       } else {
-        tece_logit_kernel<T><<<(unsigned)((a.E * a.H + 127) / 128), 128, 0, s>>>(a);
+        tece_logit_kernel<T><<<grid(a.E * a.H, 128), 128, 0, s>>>(a);
       }
       break;
-    case TECE_SOFTMAX: tece_softmax_kernel<T><<<(unsigned)(((long long)a.n_local * a.H + 127) / 128), 128, 0, s>>>(a); break;
+    case TECE_SOFTMAX: tece_softmax_kernel<T><<<grid((long long)a.n_local * a.H, 128), 128, 0, s>>>(a); break;
     case TECE_MIX:
-      if (!launch_mix_static<T, false>(a, s)) tece_mix_kernel<T, false><<<(unsigned)((a.E * a.Ca + 63) / 64), 64, 0, s>>>(a);
+    case TECE_MIX_BWD:
+      known = rank_dispatch(a.L, a.mmax, [&](auto l, auto m) {
+        constexpr int N = decltype(l)::value + 1, MM = decltype(m)::value;
+        const unsigned g = grid(a.E * N * a.Ca, 128);
+        if (stage == TECE_MIX) {
+          if (a.gate_m0) tece_mix_kernel<T, N, MM, true, false><<<g, 128, 0, s>>>(a);
+          else tece_mix_kernel<T, N, MM, false, false><<<g, 128, 0, s>>>(a);
+        } else {
+          if (a.gate_m0) tece_mix_kernel<T, N, MM, true, true><<<g, 128, 0, s>>>(a);
+          else tece_mix_kernel<T, N, MM, false, true><<<g, 128, 0, s>>>(a);
+        }
+      });
       break;
     case TECE_ROTATE_OUT:
-      if (!TECE_LM_DISPATCH(tece_rotate_out_t_kernel, (unsigned)(((long long)a.n_local * a.C + 127) / 128), 128))
-        tece_rotate_out_kernel<T><<<(unsigned)(((long long)a.n_local * a.C + 127) / 128), 128, 0, s>>>(a);
+      known = rank_dispatch(a.L, a.mmax, [&](auto l, auto m) { tece_rotate_out_kernel<T, l(), m()><<<rot_grid, kRot, 0, s>>>(a); });
       break;
     case TECE_ROTATE_OUT_BWD:
-      if (fuse_alpha) tece_rotate_out_bwd_kernel<T, true><<<(unsigned)((a.E * a.C + 127) / 128), 128, 0, s>>>(a);
-      else tece_rotate_out_bwd_kernel<T, false><<<(unsigned)((a.E * a.C + 127) / 128), 128, 0, s>>>(a);
+      known = rank_dispatch(a.L, a.mmax, [&](auto l, auto m) {
+        if (fuse_alpha) tece_rotate_out_bwd_kernel<T, l(), m(), true><<<rot_grid, kRot, 0, s>>>(a);
+        else tece_rotate_out_bwd_kernel<T, l(), m(), false><<<rot_grid, kRot, 0, s>>>(a);
+      });
       break;
     case TECE_ALPHA_BWD:  // already done by the fused kernel above when the head width allows it
-      if (!fuse_alpha) tece_alpha_bwd_kernel<T><<<(unsigned)((a.E * a.H + 127) / 128), 128, 0, s>>>(a);
+      if (!fuse_alpha) tece_alpha_bwd_kernel<T><<<grid(a.E * a.H, 128), 128, 0, s>>>(a);
       break;
-    case TECE_SOFTMAX_BWD: tece_softmax_bwd_kernel<T><<<(unsigned)(((long long)a.n_local * a.H + 127) / 128), 128, 0, s>>>(a); break;
+    case TECE_SOFTMAX_BWD: tece_softmax_bwd_kernel<T><<<grid((long long)a.n_local * a.H, 128), 128, 0, s>>>(a); break;
     case TECE_LOGIT_BWD:
-      if (fuse_alpha) tece_logit_lane_kernel<T, true><<<(unsigned)((a.E * a.C + 127) / 128), 128, 0, s>>>(a);
-      else tece_logit_bwd_kernel<T><<<(unsigned)((a.E * a.H + 127) / 128), 128, 0, s>>>(a);
+      if (fuse_alpha) tece_logit_lane_kernel<T, true><<<grid(a.E * a.C, 128), 128, 0, s>>>(a);
+      else tece_logit_bwd_kernel<T><<<grid(a.E * a.H, 128), 128, 0, s>>>(a);
       break;
-    case TECE_EDGE_SCALAR_BWD: tece_edge_scalar_bwd_kernel<T><<<(unsigned)((a.E + 127) / 128), 128, 0, s>>>(a); break;
-    case TECE_MIX_BWD:
-      if (!launch_mix_static<T, true>(a, s)) tece_mix_kernel<T, true><<<(unsigned)((a.E * a.Ca + 63) / 64), 64, 0, s>>>(a);
-      break;
+    case TECE_EDGE_SCALAR_BWD: tece_edge_scalar_bwd_kernel<T><<<grid(a.E, 128), 128, 0, s>>>(a); break;
     case TECE_ROTATE_IN_BWD:
-      if (!TECE_LM_DISPATCH(tece_rotate_in_bwd_t_kernel, (unsigned)((a.E * a.C + 127) / 128), 128))
-        tece_rotate_in_bwd_kernel<T><<<(unsigned)((a.E * a.C + 127) / 128), 128, 0, s>>>(a);
+      known = rank_dispatch(a.L, a.mmax, [&](auto l, auto m) {
+        constexpr int Lc = decltype(l)::value, Mc = decltype(m)::value;
+        constexpr int bytes = kRotWarps * 2 * (Rows<Lc, Mc>::NEP + RotInBwd<T, Lc, Mc>::kRows * 32) * (int)sizeof(T);
+        if (rot_smem_limit(tece_rotate_in_bwd_kernel<T, Lc, Mc>, bytes))
+          tece_rotate_in_bwd_kernel<T, Lc, Mc><<<(unsigned)((long long)a.n_atoms * n_col), kRot, bytes, s>>>(a);
+      });
       break;
-    case TECE_TARGET_SUM: tece_target_sum_kernel<T><<<(unsigned)(((long long)a.n_local * D * a.C + 127) / 128), 128, 0, s>>>(a); break;
-    case TECE_WIGNER_GRAD:
-      if (!TECE_LM_DISPATCH(tece_wigner_grad_t_kernel, (unsigned)((a.E + 3) / 4), 128))
-        tece_wigner_grad_kernel<T><<<(unsigned)((a.E + 3) / 4), 128, 0, s>>>(a);
+    case TECE_WIGNER_BWD:
+      known = rank_dispatch(a.L, a.mmax, [&](auto l, auto m) { tece_wigner_bwd_kernel<T, l(), m()><<<grid(a.E, kFrameThreads), kFrameThreads, 0, s>>>(a); });
       break;
-    case TECE_WIGNER_BWD: tece_wigner_bwd_kernel<T><<<(unsigned)((a.E + 63) / 64), 64, 0, s>>>(a, a.accumulate_gvec); break;
-    default: err = cudaErrorInvalidValue;
+    default: known = false;
   }
-  return err != cudaSuccess ? err : cudaGetLastError();
+  return known ? cudaGetLastError() : cudaErrorInvalidValue;
 }
 
 template cudaError_t launch_tece<float>(const TeceArgs<float>&, int, cudaStream_t);

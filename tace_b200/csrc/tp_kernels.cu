@@ -489,7 +489,7 @@ __global__ void tp_bwd_scalar_kernel(const TPArgs<T> a) {
 // edges in list order, so the result does not depend on the vector width.
 template <typename T, int W>
 __global__ void segment_sum_rows_kernel(const RowVec<T, W>* __restrict__ dxe, const int* __restrict__ rowptr, const int* __restrict__ perm,
-                                        RowVec<T, W>* __restrict__ gx, int first, int row_len) {
+                                        RowVec<T, W>* __restrict__ gx, int first, int row_len, int accumulate) {
   const int b = first + blockIdx.x;
   const int beg = rowptr[b], end = rowptr[b + 1];
   for (int k = threadIdx.x; k < row_len; k += blockDim.x) {
@@ -501,21 +501,26 @@ __global__ void segment_sum_rows_kernel(const RowVec<T, W>* __restrict__ dxe, co
 #pragma unroll
       for (int i = 0; i < W; ++i) acc.v[i] += x.v[i];
     }
+    if (accumulate) {
+      const RowVec<T, W> x = gx[(long long)b * row_len + k];
+#pragma unroll
+      for (int i = 0; i < W; ++i) acc.v[i] += x.v[i];
+    }
     gx[(long long)b * row_len + k] = acc;
   }
 }
 template <typename T>
 cudaError_t launch_segment_sum_rows(const T* dxe, const int* rowptr_src, const int* perm_src, T* gx, int first_atom, int n_atoms,
-                                    int row_len, cudaStream_t s) {
+                                    int row_len, cudaStream_t s, int accumulate) {
   if (n_atoms <= 0) return cudaSuccess;
   constexpr int W = 16 / sizeof(T);
   auto threads_for = [](int items) { const int t = (items + 31) / 32 * 32; return t < 32 ? 32 : (t > 256 ? 256 : t); };
   if (row_len % W == 0 && ((reinterpret_cast<uintptr_t>(dxe) | reinterpret_cast<uintptr_t>(gx)) & 15) == 0)
     segment_sum_rows_kernel<T, W><<<n_atoms, threads_for(row_len / W), 0, s>>>(reinterpret_cast<const RowVec<T, W>*>(dxe), rowptr_src, perm_src,
-                                                            reinterpret_cast<RowVec<T, W>*>(gx), first_atom, row_len / W);
+                                                            reinterpret_cast<RowVec<T, W>*>(gx), first_atom, row_len / W, accumulate);
   else
     segment_sum_rows_kernel<T, 1><<<n_atoms, threads_for(row_len), 0, s>>>(reinterpret_cast<const RowVec<T, 1>*>(dxe), rowptr_src, perm_src,
-                                                            reinterpret_cast<RowVec<T, 1>*>(gx), first_atom, row_len);
+                                                            reinterpret_cast<RowVec<T, 1>*>(gx), first_atom, row_len, accumulate);
   return cudaGetLastError();
 }
 
@@ -640,8 +645,8 @@ template cudaError_t launch_tp_fwd<float>(const TPArgs<float>&, cudaStream_t);
 template cudaError_t launch_tp_fwd<double>(const TPArgs<double>&, cudaStream_t);
 template cudaError_t launch_tp_bwd<float>(const TPArgs<float>&, cudaStream_t);
 template cudaError_t launch_tp_bwd<double>(const TPArgs<double>&, cudaStream_t);
-template cudaError_t launch_segment_sum_rows<float>(const float*, const int*, const int*, float*, int, int, int, cudaStream_t);
-template cudaError_t launch_segment_sum_rows<double>(const double*, const int*, const int*, double*, int, int, int, cudaStream_t);
+template cudaError_t launch_segment_sum_rows<float>(const float*, const int*, const int*, float*, int, int, int, cudaStream_t, int);
+template cudaError_t launch_segment_sum_rows<double>(const double*, const int*, const int*, double*, int, int, int, cudaStream_t, int);
 template cudaError_t launch_chunk_src_sum<float>(const float*, const int*, const int*, long long, long long, long long, float*, int, cudaStream_t);
 template cudaError_t launch_chunk_src_sum<double>(const double*, const int*, const int*, long long, long long, long long, double*, int, cudaStream_t);
 
