@@ -403,7 +403,8 @@ struct Model : ModelBase {
   int weights_missing = -1;   // entries not set yet (-1: not counted)
   T* arena = nullptr;
   long long arena_numel = 0;
-  struct DebugBuf { std::string name; const void* ptr; long long numel; };
+  // perm: the `row` elements of atom i are row perm[i] (nullptr: atom order)
+  struct DebugBuf { std::string name; const void* ptr; long long numel; const int* perm = nullptr; long long row = 0; };
   std::vector<DebugBuf> debug;
   T host_bessel[kNumBessel + 1];  // host copies of the radial frequencies and prefactor
 
@@ -654,8 +655,8 @@ struct Model : ModelBase {
   // ---- workspace ---------------------------------------------------------------------------
   static constexpr long long kChunkSlack = 8192;  // a chunk ends at an atom boundary: room for one atom's edges beyond the target
   struct LayerBufs {
-    T *h_in, *x, *xx, *gxx, *W, *H3, *Z1, *Z2, *Z3, *Hact, *M, *Gt, *gGt, *a, *A, *B2, *out, *h_out;
-    T *gh_out, *gout, *gA, *ga, *gx, *gh_in;
+    T *h_in, *x, *xx, *gxx, *W, *H3, *Z1, *Z2, *Z3, *Hact, *M, *Gt, *gGt, *a, *B2, *out, *h_out;
+    T *gh_out, *ga, *gx, *gh_in;
     T *As, *gAs, *gout_s, *hs;  // species-sorted copies used by the per-species linears
     T *B3, *gB2;                // third-order basis (reused for its gradient) and the gradient of the second-order one
     T *inv_density, *gdens;     // learned edge density: 1 / density_i and dE / d density_i
@@ -666,7 +667,7 @@ struct Model : ModelBase {
   };
   struct Bufs {
     int *row_ids, *row_split;  // owned targets without / with a ghost source (passes split around the exchange)
-    int *e_src, *e_dst, *e_orig, *perm_src, *rowptr_dst, *rowptr_src, *atom_graph, *species_perm, *species_ptr, *tile_ptr, *tc_tile_ptr;
+    int *e_src, *e_dst, *e_orig, *perm_src, *rowptr_dst, *rowptr_src, *atom_graph, *species_perm, *species_rank, *species_ptr, *tile_ptr, *tc_tile_ptr;
     int *chunk_atom_ptr, *chunk_edge_ptr, *keys_cs, *perm_cs;  // edge chunks; (chunk, source)-sorted edge list
     int n_chunks; long long chunk_rows;                        // rows held by the per-edge chunk buffers
     void* prep_temp; size_t prep_temp_bytes;
@@ -680,7 +681,7 @@ struct Model : ModelBase {
     b.e_src = ar.take<int>(E); b.e_dst = ar.take<int>(E); b.e_orig = ar.take<int>(E); b.perm_src = ar.take<int>(E);
     b.rowptr_dst = ar.take<int>(N + 1); b.rowptr_src = ar.take<int>(N + 1); b.atom_graph = ar.take<int>(N);
     b.row_ids = ar.take<int>(NL); b.row_split = ar.take<int>(2);
-    b.species_perm = ar.take<int>(NL); b.species_ptr = ar.take<int>(n_el + 1); b.tile_ptr = ar.take<int>(4 * (n_el + 1));
+    b.species_perm = ar.take<int>(NL); b.species_rank = ar.take<int>(NL); b.species_ptr = ar.take<int>(n_el + 1); b.tile_ptr = ar.take<int>(4 * (n_el + 1));
     b.tc_tile_ptr = ar.take<int>(4 * (n_el + 1));
     b.prep_temp_bytes = graph_prep_temp_bytes(E, (int)N);
     b.prep_temp = ar.take<unsigned char>(b.prep_temp_bytes);
@@ -753,8 +754,6 @@ struct Model : ModelBase {
       }
       lb.a = ar.take<T>((size_t)NL * D * C);
       lb.ga = ar.take<T>((size_t)NL * D * C);
-      lb.A = ar.take<T>((size_t)NL * D * C);
-      lb.gA = ar.take<T>((size_t)NL * D * C);
       lb.B2 = ar.take<T>((size_t)NL * p.pb.NB * C);
       lb.B3 = cfg.correlation >= 3 ? ar.take<T>((size_t)NL * p.pb3.NB * C) : nullptr;
       lb.gB2 = cfg.correlation >= 3 ? ar.take<T>((size_t)NL * p.pb.NB * C) : nullptr;
@@ -763,7 +762,6 @@ struct Model : ModelBase {
       lb.gout_s = ar.take<T>((size_t)NL * p.Dout * C);
       lb.hs = p.has_res ? ar.take<T>((size_t)NL * p.Din * C) : nullptr;
       lb.out = ar.take<T>((size_t)NL * p.Dout * C);
-      lb.gout = ar.take<T>((size_t)NL * p.Dout * C);
       lb.h_out = ar.take<T>((size_t)N * p.Dout * C);
       lb.gh_out = ar.take<T>((size_t)N * p.Dout * C);
       prev_h = lb.h_out;
@@ -806,25 +804,55 @@ struct Model : ModelBase {
     T* Cm; long long c_s1, c_s2; const T* bias;
     int accumulate;  // Cm += instead of Cm =
   };
-  // Plain (not per-species) linears: tcgen05 for fp32 models when every shape fits, CUDA cores otherwise.
-  cudaError_t run_linear(const std::vector<LinSpec>& specs, long long n_atoms, cudaStream_t s) {
-    bool tc = kTensorCore && !specs.empty() && specs.size() <= 4;
-    for (const auto& sp : specs) tc = tc && tc_linear_supported(sp.N, sp.K);
-    if (tc) {
-      TcLinearProblem probs[4];
-      for (size_t i = 0; i < specs.size(); ++i) {
-        const LinSpec& sp = specs[i];
-        probs[i] = {reinterpret_cast<const float*>(sp.A), sp.a_s1, sp.a_s2, sp.q, n_atoms, sp.K, sp.N,
-                    reinterpret_cast<const float*>(w(sp.wname_t + "_hi")), reinterpret_cast<const float*>(w(sp.wname_t + "_lo")),
-                    reinterpret_cast<float*>(sp.Cm), sp.c_s1, sp.c_s2, reinterpret_cast<const float*>(sp.bias)};
-        probs[i].accumulate = sp.accumulate;
+  // accumulate = kJoin: the product is added to that of the spec before it (same rows and result), in one pass over both K ranges
+  // where the tensor-core path takes them.
+  static constexpr int kJoin = 2;
+  // The specs of one call, a run of joined ones at a time: tcgen05 for fp32 models where every shape of the run fits, the other
+  // kernels for the rest, joined products in launches of their own.
+  template <typename Spec, typename FillTc, typename Add>
+  cudaError_t run_specs(const std::vector<Spec>& specs, long long n_atoms, cudaStream_t s, const GemmBatch<T>& empty, FillTc&& fill, Add&& add) {
+    TcLinearProblem probs[kMaxLinears];
+    int n_tc = 0;
+    std::vector<std::vector<const Spec*>> rest;  // by place in the run
+    cudaError_t err = cudaSuccess;
+    for (size_t i = 0, j; i < specs.size() && err == cudaSuccess; i = j) {
+      bool tc = kTensorCore;
+      for (j = i; j < specs.size() && (j == i || specs[j].accumulate == kJoin); ++j) tc = tc && tc_linear_supported(specs[j].N, specs[j].K);
+      for (size_t k = i; k < j && !tc; ++k) {
+        if (rest.size() <= k - i) rest.resize(k - i + 1);
+        rest[k - i].push_back(&specs[k]);
       }
-      return launch_tc_linear(probs, (int)specs.size(), dev_error, s);
+      if (!tc) continue;
+      if (n_tc + (int)(j - i) > kMaxLinears) { err = launch_tc_linear(probs, n_tc, dev_error, s); n_tc = 0; }
+      for (size_t k = i; k < j; ++k) {
+        const Spec& sp = specs[k];
+        TcLinearProblem& h = probs[n_tc++];
+        memset(&h, 0, sizeof(h));
+        h.A = reinterpret_cast<const float*>(sp.A); h.a_atom_stride = sp.a_s1; h.a_comp_stride = sp.a_s2; h.q = sp.q;
+        h.n_atoms = n_atoms; h.K = sp.K; h.N = sp.N;
+        h.Bhi = reinterpret_cast<const float*>(w(sp.wname_t + "_hi")); h.Blo = reinterpret_cast<const float*>(w(sp.wname_t + "_lo"));
+        h.C = reinterpret_cast<float*>(sp.Cm); h.c_s1 = sp.c_s1; h.c_s2 = sp.c_s2; h.bias = reinterpret_cast<const float*>(sp.bias);
+        h.accumulate = sp.accumulate == 1; h.join = sp.accumulate == kJoin;
+        fill(h, sp);
+      }
     }
+    if (err == cudaSuccess && n_tc > 0) err = launch_tc_linear(probs, n_tc, dev_error, s);
+    for (size_t level = 0; level < rest.size(); ++level)
+      for (size_t i = 0; i < rest[level].size() && err == cudaSuccess; i += kMaxProblems) {
+        GemmBatch<T> gb = empty;
+        for (size_t k = i; k < rest[level].size() && k < i + kMaxProblems; ++k) add(gb, *rest[level][k], level > 0 || rest[level][k]->accumulate == 1);
+        err = launch_gemm(gb, n_atoms, s);
+      }
+    return err;
+  }
+  // Plain (not per-species) linears.  c_map: row a of the results belongs to atom c_map[a] (nullptr: the same order).
+  cudaError_t run_linear(const std::vector<LinSpec>& specs, long long n_atoms, cudaStream_t s, const int* c_map = nullptr) {
     GemmBatch<T> gb = plain_batch(n_atoms);
-    for (const auto& sp : specs)
-      add_problem(gb, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, sp.accumulate);
-    return launch_gemm(gb, n_atoms, s);
+    gb.c_atom_map = c_map;
+    return run_specs(specs, n_atoms, s, gb, [&](TcLinearProblem& h, const LinSpec&) { h.atom_map = c_map; },
+                     [&](GemmBatch<T>& g, const LinSpec& sp, int accumulate) {
+                       add_problem(g, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, accumulate);
+                     });
   }
 
   // Per-species linears (the reference's e3nnElementLinear, tace/models/linear.py:377-481).  A holds rows of the
@@ -837,35 +865,23 @@ struct Model : ModelBase {
   };
   cudaError_t run_species_linear(const std::vector<SpeciesSpec>& specs, const Bufs& b, long long n_atoms, cudaStream_t s) {
     if (specs.empty()) return cudaSuccess;
-    bool tc = kTensorCore && specs.size() <= 4;
-    for (const auto& sp : specs) tc = tc && tc_linear_supported(sp.N, sp.K) && sp.mapped == specs[0].mapped;
-    if (tc) {
-      TcLinearProblem probs[4];
-      for (size_t i = 0; i < specs.size(); ++i) {
-        const SpeciesSpec& sp = specs[i];
-        TcLinearProblem& h = probs[i];
-        memset(&h, 0, sizeof(h));
-        h.A = reinterpret_cast<const float*>(sp.A); h.a_atom_stride = sp.a_s1; h.a_comp_stride = sp.a_s2; h.q = sp.q;
-        h.n_atoms = n_atoms; h.K = sp.K; h.N = sp.N;
-        h.Bhi = reinterpret_cast<const float*>(w(sp.wname_t + "_hi")); h.Blo = reinterpret_cast<const float*>(w(sp.wname_t + "_lo"));
-        h.C = reinterpret_cast<float*>(sp.Cm); h.c_s1 = sp.c_s1; h.c_s2 = sp.c_s2; h.bias = reinterpret_cast<const float*>(sp.bias);
-        h.n_groups = n_el; h.group_ptr = b.species_ptr; h.tile_ptr = b.tc_tile_ptr + (sp.q / 2) * (n_el + 1);
-        h.atom_map = sp.mapped ? b.species_perm : nullptr;
-        h.b_group_stride = (long long)sp.K * sp.N; h.bias_group_stride = sp.N; h.accumulate = sp.accumulate;
-        h.b_tiled = 1;  // the packed per-species hi / lo parts are K-tile-major (read once per pass, straight from DRAM)
-      }
-      return launch_tc_linear(probs, (int)specs.size(), dev_error, s);
-    }
     GemmBatch<T> gb;
     memset(&gb, 0, sizeof(gb));
-    gb.n_groups = n_el; gb.group_ptr = b.species_ptr; gb.atom_map = nullptr;
+    gb.n_groups = n_el; gb.group_ptr = b.species_ptr;
     gb.c_atom_map = specs[0].mapped ? b.species_perm : nullptr;
-    for (const auto& sp : specs) {
+    for (const auto& sp : specs)
       if (sp.mapped != specs[0].mapped) return cudaErrorInvalidValue;
-      add_problem(gb, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, sp.accumulate,
-                  (long long)sp.K * sp.N, sp.N, tiles(b, sp.q / 2));
-    }
-    return launch_gemm(gb, n_atoms, s);
+    return run_specs(specs, n_atoms, s, gb,
+                     [&](TcLinearProblem& h, const SpeciesSpec& sp) {
+                       h.n_groups = n_el; h.group_ptr = b.species_ptr; h.tile_ptr = b.tc_tile_ptr + (sp.q / 2) * (n_el + 1);
+                       h.atom_map = gb.c_atom_map;
+                       h.b_group_stride = (long long)sp.K * sp.N; h.bias_group_stride = sp.N;
+                       h.b_tiled = 1;  // the packed per-species hi / lo parts are K-tile-major (read once per pass, straight from DRAM)
+                     },
+                     [&](GemmBatch<T>& g, const SpeciesSpec& sp, int accumulate) {
+                       add_problem(g, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, accumulate,
+                                   (long long)sp.K * sp.N, sp.N, tiles(b, sp.q / 2));
+                     });
   }
 
 #define CK(expr)                                                                                 \
@@ -917,24 +933,30 @@ struct Model : ModelBase {
     }
     return s;
   }
-  // GEMM problems of one SO(2) linear over the E edges: `in` [E][in_rows][c_in] -> `out` [E][out_rows][c_out] (forward), or the
-  // gradient of the output back to the gradient of the input (backward; `out` is then the input gradient)
-  void so2_specs(std::vector<LinSpec>& sp, const std::string& pre, int which, const T* in, int in_rows, T* out, int out_rows, bool backward,
-                 int accumulate) const {
-    const So2Shape sh = so2_shape(which);
-    int off_in = 0, off_out = 0;
-    for (int m = 0; m <= sh.mm; ++m) {
-      const int K = sh.n_in[m] * sh.c_in, Nn = sh.n_out[m] * sh.c_out;
-      const std::string nm = pre + "so2." + sh.name + ".m" + std::to_string(m), nmT = pre + "so2." + sh.name + "T.m" + std::to_string(m);
-      if (!backward)
-        sp.push_back({in + (long long)off_in * sh.c_in, (long long)in_rows * sh.c_in, K, m ? 2 : 1, K, nm, nmT, Nn,
-                      out + (long long)off_out * sh.c_out, (long long)out_rows * sh.c_out, Nn, m == 0 ? w(pre + "so2." + sh.name + ".b") : nullptr, 0});
-      else  // `in` holds the gradient of the forward output, `out` receives the gradient of the forward input
-        sp.push_back({in + (long long)off_out * sh.c_out, (long long)out_rows * sh.c_out, Nn, m ? 2 : 1, Nn, nmT, nm, K,
-                      out + (long long)off_in * sh.c_in, (long long)in_rows * sh.c_in, K, nullptr, accumulate});
-      // the order-0 block of the input always spans L + 1 rows (oam_2026_07_05.py:211)
-      off_in += (m == 0) ? (L + 1) : 2 * sh.n_in[m];
-      off_out += (m == 0) ? sh.n_out[0] : 2 * sh.n_out[m];
+  // GEMM problems of SO(2) linears over the E edges: `in` [E][in_rows][c_in] -> `out` [E][out_rows][c_out] (forward), or the
+  // gradient of the output back to the gradient of the input (backward; `out` is then the input gradient, and linears of the
+  // call with the same input gradient add up)
+  struct So2Run { int which; const T* in; int in_rows; T* out; int out_rows; };
+  void so2_specs(std::vector<LinSpec>& sp, const std::string& pre, const std::vector<So2Run>& runs, bool backward) const {
+    std::vector<int> off_in(runs.size(), 0), off_out(runs.size(), 0);
+    for (int m = 0; m <= mmax; ++m) {
+      for (size_t i = 0; i < runs.size(); ++i) {
+        const So2Run& r = runs[i];
+        const So2Shape sh = so2_shape(r.which);
+        if (m > sh.mm) continue;
+        const int K = sh.n_in[m] * sh.c_in, Nn = sh.n_out[m] * sh.c_out;
+        const std::string nm = pre + "so2." + sh.name + ".m" + std::to_string(m), nmT = pre + "so2." + sh.name + "T.m" + std::to_string(m);
+        if (!backward)
+          sp.push_back({r.in + (long long)off_in[i] * sh.c_in, (long long)r.in_rows * sh.c_in, K, m ? 2 : 1, K, nm, nmT, Nn,
+                        r.out + (long long)off_out[i] * sh.c_out, (long long)r.out_rows * sh.c_out, Nn, m == 0 ? w(pre + "so2." + sh.name + ".b") : nullptr, 0});
+        else  // `in` holds the gradient of the forward output, `out` receives the gradient of the forward input
+          sp.push_back({r.in + (long long)off_out[i] * sh.c_out, (long long)r.out_rows * sh.c_out, Nn, m ? 2 : 1, Nn, nmT, nm, K,
+                        r.out + (long long)off_in[i] * sh.c_in, (long long)r.in_rows * sh.c_in, K, nullptr,
+                        i > 0 && r.out == runs[i - 1].out ? kJoin : 0});
+        // the order-0 block of the input always spans L + 1 rows (oam_2026_07_05.py:211)
+        off_in[i] += (m == 0) ? (L + 1) : 2 * sh.n_in[m];
+        off_out[i] += (m == 0) ? sh.n_out[0] : 2 * sh.n_out[m];
+      }
     }
   }
   TeceArgs<T> tece_args(const EdgeArgs<T>& ea, const Bufs& b, const LayerBufs& lb, const std::string& pre, const T* x_src, long long N,
@@ -960,20 +982,14 @@ struct Model : ModelBase {
   int tece_forward(const TeceArgs<T>& ta, const LayerBufs& lb, const std::string& pre, long long E, cudaStream_t s) {
     std::vector<LinSpec> sp;
     CKL(launch_tece(ta, TECE_ROTATE_IN, s));
-    so2_specs(sp, pre, 0, lb.tKs, t_NR, lb.tKp, t_NR, false, 0);
-    CKL(run_linear(sp, E, s)); sp.clear();
-    so2_specs(sp, pre, 1, lb.tQt, t_NR, lb.tQp, t_NR, false, 0);
+    so2_specs(sp, pre, {{0, lb.tKs, t_NR, lb.tKp, t_NR}, {1, lb.tQt, t_NR, lb.tQp, t_NR}}, false);
     CKL(run_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_LOGIT, s));
     CKL(launch_tece(ta, TECE_SOFTMAX, s));
-    so2_specs(sp, pre, 2, lb.tMw, t_NR, lb.tup, t_G + t_NF, false, 0);
-    CKL(run_linear(sp, E, s)); sp.clear();
-    so2_specs(sp, pre, 3, lb.tMw, t_NR, lb.tglu, t_NF, false, 0);
-    CKL(run_linear(sp, E, s)); sp.clear();
-    so2_specs(sp, pre, 4, lb.tMw, t_NR, lb.tcoef, t_WN, false, 0);
+    so2_specs(sp, pre, {{2, lb.tMw, t_NR, lb.tup, t_G + t_NF}, {3, lb.tMw, t_NR, lb.tglu, t_NF}, {4, lb.tMw, t_NR, lb.tcoef, t_WN}}, false);
     CKL(run_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_MIX, s));
-    so2_specs(sp, pre, 5, lb.tU, t_NF, lb.tdown, t_NR, false, 0);
+    so2_specs(sp, pre, {{5, lb.tU, t_NF, lb.tdown, t_NR}}, false);
     CKL(run_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_ROTATE_OUT, s));
     return TACE_OK;
@@ -988,18 +1004,13 @@ struct Model : ModelBase {
     CKL(launch_tece(ta, TECE_SOFTMAX_BWD, s));
     CKL(launch_tece(ta, TECE_LOGIT_BWD, s));
     CKL(launch_tece(ta, TECE_EDGE_SCALAR_BWD, s));
-    so2_specs(sp, pre, 5, lb.tgdown, t_NF, lb.tU, t_NR, true, 0);   // gU over U
+    so2_specs(sp, pre, {{5, lb.tgdown, t_NF, lb.tU, t_NR}}, true);   // gU over U
     CKL(run_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_MIX_BWD, s));                           // gup / gglu / gcoef over their forward buffers
-    so2_specs(sp, pre, 2, lb.tup, t_NR, lb.tMw, t_G + t_NF, true, 0);  // gMw over Mw
+    // gMw over Mw: the three linears that read Mw add up in one pass per order
+    so2_specs(sp, pre, {{2, lb.tup, t_NR, lb.tMw, t_G + t_NF}, {3, lb.tglu, t_NR, lb.tMw, t_NF}, {4, lb.tcoef, t_NR, lb.tMw, t_WN}}, true);
     CKL(run_linear(sp, E, s)); sp.clear();
-    so2_specs(sp, pre, 3, lb.tglu, t_NR, lb.tMw, t_NF, true, 1);
-    CKL(run_linear(sp, E, s)); sp.clear();
-    so2_specs(sp, pre, 4, lb.tcoef, t_NR, lb.tMw, t_WN, true, 1);
-    CKL(run_linear(sp, E, s)); sp.clear();
-    so2_specs(sp, pre, 0, lb.tgKp, t_NR, lb.tgKs, t_NR, true, 0);
-    CKL(run_linear(sp, E, s)); sp.clear();
-    so2_specs(sp, pre, 1, lb.tgQp, t_NR, lb.tgQt, t_NR, true, 0);
+    so2_specs(sp, pre, {{0, lb.tgKp, t_NR, lb.tgKs, t_NR}, {1, lb.tgQp, t_NR, lb.tgQt, t_NR}}, true);
     CKL(run_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_ROTATE_IN_BWD, s));
     CKL(launch_segment_sum_rows(b.dxe, b.rowptr_src, b.perm_src, lb.gx, 0, (int)N, D * C, s, /*accumulate=*/1));
@@ -1191,7 +1202,7 @@ struct Model : ModelBase {
     gp.edge_index = bt->edge_index; gp.species = bt->species; gp.graph_ptr = bt->graph_ptr;
     gp.e_src = b.e_src; gp.e_dst = b.e_dst; gp.e_orig = b.e_orig; gp.rowptr_dst = b.rowptr_dst;
     gp.perm_src = b.perm_src; gp.rowptr_src = b.rowptr_src; gp.atom_graph = b.atom_graph;
-    gp.species_perm = b.species_perm; gp.species_ptr = b.species_ptr; gp.tile_ptr = b.tile_ptr; gp.tc_tile_ptr = b.tc_tile_ptr;
+    gp.species_perm = b.species_perm; gp.species_rank = b.species_rank; gp.species_ptr = b.species_ptr; gp.tile_ptr = b.tile_ptr; gp.tc_tile_ptr = b.tc_tile_ptr;
     gp.temp = b.prep_temp; gp.temp_bytes = b.prep_temp_bytes;
     // edge chunks: one chunk (all atoms) unless the batch exceeds max_chunk_edges
     const bool chunked = E > max_chunk_edges;
@@ -1341,13 +1352,12 @@ struct Model : ModelBase {
         std::vector<LinSpec> sp;
         for (int l = 0; l <= L; ++l)
           sp.push_back({lb.a + (long long)l * l * C, (long long)D * C, C, 2 * l + 1, C, pre + "nl.l" + std::to_string(l),
-                        pre + "nlT.l" + std::to_string(l), C, lb.A + (long long)l * l * C, (long long)D * C, C,
+                        pre + "nlT.l" + std::to_string(l), C, lb.As + (long long)l * l * C, (long long)D * C, C,
                         l == 0 ? w(pre + "nl.b") : nullptr});
-        CKL(run_linear(sp, NL, s));
+        // the per-species part works in species-sorted space: this linear writes its rows there, the coefficient linears scatter into `out`
+        CKL(run_linear(sp, NL, s, b.species_rank));
       }
-      debug.push_back({"A" + ts, lb.A, NL * D * C});
-      // per-species part in species-sorted space: gather A, product basis, coefficient linears scatter into `out`
-      CKL(launch_gather_rows(lb.A, b.species_perm, lb.As, NL, D * C, s));
+      debug.push_back({"A" + ts, lb.As, NL * D * C, b.species_rank, D * C});
       if (bilinear) {
         std::vector<LinSpec> sp;
         for (int l = 0; l <= L; ++l)
@@ -1366,32 +1376,26 @@ struct Model : ModelBase {
       if (cfg.correlation >= 3) CKL(launch_pb3_fwd(lb.As, lb.B2, lb.B3, (int)NL, L, p.last ? -1 : Ln, C, s));
       {
         std::vector<SpeciesSpec> sp;
-        for (int l : p.out_ls)
+        // the products of all correlation orders add up in one pass per rank
+        for (size_t i = 0; i < p.out_ls.size(); ++i) {
+          const int l = p.out_ls[i];
+          const std::string ls = std::to_string(l);
+          T* out = lb.out + (long long)l * l * C;
           sp.push_back({bilinear ? lb.XY + (long long)l * l * 2 * C : lb.As + (long long)l * l * C, (long long)D * C * (bilinear ? 2 : 1),
-                        (long long)C * (bilinear ? 2 : 1), 2 * l + 1, C, pre + "c0.l" + std::to_string(l),
-                        pre + "c0T.l" + std::to_string(l), C, lb.out + (long long)l * l * C, (long long)p.Dout * C, C,
-                        l == 0 ? w(pre + "c.b") : nullptr, true, 0});
-        CKL(run_species_linear(sp, b, NL, s));
-        if (cfg.correlation >= 2) {
-          sp.clear();
-          for (size_t i = 0; i < p.out_ls.size(); ++i) {
-            const int l = p.out_ls[i];
+                        (long long)C * (bilinear ? 2 : 1), 2 * l + 1, C, pre + "c0.l" + ls, pre + "c0T.l" + ls, C, out,
+                        (long long)p.Dout * C, C, l == 0 ? w(pre + "c.b") : nullptr, true, 0});
+          if (cfg.correlation >= 2) {
             const int K = p.pb.k[i] * C;
-            sp.push_back({lb.B2 + (long long)p.pb.base[i] * C, (long long)p.pb.NB * C, K, 2 * l + 1, K, pre + "c1.l" + std::to_string(l),
-                          pre + "c1T.l" + std::to_string(l), C, lb.out + (long long)l * l * C, (long long)p.Dout * C, C, nullptr, true, 1});
+            sp.push_back({lb.B2 + (long long)p.pb.base[i] * C, (long long)p.pb.NB * C, K, 2 * l + 1, K, pre + "c1.l" + ls, pre + "c1T.l" + ls,
+                          C, out, (long long)p.Dout * C, C, nullptr, true, kJoin});
           }
-          CKL(run_species_linear(sp, b, NL, s));
-        }
-        if (cfg.correlation >= 3) {
-          sp.clear();
-          for (size_t i = 0; i < p.out_ls.size(); ++i) {
-            const int l = p.out_ls[i];
+          if (cfg.correlation >= 3) {
             const int K = p.pb3.k[i] * C;
-            sp.push_back({lb.B3 + (long long)p.pb3.base[i] * C, (long long)p.pb3.NB * C, K, 2 * l + 1, K, pre + "c2.l" + std::to_string(l),
-                          pre + "c2T.l" + std::to_string(l), C, lb.out + (long long)l * l * C, (long long)p.Dout * C, C, nullptr, true, 1});
+            sp.push_back({lb.B3 + (long long)p.pb3.base[i] * C, (long long)p.pb3.NB * C, K, 2 * l + 1, K, pre + "c2.l" + ls, pre + "c2T.l" + ls,
+                          C, out, (long long)p.Dout * C, C, nullptr, true, kJoin});
           }
-          CKL(run_species_linear(sp, b, NL, s));
         }
+        CKL(run_species_linear(sp, b, NL, s));
       }
       {
         std::vector<LinSpec> sp;
@@ -1464,11 +1468,10 @@ struct Model : ModelBase {
         std::vector<LinSpec> sp;
         for (int l : p.out_ls)
           sp.push_back({lb.gh_out + (long long)l * l * C, (long long)p.Dout * C, C, 2 * l + 1, C, pre + "linT.l" + std::to_string(l),
-                        pre + "lin.l" + std::to_string(l), C, lb.gout + (long long)l * l * C, (long long)p.Dout * C, C, nullptr});
-        CKL(run_linear(sp, NL, s));
+                        pre + "lin.l" + std::to_string(l), C, lb.gout_s + (long long)l * l * C, (long long)p.Dout * C, C, nullptr});
+        CKL(run_linear(sp, NL, s, b.species_rank));
       }
       // through the per-species coefficients and the product basis, in species-sorted space
-      CKL(launch_gather_rows(lb.gout, b.species_perm, lb.gout_s, NL, p.Dout * C, s));
       if (bilinear) CKL(launch_fill_zero(lb.gXY, NL * D * 2 * C, s));
       else if ((int)p.out_ls.size() != L + 1) CKL(launch_fill_zero(lb.gAs, NL * D * C, s));
       {
@@ -1477,13 +1480,13 @@ struct Model : ModelBase {
           sp.push_back({lb.gout_s + (long long)l * l * C, (long long)p.Dout * C, C, 2 * l + 1, C, pre + "c0T.l" + std::to_string(l),
                         pre + "c0.l" + std::to_string(l), C, bilinear ? lb.gXY + (long long)l * l * 2 * C : lb.gAs + (long long)l * l * C,
                         (long long)D * C * (bilinear ? 2 : 1), (long long)C * (bilinear ? 2 : 1), nullptr, false, 0});
-        CKL(run_species_linear(sp, b, NL, s));
-        if (cfg.correlation >= 2) {
+        if (cfg.correlation < 2) {
+          CKL(run_species_linear(sp, b, NL, s));
+        } else {  // the gradients of every order's basis in the same launch
           // gradient of the second-order basis: written over B2 itself, or into gB2 when the third order still needs B2
           T* g2 = cfg.correlation >= 3 ? lb.gB2 : lb.B2;
           if (cfg.correlation >= 3) {
             CKL(launch_fill_zero(lb.gB2, NL * p.pb.NB * C, s));  // ranks above the output ranks only receive third-order terms
-            sp.clear();
             for (size_t i = 0; i < p.out_ls.size(); ++i) {
               const int l = p.out_ls[i];
               const int K = p.pb3.k[i] * C;
@@ -1491,9 +1494,7 @@ struct Model : ModelBase {
                             pre + "c2.l" + std::to_string(l), K, lb.B3 + (long long)p.pb3.base[i] * C, (long long)p.pb3.NB * C, K,
                             nullptr, false, 0});
             }
-            CKL(run_species_linear(sp, b, NL, s));  // B3 now holds its gradient
           }
-          sp.clear();
           for (size_t i = 0; i < p.out_ls.size(); ++i) {
             const int l = p.out_ls[i];
             const int K = p.pb.k[i] * C;
@@ -1501,7 +1502,7 @@ struct Model : ModelBase {
                           pre + "c1.l" + std::to_string(l), K, g2 + (long long)p.pb.base[i] * C, (long long)p.pb.NB * C, K, nullptr,
                           false, 0});
           }
-          CKL(run_species_linear(sp, b, NL, s));
+          CKL(run_species_linear(sp, b, NL, s));  // B2 (gB2) and B3 now hold their gradients
           if (cfg.correlation >= 3) {
             CKL(launch_pb3_bwd(lb.As, lb.B2, lb.B3, lb.gB2, lb.gAs, (int)NL, L, p.last ? -1 : Ln, C, s));
             ++launches;
@@ -1522,13 +1523,12 @@ struct Model : ModelBase {
           }
         }
       }
-      CKL(launch_scatter_rows(lb.gAs, b.species_perm, lb.gA, NL, D * C, s));
       {
         std::vector<LinSpec> sp;
         for (int l = 0; l <= L; ++l)
-          sp.push_back({lb.gA + (long long)l * l * C, (long long)D * C, C, 2 * l + 1, C, pre + "nlT.l" + std::to_string(l),
+          sp.push_back({lb.gAs + (long long)l * l * C, (long long)D * C, C, 2 * l + 1, C, pre + "nlT.l" + std::to_string(l),
                         pre + "nl.l" + std::to_string(l), C, lb.ga + (long long)l * l * C, (long long)D * C, C, nullptr});
-        CKL(run_linear(sp, NL, s));
+        CKL(run_linear(sp, NL, s, b.species_perm));  // back to atom order
       }
       CKL(launch_gate_bwd(lb.Gt, lb.ga, lb.gGt, (int)NL, L, C, m0, s));
       if (density)  // d / d density_i, and the gradient of the unscaled linear_down output
@@ -1681,6 +1681,11 @@ struct Model : ModelBase {
     for (const auto& d : debug) {
       if (d.name == name) {
         const long long n = d.numel < numel ? d.numel : numel;
+        if (d.perm) {
+          const long long rows = n / d.row;  // whole rows
+          if (launch_gather_rows(static_cast<const T*>(d.ptr), d.perm, static_cast<T*>(dst), rows, (int)d.row, s) != cudaSuccess) return TACE_ERR_CUDA;
+          return rows * d.row;
+        }
         if (cudaMemcpyAsync(dst, d.ptr, sizeof(T) * (size_t)n, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return TACE_ERR_CUDA;
         return n;
       }

@@ -24,7 +24,7 @@
 
 namespace tace {
 
-constexpr int kMaxProblems = 4;
+constexpr int kMaxProblems = 12;
 
 template <typename T>
 struct GemmProblem {

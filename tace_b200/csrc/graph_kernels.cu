@@ -82,7 +82,7 @@ struct EdgeSort {
 };
 struct SpeciesSort {
   const int* species; int n, n_el;
-  int *perm, *ptr, *tile_ptr, *tc_tile_ptr;
+  int *perm, *rank, *ptr, *tile_ptr, *tc_tile_ptr;  // rank: place of every atom in perm
 };
 constexpr int kCountThreads = 1024, kScanItems = 4, kScanBlock = 1024 * kScanItems;
 constexpr int kSpeciesBlockAtoms = 8192;  // up to here one block sorts the atoms by species beside the edge count
@@ -147,7 +147,11 @@ __device__ void species_block(const SpeciesSort& a, int* smem) {
       base[k] = b;
     }
     __syncthreads();
-    if (z >= 0) a.perm[hist[warp * n_el + z] + rank] = i;
+    if (z >= 0) {
+      const int at = hist[warp * n_el + z] + rank;
+      a.perm[at] = i;
+      a.rank[i] = at;
+    }
     __syncthreads();
     for (int k = tid; k < 32 * n_el; k += kCountThreads) hist[k] = 0;
     __syncthreads();
@@ -348,7 +352,12 @@ size_t graph_prep_temp_bytes(long long E, int n_atoms) {
 
 int graph_prep_launches(const GraphPrepArgs& a) {
   return 6 + (a.n_atoms >= kScanBlock ? 1 : 0) + (a.split_rows && a.n_local > 0 ? 2 : 0) +
-         (a.n_local > kSpeciesBlockAtoms || a.n_elements > kSpeciesBlockElements ? 3 : 0);
+         (a.n_local > kSpeciesBlockAtoms || a.n_elements > kSpeciesBlockElements ? 4 : 0);
+}
+
+__global__ void invert_kernel(const int* __restrict__ perm, int n, int* __restrict__ rank) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) rank[perm[i]] = i;
 }
 
 cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s) {
@@ -362,7 +371,7 @@ cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s) {
   es.block_sums = take(2 * (size_t)scan_blocks);
   es.rowptr_dst = a.rowptr_dst; es.rowptr_src = a.rowptr_src;
   es.e_src = a.e_src; es.e_dst = a.e_dst; es.e_orig = a.e_orig; es.perm_src = a.perm_src;
-  SpeciesSort sp{a.species, a.n_local, a.n_elements, a.species_perm, a.species_ptr, a.tile_ptr, a.tc_tile_ptr};
+  SpeciesSort sp{a.species, a.n_local, a.n_elements, a.species_perm, a.species_rank, a.species_ptr, a.tile_ptr, a.tc_tile_ptr};
   const bool small_species = a.n_local <= kSpeciesBlockAtoms && a.n_elements <= kSpeciesBlockElements;
 
   edge_sort_init_kernel<<<(a.n_atoms + 256) / 256, 256, 0, s>>>(es, a.graph_ptr, a.n_graphs, a.atom_graph);
@@ -401,6 +410,7 @@ cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s) {
     err = cub::DeviceRadixSort::SortPairs(cub_temp, cub_bytes, keys_in, keys_out, vals_in, a.species_perm, a.n_local, 0, sbits, s);
     if (err != cudaSuccess) return err;
     lower_bound_kernel<<<(a.n_elements + 256) / 256, 256, 0, s>>>(keys_out, a.n_local, a.species_ptr, a.n_elements);
+    invert_kernel<<<(a.n_local + 255) / 256, 256, 0, s>>>(a.species_perm, a.n_local, a.species_rank);
     tile_ptr_kernel<<<1, 256, 0, s>>>(a.species_ptr, a.n_elements, a.tile_ptr, a.tc_tile_ptr);
   }
   return cudaGetLastError();

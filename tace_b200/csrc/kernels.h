@@ -183,7 +183,6 @@ struct CopySegments {
 cudaError_t launch_copy_segments(const CopySegments& c, cudaStream_t s);
 // dst[i] = src[perm[i]] (gather) / dst[perm[i]] = src[i] (scatter), rows of row_len elements
 template <typename T> cudaError_t launch_gather_rows(const T* src, const int* perm, T* dst, long long n, int row_len, cudaStream_t s);
-template <typename T> cudaError_t launch_scatter_rows(const T* src, const int* perm, T* dst, long long n, int row_len, cudaStream_t s);
 template <typename T> cudaError_t launch_add_inplace(T* dst, const T* src, long long n, cudaStream_t s);
 // dst[i, :width] += src[i, :width], rows dst_stride / src_stride elements apart
 template <typename T> cudaError_t launch_add_rows(T* dst, long long dst_stride, const T* src, long long src_stride, long long n, int width,
@@ -272,6 +271,7 @@ struct GraphPrepArgs {
   int* perm_src; int* rowptr_src;       // [E], [n_atoms+1]
   int* atom_graph;            // [n_atoms]
   int* species_perm; int* species_ptr;  // [n_local], [n_elements+1]
+  int* species_rank;          // [n_local] place of every atom in species_perm
   int* tile_ptr;              // [4][n_elements+1] for q = 1,3,5,7: 32-row tiles per species
   int* tc_tile_ptr;           // [4][n_elements+1]: (128 / q)-atom tiles per species
   void* temp; size_t temp_bytes;
@@ -319,6 +319,7 @@ struct TeceArgs {
 int tece_wigner_stride(int L, int mmax);  // entries of one edge's packed Wigner rows (tece_kernels.cu)
 template <typename T> cudaError_t launch_tece(const TeceArgs<T>& a, int stage, cudaStream_t s);
 
+constexpr int kMaxLinears = 12;  // problems of one launch
 struct TcLinearProblem {
   const float* A; long long a_atom_stride, a_comp_stride;
   int q;                 // components per atom (2l+1), <= 128
@@ -334,6 +335,7 @@ struct TcLinearProblem {
   const int* group_ptr; const int* tile_ptr; const int* atom_map;
   long long b_group_stride, bias_group_stride;
   int accumulate;        // C += instead of C =
+  int join;              // the product is added to the problem before (same rows, N and groups), in one pass over both K ranges
   int b_tiled;           // Bhi / Blo are stored K-tile-major, [groups][K/32][N][32] (b_group_stride must be N*K)
 };
 bool tc_linear_supported(int N, int K);

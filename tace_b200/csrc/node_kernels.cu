@@ -64,17 +64,16 @@ cudaError_t launch_add_inplace(T* dst, const T* src, long long n, cudaStream_t s
 }
 
 // V: the row is moved in 16-byte pieces (uint4) when its length and both base addresses allow, else element by element.
-template <typename V, bool SCATTER>
-__global__ void permute_rows_kernel(const V* __restrict__ src, const int* __restrict__ perm, V* __restrict__ dst, long long n, int row_len) {
+template <typename V>
+__global__ void gather_rows_kernel(const V* __restrict__ src, const int* __restrict__ perm, V* __restrict__ dst, long long n, int row_len) {
   const long long total = n * row_len;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
     const long long i = idx / row_len, k = idx - i * row_len;
-    const long long j = perm[i];
-    if (SCATTER) dst[j * row_len + k] = src[idx]; else dst[idx] = src[j * row_len + k];
+    dst[idx] = src[(long long)perm[i] * row_len + k];
   }
 }
-template <typename T, bool SCATTER>
-cudaError_t launch_permute_rows(const T* src, const int* perm, T* dst, long long n, int row_len, cudaStream_t s) {
+template <typename T>
+cudaError_t launch_gather_rows(const T* src, const int* perm, T* dst, long long n, int row_len, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   constexpr int per = 16 / sizeof(T);
   const bool wide = row_len % per == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
@@ -82,18 +81,10 @@ cudaError_t launch_permute_rows(const T* src, const int* perm, T* dst, long long
   const long long blocks = (n * len + 255) / 256;
   const unsigned grid = (unsigned)(blocks < 148 * 32 ? blocks : 148 * 32);
   if (wide)
-    permute_rows_kernel<uint4, SCATTER><<<grid, 256, 0, s>>>(reinterpret_cast<const uint4*>(src), perm, reinterpret_cast<uint4*>(dst), n, len);
+    gather_rows_kernel<uint4><<<grid, 256, 0, s>>>(reinterpret_cast<const uint4*>(src), perm, reinterpret_cast<uint4*>(dst), n, len);
   else
-    permute_rows_kernel<T, SCATTER><<<grid, 256, 0, s>>>(src, perm, dst, n, len);
+    gather_rows_kernel<T><<<grid, 256, 0, s>>>(src, perm, dst, n, len);
   return cudaGetLastError();
-}
-template <typename T>
-cudaError_t launch_gather_rows(const T* src, const int* perm, T* dst, long long n, int row_len, cudaStream_t s) {
-  return launch_permute_rows<T, false>(src, perm, dst, n, row_len, s);
-}
-template <typename T>
-cudaError_t launch_scatter_rows(const T* src, const int* perm, T* dst, long long n, int row_len, cudaStream_t s) {
-  return launch_permute_rows<T, true>(src, perm, dst, n, row_len, s);
 }
 
 template <typename T>
@@ -660,7 +651,6 @@ __global__ void one_hot_kernel(const int* __restrict__ species, long long n, int
   template cudaError_t launch_readout_linear_bwd<T>(T*, long long, const T*, const T*, const int*, const int*, int, int, cudaStream_t); \
   template cudaError_t launch_add_inplace<T>(T*, const T*, long long, cudaStream_t);                          \
   template cudaError_t launch_gather_rows<T>(const T*, const int*, T*, long long, int, cudaStream_t);         \
-  template cudaError_t launch_scatter_rows<T>(const T*, const int*, T*, long long, int, cudaStream_t);        \
   template cudaError_t launch_species_gather<T>(const T*, const int*, T*, int, int, cudaStream_t);            \
   template cudaError_t launch_gate_fwd<T>(const T*, T*, int, int, int, int, cudaStream_t);                    \
   template cudaError_t launch_gate_bwd<T>(const T*, const T*, T*, int, int, int, int, cudaStream_t);          \

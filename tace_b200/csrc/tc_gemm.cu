@@ -120,13 +120,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 // One linear problem of a launch: C[(atom, m), :] = A[(atom, m), 0:K] @ B[0:N, 0:K]^T (+ bias).
 // Rows are (atom, component) pairs; the 3-D tensor map of A is {K, q, atoms} with box {32, q, R},
 // R = 128 / q atoms per tile, so a tile's rows land in shared memory in (atom, m) order.
-struct TcProblem {
+// Several products can share a result: their K ranges are walked one after the other in the same accumulators.
+struct TcSegment {
   CUtensorMap tmA, tmBhi, tmBlo;  // B maps are 3-D {K, N, groups}
+  int num_k;             // 32-wide K steps
+  int b_tiled;           // B maps are 4-D {32, N, K/32, groups} over K-tile-major weights
+};
+struct TcProblem {
   float* C;
   const float* bias;     // [N] (per group) or nullptr
   long long c_s1, c_s2;  // atom stride / component stride of C rows (elements)
   long long bias_group_stride;
-  int q, R, n_atoms, N, K;
+  int q, R, n_atoms, N;
+  int seg0, num_k;       // first of its segments, K steps of all of them
   // per-species problems: atoms are sorted by species, group g owns atoms [group_ptr[g], group_ptr[g+1]) and
   // R-atom tiles [tile_ptr[g], tile_ptr[g+1]); both arrays live in device memory.  n_groups == 0: one group.
   int n_groups;
@@ -134,11 +140,11 @@ struct TcProblem {
   const int* tile_ptr;
   const int* atom_map;   // row of C for sorted atom a is atom_map[a]; nullptr: identity
   int accumulate;        // C += instead of C =
-  int b_tiled;           // B maps are 4-D {32, N, K/32, groups} over K-tile-major weights
   int table;             // offset of its row pointers in the kernel's shared-memory tables, -1: read from global memory
 };
-constexpr int kTcMaxProblems = 4;
+constexpr int kTcMaxProblems = kMaxLinears;
 struct TcBatch {
+  TcSegment seg[kTcMaxProblems];
   TcProblem p[kTcMaxProblems];
   int n_problems;
   int tile_start[kTcMaxProblems + 1];  // prefix sum of the problems' tile counts
@@ -163,7 +169,7 @@ struct TcSmem {
   static constexpr int kThreads = 448, kSplitWarps = 4, kEpilogueThreads = 256;
   static constexpr int kTmemCols = 512;                  // accumulators [0, 2 BN) | per stage 32 columns high part, 32 residual
   static constexpr int kTmemA = 2 * BN;                  // first activation column
-  static constexpr int kBarrierBytes = 256;
+  static constexpr int kBarrierBytes = 256;  // and the tile counts of the problems
   // result staging: per epilogue warp sixteen rows x 32 columns, and the addresses of its 32 rows
   static constexpr int kStoreBytes = 8 * 16 * 128, kRowBytes = 8 * 32 * 8;
   // row pointers of the species and tile tables of the grouped problems, copied in once (a tile is found by a search over them)
@@ -247,7 +253,7 @@ __device__ __forceinline__ TileInfo decode_tile(const TcBatch& b, const int* til
   TileInfo t;
   t.prob = pi;
   t.n0 = (local - mt * tiles_n) * BN;
-  t.num_k = P.K / kBK;
+  t.num_k = P.num_k;
   if (P.n_groups > 0) {
     const int* tile_ptr = P.table >= 0 ? tables + P.table : P.tile_ptr;
     const int* group_ptr = P.table >= 0 ? tables + P.table + P.n_groups + 1 : P.group_ptr;
@@ -343,17 +349,20 @@ __global__ void __launch_bounds__(TcSmem<BN>::kThreads, 1) tc_gemm_kernel(const 
         const TileInfo t = decode_tile<BN>(batch, tile_start, tables, tile);
         const TcProblem& P = batch.p[t.prob];
         const uint32_t a_bytes = (uint32_t)P.R * P.q * kBK * 4;
-        for (int ks = 0; ks < t.num_k; ++ks, ++step) {
+        const TcSegment* G = &batch.seg[P.seg0];
+        int left = G->num_k, ks = 0;  // K steps left in the segment, position in it
+        for (int k = 0; k < t.num_k; ++k, ++ks, --left, ++step) {
+          if (left == 0) { ++G; left = G->num_k; ks = 0; }
           const int s = step % kStages, ph = (step / kStages) & 1;
           if (!mbar_wait(empty_bar(s), ph ^ 1, abort_flag, batch.error, 1, batch.spin_limit)) { ok = false; break; }
           mbar_expect_tx(raw_bar(s), a_bytes + 2 * S::kTileBBytes + batch.extra_tx);
-          tma_load_3d(stage_a(s), &P.tmA, raw_bar(s), ks * kBK, 0, t.atom0);
-          if (P.b_tiled) {  // weights stored K-tile-major: one contiguous block per (k-step, n-tile)
-            tma_load_4d(stage_bhi(s), &P.tmBhi, raw_bar(s), 0, t.n0, ks, t.group);
-            tma_load_4d(stage_blo(s), &P.tmBlo, raw_bar(s), 0, t.n0, ks, t.group);
+          tma_load_3d(stage_a(s), &G->tmA, raw_bar(s), ks * kBK, 0, t.atom0);
+          if (G->b_tiled) {  // weights stored K-tile-major: one contiguous block per (k-step, n-tile)
+            tma_load_4d(stage_bhi(s), &G->tmBhi, raw_bar(s), 0, t.n0, ks, t.group);
+            tma_load_4d(stage_blo(s), &G->tmBlo, raw_bar(s), 0, t.n0, ks, t.group);
           } else {
-            tma_load_3d(stage_bhi(s), &P.tmBhi, raw_bar(s), ks * kBK, t.n0, t.group);
-            tma_load_3d(stage_blo(s), &P.tmBlo, raw_bar(s), ks * kBK, t.n0, t.group);
+            tma_load_3d(stage_bhi(s), &G->tmBhi, raw_bar(s), ks * kBK, t.n0, t.group);
+            tma_load_3d(stage_blo(s), &G->tmBlo, raw_bar(s), ks * kBK, t.n0, t.group);
           }
         }
       }
@@ -606,14 +615,24 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
     return cudaErrorInvalidValue;
   const int sms = sms_of[dev];
   bool all128 = true, one = true;
+  int first[kTcMaxProblems + 1], n_results = 0, steps_of[kTcMaxProblems];  // results: runs of problems joined to their first one
   for (int i = 0; i < n_problems; ++i) {
     const TcLinearProblem& h = probs[i];
     if (!tc_linear_supported(h.N, h.K) || h.q < 1 || h.q > 128 || (h.a_atom_stride & 3) || (h.a_comp_stride & 3) || (h.c_s1 & 3) ||
         (h.c_s2 & 3))
       return cudaErrorInvalidValue;
+    if (h.join) {
+      if (i == 0 || h.q != probs[i - 1].q || h.N != probs[i - 1].N || h.n_atoms != probs[i - 1].n_atoms || h.n_groups != probs[i - 1].n_groups)
+        return cudaErrorInvalidValue;
+      steps_of[n_results - 1] += h.K / kBK;
+    } else {
+      first[n_results] = i;
+      steps_of[n_results++] = h.K / kBK;
+    }
     all128 = all128 && (h.N % 128 == 0);
-    one = one && (h.K / kBK <= kChunk);
   }
+  first[n_results] = n_problems;
+  for (int i = 0; i < n_results; ++i) one = one && steps_of[i] <= kChunk;
   const int bn = all128 ? 128 : 64;
   TcBatch b;
   memset(&b, 0, sizeof(b));
@@ -623,31 +642,40 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
   b.extra_tx = g_test_extra_tx;
   // long K loops first: tiles are dealt round robin, and the short ones fill what the long ones leave of the last round
   int order[kTcMaxProblems];
-  for (int i = 0; i < n_problems; ++i) {
+  for (int i = 0; i < n_results; ++i) {
     int j = i;
-    for (; j > 0 && probs[order[j - 1]].K < probs[i].K; --j) order[j] = order[j - 1];
+    for (; j > 0 && steps_of[order[j - 1]] < steps_of[i]; --j) order[j] = order[j - 1];
     order[j] = i;
   }
-  int tiles = 0, table = 0;
-  for (int i = 0; i < n_problems; ++i) {
-    const TcLinearProblem& h = probs[order[i]];
+  int tiles = 0, table = 0, segs = 0;
+  for (int i = 0; i < n_results; ++i) {
+    const TcLinearProblem& h = probs[first[order[i]]];
     if (h.n_atoms <= 0) continue;
     TcProblem& P = b.p[b.n_problems];
-    P.q = h.q; P.R = kBM / h.q; P.n_atoms = (int)h.n_atoms; P.N = h.N; P.K = h.K;
+    P.q = h.q; P.R = kBM / h.q; P.n_atoms = (int)h.n_atoms; P.N = h.N;
     P.C = h.C; P.bias = h.bias; P.c_s1 = h.c_s1; P.c_s2 = h.c_s2; P.bias_group_stride = h.bias_group_stride;
     P.n_groups = h.n_groups; P.group_ptr = h.group_ptr; P.tile_ptr = h.tile_ptr; P.atom_map = h.atom_map;
     P.accumulate = h.accumulate;
     P.table = -1;
-    if (h.n_groups > 0 && table + 2 * (h.n_groups + 1) <= TcSmem<128>::kTableInts) { P.table = table; table += 2 * (h.n_groups + 1); }
+    for (int k = 0; k < b.n_problems && h.n_groups > 0; ++k)  // the tables of an earlier problem
+      if (b.p[k].n_groups == h.n_groups && b.p[k].tile_ptr == h.tile_ptr && b.p[k].group_ptr == h.group_ptr) P.table = b.p[k].table;
+    if (h.n_groups > 0 && P.table < 0 && table + 2 * (h.n_groups + 1) <= TcSmem<128>::kTableInts) { P.table = table; table += 2 * (h.n_groups + 1); }
     const int groups = h.n_groups > 0 ? h.n_groups : 1;
     if (h.n_groups > 0 && (!h.group_ptr || !h.tile_ptr)) return cudaErrorInvalidValue;
-    P.b_tiled = h.b_tiled;
-    if (h.b_tiled && groups > 1 && h.b_group_stride != (long long)h.N * h.K) return cudaErrorInvalidValue;
-    if (!make_map_3d(&P.tmA, h.A, h.n_atoms, h.q, h.K, h.a_atom_stride, h.a_comp_stride, P.R)) return cudaErrorInvalidValue;
-    if (h.b_tiled ? (!make_map_b_tiled(&P.tmBhi, h.Bhi, groups, h.N, h.K, bn) || !make_map_b_tiled(&P.tmBlo, h.Blo, groups, h.N, h.K, bn))
-                  : (!make_map_b(&P.tmBhi, h.Bhi, groups, h.N, h.K, h.b_group_stride, bn) ||
-                     !make_map_b(&P.tmBlo, h.Blo, groups, h.N, h.K, h.b_group_stride, bn)))
-      return cudaErrorInvalidValue;
+    P.seg0 = segs;
+    for (int k = first[order[i]]; k < first[order[i] + 1]; ++k) {
+      const TcLinearProblem& g = probs[k];
+      TcSegment& G = b.seg[segs++];
+      G.num_k = g.K / kBK;
+      G.b_tiled = g.b_tiled;
+      P.num_k += G.num_k;
+      if (g.b_tiled && groups > 1 && g.b_group_stride != (long long)g.N * g.K) return cudaErrorInvalidValue;
+      if (!make_map_3d(&G.tmA, g.A, g.n_atoms, g.q, g.K, g.a_atom_stride, g.a_comp_stride, P.R)) return cudaErrorInvalidValue;
+      if (g.b_tiled ? (!make_map_b_tiled(&G.tmBhi, g.Bhi, groups, g.N, g.K, bn) || !make_map_b_tiled(&G.tmBlo, g.Blo, groups, g.N, g.K, bn))
+                    : (!make_map_b(&G.tmBhi, g.Bhi, groups, g.N, g.K, g.b_group_stride, bn) ||
+                       !make_map_b(&G.tmBlo, g.Blo, groups, g.N, g.K, g.b_group_stride, bn)))
+        return cudaErrorInvalidValue;
+    }
     b.tile_start[b.n_problems] = tiles;
     tiles += (int)((h.n_atoms + P.R - 1) / P.R + h.n_groups) * (h.N / bn);
     ++b.n_problems;
