@@ -14,7 +14,7 @@
 // 16 through a ring of three cp.async stages.  The tiles are small because the systems are (a 256-atom cell has 2 304 rows in
 // all ranks of a linear together: 144 tiles for 148 SMs), and what bound the former 64 x 64 CUDA-core tiles was one block per
 // four SMs walking its K loop with nothing in flight: K = N = 64 on those rows 18 -> 5 us, the 10 944 x 704 x 64 GEMMs of the
-// radial MLP 139 / 255 -> 43 / 41 us.
+// radial MLP 139 / 255 -> 48 / 45 us.
 // FP32 shapes that the tcgen05 kernel does not take: CUDA cores, 32 x 64 x 16 tiles, 256 threads, 2 x 4 outputs per thread.
 #pragma once
 #include <cuda_runtime.h>
