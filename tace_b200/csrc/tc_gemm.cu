@@ -133,6 +133,7 @@ struct TcProblem {
   long long bias_group_stride;
   int q, R, n_atoms, N;
   int seg0, num_k;       // first of its segments, K steps of all of them
+  int row_tiles;         // of a plain problem
   // per-species problems: atoms are sorted by species, group g owns atoms [group_ptr[g], group_ptr[g+1]) and
   // R-atom tiles [tile_ptr[g], tile_ptr[g+1]); both arrays live in device memory.  n_groups == 0: one group.
   int n_groups;
@@ -141,12 +142,13 @@ struct TcProblem {
   const int* atom_map;   // row of C for sorted atom a is atom_map[a]; nullptr: identity
   int accumulate;        // C += instead of C =
   int table;             // offset of its row pointers in the kernel's shared-memory tables, -1: read from global memory
+  int copy_table;        // not yet copied for an earlier problem
 };
 constexpr int kTcMaxProblems = kMaxLinears;
 struct TcBatch {
   TcSegment seg[kTcMaxProblems];
   TcProblem p[kTcMaxProblems];
-  int n_problems;
+  int n_problems, n_segments;
   int tile_start[kTcMaxProblems + 1];  // prefix sum of the problems' tile counts
   int* error;
   uint32_t spin_limit;   // polls per wait before a role gives up (kSpinLimit; smaller in the test mode)
@@ -187,6 +189,9 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z, int w) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
@@ -300,27 +305,39 @@ __global__ void __launch_bounds__(TcSmem<BN>::kThreads, 1) tc_gemm_kernel(const 
   int* tile_start = reinterpret_cast<int*>(misc + 16);  // [n_problems + 1]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = 0; i < batch.n_problems; ++i) {
-    const TcProblem& P = batch.p[i];
-    if (P.n_groups > 0 && P.table >= 0)
-      for (int k = tid; k <= P.n_groups; k += S::kThreads) {
-        tables[P.table + k] = P.tile_ptr[k];
-        tables[P.table + P.n_groups + 1 + k] = P.group_ptr[k];
-      }
+  // The prologue is a third of a launch with one tile per SM (5.3 us for 288 rows of K = N = 64), so its parts run side by side:
+  // warp 0 counts the tiles, a lane per problem, and has the tensor maps fetched; warp 1 allocates; warp 2 sets the barriers up;
+  // the others copy the tables.
+  if (warp == 0) {
+    const TcProblem& P = batch.p[lane < batch.n_problems ? lane : 0];
+    int count = 0;
+    if (lane < batch.n_problems) count = (P.n_groups > 0 ? P.tile_ptr[P.n_groups] : P.row_tiles) * (P.N / BN);
+    int sum = count;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
+    }
+    if (lane <= kTcMaxProblems) tile_start[lane] = sum - count;  // past the last problem: the total
+    for (int m = lane; m < 3 * batch.n_segments; m += 32) {
+      const TcSegment& G = batch.seg[m / 3];
+      prefetch_map(m % 3 == 0 ? &G.tmA : m % 3 == 1 ? &G.tmBhi : &G.tmBlo);
+    }
   }
-  if (tid == 0) {  // `ready` takes one arrival per splitter warp
+  if (warp > 2)
+    for (int i = 0; i < batch.n_problems; ++i) {
+      const TcProblem& P = batch.p[i];
+      if (P.n_groups > 0 && P.copy_table)
+        for (int k = tid - 96; k <= P.n_groups; k += S::kThreads - 96) {
+          tables[P.table + k] = P.tile_ptr[k];
+          tables[P.table + P.n_groups + 1 + k] = P.group_ptr[k];
+        }
+    }
+  if (tid == 64) {  // `ready` takes one arrival per splitter warp
     for (int s = 0; s < kStages; ++s) { mbar_init(raw_bar(s), 1); mbar_init(ready_bar(s), S::kSplitWarps); mbar_init(empty_bar(s), 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), S::kEpilogueThreads); }
     mbar_init(drain_bar, 1);
     *abort_flag = 0;
-    int acc = 0;
-    for (int i = 0; i < batch.n_problems; ++i) {
-      const TcProblem& P = batch.p[i];
-      tile_start[i] = acc;
-      const int tiles_m = P.n_groups > 0 ? P.tile_ptr[P.n_groups] : (P.n_atoms + P.R - 1) / P.R;
-      acc += tiles_m * (P.N / BN);
-    }
-    for (int i = batch.n_problems; i <= kTcMaxProblems; ++i) tile_start[i] = acc;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {  // two accumulators of BN fp32 columns
@@ -659,7 +676,7 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
     P.table = -1;
     for (int k = 0; k < b.n_problems && h.n_groups > 0; ++k)  // the tables of an earlier problem
       if (b.p[k].n_groups == h.n_groups && b.p[k].tile_ptr == h.tile_ptr && b.p[k].group_ptr == h.group_ptr) P.table = b.p[k].table;
-    if (h.n_groups > 0 && P.table < 0 && table + 2 * (h.n_groups + 1) <= TcSmem<128>::kTableInts) { P.table = table; table += 2 * (h.n_groups + 1); }
+    if (h.n_groups > 0 && P.table < 0 && table + 2 * (h.n_groups + 1) <= TcSmem<128>::kTableInts) { P.table = table; P.copy_table = 1; table += 2 * (h.n_groups + 1); }
     const int groups = h.n_groups > 0 ? h.n_groups : 1;
     if (h.n_groups > 0 && (!h.group_ptr || !h.tile_ptr)) return cudaErrorInvalidValue;
     P.seg0 = segs;
@@ -677,9 +694,11 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
         return cudaErrorInvalidValue;
     }
     b.tile_start[b.n_problems] = tiles;
-    tiles += (int)((h.n_atoms + P.R - 1) / P.R + h.n_groups) * (h.N / bn);
+    P.row_tiles = (int)((h.n_atoms + P.R - 1) / P.R);
+    tiles += (P.row_tiles + h.n_groups) * (h.N / bn);
     ++b.n_problems;
   }
+  b.n_segments = segs;
   for (int i = b.n_problems; i <= kTcMaxProblems; ++i) b.tile_start[i] = tiles;
   if (tiles == 0) return cudaSuccess;
   if (bn == 128) return one ? launch_tc<128, true>(b, dev, sms, s) : launch_tc<128, false>(b, dev, sms, s);
