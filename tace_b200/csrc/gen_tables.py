@@ -435,6 +435,8 @@ def gen_interaction_wide(L, Lin, out, paths, lay, Ks, xoff):
                 for m1 in range(2 * l1 + 1):
                     o(f"      F2 d{l1}_{m1}[NV]; {V} d{l1}_{m1}[v] = F2{{0.0f, 0.0f}};")
         o(f"      F2 w{p}[NV]; wf.template get<{ip}>(w{p});")
+        if scalar_src:  # one source component: weighted once per path instead of every row of the message gradient
+            o(f"      {V} w{p}[v] = mul2(w{p}[v], x{l1}_0[v]);")
         started = set()
         for m3 in range(2 * l3 + 1):
             used = [m1 for m1 in range(2 * l1 + 1) if (p, m1, m3) in gi]
@@ -448,9 +450,12 @@ def gen_interaction_wide(L, Lin, out, paths, lay, Ks, xoff):
                 else:
                     started.add(m1)
                     o(f"      F2 u{p}_{m1}[NV]; {V} u{p}_{m1}[v] = mul2s({e}, g{p}_{m3}[v]);")
-            o(f"      F2 h{p}_{m3}[NV]; {V} h{p}_{m3}[v] = mul2(w{p}[v], g{p}_{m3}[v]);")
-            for m1 in used:
-                o(f"      const float t{p}_{m1}_{m3} = dot2<NV>(x{l1}_{m1}, h{p}_{m3});")
+            if scalar_src:
+                o(f"      const float t{p}_0_{m3} = dot2<NV>(w{p}, g{p}_{m3});")
+            else:
+                o(f"      F2 h{p}_{m3}[NV]; {V} h{p}_{m3}[v] = mul2(w{p}[v], g{p}_{m3}[v]);")
+                for m1 in used:
+                    o(f"      const float t{p}_{m1}_{m3} = dot2<NV>(x{l1}_{m1}, h{p}_{m3});")
             for m2 in range(2 * l2 + 1):
                 for m1 in used:
                     if K[m1, m2, m3] != 0.0:

@@ -11,7 +11,7 @@
 //
 // Measured against one channel per thread, on B200 at rank 3, 128 channels, 2 407 targets, 150 400 edges: backward 1.51 -> 1.04 ms
 // (FMA pipe 62 % busy, L1 68 % of its wavefronts), forward 0.80 -> 0.54 ms (L1 81 %: per edge 368 wavefronts of table, 320 of
-// coupling rows, 64 of source rows), scalar source 0.29 -> 0.15 and 0.11 -> 0.08 ms; rank 2, 64 channels, 131 072 targets,
+// coupling rows, 64 of source rows), scalar source forward 0.11 -> 0.08 ms; rank 2, 64 channels, 131 072 targets,
 // 5.5 M edges: 10.4 -> 7.2 and 5.1 -> 3.9 ms; 32 targets of 42 edges: 51 -> 10 and 31 -> 13 us.
 #include <cstdint>
 #include "kernels.h"
@@ -261,7 +261,7 @@ __global__ void __maxnreg__(168) tp_fwd_wide_kernel(const TPArgs<float> a) {
 template <typename TP, int NV, int C>
 struct WideBwdShape {
   static constexpr int CW = C / (64 * NV);       // warps per edge
-  static constexpr int kWarps = CW > 1 && TP::NX > 1 ? 8 : 4, EW = kWarps / CW;  // edges in flight per block
+  static constexpr int kWarps = CW > 1 ? 8 : 4, EW = kWarps / CW;  // edges in flight per block
   static constexpr int NRED = TP::D + 2;          // dY | dE/d(length) | dE/d(envelope)
   static constexpr int kMsgFloats = TP::NM * C, kGFloats = kWideBatch * TP::GVS, kRedFloats = CW > 1 ? kWideBatch * CW * NRED : 0;
   static constexpr int kBytes = (kMsgFloats + kGFloats + kRedFloats) * 4;
@@ -357,7 +357,7 @@ __device__ __forceinline__ void wide_bwd_row(const TPArgs<float>& a, int i, unsi
     for (int e = ew; e < nb; e += S::EW) {
       WideRow<NV, C> xs;
       xs.x = a.x + (long long)esrc[e] * (TP::NX * C) + c0 + lane;
-      if constexpr (TP::NX > 1) xs.dx = a.dxe + (long long)(e0 + e - a.e_base) * (TP::NX * C) + c0 + lane;
+      xs.dx = a.dxe + (long long)(e0 + e - a.e_base) * (TP::NX * C) + c0 + lane;
       wf.row = wf.row_next;
       wf.row_next = table + (long long)ek[e + S::EW < nb ? e + S::EW : e] * ROW;
       wf.t = et[e];
@@ -429,6 +429,112 @@ __global__ void __maxnreg__(128) tp_bwd_wide_kernel(const TPArgs<float> a) {
   }
 }
 
+// ---- backward, scalar source (the first interaction) --------------------------------------------------------------------
+// The message gradient of a target is D rows only, so a warp keeps it in registers over the edges it works on, for all of its C
+// channels, and nothing but the sums over the channels remains to be exchanged: the D - 1 derivatives that count (that of Y_00
+// does not, sh_grad), dE/d(length) and dE/d(envelope) leave one halving exchange together.  No barrier; lane e of a batch
+// builds edge e's coupling row, the next edge's source row is on its way. Shares of a target's edges go to neighbouring warps.
+// With the gradient rows in shared memory, two warps per edge at 128 channels and two exchanges, the LSU was 73 % busy with them;
+// what is left are the table entries.  Rank 2, 64 channels, 5.5 M edges: 2.82 -> 1.94 ms; rank 3, 64 channels, 1 372 targets of 42 edges:
+// 47 -> 36 us; rank 3, 128 channels, 2.8 M edges: 2.56 -> 2.16 ms, 150 400 edges: 148 -> 125 us.
+template <int NV, int D>
+struct WideMsgRegs {
+  F2 g[D][NV];
+  template <int K> __device__ __forceinline__ void load(F2 (&r)[NV]) const {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) r[v] = g[K][v];
+  }
+};
+template <int NV>
+struct WideRowRegs {
+  F2 x[NV];
+  template <int K> __device__ __forceinline__ void load(F2 (&r)[NV]) const {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) r[v] = x[v];
+  }
+};
+template <typename TP, int C, bool ENV>
+__global__ void __launch_bounds__(128, C == 64 ? 5 : 3) tp_bwd_scalar_wide_kernel(const TPArgs<float> a, int shares) {
+  static_assert(TP::NX == 1 && TP::NM == TP::D, "one source component, one path per rank");
+  constexpr int NV = C / 64, D = TP::D, ROW = 4 * C * TP::NP, NSUM = D + (ENV && D < 16 ? 1 : 0);
+  __shared__ __align__(16) float coupling[4][kWideBatch * TP::GVS];
+  __shared__ __align__(16) float4 meta[4][kWideBatch];  // source, table interval, place in it, envelope
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int unit = blockIdx.x * 4 + warp, i = unit / shares, share = unit - i * shares;
+  if (i >= a.n_seg) return;
+  int beg = a.rowptr[i], end = a.rowptr[i + 1];
+  const int deg = end - beg, lo = beg + deg * share / shares;
+  end = beg + deg * (share + 1) / shares;
+  beg = lo;
+  if (beg >= end) return;
+  WideMsgRegs<NV, D> gm;
+  const float* gMi = a.gM + (long long)i * (D * C) + lane;
+#pragma unroll
+  for (int k = 0; k < D; ++k)
+#pragma unroll
+    for (int v = 0; v < NV; ++v) gm.g[k][v] = F2{gMi[k * C + 64 * v], gMi[k * C + 64 * v + 32]};
+  float* Gs = coupling[warp];
+  float4* ms = meta[warp];
+  const float* table = a.rtab + 4 * lane;
+  auto load_x = [&](int src, WideRowRegs<NV>& x) {
+    const float* p = a.x + (long long)src * C + lane;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) x.x[v] = F2{__ldg(p + 64 * v), __ldg(p + 64 * v + 32)};
+  };
+  for (int e0 = beg; e0 < end; e0 += kWideBatch) {
+    const int nb = min(kWideBatch, end - e0);
+    __syncwarp();
+    if (lane < nb) {
+      int k;
+      float t, u = 1.0f;
+      interval_of(a, a.dlen[e0 + lane], k, t);
+      if constexpr (ENV) u = a.env[e0 + lane];
+      ms[lane] = make_float4(__int_as_float(a.e_src[e0 + lane]), __int_as_float(k), t, u);
+      float y[D];
+      load_Y<D>(a.Y, e0 + lane, y);
+      TP::template build_v<0>(y, Gs + lane * TP::GVS);
+    }
+    __syncwarp();
+    WideWeights<TP, 0, TP::NP, NV, C, ENV, true, (NV == 1 ? TP::NP : 2)> wf;
+    WideRowRegs<NV> xn;
+    float4 m = ms[0];
+    load_x(__float_as_int(m.x), xn);
+    wf.row_next = table + (long long)__float_as_int(m.y) * ROW;
+    wf.start(wf.row_next);
+    for (int e = 0; e < nb; ++e) {
+      const float4 mn = ms[e + 1 < nb ? e + 1 : e];
+      WideRowRegs<NV> xs = xn;
+      load_x(__float_as_int(mn.x), xn);
+      wf.row = wf.row_next;
+      wf.row_next = table + (long long)__float_as_int(mn.y) * ROW;
+      wf.t = m.z;
+      if constexpr (ENV) wf.u = m.w;
+      m = mn;
+      wf.dr = F2{0.0f, 0.0f};
+      wf.du = F2{0.0f, 0.0f};
+      float dY[D], sum[NSUM];
+#pragma unroll
+      for (int k = 0; k < D; ++k) dY[k] = 0.0f;
+      TP::template bwd_v<NV>(xs, gm, Gs + e * TP::GVS, wf, dY);
+#pragma unroll
+      for (int k = 1; k < D; ++k) sum[k] = dY[k];
+      sum[0] = (wf.dr.x + wf.dr.y) * (ENV ? wf.u * a.rt_inv_h : a.rt_inv_h);
+      float du = wf.du.x + wf.du.y;
+      if constexpr (NSUM > D) sum[D] = du;
+      else if constexpr (ENV) du = wide_warp_sum(du);
+      int k;
+      const float v = wide_warp_sums<NSUM>(sum, lane, k);
+      float* dst = k == 0 ? a.ddlen + (e0 + e) : a.dY + (long long)(e0 + e) * D + k;
+      bool add = k == 0 ? a.accumulate_ddlen : a.accumulate_dY;
+      if constexpr (NSUM > D) { if (k == D) { dst = a.denv + (e0 + e); add = a.accumulate_denv; } }
+      if (k < NSUM) *dst = add ? *dst + v : v;
+      if constexpr (ENV && NSUM == D) {
+        if (lane == 31) { float* de = a.denv + (e0 + e); *de = a.accumulate_denv ? *de + du : du; }
+      }
+    }
+  }
+}
+
 // ---- launchers ----------------------------------------------------------------------------------------------------
 constexpr int kWideMaxDevices = 64;
 
@@ -482,7 +588,16 @@ cudaError_t launch_wide_bwd_k(const TPArgs<float>& a, cudaStream_t s) {
 }
 template <typename TP, int C, bool ENV>
 cudaError_t launch_wide_bwd(const TPArgs<float>& a, cudaStream_t s) {
-  return a.row_ids ? launch_wide_bwd_k<TP, 1, C, ENV, true>(a, s) : launch_wide_bwd_k<TP, 1, C, ENV, false>(a, s);
+  if constexpr (TP::NX == 1) {
+    if (a.row_ids) return cudaErrorInvalidValue;  // partial passes exist where source features are exchanged, not here
+    // Shares per target: enough warps for three rounds of what the chip holds, while a share keeps at least eight edges.
+    int shares = 1;
+    while ((long long)a.n_seg * shares < 3 * 148 * 16 && a.n_edges >= 16LL * shares * a.n_seg && shares < 16) shares *= 2;
+    tp_bwd_scalar_wide_kernel<TP, C, ENV><<<(unsigned)(((long long)a.n_seg * shares + 3) / 4), 128, 0, s>>>(a, shares);
+    return cudaGetLastError();
+  } else {
+    return a.row_ids ? launch_wide_bwd_k<TP, 1, C, ENV, true>(a, s) : launch_wide_bwd_k<TP, 1, C, ENV, false>(a, s);
+  }
 }
 template <typename TP>
 cudaError_t wide_fwd_t(const TPArgs<float>& a, cudaStream_t s) {
