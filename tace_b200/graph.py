@@ -4,6 +4,7 @@
 
 from __future__ import annotations
 
+import functools
 import math
 from typing import Dict, Sequence
 
@@ -11,18 +12,28 @@ import numpy as np
 import torch
 
 from . import lib as _lib
-from .neighbour_list import _list_on_device, complete_cell
+from .neighbour_list import _list_at, complete_cell
+
+
+@functools.lru_cache(maxsize=16)
+def _element_table(model_numbers: tuple) -> np.ndarray:
+    table = np.full(max(max(model_numbers), 118) + 1, -1, dtype=np.int64)
+    for i, z in enumerate(sorted(model_numbers)):
+        table[z] = i
+    return table
 
 
 def z_to_index(atomic_numbers: Sequence[int], model_numbers: Sequence[int]) -> np.ndarray:
     """tace/dataset/element.py:41-61 (TorchElement.z2idx): position of each Z in the sorted element list."""
-    table = np.full(max(max(model_numbers), int(np.max(atomic_numbers))) + 1, -1, dtype=np.int64)
-    for i, z in enumerate(sorted(model_numbers)):
-        table[z] = i
-    idx = table[np.asarray(atomic_numbers, dtype=np.int64)]
-    if (idx < 0).any():
-        raise ValueError("structure contains an element the model was not built for")
-    return idx
+    table = _element_table(tuple(map(int, model_numbers)))
+    numbers = np.asarray(atomic_numbers, dtype=np.int64)
+    if len(numbers) and numbers.max() < len(table):
+        idx = table[numbers]
+        if idx.min() >= 0:
+            return idx
+    elif len(numbers) == 0:
+        return numbers
+    raise ValueError("structure contains an element the model was not built for")
 
 
 def build_batch(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cutoff: float, dtype: torch.dtype,
@@ -42,18 +53,13 @@ def build_batch(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cuto
         cells = np.stack([complete_cell(c, positions[a:b], p, cutoff)
                           for c, p, a, b in zip(lattice_host, pbc_host, ptr_host[:-1], ptr_host[1:])])
     species_host = np.asarray(batch["species"]) if "species" in batch else z_to_index(np.asarray(batch["atomic_numbers"]), model_numbers)
-    real = np.float64 if dtype == torch.float64 else np.float32
     n, b = len(positions), len(lattice_host)
-    fields = [("pos64", positions, np.float64, (n, 3)), ("cells", cells, np.float64, (b, 3, 3)),
-              ("ptr", ptr_host, np.int64, (b + 1,)), ("batch", np.asarray(batch["batch"]), np.int64, (n,)),
-              ("positions", positions, real, (n, 3)), ("lattice", lattice_host, real, (b, 3, 3)),
-              ("ptr32", ptr_host, np.int32, (b + 1,)), ("species", species_host, np.int32, (n,)), ("pbc", pbc_host, np.uint8, (b, 3))]
-    up = _upload(fields, device)
-    pos64 = up["pos64"]
-    edge_index, shifts = _list_on_device(pos64, up["cells"], up["pbc"], up["ptr32"], cutoff, -1, dtype)
+    up, at = _upload(n, b, np.float64 if dtype == torch.float64 else np.float32,
+                     (positions, cells, ptr_host, batch["batch"], positions, lattice_host, ptr_host, species_host, pbc_host), device)
+    edge_index, shifts = _list_at(device, n, b, (at["pos64"], at["cells"], at["pbc"], at["ptr32"]), cutoff, -1, dtype)
     node_attrs = torch.empty(n, n_el, dtype=dtype, device=device)
     with _lib.on_device(device):
-        _lib.check(_lib.load().tace_one_hot(up["species"].data_ptr(), n, n_el, _lib.dtype_code(dtype), node_attrs.data_ptr(),
+        _lib.check(_lib.load().tace_one_hot(at["species"], n, n_el, _lib.dtype_code(dtype), node_attrs.data_ptr(),
                                             _lib.stream_of(device)), "tace_one_hot")
     return {
         "positions": up["positions"],
@@ -70,27 +76,43 @@ def build_batch(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cuto
 _STAGED_BYTES = 1 << 20  # up to here the fields travel as one block; above, the copy into the block costs more than the transfers it saves
 
 
-def _upload(fields, device: torch.device) -> Dict[str, torch.Tensor]:
-    """Host fields (name, values, type, shape) on the device.  A small batch is packed into one pinned block, every field at a
-    multiple of 16 bytes and already in its final type: one transfer instead of one transfer and one conversion kernel per
-    field (nine fields of a 32-atom cell: 150 us of host work before, 35 us now).  The pinned block comes from torch's caching
-    host allocator, which keeps it until the transfer has finished."""
+@functools.lru_cache(maxsize=64)
+def _layout(n: int, b: int, real):
+    """Places of the fields of ``n`` atoms in ``b`` structures in one block: (name, type, shape, offset) of each, and the size."""
     at, places = 0, []
-    for _, _, kind, shape in fields:
-        size = math.prod(shape)
-        places.append((at, at + size * _BYTES[kind]))
-        at += (size * _BYTES[kind] + 15) & ~15
-    if at > _STAGED_BYTES:
-        return {name: torch.as_tensor(values).to(device, non_blocking=True).to(_TORCH[kind]).reshape(shape).contiguous()
-                for name, values, kind, shape in fields}
-    block = torch.empty(max(at, 16), dtype=torch.uint8, pin_memory=True)
+    for name, kind, shape in (("pos64", np.float64, (n, 3)), ("cells", np.float64, (b, 3, 3)), ("ptr", np.int64, (b + 1,)),
+                              ("batch", np.int64, (n,)), ("positions", real, (n, 3)), ("lattice", real, (b, 3, 3)),
+                              ("ptr32", np.int32, (b + 1,)), ("species", np.int32, (n,)), ("pbc", np.uint8, (b, 3))):
+        places.append((name, kind, shape, at))
+        at += (math.prod(shape) * _BYTES[kind] + 15) & ~15
+    return tuple(places), at
+
+
+_RETURNED = ("batch", "ptr", "positions", "lattice", "species")  # fields of the model's input; the others only go to the list kernels
+
+
+def _upload(n: int, b: int, real, values, device: torch.device):
+    """Host values (in the order of ``_layout``) on the device: (tensors, addresses) by name.  A small batch is packed into one
+    pinned block, every field at a multiple of 16 bytes and already in its final type: one transfer instead of one transfer and
+    one conversion kernel per field.  The pinned block comes from torch's caching host allocator, which keeps it until the
+    transfer has finished."""
+    places, size = _layout(n, b, real)
+    if size > _STAGED_BYTES:
+        up = {name: torch.as_tensor(v).to(device, non_blocking=True).to(_TORCH[kind]).reshape(shape).contiguous()
+              for (name, kind, shape, _), v in zip(places, values)}
+        return up, {name: t.data_ptr() for name, t in up.items()}
+    block = torch.empty(max(size, 16), dtype=torch.uint8, pin_memory=True)
     host = block.numpy()
-    for (_, values, kind, shape), (lo, hi) in zip(fields, places):
-        host[lo:hi].view(kind).reshape(shape)[...] = values
+    for (_, kind, shape, lo), v in zip(places, values):
+        np.ndarray(shape, kind, host, lo)[...] = v
     dev = block.to(device, non_blocking=True)
-    typed = {kind: dev.view(_TORCH[kind]) for kind in {f[2] for f in fields}}
-    return {name: typed[kind].as_strided(shape, _STRIDES[len(shape)], lo // _BYTES[kind])
-            for (name, _, kind, shape), (lo, _) in zip(fields, places)}
+    base, typed, up = dev.data_ptr(), {}, {}
+    for name, kind, shape, lo in places:
+        if name in _RETURNED:
+            if kind not in typed:
+                typed[kind] = dev.view(_TORCH[kind])
+            up[name] = typed[kind].as_strided(shape, _STRIDES[len(shape)], lo // _BYTES[kind])
+    return up, {name: base + lo for name, _, _, lo in places}
 
 
 _TORCH = {np.float64: torch.float64, np.float32: torch.float32, np.int64: torch.int64, np.int32: torch.int32, np.uint8: torch.uint8}

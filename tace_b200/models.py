@@ -523,7 +523,7 @@ class TensorModel(torch.nn.Module):
             graph_ptr = ready(data["ptr"], torch.int32)
             n_graphs = int(graph_ptr.numel() - 1)
             batch.positions = real(data["positions"]).data_ptr()
-            batch.lattice = real(data["lattice"]).reshape(-1, 3, 3).data_ptr()
+            batch.lattice = real(data["lattice"]).data_ptr()
             batch.edge_shifts = real(data["edge_shifts"]).data_ptr()
         keep.append(graph_ptr)
         batch.n_atoms, batch.n_local, batch.n_edges, batch.n_graphs = n_atoms, n_local, E, n_graphs
@@ -561,8 +561,13 @@ class TensorModel(torch.nn.Module):
         else:
             for k, shape in shapes.items():
                 res[k] = torch.empty(shape, dtype=dtype, device=device)
-        for k in shapes:
-            setattr(out, k, res[k].data_ptr())
+        if block is not None:
+            base, width = block.data_ptr(), block.element_size()
+            for k, place in places.items():
+                setattr(out, k, base + place * width)
+        else:
+            for k in shapes:
+                setattr(out, k, res[k].data_ptr())
 
         exchange_cb = None
         if self.lmp and n_atoms != n_local and self.readout_fn.num_layers > 1:
@@ -587,6 +592,7 @@ class TensorModel(torch.nn.Module):
                 return int(nbytes.value)
 
             shape_key = (n_atoms, n_local, E, n_graphs, device.index)
+            asked = False  # nbytes holds this batch's size
 
             def set_limit(limit: int) -> None:
                 if limit != self._auto_chunk:
@@ -604,7 +610,7 @@ class TensorModel(torch.nn.Module):
                 for limit in (whole, self._auto_chunk):  # the whole batch, else the chunk size chosen last time
                     if limit is not None and limit <= whole and not fits:
                         set_limit(limit)
-                        fits = needed() <= held
+                        fits = asked = needed() <= held
                 if not fits:
                     free, _total = torch.cuda.mem_get_info(device)
                     budget = 0.8 * (free + (self._workspace.numel() if self._workspace is not None else 0))
@@ -617,8 +623,7 @@ class TensorModel(torch.nn.Module):
                             raise _lib.TaceError(f"tace_b200: this batch needs {needed() / 2**30:.1f} GiB of workspace with the TECE edge block "
                                                  f"(all per-edge tensors resident), {budget / 2**30:.1f} GiB are available; use smaller batches")
             if shape_key != self._sized_for or self._workspace is None:
-                needed()
-                self._sized_bytes = int(nbytes.value)
+                self._sized_bytes = int(nbytes.value) if asked else needed()
                 self._sized_for = shape_key
             ws = self._get_workspace(self._sized_bytes, device)
             ws_ptr = (ws.data_ptr() + 255) & ~255

@@ -8,6 +8,7 @@ structures); ``get_neighborhood`` keeps the reference signature and numpy return
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional, Tuple, Union
 
 import numpy as np
@@ -63,25 +64,36 @@ _SHIFT_TYPES = {torch.int32: -1, torch.float32: _lib.TACE_F32, torch.float64: _l
 def _list_on_device(positions: torch.Tensor, lattice: torch.Tensor, pbc: torch.Tensor, graph_ptr: torch.Tensor, cutoff: float,
                     n_targets: int, shift_dtype: torch.dtype) -> Tuple[torch.Tensor, torch.Tensor]:
     """``neighbor_list_batch`` on arguments that have its types and layout already; shifts as ``shift_dtype``."""
-    lib = _lib.load()
-    dev = positions.device
-    n, b = positions.shape[0], lattice.shape[0]
+    return _list_at(positions.device, positions.shape[0], lattice.shape[0],
+                    (positions.data_ptr(), lattice.data_ptr(), pbc.data_ptr(), graph_ptr.data_ptr()), cutoff, n_targets, shift_dtype)
+
+
+@functools.lru_cache(maxsize=256)
+def _workspace_bytes(n: int, b: int) -> int:
     need = ctypes.c_size_t()
-    _lib.check(lib.tace_nl_workspace_bytes(n, b, ctypes.byref(need)), "tace_nl_workspace_bytes")
+    _lib.check(_lib.load().tace_nl_workspace_bytes(n, b, ctypes.byref(need)), "tace_nl_workspace_bytes")
+    return int(need.value) + 256
+
+
+def _list_at(dev: torch.device, n: int, b: int, inputs, cutoff: float, n_targets: int,
+             shift_dtype: torch.dtype) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``_list_on_device`` for inputs given by their addresses (positions, cells, pbc, graph pointers)."""
+    lib = _lib.load()
+    need = _workspace_bytes(n, b)
     # one scratch from torch's caching allocator: row pointers | counts | the library's workspace
     rows, counts = 8 * (n + 1), 4 * n
-    scratch = torch.empty(rows + counts + int(need.value) + 256, dtype=torch.uint8, device=dev)
+    scratch = torch.empty(rows + counts + need, dtype=torch.uint8, device=dev)
     row_ptr = scratch.data_ptr()
     work = row_ptr + rows + counts
-    args = (positions.data_ptr(), lattice.data_ptr(), pbc.data_ptr(), graph_ptr.data_ptr(), b, n, n_targets, float(cutoff))
+    args = (*inputs, b, n, n_targets, float(cutoff))
     with _lib.on_device(dev):
         stream = _lib.stream_of(dev)
-        _lib.check(lib.tace_nl_rows(*args, row_ptr + rows, row_ptr, work, int(need.value) + 256, stream), "tace_nl_rows")
+        _lib.check(lib.tace_nl_rows(*args, row_ptr + rows, row_ptr, work, need, stream), "tace_nl_rows")
         n_edges = int(scratch[8 * n:8 * n + 8].view(torch.int64).item())
         edge_index = torch.empty(2, n_edges, dtype=torch.int64, device=dev)
         shifts = torch.empty(n_edges, 3, dtype=shift_dtype, device=dev)
         _lib.check(lib.tace_nl_fill_rows(*args, row_ptr, n_edges, edge_index.data_ptr(), shifts.data_ptr(), _SHIFT_TYPES[shift_dtype],
-                                         work, int(need.value) + 256, stream), "tace_nl_fill_rows")
+                                         work, need, stream), "tace_nl_fill_rows")
     return edge_index, shifts
 
 
