@@ -11,6 +11,7 @@ optional: when it is installed the class derives from its ``ModelInterface``.
 
 from __future__ import annotations
 
+import functools
 from pathlib import Path
 from typing import Callable, Dict, List, Optional, Union
 
@@ -39,6 +40,11 @@ def tace_b200_nl(positions: torch.Tensor, cell: torch.Tensor, pbc, cutoff: float
     edge_index, shifts = neighbor_list_batch(positions.to(torch.float64), cell.to(torch.float64), pbc_t.contiguous(), ptr, float(cutoff))
     mapping_system = system_idx[edge_index[0]]
     return edge_index, mapping_system, shifts
+
+
+@functools.lru_cache(maxsize=16)
+def _periodic_rows(pbc: tuple, n_systems: int, device: torch.device) -> torch.Tensor:
+    return torch.tensor([pbc], dtype=torch.uint8, device=device).expand(n_systems, 3).contiguous()
 
 
 class TACETorchSimCalc(_Base):
@@ -102,6 +108,7 @@ class TACETorchSimCalc(_Base):
         self.n_systems = len(counts)
         self.n_atoms_per_system = counts.tolist()
         self.ptr = torch.cat([counts.new_zeros(1), counts.cumsum(0)])
+        self._ptr32 = self.ptr.to(torch.int32)
 
     def _setup_node_attrs(self, atomic_numbers: torch.Tensor) -> None:
         if int(atomic_numbers.max()) >= self._z_table.numel():
@@ -129,8 +136,15 @@ class TACETorchSimCalc(_Base):
             if not hasattr(self, "system_idx") or not torch.equal(sidx, self.system_idx):
                 self._setup_ptr(sidx)
                 self.system_idx = sidx
-        edge_index, _mapping, unit_shifts = self.neighbor_list_fn(state.positions, state.row_vector_cell, state.pbc, self.r_max,
-                                                                  self.system_idx)
+        pbc = state.pbc
+        if (self.neighbor_list_fn is tace_b200_nl and isinstance(pbc, (tuple, list)) and len(pbc) == 3
+                and all(isinstance(p, (bool, int)) for p in pbc) and state.row_vector_cell.numel() == 9 * self.n_systems):
+            # this package's own list, without working the systems' offsets out again (they belong to `system_idx`) and
+            # without the edges' system indices, which the model does not read
+            rows = _periodic_rows(tuple(map(bool, pbc)), self.n_systems, state.positions.device)
+            edge_index, unit_shifts = neighbor_list_batch(state.positions, state.row_vector_cell, rows, self._ptr32, self.r_max)
+        else:
+            edge_index, _mapping, unit_shifts = self.neighbor_list_fn(state.positions, state.row_vector_cell, pbc, self.r_max, self.system_idx)
         out = self.model({
             "ptr": self.ptr, "node_attrs": self.node_attrs, "species": self.species, "batch": self.system_idx, "pbc": state.pbc,
             "lattice": state.row_vector_cell, "positions": state.positions, "edge_index": edge_index, "edge_shifts": unit_shifts,
