@@ -23,7 +23,6 @@ namespace {
 
 constexpr int kWideBatch = 16;  // edges whose coupling rows are in shared memory at a time
 constexpr int kWideListRows = 8;
-constexpr int kWideFewBlocks = 1184;  // eight blocks per SM
 
 // Entry `it` of the part of a partial pass' row list this launch works on, -1 past its end (see tp_row in tp_kernels.cu).
 __device__ __forceinline__ int wide_row(const TPArgs<float>& a, int it) {
@@ -203,7 +202,7 @@ __device__ __forceinline__ void wide_fwd_group(const TPArgs<float>& a, int i, in
   wide_fwd_warp<TP, NV, C, ENV, GRP>(a, lo, hi, c0, Gs, acc);
   constexpr int NOUT = TP::v_nout(GRP);
   if constexpr (ES > 1) {
-    float* buf = reinterpret_cast<float*>(smem + GRP * S::kAccBytes) + lane;
+    float* buf = reinterpret_cast<float*>(smem) + lane;
     for (int s = 1; s < ES; ++s) {
       __syncthreads();
       if (es == s) {
@@ -238,8 +237,7 @@ __global__ void __maxnreg__(168) tp_fwd_wide_kernel(const TPArgs<float> a) {
   using S = WideFwdShape<TP, NV, C>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5;
-  const int grp = warp % TP::NGV, rest = warp / TP::NGV;
-  const int es = ES == 1 ? 0 : rest, tgt = ES == 1 ? rest : 0;
+  const int grp = ES == 1 ? warp % TP::NGV : (int)blockIdx.z, es = ES == 1 ? 0 : warp, tgt = ES == 1 ? warp / TP::NGV : 0;
   constexpr int NT = ES == 1 ? S::TPB : 1;
   float* Gs = reinterpret_cast<float*>(smem + warp * S::kGBytes);
   constexpr int ROWS = LIST ? kWideListRows : 1;
@@ -553,22 +551,24 @@ template <typename TP, int NV, int C, bool ENV, int ES, bool LIST>
 cudaError_t launch_wide_fwd_k(const TPArgs<float>& a, cudaStream_t s) {
   using S = WideFwdShape<TP, NV, C>;
   static bool done[kWideMaxDevices] = {};
-  constexpr int warps = TP::NGV * (ES == 1 ? S::TPB : ES), nt = ES == 1 ? S::TPB : 1;
-  constexpr int g = warps * S::kGBytes, acc = ES > 1 ? TP::NGV * S::kAccBytes : 0, bytes = g > acc ? g : acc;
+  constexpr int warps = ES == 1 ? TP::NGV * S::TPB : ES, nt = ES == 1 ? S::TPB : 1;
+  constexpr int g = warps * S::kGBytes, acc = ES > 1 ? S::kAccBytes : 0, bytes = g > acc ? g : acc;
   auto kernel = tp_fwd_wide_kernel<TP, NV, C, ENV, ES, LIST>;
   const cudaError_t e = allow_smem(kernel, bytes, done);
   if (e != cudaSuccess) return e;
   const int per = nt * (LIST ? kWideListRows : 1);
-  kernel<<<dim3((a.n_seg + per - 1) / per, S::CW), warps * 32, bytes, s>>>(a);
+  kernel<<<dim3((a.n_seg + per - 1) / per, S::CW, ES == 1 ? 1 : TP::NGV), warps * 32, bytes, s>>>(a);
   return cudaGetLastError();
 }
-// Few targets: four warps share the edges of a target, so that a cell of some dozen atoms does not walk its edge lists with one
-// warp per SM (32 atoms, 42 edges each, rank 2, 64 channels: see the launcher's rule below).
+// Few targets: four warps share the edges of a (target, group), so that a cell of some dozen atoms does not walk its edge lists
+// with one warp per SM.  What a share costs besides its edges (coupling rows, sums through shared memory) weighs more the fewer
+// edges it has, so the line moves with their number: at 62 edges per target and 128 channels shares win up to 864 blocks
+// (126 -> 115 us, 576: 76 -> 72) and are even at 1 152, at 42 edges and 64 channels up to 500 (42 -> 40 us; 864: 50 -> 57).
 template <typename TP, int C, bool ENV>
 cudaError_t launch_wide_fwd(const TPArgs<float>& a, cudaStream_t s) {
   if (a.row_ids) return launch_wide_fwd_k<TP, 1, C, ENV, 1, true>(a, s);
   const long long blocks = (long long)a.n_seg * (C / 64);
-  if (a.split_sums && blocks <= kWideFewBlocks && a.n_edges >= 16LL * a.n_seg) return launch_wide_fwd_k<TP, 1, C, ENV, 4, false>(a, s);
+  if (a.split_sums && blocks * a.n_seg <= 15LL * a.n_edges && a.n_edges >= 16LL * a.n_seg) return launch_wide_fwd_k<TP, 1, C, ENV, 4, false>(a, s);
   return launch_wide_fwd_k<TP, 1, C, ENV, 1, false>(a, s);
 }
 template <typename TP, int NV, int C, bool ENV, bool LIST>
@@ -590,9 +590,13 @@ template <typename TP, int C, bool ENV>
 cudaError_t launch_wide_bwd(const TPArgs<float>& a, cudaStream_t s) {
   if constexpr (TP::NX == 1) {
     if (a.row_ids) return cudaErrorInvalidValue;  // partial passes exist where source features are exchanged, not here
-    // Shares per target: enough warps for three rounds of what the chip holds, while a share keeps at least eight edges.
+    // Shares per target: warps for three rounds of what the chip holds, while a share keeps at least eight edges; down to two
+    // edges while there are fewer than eight warps per SM, because then the walk over a share is all that is waited for
+    // (32 targets of 42 edges: 10.5 -> 4.6 us; with 500 targets such shares cost 15 -> 19 us).
     int shares = 1;
-    while ((long long)a.n_seg * shares < 3 * 148 * 16 && a.n_edges >= 16LL * shares * a.n_seg && shares < 16) shares *= 2;
+    while (shares < 16 && (((long long)a.n_seg * shares < 3 * 148 * 16 && a.n_edges >= 16LL * shares * a.n_seg) ||
+                           ((long long)a.n_seg * shares < 8 * 148 && a.n_edges >= 4LL * shares * a.n_seg)))
+      shares *= 2;
     tp_bwd_scalar_wide_kernel<TP, C, ENV><<<(unsigned)(((long long)a.n_seg * shares + 3) / 4), 128, 0, s>>>(a, shares);
     return cudaGetLastError();
   } else {
