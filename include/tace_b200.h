@@ -351,7 +351,9 @@ int tace_nl_build_noalloc(const double* positions, const double* lattice, const 
  *   fp64 difference as tace_edge_vectors).
  * tace_rows_gather: dst[r,:] = src[index[r],:] for r < n_rows (packs a halo message; elem_bytes 4 or 8).
  * tace_rows_scatter_add: dst[index[r],:] += src[r,:]; the indices of one call must be distinct (unpacks
- *   gradients returned by a neighbouring domain, tace/models/lammps.py:105-129); float / double rows. */
+ *   gradients returned by a neighbouring domain, tace/models/lammps.py:105-129); float / double rows.
+ * tace_rows_segment_add: dst[targets[t],:] += src[order[j],:] for j = ptr[t] .. ptr[t+1]-1, in that order; the targets
+ *   must be distinct (the same for all periodic images of the atoms at once). */
 int tace_md_kick_drift(double* positions, double* velocities, const void* forces, int32_t force_dtype, const double* inv_mass,
                        int64_t n_atoms, double kick, double dt, tace_stream_t stream);
 int tace_md_langevin(double* velocities, const double* inv_mass, const int64_t* ids, int64_t n_atoms, double c1,
@@ -370,6 +372,8 @@ int tace_edges_compact(const double* positions, const int64_t* edge_index, int64
                        tace_stream_t stream);
 int tace_rows_gather(const void* src, const int64_t* index, int64_t n_rows, int32_t row_len, int32_t elem_bytes, void* dst,
                      tace_stream_t stream);
+int tace_rows_segment_add(const void* src, const int64_t* order, const int64_t* targets, const int64_t* ptr, int64_t n_targets,
+                          int32_t row_len, int32_t elem_bytes, void* dst, tace_stream_t stream);
 int tace_rows_scatter_add(const void* src, const int64_t* index, int64_t n_rows, int32_t row_len, int32_t elem_bytes, void* dst,
                           tace_stream_t stream);
 

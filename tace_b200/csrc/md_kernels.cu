@@ -81,6 +81,22 @@ __global__ void rows_kernel(const V* __restrict__ src, const int64_t* __restrict
   }
 }
 
+// dst[targets[t]] += src[order[j]] for j in [ptr[t], ptr[t+1]), in that order: the rows that a halo exchange brings back for one
+// atom from up to 26 periodic images in one launch instead of one per image.
+template <typename V>
+__global__ void rows_segment_add_kernel(const V* __restrict__ src, const int64_t* __restrict__ order, const int64_t* __restrict__ targets,
+                                        const int64_t* __restrict__ ptr, long long n_targets, int row_len, V* __restrict__ dst) {
+  const long long total = n_targets * row_len;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < total; k += (long long)gridDim.x * blockDim.x) {
+    const long long t = k / row_len;
+    const int c = (int)(k - t * row_len);
+    V* d = dst + targets[t] * row_len + c;
+    V acc = *d;
+    for (long long j = ptr[t]; j < ptr[t + 1]; ++j) acc = acc + src[order[j] * row_len + c];
+    *d = acc;
+  }
+}
+
 inline unsigned grid_for(long long total, int block) {
   long long g = (total + block - 1) / block;
   const long long cap = 148LL * 16;
@@ -281,6 +297,19 @@ int rows_dispatch(const void* src, const int64_t* idx, int64_t n_rows, int32_t r
 extern "C" int tace_rows_gather(const void* src, const int64_t* index, int64_t n_rows, int32_t row_len, int32_t elem_bytes,
                                 void* dst, tace_stream_t stream) {
   return rows_dispatch<true>(src, index, n_rows, row_len, elem_bytes, dst, stream);
+}
+extern "C" int tace_rows_segment_add(const void* src, const int64_t* order, const int64_t* targets, const int64_t* ptr, int64_t n_targets,
+                                     int32_t row_len, int32_t elem_bytes, void* dst, tace_stream_t stream) {
+  if (n_targets < 0 || row_len <= 0 || (elem_bytes != 4 && elem_bytes != 8)) return TACE_ERR_INVALID_ARGUMENT;
+  if (n_targets == 0) return TACE_OK;
+  if (!src || !order || !targets || !ptr || !dst) return TACE_ERR_INVALID_ARGUMENT;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const unsigned grid = grid_for(n_targets * row_len, 256);
+  if (elem_bytes == 4)
+    rows_segment_add_kernel<float><<<grid, 256, 0, s>>>(static_cast<const float*>(src), order, targets, ptr, n_targets, row_len, static_cast<float*>(dst));
+  else
+    rows_segment_add_kernel<double><<<grid, 256, 0, s>>>(static_cast<const double*>(src), order, targets, ptr, n_targets, row_len, static_cast<double*>(dst));
+  return cudaGetLastError() == cudaSuccess ? TACE_OK : TACE_ERR_CUDA;
 }
 extern "C" int tace_rows_scatter_add(const void* src, const int64_t* index, int64_t n_rows, int32_t row_len, int32_t elem_bytes,
                                      void* dst, tace_stream_t stream) {

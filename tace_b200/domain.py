@@ -97,6 +97,7 @@ class HaloPlan:
     send_index: Dict[int, torch.Tensor] = field(default_factory=dict)   # owned-local rows sent to each peer
     send_parts: Dict[int, List[Tuple[int, int]]] = field(default_factory=dict)  # (start, count) per periodic shift
     recv_slice: Dict[int, Tuple[int, int]] = field(default_factory=dict)  # (offset, count) in the ghost block
+    add_lists: Dict[int, Tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = field(default_factory=dict)  # HaloExchange._add_rows
     ghost_shift: Optional[torch.Tensor] = None   # int64 [n_ghost, 3] periodic image of each ghost
     ghost_owner: Optional[torch.Tensor] = None   # int64 [n_ghost] owning rank
     ghost_owner_index: Optional[torch.Tensor] = None  # int64 [n_ghost] row on the owning rank
@@ -234,13 +235,16 @@ class HaloExchange:
 
     # -- helpers -----------------------------------------------------------------------------------
     @staticmethod
-    def _gather_rows(src2: torch.Tensor, idx: torch.Tensor) -> torch.Tensor:
+    def _gather_rows(src2: torch.Tensor, idx: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Packed copy of rows ``idx``: the library's gather kernel on the GPU, torch on the CPU (tests)."""
-        if not src2.is_cuda or src2.element_size() not in (4, 8) or not src2.is_contiguous():
-            return src2.index_select(0, idx).contiguous()
+        if (not src2.is_cuda or src2.element_size() not in (4, 8) or not src2.is_contiguous()
+                or (out is not None and not out.is_contiguous())):
+            rows = src2.index_select(0, idx).contiguous()
+            return rows if out is None else out.copy_(rows)
         from . import lib as _lib
 
-        out = torch.empty(idx.numel(), src2.shape[1], dtype=src2.dtype, device=src2.device)
+        if out is None:
+            out = torch.empty(idx.numel(), src2.shape[1], dtype=src2.dtype, device=src2.device)
         with torch.cuda.device(src2.device):
             _lib.check(_lib.load().tace_rows_gather(src2.data_ptr(), idx.data_ptr(), idx.numel(), src2.shape[1], src2.element_size(),
                                                     out.data_ptr(), torch.cuda.current_stream(src2.device).cuda_stream),
@@ -248,7 +252,7 @@ class HaloExchange:
         return out
 
     def _add_rows(self, dst2: torch.Tensor, q: int, rows: torch.Tensor) -> None:
-        """dst2[send_index[q]] += rows, one launch per periodic shift (indices are distinct within a shift)."""
+        """dst2[send_index[q]] += rows: one launch, every atom's rows added in the order of its periodic images."""
         idx = self.plan.send_index[q]
         if not dst2.is_cuda or dst2.dtype not in (torch.float32, torch.float64) or not dst2.is_contiguous():
             dst2[: self.plan.n_owned].index_add_(0, idx, rows)
@@ -257,13 +261,16 @@ class HaloExchange:
 
         lib = _lib.load()
         rows = rows.contiguous()
-        width = dst2.shape[1]
-        with torch.cuda.device(dst2.device):
-            stream = torch.cuda.current_stream(dst2.device).cuda_stream
-            for start, count in self.plan.send_parts[q]:
-                _lib.check(lib.tace_rows_scatter_add(rows.data_ptr() + start * width * rows.element_size(),
-                                                     idx.data_ptr() + start * 8, count, width, rows.element_size(),
-                                                     dst2.data_ptr(), stream), "tace_rows_scatter_add")
+        lists = self.plan.add_lists.get(q)
+        if lists is None:  # once per partition: the rows of every atom together, images in the order they are sent in
+            atoms, order = torch.sort(idx, stable=True)
+            targets, counts = torch.unique_consecutive(atoms, return_counts=True)
+            lists = self.plan.add_lists[q] = (order, targets, torch.cat([counts.new_zeros(1), counts.cumsum(0)]))
+        order, targets, ptr = lists
+        with _lib.on_device(dst2.device):
+            _lib.check(lib.tace_rows_segment_add(rows.data_ptr(), order.data_ptr(), targets.data_ptr(), ptr.data_ptr(), targets.numel(),
+                                                 dst2.shape[1], rows.element_size(), dst2.data_ptr(), _lib.stream_of(dst2.device)),
+                       "tace_rows_segment_add")
 
     def _p2p(self, sends: List[Tuple[torch.Tensor, int]], recvs: List[Tuple[torch.Tensor, int]]) -> None:
         import torch.distributed as dist
@@ -291,7 +298,7 @@ class HaloExchange:
             sidx = p.send_index[q]
             if q == p.rank:
                 if cnt:
-                    dst2[n + off:n + off + cnt].copy_(self._gather_rows(src2, sidx))
+                    self._gather_rows(src2, sidx, out=dst2[n + off:n + off + cnt])
                 continue
             if sidx.numel():
                 sends.append((self._gather_rows(src2, sidx), q))
@@ -315,7 +322,7 @@ class HaloExchange:
             sidx = p.send_index[q]
             if q == p.rank:
                 if cnt:
-                    landed[q] = src2[n + off:n + off + cnt].clone()
+                    landed[q] = src2[n + off:n + off + cnt]  # ghost rows: nothing below writes to them
                 continue
             if cnt:
                 sends.append((src2[n + off:n + off + cnt].contiguous(), q))
