@@ -36,6 +36,16 @@ def z_to_index(atomic_numbers: Sequence[int], model_numbers: Sequence[int]) -> n
     raise ValueError("structure contains an element the model was not built for")
 
 
+def _checked_species(species, n_atoms: int, n_elements: int) -> np.ndarray:
+    """A caller's own element indices, one per atom and inside the model's list (on the device they index tables)."""
+    species = np.asarray(species).reshape(-1)
+    if len(species) != n_atoms:
+        raise ValueError(f"species holds {len(species)} entries for {n_atoms} atoms")
+    if n_atoms and not (0 <= species.min() and species.max() < n_elements):
+        raise ValueError(f"species must hold indices in 0..{n_elements - 1} (the model's element list)")
+    return species
+
+
 def build_batch(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cutoff: float, dtype: torch.dtype,
                 device: torch.device) -> Dict[str, torch.Tensor]:
     """``batch`` as returned by ``tace_b200.synth.collate``: host numpy arrays or (pinned) CPU
@@ -52,8 +62,9 @@ def build_batch(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cuto
     else:
         cells = np.stack([complete_cell(c, positions[a:b], p, cutoff)
                           for c, p, a, b in zip(lattice_host, pbc_host, ptr_host[:-1], ptr_host[1:])])
-    species_host = np.asarray(batch["species"]) if "species" in batch else z_to_index(np.asarray(batch["atomic_numbers"]), model_numbers)
     n, b = len(positions), len(lattice_host)
+    species_host = (_checked_species(batch["species"], n, n_el) if "species" in batch
+                    else z_to_index(np.asarray(batch["atomic_numbers"]), model_numbers))
     up, at = _upload(n, b, np.float64 if dtype == torch.float64 else np.float32,
                      (positions, cells, ptr_host, batch["batch"], positions, lattice_host, ptr_host, species_host, pbc_host), device)
     edge_index, shifts = _list_at(device, n, b, (at["pos64"], at["cells"], at["pbc"], at["ptr32"]), cutoff, -1, dtype)
