@@ -125,7 +125,8 @@ typedef struct {
   int32_t n_graphs;
   const void* positions;     /* [n_atoms,3] or NULL */
   const void* lattice;       /* [n_graphs,3,3] row vectors, or NULL */
-  const int32_t* species;    /* [n_atoms] index into the model's element list */
+  const int32_t* species;    /* [n_atoms] index into the model's element list; an index outside it gives that atom's graph
+                                NaN as energy (such an atom is never used to address anything) */
   const int32_t* graph_ptr;  /* [n_graphs+1] first atom of each graph (atoms sorted by graph) */
   const int64_t* edge_index; /* [2,n_edges]: row 0 = source, row 1 = target (any order) */
   const void* edge_shifts;   /* [n_edges,3] or NULL */
@@ -289,7 +290,8 @@ int tace_nl_fill_rows(const double* positions, const double* lattice, const uint
                       int64_t n_atoms, int64_t n_targets, double cutoff, const int64_t* row_ptr, int64_t n_edges, int64_t* edge_index,
                       void* edge_shifts, int32_t shift_type, void* workspace, size_t workspace_bytes, tace_stream_t stream);
 
-/* out[i][:] = one-hot row of species[i] among n_elements, as reals of `dtype` (TACE_F32 / TACE_F64). */
+/* out[i][:] = one-hot row of species[i] among n_elements, as reals of `dtype` (TACE_F32 / TACE_F64); a row of zeros for an index
+ * outside [0, n_elements). */
 int tace_one_hot(const int32_t* species, int64_t n, int32_t n_elements, int32_t dtype, void* out, tace_stream_t stream);
 
 /* Neighbour list in one call that allocates nothing.  No counterpart in the reference.

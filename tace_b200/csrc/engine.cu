@@ -667,7 +667,7 @@ struct Model : ModelBase {
   };
   struct Bufs {
     int *row_ids, *row_split;  // owned targets without / with a ghost source (passes split around the exchange)
-    int *e_src, *e_dst, *e_orig, *perm_src, *rowptr_dst, *rowptr_src, *atom_graph, *species_perm, *species_rank, *species_ptr, *tile_ptr, *tc_tile_ptr;
+    int *e_src, *e_dst, *e_orig, *perm_src, *rowptr_dst, *rowptr_src, *atom_graph, *species, *species_perm, *species_rank, *species_ptr, *tile_ptr, *tc_tile_ptr;
     int *chunk_atom_ptr, *chunk_edge_ptr, *keys_cs, *perm_cs;  // edge chunks; (chunk, source)-sorted edge list
     int n_chunks; long long chunk_rows;                        // rows held by the per-edge chunk buffers
     void* prep_temp; size_t prep_temp_bytes;
@@ -680,7 +680,7 @@ struct Model : ModelBase {
   size_t layout(Arena& ar, Bufs& b, long long N, long long NL, long long E, int B) {
     b.e_src = ar.take<int>(E); b.e_dst = ar.take<int>(E); b.e_orig = ar.take<int>(E); b.perm_src = ar.take<int>(E);
     b.rowptr_dst = ar.take<int>(N + 1); b.rowptr_src = ar.take<int>(N + 1); b.atom_graph = ar.take<int>(N);
-    b.row_ids = ar.take<int>(NL); b.row_split = ar.take<int>(2);
+    b.species = ar.take<int>(N); b.row_ids = ar.take<int>(NL); b.row_split = ar.take<int>(2);
     b.species_perm = ar.take<int>(NL); b.species_rank = ar.take<int>(NL); b.species_ptr = ar.take<int>(n_el + 1); b.tile_ptr = ar.take<int>(4 * (n_el + 1));
     b.tc_tile_ptr = ar.take<int>(4 * (n_el + 1));
     b.prep_temp_bytes = graph_prep_temp_bytes(E, (int)N);
@@ -1202,7 +1202,7 @@ struct Model : ModelBase {
     gp.edge_index = bt->edge_index; gp.species = bt->species; gp.graph_ptr = bt->graph_ptr;
     gp.e_src = b.e_src; gp.e_dst = b.e_dst; gp.e_orig = b.e_orig; gp.rowptr_dst = b.rowptr_dst;
     gp.perm_src = b.perm_src; gp.rowptr_src = b.rowptr_src; gp.atom_graph = b.atom_graph;
-    gp.species_perm = b.species_perm; gp.species_rank = b.species_rank; gp.species_ptr = b.species_ptr; gp.tile_ptr = b.tile_ptr; gp.tc_tile_ptr = b.tc_tile_ptr;
+    gp.species_safe = b.species; gp.species_perm = b.species_perm; gp.species_rank = b.species_rank; gp.species_ptr = b.species_ptr; gp.tile_ptr = b.tile_ptr; gp.tc_tile_ptr = b.tc_tile_ptr;
     gp.temp = b.prep_temp; gp.temp_bytes = b.prep_temp_bytes;
     // edge chunks: one chunk (all atoms) unless the batch exceeds max_chunk_edges
     const bool chunked = E > max_chunk_edges;
@@ -1255,7 +1255,7 @@ struct Model : ModelBase {
       ea.dH1[t] = dh1_buffer(b.lay[t]);
     }
     ea.rp.env_after_mlp = env_after ? 1 : 0;
-    ea.species = bt->species;
+    ea.species = b.species;
     ea.env = b.env; ea.denv = b.denv; ea.add_denv = 1;
     ea.dlen = b.dlen; ea.ddlen = b.ddlen;
     ea.vec = b.vec; ea.Y = b.Y; ea.dY = b.dY; ea.g = b.g; ea.n_valid = b.rowptr_dst + N; ea.edge_forces = static_cast<T*>(o->edge_forces);
@@ -1270,7 +1270,7 @@ struct Model : ModelBase {
     // ---- layers, forward
     bool wigner_done = false, tece_seen = false;
     PH("embed");
-    CKL(launch_species_gather(w("emb"), bt->species, b.lay[0].h_in, (int)N, C, s));
+    CKL(launch_species_gather(w("emb"), b.species, b.lay[0].h_in, (int)N, C, s));
     for (int t = 0; t < NL_; ++t) {
       const LayerPlan& p = layers[t];
       LayerBufs& lb = b.lay[t];
@@ -1432,7 +1432,7 @@ struct Model : ModelBase {
     ZblArgs<T> za;
     memset(&za, 0, sizeof(za));
     if (zbl) {  // pair repulsion per atom, summed over the incoming edges
-      za.rowptr_dst = b.rowptr_dst; za.e_src = b.e_src; za.e_dst = b.e_dst; za.species = bt->species; za.dlen = b.dlen;
+      za.rowptr_dst = b.rowptr_dst; za.e_src = b.e_src; za.e_dst = b.e_dst; za.species = b.species; za.dlen = b.dlen;
       za.z = w("zbl.z"); za.rcov = w("zbl.rcov"); za.par = w("zbl.par"); za.p = cfg.envelope_p; za.n = (int)NL; za.E = E;
       za.node = b.zbl_node;
       CKL(launch_zbl_fwd(za, s));
@@ -1448,7 +1448,7 @@ struct Model : ModelBase {
     }
     CKL(launch_readout(ra, s));
     if (o->energy) {
-      CKL(launch_graph_energy(b.e_scaled, w("e0"), bt->species, bt->graph_ptr, bt->fidelity, n_el, static_cast<T*>(o->energy), B, NL,
+      CKL(launch_graph_energy(b.e_scaled, w("e0"), b.species, bt->graph_ptr, bt->fidelity, n_el, static_cast<T*>(o->energy), B, NL,
                               b.energy_partial, s));
       if (graph_energy_slices(NL, B) > 1) ++launches;  // the slice sums are added by a second kernel
     }

@@ -81,19 +81,24 @@ struct EdgeSort {
   int *e_src, *e_dst, *e_orig, *perm_src;
 };
 struct SpeciesSort {
-  const int* species; int n, n_el;
+  const int* species; int n, n_el;  // species: inside [0, n_el)
   int *perm, *rank, *ptr, *tile_ptr, *tc_tile_ptr;  // rank: place of every atom in perm
 };
 constexpr int kCountThreads = 1024, kScanItems = 4, kScanBlock = 1024 * kScanItems;
 constexpr int kSpeciesBlockAtoms = 8192;  // up to here one block sorts the atoms by species beside the edge count
 constexpr int kSpeciesBlockElements = 256;
 
-__global__ void edge_sort_init_kernel(EdgeSort a, const int* __restrict__ graph_ptr, int n_graphs, int* atom_graph) {
+// Also copies the species, with 0 in the place of an index outside the element list: everything downstream addresses tables,
+// counters and sorted rows with them.  (The read-out sees the caller's own index and gives such an atom a NaN.)
+__global__ void edge_sort_init_kernel(EdgeSort a, const int* __restrict__ graph_ptr, int n_graphs, int* atom_graph,
+                                      const int* __restrict__ species_in, int n_el, int* __restrict__ species) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i > a.n) return;
   a.cur_dst[i] = 0;
   a.cur_src[i] = 0;
   if (i == a.n) return;
+  const int z = species_in[i];
+  species[i] = (unsigned)z < (unsigned)n_el ? z : 0;
   int lo = 0, hi = n_graphs;  // largest g with graph_ptr[g] <= i
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -371,10 +376,11 @@ cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s) {
   es.block_sums = take(2 * (size_t)scan_blocks);
   es.rowptr_dst = a.rowptr_dst; es.rowptr_src = a.rowptr_src;
   es.e_src = a.e_src; es.e_dst = a.e_dst; es.e_orig = a.e_orig; es.perm_src = a.perm_src;
-  SpeciesSort sp{a.species, a.n_local, a.n_elements, a.species_perm, a.species_rank, a.species_ptr, a.tile_ptr, a.tc_tile_ptr};
+  SpeciesSort sp{a.species_safe, a.n_local, a.n_elements, a.species_perm, a.species_rank, a.species_ptr, a.tile_ptr, a.tc_tile_ptr};
   const bool small_species = a.n_local <= kSpeciesBlockAtoms && a.n_elements <= kSpeciesBlockElements;
 
-  edge_sort_init_kernel<<<(a.n_atoms + 256) / 256, 256, 0, s>>>(es, a.graph_ptr, a.n_graphs, a.atom_graph);
+  edge_sort_init_kernel<<<(a.n_atoms + 256) / 256, 256, 0, s>>>(es, a.graph_ptr, a.n_graphs, a.atom_graph, a.species, a.n_elements,
+                                                                a.species_safe);
   long long blocks = (a.E + kCountThreads - 1) / kCountThreads;
   if (blocks > 2 * 148) blocks = 2 * 148;
   const size_t smem = small_species ? sizeof(int) * (33 * (size_t)a.n_elements + 1) : 0;
@@ -406,7 +412,7 @@ cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s) {
   if (!small_species) {  // species-sorted permutation of the local atoms
     int sbits = 1;
     while ((1 << sbits) < a.n_elements + 1 && sbits < 31) ++sbits;
-    iota_and_key32_kernel<<<(a.n_local + 255) / 256, 256, 0, s>>>(a.species, keys_in, vals_in, a.n_local);
+    iota_and_key32_kernel<<<(a.n_local + 255) / 256, 256, 0, s>>>(a.species_safe, keys_in, vals_in, a.n_local);
     err = cub::DeviceRadixSort::SortPairs(cub_temp, cub_bytes, keys_in, keys_out, vals_in, a.species_perm, a.n_local, 0, sbits, s);
     if (err != cudaSuccess) return err;
     lower_bound_kernel<<<(a.n_elements + 256) / 256, 256, 0, s>>>(keys_out, a.n_local, a.species_ptr, a.n_elements);

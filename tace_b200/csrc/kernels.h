@@ -106,7 +106,7 @@ struct ReadoutArgs {
   const T* W2;       // [H]
   const T* scale;    // [n_el]
   const T* e0;       // [n_el]
-  const int* species;
+  const int* species;  // the caller's: an atom outside the element list gets a NaN (its row in every table is that of element 0)
   const int* atom_graph;  // [n] graph of each atom
   const int* graph_ptr;   // [B+1]
   const int* rowptr_dst;  // [n+1] to count a graph's edges
@@ -270,6 +270,7 @@ struct GraphPrepArgs {
   int* row_split;             // [2]
   int* perm_src; int* rowptr_src;       // [E], [n_atoms+1]
   int* atom_graph;            // [n_atoms]
+  int* species_safe;          // [n_atoms] species, 0 for an index outside [0, n_elements)
   int* species_perm; int* species_ptr;  // [n_local], [n_elements+1]
   int* species_rank;          // [n_local] place of every atom in species_perm
   int* tile_ptr;              // [4][n_elements+1] for q = 1,3,5,7: 32-row tiles per species

@@ -474,10 +474,12 @@ __global__ void readout_kernel(const ReadoutArgs<T> a, int with_t) {
       e += warp_sum(acc);
     }
     if (a.zbl && !a.zbl_after) e += a.zbl[i];
-    const int z = f * a.n_el + a.species[i];
+    const int zi = a.species[i];
+    const bool known = (unsigned)zi < (unsigned)a.n_el;
+    const int z = f * a.n_el + (known ? zi : 0);
     const int n_nodes = a.graph_ptr[g + 1] - a.graph_ptr[g];
     const int n_edges = a.rowptr_dst[a.graph_ptr[g + 1]] - a.rowptr_dst[a.graph_ptr[g]];
-    const T sc = (n_nodes == 1 && n_edges == 0) ? T(0) : a.scale[z];
+    const T sc = !known ? T(NAN) : (n_nodes == 1 && n_edges == 0) ? T(0) : a.scale[z];
     const T es = (a.zbl && a.zbl_after) ? e * sc + a.zbl[i] : e * sc;
     if (lane == 0) {
       a.e_scaled[i] = es;

@@ -44,3 +44,28 @@ def test_replay_with_changing_edge_counts(kw):
             if v is not None:
                 assert torch.equal(v, r[k]), k
     assert model.device_error() == 0
+
+
+@pytest.mark.parametrize("reps", [2, 13])  # species sorted by one block, by the device-wide sort
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_species_outside_the_element_list_give_nan_in_their_graph_only(reps, dtype):
+    """An index that a caller puts on the device wrongly addresses nothing: its structure's energy is NaN, the other one's and the
+    next evaluation's are what they were (the captured pass included)."""
+    good = synth.fcc_supercell(reps, 3.61, 0.05, seed=4, species=(13, 29), fractions=(0.5, 0.5))
+    other = synth.fcc_supercell(2, 3.61, 0.05, seed=5, species=(13, 29), fractions=(0.5, 0.5))
+    model, _, _ = make_models(2, 64, [13, 29], 3.0, 12.0, dtype, targets=("energy", "forces"))
+    data = build_batch(synth.collate([good, other]), [13, 29], 3.0, dtype, DEV)
+    want = {k: v.clone() for k, v in model(data).items() if v is not None}
+    n = len(good["positions"])
+    wrong = data["species"].clone()
+    wrong[n + 1], wrong[n + 4], wrong[n + 5], wrong[n + 9] = -1, 2, 1 << 20, -(1 << 31)
+    tol = dict(rtol=0.0, atol=(1e-4 if dtype == torch.float32 else 1e-9) * n)
+    for _ in range(3):
+        out = model(dict(data, species=wrong))
+        assert torch.isnan(out["energy"][1]) and torch.isnan(out["node_energy"][[n + 1, n + 4, n + 5, n + 9]]).all()
+        assert torch.allclose(out["energy"][0], want["energy"][0], **tol)
+        assert torch.isfinite(out["forces"][:n]).all() and torch.isfinite(out["node_energy"][:n]).all()
+    for _ in range(2):
+        out = model(data)
+        assert torch.allclose(out["energy"], want["energy"], **tol) and torch.isfinite(out["forces"]).all()
+    assert model.device_error() == 0
