@@ -14,9 +14,11 @@ from __future__ import annotations
 
 import copy
 import ctypes
+import operator
 import os
 import math
-from typing import Any, Dict, List, Optional, Union
+from itertools import chain
+from typing import Any, Dict, List, Optional, Tuple, Union
 
 import numpy as np
 import torch
@@ -292,6 +294,20 @@ class _Flags:
     pass
 
 
+_version_of = operator.attrgetter("_version")
+
+
+class _WeightTree:
+    """The dictionaries of every module below ``root`` and what they hold now (``TensorModel._weights_version``)."""
+
+    def __init__(self, root: torch.nn.Module, generation: int):
+        self.root, self.generation = root, generation
+        dicts = [d for m in root.modules() for d in (m._modules, m._parameters, m._buffers)]
+        self.filled, self.empty = [d for d in dicts if d], [d for d in dicts if not d]
+        self.items = list(chain.from_iterable(map(dict.values, self.filled)))
+        self.tensors = [t for t in self.items if isinstance(t, torch.Tensor)]
+
+
 class TensorModel(torch.nn.Module):
     """``TensorModel(readout_fn)`` with the reference's ``forward(data)`` contract."""
 
@@ -303,7 +319,7 @@ class TensorModel(torch.nn.Module):
         self.fidelity_idx = 0
         self._handle = None
         self._handle_key = None
-        self._weight_dicts = None
+        self._weight_tree, self._weight_generation = None, 0
         self._workspace = None
         self._graph_mode = os.environ.get("TACE_B200_GRAPHS", "1") != "0"
         self._sized_for, self._sized_bytes = None, 0  # batch shape the workspace size was last computed for
@@ -360,12 +376,19 @@ class TensorModel(torch.nn.Module):
         return [int(z) for z in self.readout_fn.atomic_numbers.cpu().tolist()]
 
     # ---- native model handle ----------------------------------------------------------------------
-    def _weights_version(self) -> int:
-        """Sum of the version counters of every parameter and buffer: changes when a weight is written in place.  Walks the
-        modules' own dictionaries (building a state_dict cost 0.25 ms per evaluation)."""
-        if self._weight_dicts is None or self._weight_dicts[0] is not self.readout_fn:
-            self._weight_dicts = (self.readout_fn, [d for m in self.readout_fn.modules() for d in (m._parameters, m._buffers) if d])
-        return sum(t._version for d in self._weight_dicts[1] for t in d.values() if t is not None)
+    def _weights_version(self) -> Tuple[int, int]:
+        """Changes when a parameter or buffer is written in place (version counters) or when one is replaced, registered or
+        removed anywhere below ``readout_fn``, submodules included.  Walks the modules' own dictionaries, kept from the last
+        change together with everything that they held: an object that is still held cannot share its identity with a new one.
+        (A state_dict per evaluation cost 0.25 ms; this walk 10 us for 47 modules with 49 tensors.)"""
+        held = self._weight_tree
+        if held is not None and held.root is self.readout_fn and not any(held.empty):
+            now = list(chain.from_iterable(map(dict.values, held.filled)))
+            if len(now) == len(held.items) and all(map(operator.is_, now, held.items)):
+                return held.generation, sum(map(_version_of, held.tensors))
+        self._weight_generation += 1
+        self._weight_tree = held = _WeightTree(self.readout_fn, self._weight_generation)
+        return held.generation, sum(map(_version_of, held.tensors))
 
     def _native(self, device: torch.device):
         rf = self.readout_fn
@@ -464,7 +487,7 @@ class TensorModel(torch.nn.Module):
     def __getstate__(self):
         state = self.__dict__.copy()
         state["_handle"], state["_handle_key"], state["_workspace"] = None, None, None
-        state["_exchange_stream"], state["_weight_dicts"] = None, None
+        state["_exchange_stream"], state["_weight_tree"] = None, None
         return state
 
     def _get_workspace(self, nbytes: int, device: torch.device) -> torch.Tensor:

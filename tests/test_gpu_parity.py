@@ -540,3 +540,30 @@ def test_tabulated_radial_weights_match_the_per_edge_mlp(L, C, radial):
         print(f"table vs {what}: dE/atom = {de:.3e}, dF = {df:.3e}")
         assert de <= 2e-6 and df <= 2e-5, what
     assert model.device_error() == 0
+
+
+def test_replaced_weights_reach_the_device():
+    """A submodule exchanged inside the model, a parameter exchanged and one written in place: each evaluation uses the weights of
+    the moment (compared with a model that was built with them)."""
+    import copy
+    data = to_device(oracle_batch([synth.fcc_supercell(2, 3.61, 0.05, seed=3, species=(13, 29), fractions=(0.5, 0.5))], [13, 29], 3.0,
+                                  torch.float64), torch.device("cuda:0"))
+    model, _, _ = make_models(1, 32, [13, 29], 3.0, 12.0, torch.float64)
+    part = model.readout_fn.get_submodule("representation.interactions.0")
+    energies = [model(data)["energy"].clone()]
+
+    def check():
+        fresh, _, _ = make_models(1, 32, [13, 29], 3.0, 12.0, torch.float64)
+        fresh.load_state_dict(model.state_dict())
+        energies.append(model(data)["energy"].clone())
+        assert torch.equal(energies[-1], fresh(data)["energy"]) and not torch.equal(energies[-1], energies[-2])
+
+    new = copy.deepcopy(part.linear_up)
+    new.weight.data = 1.5 * new.weight.data
+    part.linear_up = new
+    check()
+    part.linear_up.weight = torch.nn.Parameter(0.5 * part.linear_up.weight.detach())
+    check()
+    with torch.no_grad():
+        part.linear_up.weight.mul_(3.0)
+    check()
