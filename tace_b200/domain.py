@@ -97,7 +97,7 @@ class HaloPlan:
     send_index: Dict[int, torch.Tensor] = field(default_factory=dict)   # owned-local rows sent to each peer
     send_parts: Dict[int, List[Tuple[int, int]]] = field(default_factory=dict)  # (start, count) per periodic shift
     recv_slice: Dict[int, Tuple[int, int]] = field(default_factory=dict)  # (offset, count) in the ghost block
-    add_lists: Dict[int, Tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = field(default_factory=dict)  # HaloExchange._add_rows
+    add_lists: Dict[int, Tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = field(default_factory=dict)  # segment_lists(send_index[q])
     ghost_shift: Optional[torch.Tensor] = None   # int64 [n_ghost, 3] periodic image of each ghost
     ghost_owner: Optional[torch.Tensor] = None   # int64 [n_ghost] owning rank
     ghost_owner_index: Optional[torch.Tensor] = None  # int64 [n_ghost] row on the owning rank
@@ -111,6 +111,16 @@ def _in_box(frac: torch.Tensor, lo: np.ndarray, hi: np.ndarray) -> torch.Tensor:
 
 def _overlaps(lo_a, hi_a, lo_b, hi_b) -> bool:
     return bool(np.all(lo_a < hi_b) and np.all(lo_b < hi_a))
+
+
+def segment_lists(index: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """``dst[index] += rows`` as sums of segments: rows ``order[ptr[t]:ptr[t + 1]]`` belong to row ``targets[t]`` of ``dst``, in the
+    order in which they come.  Waits for the device (the number of targets is a shape)."""
+    if index.numel() == 0:
+        return index, index, index.new_zeros(1)
+    atoms, order = torch.sort(index, stable=True)
+    targets, counts = torch.unique_consecutive(atoms, return_counts=True)
+    return order, targets, torch.cat([counts.new_zeros(1), counts.cumsum(0)])
 
 
 def build_halo_plan(grid: DomainGrid, rank: int, frac_by_rank: Sequence[torch.Tensor], ghost_width: Sequence[float]) -> HaloPlan:
@@ -188,6 +198,7 @@ def build_halo_plan(grid: DomainGrid, rank: int, frac_by_rank: Sequence[torch.Te
         plan.send_index.setdefault(q, torch.zeros(0, dtype=torch.int64, device=dev))
         plan.send_parts.setdefault(q, [])
         plan.recv_slice.setdefault(q, (plan.n_ghost, 0))
+        plan.add_lists[q] = segment_lists(plan.send_index[q])
     return plan
 
 
@@ -210,6 +221,9 @@ class HaloExchange:
 
     def __init__(self, plan: HaloPlan, group=None):
         self.plan = plan
+        for q, idx in plan.send_index.items():
+            if q not in plan.add_lists:  # a plan that build_halo_plan did not make: now, because the host must not wait inside an exchange
+                plan.add_lists[q] = segment_lists(idx)
         self.group = group
         self.calls = 0
         self.bytes_sent = 0
@@ -261,12 +275,7 @@ class HaloExchange:
 
         lib = _lib.load()
         rows = rows.contiguous()
-        lists = self.plan.add_lists.get(q)
-        if lists is None:  # once per partition: the rows of every atom together, images in the order they are sent in
-            atoms, order = torch.sort(idx, stable=True)
-            targets, counts = torch.unique_consecutive(atoms, return_counts=True)
-            lists = self.plan.add_lists[q] = (order, targets, torch.cat([counts.new_zeros(1), counts.cumsum(0)]))
-        order, targets, ptr = lists
+        order, targets, ptr = self.plan.add_lists[q]
         with _lib.on_device(dst2.device):
             _lib.check(lib.tace_rows_segment_add(rows.data_ptr(), order.data_ptr(), targets.data_ptr(), ptr.data_ptr(), targets.numel(),
                                                  dst2.shape[1], rows.element_size(), dst2.data_ptr(), _lib.stream_of(dst2.device)),

@@ -187,3 +187,28 @@ def test_halo_wider_than_cell_is_rejected():
     dg = DomainGrid((1, 1, 1))
     with pytest.raises(ValueError):
         build_halo_plan(dg, 0, [torch.rand(4, 3, dtype=torch.float64)], [1.2, 0.3, 0.3])
+
+
+@pytest.mark.parametrize("grid", [(1, 1, 1), (2, 1, 1), (2, 2, 2)])
+def test_plans_carry_the_lists_of_their_row_sums(grid):
+    """The segments of every peer's rows exist when the plan does (nothing is worked out, and waited for, inside an exchange), and
+    adding them up in order gives what index_add gives."""
+    rng = np.random.default_rng(7)
+    dg = DomainGrid(grid)
+    frac = torch.tensor(rng.random((60, 3)))
+    owner = dg.owner_of(frac)
+    frac_by_rank = [frac[owner == r] for r in range(dg.world_size)]
+    for r in range(dg.world_size):
+        plan = build_halo_plan(dg, r, frac_by_rank, (0.4, 0.4, 0.4))
+        assert set(plan.add_lists) == set(plan.send_index)
+        for q, idx in plan.send_index.items():
+            order, targets, ptr = plan.add_lists[q]
+            rows, dst = torch.randn(idx.numel(), 2, dtype=torch.float64), torch.randn(plan.n_owned, 2, dtype=torch.float64)
+            ref = dst.clone().index_add_(0, idx, rows)
+            assert targets.unique().numel() == targets.numel() == ptr.numel() - 1 and int(ptr[-1]) == idx.numel()
+            for t, i in enumerate(targets.tolist()):
+                part = order[int(ptr[t]):int(ptr[t + 1])]
+                assert torch.equal(part, part.sort().values)  # images in the order they are sent in
+                for j in part.tolist():
+                    dst[i] += rows[j]
+            assert torch.allclose(dst, ref, rtol=0, atol=1e-14)

@@ -14,6 +14,7 @@ import torch
 from helpers import make_models, oracle_batch
 from tace_b200 import lib as _lib
 from tace_b200 import synth
+from tace_b200.domain import DomainGrid, HaloExchange, build_halo_plan
 from tace_b200.md import ACCEL, DomainMD, masses_for, maxwell_boltzmann
 
 pytestmark = pytest.mark.gpu
@@ -362,3 +363,21 @@ def test_one_process_two_devices(dtype):
         out = model(to_device(data, dev))
         check_parity(out, oracle(data), data["ptr"], dtype, f"L3 C128 on {dev}")
         assert model.device_error() == 0
+
+
+def test_the_first_exchange_of_a_partition_makes_no_host_wait():
+    frac = torch.rand(200, 3, generator=torch.Generator().manual_seed(2), dtype=torch.float64).to(DEV)
+    ex = HaloExchange(build_halo_plan(DomainGrid((1, 1, 1)), 0, [frac], (0.3, 0.3, 0.3)))
+    rows = torch.randn(200 + ex.plan.n_ghost, 5, dtype=torch.float32, device=DEV)
+    out, back = torch.empty_like(rows), torch.empty_like(rows)
+    torch.cuda.synchronize()
+    before = torch.cuda.get_sync_debug_mode()
+    torch.cuda.set_sync_debug_mode("error")
+    try:
+        ex.forward_exchange(rows, out)
+        ex.reverse_exchange(out, back)
+    finally:
+        torch.cuda.set_sync_debug_mode(before)
+    ref = out.double().cpu()
+    ref[:200].index_add_(0, ex.plan.send_index[0].cpu(), out[200:].double().cpu())
+    assert (back.double().cpu() - ref).abs().max().item() <= 1e-5  # at most 7 images: 7 additions of 2^-24 of a sum below 20
