@@ -13,6 +13,7 @@
 // positions and explicit round-to-nearest multiplies/adds (no FMA contraction), so the edge set
 // is bit-identical to a brute-force fp64 enumeration evaluated in the same order.
 #include <cub/cub.cuh>
+#include <thrust/iterator/transform_iterator.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -146,29 +147,30 @@ __global__ void nl_bin_kernel(const double* __restrict__ pos, const GraphBins* _
 }
 
 // Exclusive scan of one value per thread over a block of 1 024; `total` is the block's sum.
-__device__ __forceinline__ int scan_1024(int v, int* warp_sums, int& total) {
+template <typename V>
+__device__ __forceinline__ V scan_1024(V v, V* warp_sums, V& total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int x = v;
+  V x = v;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const int o = __shfl_up_sync(0xffffffffu, x, off);
+    const V o = __shfl_up_sync(0xffffffffu, x, off);
     if (lane >= off) x += o;
   }
   __syncthreads();  // warp_sums may still be read from an earlier scan
   if (lane == 31) warp_sums[warp] = x;
   __syncthreads();
   if (warp == 0) {
-    int w = warp_sums[lane];
+    V w = warp_sums[lane];
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, w, off);
+      const V o = __shfl_up_sync(0xffffffffu, w, off);
       if (lane >= off) w += o;
     }
     warp_sums[lane] = w;
   }
   __syncthreads();
   total = warp_sums[31];
-  return x - v + (warp ? warp_sums[warp - 1] : 0);
+  return x - v + (warp ? warp_sums[warp - 1] : V(0));
 }
 
 // The whole preparation of a small batch (bins, atoms sorted by bin in index order, bin starts) in one block: five launches, one
@@ -231,11 +233,12 @@ __global__ void __launch_bounds__(1024) nl_small_prepare_kernel(const double* __
     atoms_sorted[b + r] = i;
   }
 }
-// row_ptr[i] = counts[0] + ... + counts[i - 1], i = 0..n, in one block
+// row_ptr[i] = counts[0] + ... + counts[i - 1], i = 0..n, in one block.  Summed in 64 bits: 46 342 atoms that all see each other
+// have 2^31 edges.
 __global__ void __launch_bounds__(1024) nl_row_ptr_kernel(const int* __restrict__ counts, int n, int64_t* row_ptr) {
-  __shared__ int warp_sums[32];
+  __shared__ int64_t warp_sums[32];
   const int per = (n + 1023) / 1024, i0 = threadIdx.x * per, i1 = min(i0 + per, n);
-  int sum = 0, total;
+  int64_t sum = 0, total;
   for (int i = i0; i < i1; ++i) sum += counts[i];
   int64_t at = scan_1024(sum, warp_sums, total);
   for (int i = i0; i < i1; ++i) { row_ptr[i] = at; at += counts[i]; }
@@ -363,13 +366,17 @@ __global__ void __launch_bounds__(128) nl_search_kernel(const double* __restrict
   if (!FILL && lane == 0) counts[i] = count;
 }
 
+// Counts as 64-bit numbers: a device-wide scan adds up in the type of what it reads.
+struct Widen { __host__ __device__ int64_t operator()(int x) const { return x; } };
+inline auto widened(const int* counts) { return thrust::make_transform_iterator(counts, Widen()); }
+
 inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 inline int nl_max_cells(int n_atoms, int n_graphs) { return 2 * n_atoms + n_graphs + 1; }
 size_t nl_cub_bytes(int n_atoms) {
   size_t sort = 0, scan = 0;
   if (n_atoms <= 0) return 0;
   cub::DeviceRadixSort::SortPairs(nullptr, sort, (const int*)nullptr, (int*)nullptr, (const int*)nullptr, (int*)nullptr, n_atoms);
-  cub::DeviceScan::InclusiveSum(nullptr, scan, (const int*)nullptr, (int64_t*)nullptr, n_atoms);
+  cub::DeviceScan::InclusiveSum(nullptr, scan, widened(nullptr), (int64_t*)nullptr, n_atoms);
   return sort > scan ? sort : scan;
 }
 size_t nl_workspace_bytes(int n_atoms, int n_graphs) {
@@ -432,7 +439,7 @@ cudaError_t nl_row_ptr(const int* counts, int n_atoms, int64_t* row_ptr, void* c
   }
   nl_zero_first_kernel<<<1, 1, 0, s>>>(row_ptr);
   size_t bytes = nl_cub_bytes(n_atoms);
-  return cub::DeviceScan::InclusiveSum(cub_temp, bytes, counts, row_ptr + 1, n_atoms, s);
+  return cub::DeviceScan::InclusiveSum(cub_temp, bytes, widened(counts), row_ptr + 1, n_atoms, s);
 }
 
 // prepared: the workspace still holds what a count of the same structures left there

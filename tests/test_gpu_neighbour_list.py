@@ -103,3 +103,23 @@ def test_rows_entry_equals_the_count_and_fill_pair(n_mol, copies):
     assert lib.tace_nl_fill(*args, rows.data_ptr(), E, ei2.data_ptr(), es2.data_ptr(), work.data_ptr(), work.numel(), 0) == 0
     assert E > 0 or n_mol == 1
     assert torch.equal(ei, ei2) and torch.equal(es, es2.double())
+
+
+@pytest.mark.parametrize("n", [46500, 66000])  # row pointers in one block, by the device-wide scan (from 65 537 atoms)
+def test_row_pointers_past_two_to_the_31_edges(n):
+    """Every atom of a small open cluster sees every other one: n (n - 1) edges, 2.16e9 and 4.36e9 of them, counted but not stored."""
+    import ctypes
+    from tace_b200 import lib as _lib
+    lib, dev = _lib.load(), torch.device("cuda:0")
+    pos = torch.rand(n, 3, generator=torch.Generator().manual_seed(n), dtype=torch.float64).to(dev)
+    lat = (4.0 * torch.eye(3, dtype=torch.float64, device=dev))[None].contiguous()
+    pbc = torch.zeros(1, 3, dtype=torch.uint8, device=dev)
+    ptr = torch.tensor([0, n], dtype=torch.int32, device=dev)
+    need = ctypes.c_size_t()
+    assert lib.tace_nl_workspace_bytes(n, 1, ctypes.byref(need)) == 0
+    work = torch.empty(need.value, dtype=torch.uint8, device=dev)
+    counts, rows = torch.empty(n, dtype=torch.int32, device=dev), torch.empty(n + 1, dtype=torch.int64, device=dev)
+    assert lib.tace_nl_rows(pos.data_ptr(), lat.data_ptr(), pbc.data_ptr(), ptr.data_ptr(), 1, n, -1, 2.0, counts.data_ptr(), rows.data_ptr(),
+                            work.data_ptr(), work.numel(), 0) == 0
+    assert (counts == n - 1).all()
+    assert torch.equal(rows, (n - 1) * torch.arange(n + 1, dtype=torch.int64, device=dev))
