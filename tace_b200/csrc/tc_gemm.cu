@@ -70,6 +70,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   atomicCAS(error, 0, code);
   return false;
 }
+// The same for a warp whose lanes go on together: the lanes may read the abort flag at different times, and what follows a wait
+// are instructions for all of them (tcgen05.ld / st, __syncwarp), so all leave when one does.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* error, int code, uint32_t limit) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error, code, limit));
+}
 // K-major operand tile with 128-byte rows and 128-byte swizzle: 8-row groups are 1024 bytes apart.
 __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
   uint64_t d = 0;
@@ -412,7 +417,7 @@ __global__ void __launch_bounds__(TcSmem<BN>::kThreads, 1) tc_gemm_kernel(const 
           const bool chunk_end = (ks % kChunk) == kChunk - 1 || ks == num_k - 1;
           if (chunk_begin) ok = mbar_wait(acc_empty(a), ((chunk >> 1) & 1) ^ 1, abort_flag, batch.error, 4, batch.spin_limit);
           ok = ok && mbar_wait(ready_bar(s), ph, abort_flag, batch.error, 2, batch.spin_limit);
-          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }  // as in warp_wait, one vote for both waits
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t d = tmem + a * BN;
           const uint64_t stage_off = (uint64_t)((uint32_t)(s * S::kStageBytes) >> 4);
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(TcSmem<BN>::kThreads, 1) tc_gemm_kernel(const 
       const TileInfo t = decode_tile<BN>(batch, tile_start, tables, tile);
       for (int ks = 0; ks < t.num_k; ++ks, ++step) {
         const int s = step % kStages, ph = (step / kStages) & 1;
-        if (!mbar_wait(raw_bar(s), ph, abort_flag, batch.error, 3, batch.spin_limit)) { ok = false; break; }
+        if (!warp_wait(raw_bar(s), ph, abort_flag, batch.error, 3, batch.spin_limit)) { ok = false; break; }
         // one thread per row (= TMEM lane): the row's eight 16-byte pieces sit at positions j ^ (row & 7) of its 128 bytes
         // (the swizzle the TMA unit wrote); high parts go to 32 TMEM columns of the stage, residuals to the next 32
         const int row = (warp & 3) * 32 + lane;
@@ -502,7 +507,7 @@ __global__ void __launch_bounds__(TcSmem<BN>::kThreads, 1) tc_gemm_kernel(const 
       const int n_chunks = (t.num_k + kChunk - 1) / kChunk;
       for (int cin = 0; cin < n_chunks; ++cin, ++chunk) {
         const int a = chunk & 1;
-        if (!mbar_wait(acc_full(a), (chunk >> 1) & 1, abort_flag, batch.error, 5, batch.spin_limit)) { ok = false; break; }
+        if (!warp_wait(acc_full(a), (chunk >> 1) & 1, abort_flag, batch.error, 5, batch.spin_limit)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int c = 0; c < HN / 32; ++c) {

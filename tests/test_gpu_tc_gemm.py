@@ -80,3 +80,28 @@ def test_an_expired_wait_is_reported_and_leaves_the_device_usable():
     assert int(err.item()) == 0
     ref = A.double().cpu() @ B.double().T
     assert (C.cpu().double() - ref).abs().max().item() <= 2e-6 * ref.abs().max().item()
+
+
+@pytest.mark.parametrize("N,K", [(128, 64), (128, 512), (64, 64), (64, 512)])  # the four instances: tile width, one chunk or several
+def test_every_instance_returns_from_an_expired_wait(N, K):
+    """As above, with more tiles than SMs: every warp of every block has to leave as a whole."""
+    lib, dev = _lib.load(), torch.device("cuda:0")
+    M = 128 * 400
+    A = torch.randn(M, K, device=dev)
+    hi, lo = (torch.from_numpy(x).to(dev) for x in split_tf32(torch.randn(N, K).numpy()))
+    C, err = torch.zeros(M, N, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    call = lambda: lib.tace_tc_gemm_f32(A.data_ptr(), K, hi.data_ptr(), lo.data_ptr(), C.data_ptr(), N, M, N, K, err.data_ptr(),
+                                        torch.cuda.current_stream().cuda_stream)
+    assert lib.tace_tc_gemm_set_test_mode(2048, 16) == 0
+    try:
+        assert call() == 0
+        torch.cuda.synchronize()
+    finally:
+        assert lib.tace_tc_gemm_set_test_mode(0, 0) == 0
+    assert int(err.item()) in (1, 2, 3, 4, 5)
+    err.zero_()
+    assert call() == 0
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    ref = A[:512].double() @ (hi.double() + lo.double()).T
+    assert (C[:512].double() - ref).abs().max().item() <= 2e-6 * ref.abs().max().item() * max(1.0, (K / 64) ** 0.5)

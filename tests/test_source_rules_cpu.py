@@ -1,0 +1,24 @@
+"""Rules of the kernel sources that no run can show broken without hanging a GPU, checked by reading."""
+import os
+import re
+
+from conftest import ROOT
+
+
+def test_warps_of_the_tensor_core_gemm_leave_a_wait_as_a_whole():
+    """A bounded wait that gives up is seen by the lanes of a warp at different times.  Wherever a wait is followed by instructions
+    of the whole warp (tcgen05.ld / st / wait, __syncwarp), its result has to be voted on first; only the TMA producer waits in a
+    single lane."""
+    src = open(os.path.join(ROOT, "tace_b200", "csrc", "tc_gemm.cu")).read()
+    roles = re.split(r"// ---- (TMA producer|MMA issuer|operand splitters|epilogue)", src)[1:]
+    bodies = dict(zip(roles[::2], roles[1::2]))
+    assert len(bodies) == 4
+    assert re.match(r"\s*if \(lane == 0\) \{", bodies["TMA producer"])
+    for role in ("operand splitters", "epilogue"):
+        body = bodies[role].split("tcgen05.dealloc")[0]
+        assert "sync.aligned" in body or "tmem_" in body
+        assert re.search(r"\bwarp_wait\(", body) and not re.search(r"\bmbar_wait\(", body), role
+    issuer = bodies["MMA issuer"]
+    last_wait = issuer.rindex("mbar_wait(")
+    assert "__all_sync(" in issuer[last_wait:issuer.index("umma_tf32_ts(")]
+    assert "__all_sync(" in src[src.index("bool warp_wait("):src.index("umma_desc(")]
