@@ -74,6 +74,23 @@ def export_tace(model: TensorModel, path: str) -> None:
                 "embedding_property": [], "statistics": rf.statistics}, path)
 
 
+def _fetch(results):
+    """Function that brings one of ``results`` to the host.  Small results of ``TensorModel`` are views of one allocation, which
+    then comes in one transfer; anything else (large results, a small part of the allocation, the results of an object put in the
+    model's place) comes one by one."""
+    block = results[0]._base if results else None
+    if (block is None or block.dim() != 1 or block.numel() > 2 * sum(x.numel() for x in results) + 64
+            or not all(x._base is block and x.dtype == block.dtype and x.is_contiguous() for x in results)):
+        return lambda x: x.cpu().numpy()
+    host, first = block.cpu().numpy(), block.storage_offset()
+
+    def part(x):
+        at = x.storage_offset() - first
+        return host[at:at + x.numel()].reshape(x.shape)
+
+    return part
+
+
 class TACEAseCalc(Calculator):
     def __init__(self, model: Union[str, TensorModel], *, dtype: Optional[str] = None, device: Optional[str] = None,
                  fidelity_idx: Optional[int] = None, target_property: Optional[List[str]] = None,
@@ -110,20 +127,14 @@ class TACEAseCalc(Calculator):
             "ptr": np.array([0, n], dtype=np.int64),
         }
         data = build_batch(host, self.atomic_numbers, self.cutoff, self.dtype, self.device)
-        with torch.no_grad():
-            outs, block = self.model._evaluate(data)
-        if block is not None:  # every result in one transfer
-            host, size = block.cpu().numpy(), block.element_size()
-            at = lambda x: (x.data_ptr() - block.data_ptr()) // size
-            fetch = lambda x: host[at(x):at(x) + x.numel()].reshape(x.shape)
-        else:
-            fetch = lambda x: x.cpu().numpy()
+        outs = self.model(data)
+        fetch = _fetch([outs[p] for p in self.target_property if outs.get(p) is not None])
         self.results = {}
         for p in self.target_property:
             if outs.get(p) is None:
                 continue
             if p == "energy":
-                self.results["energy"] = float(fetch(outs[p])[0])
+                self.results["energy"] = float(fetch(outs[p]).item())
                 self.results["free_energy"] = self.results["energy"]
             elif p in ("stress", "virials"):
                 self.results[p] = fetch(outs[p]).squeeze(0)

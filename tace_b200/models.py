@@ -505,11 +505,6 @@ class TensorModel(torch.nn.Module):
     # ---- forward -------------------------------------------------------------------------------------
     @torch.no_grad()
     def forward(self, data: Dict[str, torch.Tensor]) -> Dict[str, Optional[torch.Tensor]]:
-        return self._evaluate(data)[0]
-
-    def _evaluate(self, data: Dict[str, torch.Tensor]):
-        """(results, block): ``block`` is the one allocation the results are views of when they are small, so that a caller who
-        wants them on the host fetches them in one transfer; None when they are separate."""
         lib = _lib.load()
         dtype = self.get_model_dtype()
         node_attrs = data.get("node_attrs")
@@ -538,7 +533,7 @@ class TensorModel(torch.nn.Module):
             if n_atoms == 0:  # a rank of a domain decomposition that neither owns nor sees any atom
                 zeros = lambda *shape: torch.zeros(*shape, dtype=dtype, device=device)
                 return {"energy": zeros(1), "node_energy": zeros(0), "forces": zeros(0, 3) if flags.compute_forces else None,
-                        "virials": None, "stress": None, "edge_forces": zeros(0, 3)}, None
+                        "virials": None, "stress": None, "edge_forces": zeros(0, 3)}
             # an empty edge list (a rank that owns no atom) still has to say "edge-vector mode": never a NULL pointer
             vec = data["edge_vector"] if E > 0 else torch.zeros(1, 3, dtype=dtype, device=device)
             batch.edge_vector = real(vec).data_ptr()
@@ -573,7 +568,7 @@ class TensorModel(torch.nn.Module):
         if flags.compute_edge_forces or self.lmp:
             shapes["edge_forces"] = (E, 3)
         sizes = {k: math.prod(s) for k, s in shapes.items()}
-        block = None
+        block = None  # small results are views of one allocation: a caller who wants them on the host fetches them in one transfer
         if sum(sizes.values()) <= _RESULT_BLOCK:
             at, places = 0, {}
             for k, size in sizes.items():
@@ -665,7 +660,7 @@ class TensorModel(torch.nn.Module):
                 # the handle must never keep a pointer to a callback object that dies with this frame
                 if exchange_cb is not None:
                     lib.tace_set_exchange(handle, _lib.EXCHANGE_FN(0), None)
-        return res, block
+        return res
 
     def _make_exchange(self, lmp_data, dtype: torch.dtype, device: torch.device, sync: bool = True, stream=None):
         """ctypes callback handing the workspace rows to ``lmp_data.forward_exchange`` /

@@ -39,6 +39,32 @@ def test_ase_calculator_matches_oracle_and_pt_roundtrip(tmp_path):
     assert set(calc.implemented_properties) >= {"energy", "free_energy", "forces", "stress"}
 
 
+def test_ase_calculator_calls_the_model_as_a_module():
+    """Forward hooks run, and an object put in the model's place is used through its call: here the mean of two models, whose
+    results are separate tensors and whose energy has no dimension."""
+    s = synth.fcc_supercell(2, 3.61, 0.05, seed=0, species=(13, 29), fractions=(0.5, 0.5))
+    models = [make_models(2, 32, [13, 29], 4.0, 20.0, torch.float64, seed=k)[0] for k in (0, 5)]
+    singles = []
+    for model in models:
+        calls = []
+        handle = model.register_forward_hook(lambda *_: calls.append(1))
+        calc = TACEAseCalc(model, device="cuda:0")
+        calc.calculate(FakeAtoms(s))
+        handle.remove()
+        assert len(calls) == 1
+        singles.append(calc.results)
+
+    def mean(data):
+        a, b = (m(data) for m in models)
+        return {"energy": (0.5 * (a["energy"] + b["energy"]))[0], "forces": 0.5 * (a["forces"] + b["forces"]), "stress": None}
+
+    calc.model = mean
+    calc.calculate(FakeAtoms(s))
+    assert set(calc.results) == {"energy", "free_energy", "forces"}
+    assert abs(calc.results["energy"] - 0.5 * (singles[0]["energy"] + singles[1]["energy"])) < 1e-10
+    assert np.abs(calc.results["forces"] - 0.5 * (singles[0]["forces"] + singles[1]["forces"])).max() < 1e-12
+
+
 class FakeLammpsData:
     """Single-rank stand-in for the Kokkos ML-IAP data object: local atoms plus periodic ghost copies."""
 
