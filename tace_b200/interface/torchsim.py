@@ -11,7 +11,6 @@ optional: when it is installed the class derives from its ``ModelInterface``.
 
 from __future__ import annotations
 
-import functools
 from pathlib import Path
 from typing import Callable, Dict, List, Optional, Union
 
@@ -42,11 +41,6 @@ def tace_b200_nl(positions: torch.Tensor, cell: torch.Tensor, pbc, cutoff: float
     return edge_index, mapping_system, shifts
 
 
-@functools.lru_cache(maxsize=16)
-def _periodic_rows(pbc: tuple, n_systems: int, device: torch.device) -> torch.Tensor:
-    return torch.tensor([pbc], dtype=torch.uint8, device=device).expand(n_systems, 3).contiguous()
-
-
 class TACETorchSimCalc(_Base):
     def __init__(self, model: Union[str, Path, TensorModel, None] = None, *, device: Optional[torch.device] = None,
                  dtype: torch.dtype = torch.float32, neighbor_list_fn: Optional[Callable] = None, compute_forces: bool = True,
@@ -61,6 +55,7 @@ class TACETorchSimCalc(_Base):
         self._compute_forces, self._compute_stress = bool(compute_forces), bool(compute_stress)
         self.neighbor_list_fn = tace_b200_nl if neighbor_list_fn is None else neighbor_list_fn
         self._memory_scales_with = "n_atoms_x_density"
+        self._rows = (None, None)  # see _periodic_rows
         model = load_tace(model, self._device, dtype=dtype, target_property=target_property).to(self._device)
         self._dtype = model.get_model_dtype()
         model.flags.compute_forces = self._compute_forces
@@ -119,6 +114,14 @@ class TACETorchSimCalc(_Base):
         self.species = species.to(torch.int32)
         self.node_attrs = torch.nn.functional.one_hot(species, len(self._z_list)).to(self._dtype)
 
+    def _periodic_rows(self, pbc: tuple, device: torch.device) -> torch.Tensor:
+        """``pbc`` once per system, kept for the next call like the other tensors made from the systems' shape (in this object: a
+        table shared by all calculators would be read on streams and freed at times that nothing orders)."""
+        key = (pbc, self.n_systems, device)
+        if self._rows[0] != key:
+            self._rows = (key, torch.tensor([pbc], dtype=torch.uint8, device=device).expand(self.n_systems, 3).contiguous())
+        return self._rows[1]
+
     def forward(self, state, **_kwargs) -> Dict[str, torch.Tensor]:
         if self.atomic_numbers_in_init:
             if state.positions.shape[0] != self.atomic_numbers.shape[0]:
@@ -141,8 +144,9 @@ class TACETorchSimCalc(_Base):
                 and all(isinstance(p, (bool, int)) for p in pbc) and state.row_vector_cell.numel() == 9 * self.n_systems):
             # this package's own list, without working the systems' offsets out again (they belong to `system_idx`) and
             # without the edges' system indices, which the model does not read
-            rows = _periodic_rows(tuple(map(bool, pbc)), self.n_systems, state.positions.device)
-            edge_index, unit_shifts = neighbor_list_batch(state.positions, state.row_vector_cell, rows, self._ptr32, self.r_max)
+            edge_index, unit_shifts = neighbor_list_batch(state.positions, state.row_vector_cell,
+                                                          self._periodic_rows(tuple(map(bool, pbc)), state.positions.device),
+                                                          self._ptr32, self.r_max)
         else:
             edge_index, _mapping, unit_shifts = self.neighbor_list_fn(state.positions, state.row_vector_cell, pbc, self.r_max, self.system_idx)
         out = self.model({

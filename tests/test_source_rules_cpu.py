@@ -22,3 +22,20 @@ def test_warps_of_the_tensor_core_gemm_leave_a_wait_as_a_whole():
     last_wait = issuer.rindex("mbar_wait(")
     assert "__all_sync(" in issuer[last_wait:issuer.index("umma_tf32_ts(")]
     assert "__all_sync(" in src[src.index("bool warp_wait("):src.index("umma_desc(")]
+
+
+def test_no_cached_function_hands_out_device_tensors():
+    """A tensor kept by a function for the whole process is made on one stream and read on others, and freed when the cache is full,
+    with nothing to order it.  What is cached per function are plain host values."""
+    import importlib
+    import pkgutil
+
+    import tace_b200
+
+    cached = set()
+    for info in pkgutil.walk_packages(tace_b200.__path__, "tace_b200."):
+        if info.name.endswith(".libtace_b200"):  # the kernel library, not a Python module
+            continue
+        module = importlib.import_module(info.name)
+        cached |= {f"{f.__module__}.{f.__name__}" for f in vars(module).values() if hasattr(f, "cache_info")}
+    assert cached == {"tace_b200.graph._element_table", "tace_b200.graph._layout", "tace_b200.neighbour_list._workspace_bytes"}
