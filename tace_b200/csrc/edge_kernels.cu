@@ -343,14 +343,14 @@ template <typename T>
 cudaError_t launch_silu(const T* in, T* out, long long n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   const long long blocks = (n + 255) / 256;
-  silu_kernel<T><<<(unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, s>>>(in, out, n);
+  silu_kernel<T><<<(unsigned)(blocks < 32 * kSMs ? blocks : 32 * kSMs), 256, 0, s>>>(in, out, n);
   return cudaGetLastError();
 }
 template <typename T>
 cudaError_t launch_silu_grad_mul(T* g, const T* z, long long n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   const long long blocks = (n + 255) / 256;
-  silu_grad_mul_kernel<T><<<(unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, s>>>(g, z, n);
+  silu_grad_mul_kernel<T><<<(unsigned)(blocks < 32 * kSMs ? blocks : 32 * kSMs), 256, 0, s>>>(g, z, n);
   return cudaGetLastError();
 }
 template <typename T>

@@ -214,8 +214,8 @@ struct ModelBase {
   // the workspace, the graph is launched on the caller's stream, and results are copied out, so
   // the caller's input and output pointers may change freely between calls.
   // The edge count of a structure that moves changes with every evaluation, so graphs are captured for a capacity: the
-  // count rounded up to a step of at most 1/16 of it (1/32 above 2 048 edges), the staged edge list padded with edges that
-  // belong to no atom.  Above 131 072 edges a pass is long enough for its launches to hide and the padding rows would
+  // count rounded up to a multiple of 64 (up to 2 048 edges) or of a power of two between 1/32 and 1/16 of it, the staged edge
+  // list padded with edges that belong to no atom.  Above 131 072 edges a pass is long enough for its launches to hide and the padding rows would
   // cost more than they save: exact counts there.
   static int64_t round_edges(int64_t E) {  // a multiple of its own step, so rounding it again changes nothing
     if (E <= 0 || E > (1 << 17)) return E;

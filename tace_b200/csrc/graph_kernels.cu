@@ -382,7 +382,7 @@ cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s) {
   edge_sort_init_kernel<<<(a.n_atoms + 256) / 256, 256, 0, s>>>(es, a.graph_ptr, a.n_graphs, a.atom_graph, a.species, a.n_elements,
                                                                 a.species_safe);
   long long blocks = (a.E + kCountThreads - 1) / kCountThreads;
-  if (blocks > 2 * 148) blocks = 2 * 148;
+  if (blocks > 2 * kSMs) blocks = 2 * kSMs;
   const size_t smem = small_species ? sizeof(int) * (33 * (size_t)a.n_elements + 1) : 0;
   if (blocks + small_species > 0)
     edge_count_kernel<<<(unsigned)(blocks + small_species), kCountThreads, smem, s>>>(es, sp, small_species ? 1 : 0);

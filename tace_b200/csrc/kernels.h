@@ -6,6 +6,10 @@
 
 namespace tace {
 
+// Multiprocessors of a B200: the unit of the launch rules (grids of grid-stride kernels, shares of a target's edges).  Results do
+// not depend on it beyond the order of the sums that split_sums allows to be cut.
+constexpr int kSMs = 148;
+
 constexpr int kMaxLayers = 4;
 
 
@@ -59,6 +63,9 @@ struct TPArgs {
 template <typename T> cudaError_t launch_tp_fwd(const TPArgs<T>& a, cudaStream_t s);
 template <typename T> cudaError_t launch_tp_bwd(const TPArgs<T>& a, cudaStream_t s);
 // the fp32 kernels with several channels per thread (tp_wide_kernels.cu), taken by the two above where they apply
+// 64 and 128 channels: the widths of the configurations measured here.  Wider multiples of 64 would fit the layout (C / 64
+// warps per edge, C / 64 blocks per target); they are not instantiated and not measured.  32 and 96
+// channels would leave lanes without a pair.
 inline bool tp_wide_channels(int C) { return C == 64 || C == 128; }
 void tp_wide_table(const float* in, float* out, long long rows, int C);  // table layout these kernels read
 bool tp_wide_supported(const TPArgs<float>& a);

@@ -11,6 +11,7 @@
 #include <type_traits>
 
 #include "../../include/tace_b200.h"
+#include "kernels.h"
 
 namespace tace {
 namespace {
@@ -99,7 +100,7 @@ __global__ void rows_segment_add_kernel(const V* __restrict__ src, const int64_t
 
 inline unsigned grid_for(long long total, int block) {
   long long g = (total + block - 1) / block;
-  const long long cap = 148LL * 16;
+  const long long cap = 16LL * kSMs;
   return (unsigned)(g < 1 ? 1 : (g > cap ? cap : g));
 }
 

@@ -18,7 +18,7 @@ __global__ void fill_zero_kernel(T* p, long long n) {
 template <typename T>
 cudaError_t launch_fill_zero(T* p, long long n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  const int blocks = (int)(((n + 255) / 256 < 148LL * 16) ? (n + 255) / 256 : 148LL * 16);
+  const int blocks = (int)(((n + 255) / 256 < 16LL * kSMs) ? (n + 255) / 256 : 16LL * kSMs);
   fill_zero_kernel<T><<<blocks, 256, 0, s>>>(p, n);
   return cudaGetLastError();
 }
@@ -47,7 +47,7 @@ cudaError_t launch_copy_segments(const CopySegments& c, cudaStream_t s) {
   long long most = 0;
   for (int k = 0; k < c.n; ++k) most = c.bytes[k] > most ? c.bytes[k] : most;
   const long long blocks = (most / 16 + 255) / 256;
-  copy_segments_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks > 148 * 8 ? 148 * 8 : blocks), 256, 0, s>>>(c);
+  copy_segments_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks > 8 * kSMs ? 8 * kSMs : blocks), 256, 0, s>>>(c);
   return cudaGetLastError();
 }
 
@@ -58,7 +58,7 @@ __global__ void add_inplace_kernel(T* dst, const T* src, long long n) {
 template <typename T>
 cudaError_t launch_add_inplace(T* dst, const T* src, long long n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  const int blocks = (int)(((n + 255) / 256 < 148LL * 16) ? (n + 255) / 256 : 148LL * 16);
+  const int blocks = (int)(((n + 255) / 256 < 16LL * kSMs) ? (n + 255) / 256 : 16LL * kSMs);
   add_inplace_kernel<T><<<blocks, 256, 0, s>>>(dst, src, n);
   return cudaGetLastError();
 }
@@ -79,7 +79,7 @@ cudaError_t launch_gather_rows(const T* src, const int* perm, T* dst, long long 
   const bool wide = row_len % per == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
   const int len = wide ? row_len / per : row_len;
   const long long blocks = (n * len + 255) / 256;
-  const unsigned grid = (unsigned)(blocks < 148 * 32 ? blocks : 148 * 32);
+  const unsigned grid = (unsigned)(blocks < 32 * kSMs ? blocks : 32 * kSMs);
   if (wide)
     gather_rows_kernel<uint4><<<grid, 256, 0, s>>>(reinterpret_cast<const uint4*>(src), perm, reinterpret_cast<uint4*>(dst), n, len);
   else
@@ -590,7 +590,7 @@ cudaError_t launch_readout(const ReadoutArgs<T>& a, cudaStream_t s) {
   const size_t smem = (with_t ? 2 : 1) * w1 + per_warp;
   if (smem > 48 * 1024) return cudaErrorInvalidValue;
   const int blocks = (a.n + warps - 1) / warps;
-  readout_kernel<T><<<blocks < 1184 ? blocks : 1184, warps * 32, smem, s>>>(a, with_t);
+  readout_kernel<T><<<blocks < 8 * kSMs ? blocks : 8 * kSMs, warps * 32, smem, s>>>(a, with_t);
   return cudaGetLastError();
 }
 

@@ -1,7 +1,6 @@
-// FP32-accurate dense GEMM on the 5th-generation tensor cores (tcgen05 + TMEM + TMA), used for
-// the last layer of the radial MLP and its transpose (the reference's mlpLinear torch.mm,
-// tace/models/linear.py:267-276, which produces the per-edge tensor-product weights
-// [edges, paths*channels]).
+// FP32-accurate dense GEMM on the 5th-generation tensor cores (tcgen05 + TMEM + TMA): every fp32 linear whose widths are
+// multiples of 64 and 32 - per-rank and per-species linears (tace/models/linear.py:377-481), the SO(2) linears of the edge
+// block, and the layers of the radial MLP where they are evaluated per edge (tace/models/linear.py:267-276).
 //
 //   C[M, N] = A[M, K] @ B[N, K]^T        (both operands K-major, C row-major, all fp32)
 //
@@ -15,7 +14,7 @@
 //
 // One persistent CTA per SM walks its share of 128 x BN output tiles with specialised warps: a TMA
 // producer fills a ring of {A, B_hi, B_lo} per 32-wide K step (four stages at BN = 128, six at BN = 64),
-// four warps split A, one thread issues the tcgen05.mma instructions into one of two TMEM
+// four warps split A, one warp (through its elected lane) issues the tcgen05.mma instructions into one of two TMEM
 // accumulators, and eight epilogue warps drain the other accumulator (tcgen05.ld of their 32 lanes, rows stored whole), so
 // loads, splitting, tensor-core work and stores overlap.  The tensor core adds into its accumulator with truncation, an error that
 // grows linearly with the number of accumulated instructions; long K loops are therefore cut

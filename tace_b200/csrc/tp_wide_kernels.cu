@@ -1,5 +1,5 @@
 // Interaction tensor product for fp32 models with tabulated radial weights and 64 or 128 channels: a thread owns 2 NV channels of
-// an edge instead of one.  (tp_kernels.cu keeps the general kernels: fp64, weights in memory, other channel counts.)
+// an edge instead of one (NV = 1; with a scalar source, where a warp takes all channels, NV = channels / 64).  (tp_kernels.cu keeps the general kernels: fp64, weights in memory, other channel counts.)
 //
 // What bounds the contraction is FP32 work and, just below it, the shared-memory / L1 path, so both are what this layout
 // saves.  A coupling entry G is read from shared memory once per warp and edge (a broadcast 128-bit read costs two
@@ -23,6 +23,7 @@ namespace {
 
 constexpr int kWideBatch = 16;  // edges whose coupling rows are in shared memory at a time
 constexpr int kWideListRows = 8;
+constexpr int kPairs = 1;       // pairs of channels of a thread where source features have a rank (NV = 1 in the text above)
 
 // Entry `it` of the part of a partial pass' row list this launch works on, -1 past its end (see tp_row in tp_kernels.cu).
 __device__ __forceinline__ int wide_row(const TPArgs<float>& a, int it) {
@@ -125,25 +126,25 @@ struct WideWeights {
 // in the warp's own shared memory, then the warp walks over the batch, the source components of the next edge and the table
 // entries of the next paths on their way.  ES warps share the edges of a target when there are too few targets to fill the
 // chip; their sums are added in a fixed order.
-template <typename TP, int NV, int C, bool ENV, int GRP>
-__device__ __forceinline__ void wide_fwd_warp(const TPArgs<float>& a, int beg, int end, int c0, float* Gs, F2 (&acc)[TP::OUTMAX][NV]) {
+template <typename TP, int C, bool ENV, int GRP>
+__device__ __forceinline__ void wide_fwd_warp(const TPArgs<float>& a, int beg, int end, int c0, float* Gs, F2 (&acc)[TP::OUTMAX][kPairs]) {
   constexpr int GS = TP::GVMAX, NX = TP::v_nx(GRP);
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int k = 0; k < TP::OUTMAX; ++k)
 #pragma unroll
-    for (int v = 0; v < NV; ++v) acc[k][v] = F2{0.0f, 0.0f};
+    for (int v = 0; v < kPairs; ++v) acc[k][v] = F2{0.0f, 0.0f};
   if (beg >= end) return;
   const float* table = a.rtab + 4 * c0 + 4 * lane;
   const float* x0 = a.x + TP::v_x0(GRP) * C + c0 + lane;
   constexpr int ROW = 4 * C * TP::NP;
-  WideWeights<TP, TP::v_p0(GRP), TP::v_np(GRP), NV, C, ENV, false, 2> wf;
-  auto load_x = [&](int src, F2 (&x)[TP::INMAX][NV]) {
+  WideWeights<TP, TP::v_p0(GRP), TP::v_np(GRP), kPairs, C, ENV, false, 2> wf;
+  auto load_x = [&](int src, F2 (&x)[TP::INMAX][kPairs]) {
     const float* p = x0 + (long long)src * (TP::NX * C);
 #pragma unroll
     for (int k = 0; k < NX; ++k)
 #pragma unroll
-      for (int v = 0; v < NV; ++v) x[k][v] = F2{__ldg(p + k * C + 64 * v), __ldg(p + k * C + 64 * v + 32)};
+      for (int v = 0; v < kPairs; ++v) x[k][v] = F2{__ldg(p + k * C + 64 * v), __ldg(p + k * C + 64 * v + 32)};
   };
   for (int e0 = beg; e0 < end; e0 += kWideBatch) {
     const int nb = min(kWideBatch, end - e0);
@@ -155,7 +156,7 @@ __device__ __forceinline__ void wide_fwd_warp(const TPArgs<float>& a, int beg, i
       interval_of(a, a.dlen[e0 + lane], k, t);
       if constexpr (ENV) u = a.env[e0 + lane];
     }
-    F2 xn[TP::INMAX][NV];
+    F2 xn[TP::INMAX][kPairs];
     load_x(__shfl_sync(0xffffffffu, src, 0), xn);
     wf.row_next = table + (long long)__shfl_sync(0xffffffffu, k, 0) * ROW;
     wf.start(wf.row_next);
@@ -166,40 +167,40 @@ __device__ __forceinline__ void wide_fwd_warp(const TPArgs<float>& a, int beg, i
     }
     __syncwarp();
     for (int e = 0; e < nb; ++e) {
-      F2 x[TP::INMAX][NV];
+      F2 x[TP::INMAX][kPairs];
 #pragma unroll
       for (int k2 = 0; k2 < NX; ++k2)
 #pragma unroll
-        for (int v = 0; v < NV; ++v) x[k2][v] = xn[k2][v];
+        for (int v = 0; v < kPairs; ++v) x[k2][v] = xn[k2][v];
       const int nxt = e + 1 < nb ? e + 1 : e;
       load_x(__shfl_sync(0xffffffffu, src, nxt), xn);
       wf.row = wf.row_next;
       wf.row_next = table + (long long)__shfl_sync(0xffffffffu, k, nxt) * ROW;
       wf.t = __shfl_sync(0xffffffffu, t, e);
       if constexpr (ENV) wf.u = __shfl_sync(0xffffffffu, u, e);
-      TP::template fwd_v<GRP, NV>(x, Gs + e * GS, wf, acc);
+      TP::template fwd_v<GRP, kPairs>(x, Gs + e * GS, wf, acc);
     }
   }
 }
 
-template <typename TP, int NV, int C>
+template <typename TP, int C>
 struct WideFwdShape {
-  static constexpr int CW = C / (64 * NV);                             // channel shares of a target (gridDim.y)
+  static constexpr int CW = C / (64 * kPairs);                             // channel shares of a target (gridDim.y)
   static constexpr int TPB = TP::NGV >= 3 ? 1 : 4 / TP::NGV;          // targets per block
   static constexpr int kGBytes = kWideBatch * TP::GVMAX * 4;          // coupling rows of one warp
-  static constexpr int kAccBytes = TP::OUTMAX * 2 * NV * 32 * 4;      // sums of one warp
+  static constexpr int kAccBytes = TP::OUTMAX * 2 * kPairs * 32 * 4;      // sums of one warp
 };
 
-template <typename TP, int NV, int C, bool ENV, int ES, int GRP>
+template <typename TP, int C, bool ENV, int ES, int GRP>
 __device__ __forceinline__ void wide_fwd_group(const TPArgs<float>& a, int i, int es, unsigned char* smem, float* Gs) {
-  using S = WideFwdShape<TP, NV, C>;
-  const int lane = threadIdx.x & 31, c0 = blockIdx.y * 64 * NV;
-  F2 acc[TP::OUTMAX][NV];
+  using S = WideFwdShape<TP, C>;
+  const int lane = threadIdx.x & 31, c0 = blockIdx.y * 64 * kPairs;
+  F2 acc[TP::OUTMAX][kPairs];
   int beg = 0, end = 0;
   if (i >= 0) { beg = a.rowptr[i]; end = a.rowptr[i + 1]; }
   const int deg = end - beg;
   const int lo = ES == 1 ? beg : beg + deg * es / ES, hi = ES == 1 ? end : beg + deg * (es + 1) / ES;
-  wide_fwd_warp<TP, NV, C, ENV, GRP>(a, lo, hi, c0, Gs, acc);
+  wide_fwd_warp<TP, C, ENV, GRP>(a, lo, hi, c0, Gs, acc);
   constexpr int NOUT = TP::v_nout(GRP);
   if constexpr (ES > 1) {
     float* buf = reinterpret_cast<float*>(smem) + lane;
@@ -209,14 +210,14 @@ __device__ __forceinline__ void wide_fwd_group(const TPArgs<float>& a, int i, in
 #pragma unroll
         for (int k = 0; k < NOUT; ++k)
 #pragma unroll
-          for (int v = 0; v < NV; ++v) { buf[(2 * (k * NV + v)) * 32] = acc[k][v].x; buf[(2 * (k * NV + v) + 1) * 32] = acc[k][v].y; }
+          for (int v = 0; v < kPairs; ++v) { buf[(2 * (k * kPairs + v)) * 32] = acc[k][v].x; buf[(2 * (k * kPairs + v) + 1) * 32] = acc[k][v].y; }
       }
       __syncthreads();
       if (es == 0) {
 #pragma unroll
         for (int k = 0; k < NOUT; ++k)
 #pragma unroll
-          for (int v = 0; v < NV; ++v) { acc[k][v].x += buf[(2 * (k * NV + v)) * 32]; acc[k][v].y += buf[(2 * (k * NV + v) + 1) * 32]; }
+          for (int v = 0; v < kPairs; ++v) { acc[k][v].x += buf[(2 * (k * kPairs + v)) * 32]; acc[k][v].y += buf[(2 * (k * kPairs + v) + 1) * 32]; }
       }
     }
     if (es != 0) return;
@@ -226,15 +227,15 @@ __device__ __forceinline__ void wide_fwd_group(const TPArgs<float>& a, int i, in
 #pragma unroll
   for (int k = 0; k < NOUT; ++k)
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
+    for (int v = 0; v < kPairs; ++v) {
       Mi[TP::template vmap<GRP>(k) * C + 64 * v] = acc[k][v].x;
       Mi[TP::template vmap<GRP>(k) * C + 64 * v + 32] = acc[k][v].y;
     }
 }
 
-template <typename TP, int NV, int C, bool ENV, int ES, bool LIST>
+template <typename TP, int C, bool ENV, int ES, bool LIST>
 __global__ void __maxnreg__(168) tp_fwd_wide_kernel(const TPArgs<float> a) {
-  using S = WideFwdShape<TP, NV, C>;
+  using S = WideFwdShape<TP, C>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5;
   const int grp = ES == 1 ? warp % TP::NGV : (int)blockIdx.z, es = ES == 1 ? 0 : warp, tgt = ES == 1 ? warp / TP::NGV : 0;
@@ -246,9 +247,9 @@ __global__ void __maxnreg__(168) tp_fwd_wide_kernel(const TPArgs<float> a) {
     int i = it < a.n_seg ? it : -1;
     if constexpr (LIST) i = wide_row(a, it);
     if (ES == 1 && i < 0) break;
-    if (grp == 0) wide_fwd_group<TP, NV, C, ENV, ES, 0>(a, i, es, smem, Gs);
-    else if (grp == 1) { if constexpr (TP::NGV > 1) wide_fwd_group<TP, NV, C, ENV, ES, 1>(a, i, es, smem, Gs); }
-    else { if constexpr (TP::NGV > 2) wide_fwd_group<TP, NV, C, ENV, ES, 2>(a, i, es, smem, Gs); }
+    if (grp == 0) wide_fwd_group<TP, C, ENV, ES, 0>(a, i, es, smem, Gs);
+    else if (grp == 1) { if constexpr (TP::NGV > 1) wide_fwd_group<TP, C, ENV, ES, 1>(a, i, es, smem, Gs); }
+    else { if constexpr (TP::NGV > 2) wide_fwd_group<TP, C, ENV, ES, 2>(a, i, es, smem, Gs); }
   }
 }
 
@@ -256,9 +257,9 @@ __global__ void __maxnreg__(168) tp_fwd_wide_kernel(const TPArgs<float> a) {
 // One block per target (and, with gridDim.y > 1, per share of its edges): the message gradient of the target sits in shared
 // memory, the coupling rows of a batch are built by all warps together (warp g: path group g, lane: edge), then CW warps work
 // on an edge at a time.  Everything the pass produces belongs to one edge, so edges can be dealt to warps and blocks freely.
-template <typename TP, int NV, int C>
+template <typename TP, int C>
 struct WideBwdShape {
-  static constexpr int CW = C / (64 * NV);       // warps per edge
+  static constexpr int CW = C / (64 * kPairs);       // warps per edge
   static constexpr int kWarps = CW > 1 ? 8 : 4, EW = kWarps / CW;  // edges in flight per block
   static constexpr int NRED = TP::D + 2;          // dY | dE/d(length) | dE/d(envelope)
   static constexpr int kMsgFloats = TP::NM * C, kGFloats = kWideBatch * TP::GVS, kRedFloats = CW > 1 ? kWideBatch * CW * NRED : 0;
@@ -304,15 +305,15 @@ __device__ __forceinline__ float wide_warp_sum(float v) {
   return v;
 }
 
-template <typename TP, int NV, int C, bool ENV>
+template <typename TP, int C, bool ENV>
 __device__ __forceinline__ void wide_bwd_row(const TPArgs<float>& a, int i, unsigned char* smem, int* esrc, int* ek, float* et, float* eu) {
-  using S = WideBwdShape<TP, NV, C>;
+  using S = WideBwdShape<TP, C>;
   constexpr int D = TP::D, ROW = 4 * C * TP::NP;
   float* gMs = reinterpret_cast<float*>(smem);
   float* Gs = gMs + S::kMsgFloats;
   float* red = Gs + S::kGFloats;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int cw = warp % S::CW, ew = warp / S::CW, c0 = cw * 64 * NV;
+  const int cw = warp % S::CW, ew = warp / S::CW, c0 = cw * 64 * kPairs;
   int beg = a.rowptr[i], end = a.rowptr[i + 1];
   if (gridDim.y > 1) {
     const int deg = end - beg, lo = beg + deg * (int)blockIdx.y / (int)gridDim.y;
@@ -328,7 +329,7 @@ __device__ __forceinline__ void wide_bwd_row(const TPArgs<float>& a, int i, unsi
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   const float* table = a.rtab + 4 * c0 + 4 * lane;
-  WideMsg<NV, C> gm;
+  WideMsg<kPairs, C> gm;
   gm.g = gMs + c0 + lane;
   for (int e0 = beg; e0 < end; e0 += kWideBatch) {
     const int nb = min(kWideBatch, end - e0);
@@ -347,13 +348,13 @@ __device__ __forceinline__ void wide_bwd_row(const TPArgs<float>& a, int i, unsi
     }
     if (e0 == beg) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    WideWeights<TP, 0, TP::NP, NV, C, ENV, true, 1> wf;
+    WideWeights<TP, 0, TP::NP, kPairs, C, ENV, true, 1> wf;
     if (ew < nb) {
       wf.row_next = table + (long long)ek[ew] * ROW;
       wf.start(wf.row_next);
     }
     for (int e = ew; e < nb; e += S::EW) {
-      WideRow<NV, C> xs;
+      WideRow<kPairs, C> xs;
       xs.x = a.x + (long long)esrc[e] * (TP::NX * C) + c0 + lane;
       xs.dx = a.dxe + (long long)(e0 + e - a.e_base) * (TP::NX * C) + c0 + lane;
       wf.row = wf.row_next;
@@ -365,7 +366,7 @@ __device__ __forceinline__ void wide_bwd_row(const TPArgs<float>& a, int i, unsi
       float dY[D];
 #pragma unroll
       for (int k = 0; k < D; ++k) dY[k] = 0.0f;
-      TP::template bwd_v<NV>(xs, gm, Gs + e * TP::GVS, wf, dY);
+      TP::template bwd_v<kPairs>(xs, gm, Gs + e * TP::GVS, wf, dY);
       int k;
       const float v = wide_warp_sums<D>(dY, lane, k);
       float dr = wide_warp_sum(wf.dr.x + wf.dr.y) * a.rt_inv_h, du = 0.0f;
@@ -411,7 +412,7 @@ __device__ __forceinline__ void wide_bwd_row(const TPArgs<float>& a, int i, unsi
   }
 }
 
-template <typename TP, int NV, int C, bool ENV, bool LIST>
+template <typename TP, int C, bool ENV, bool LIST>
 __global__ void __maxnreg__(128) tp_bwd_wide_kernel(const TPArgs<float> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int esrc[kWideBatch], ek[kWideBatch];
@@ -420,10 +421,10 @@ __global__ void __maxnreg__(128) tp_bwd_wide_kernel(const TPArgs<float> a) {
     for (int it = blockIdx.x * kWideListRows; it < ((int)blockIdx.x + 1) * kWideListRows; ++it) {
       const int i = wide_row(a, it);
       if (i < 0) break;
-      wide_bwd_row<TP, NV, C, ENV>(a, i, smem, esrc, ek, et, eu);
+      wide_bwd_row<TP, C, ENV>(a, i, smem, esrc, ek, et, eu);
     }
   } else {
-    wide_bwd_row<TP, NV, C, ENV>(a, blockIdx.x, smem, esrc, ek, et, eu);
+    wide_bwd_row<TP, C, ENV>(a, blockIdx.x, smem, esrc, ek, et, eu);
   }
 }
 
@@ -547,13 +548,13 @@ cudaError_t allow_smem(K kernel, int bytes, bool (&done)[kWideMaxDevices]) {
   return e;
 }
 
-template <typename TP, int NV, int C, bool ENV, int ES, bool LIST>
+template <typename TP, int C, bool ENV, int ES, bool LIST>
 cudaError_t launch_wide_fwd_k(const TPArgs<float>& a, cudaStream_t s) {
-  using S = WideFwdShape<TP, NV, C>;
+  using S = WideFwdShape<TP, C>;
   static bool done[kWideMaxDevices] = {};
   constexpr int warps = ES == 1 ? TP::NGV * S::TPB : ES, nt = ES == 1 ? S::TPB : 1;
   constexpr int g = warps * S::kGBytes, acc = ES > 1 ? S::kAccBytes : 0, bytes = g > acc ? g : acc;
-  auto kernel = tp_fwd_wide_kernel<TP, NV, C, ENV, ES, LIST>;
+  auto kernel = tp_fwd_wide_kernel<TP, C, ENV, ES, LIST>;
   const cudaError_t e = allow_smem(kernel, bytes, done);
   if (e != cudaSuccess) return e;
   const int per = nt * (LIST ? kWideListRows : 1);
@@ -566,23 +567,23 @@ cudaError_t launch_wide_fwd_k(const TPArgs<float>& a, cudaStream_t s) {
 // (126 -> 115 us, 576: 76 -> 72) and are even at 1 152, at 42 edges and 64 channels up to 500 (42 -> 40 us; 864: 50 -> 57).
 template <typename TP, int C, bool ENV>
 cudaError_t launch_wide_fwd(const TPArgs<float>& a, cudaStream_t s) {
-  if (a.row_ids) return launch_wide_fwd_k<TP, 1, C, ENV, 1, true>(a, s);
+  if (a.row_ids) return launch_wide_fwd_k<TP, C, ENV, 1, true>(a, s);
   const long long blocks = (long long)a.n_seg * (C / 64);
-  if (a.split_sums && blocks * a.n_seg <= 15LL * a.n_edges && a.n_edges >= 16LL * a.n_seg) return launch_wide_fwd_k<TP, 1, C, ENV, 4, false>(a, s);
-  return launch_wide_fwd_k<TP, 1, C, ENV, 1, false>(a, s);
+  if (a.split_sums && blocks * a.n_seg <= 15LL * a.n_edges && a.n_edges >= 16LL * a.n_seg) return launch_wide_fwd_k<TP, C, ENV, 4, false>(a, s);
+  return launch_wide_fwd_k<TP, C, ENV, 1, false>(a, s);
 }
-template <typename TP, int NV, int C, bool ENV, bool LIST>
+template <typename TP, int C, bool ENV, bool LIST>
 cudaError_t launch_wide_bwd_k(const TPArgs<float>& a, cudaStream_t s) {
-  using S = WideBwdShape<TP, NV, C>;
+  using S = WideBwdShape<TP, C>;
   static bool done[kWideMaxDevices] = {};
-  auto kernel = tp_bwd_wide_kernel<TP, NV, C, ENV, LIST>;
+  auto kernel = tp_bwd_wide_kernel<TP, C, ENV, LIST>;
   const cudaError_t e = allow_smem(kernel, S::kBytes, done);
   if (e != cudaSuccess) return e;
   // Blocks per target: as many as it takes to give every SM several rounds of blocks (a last round that is nearly empty
   // costs a whole one), while a share keeps at least eight edges to pay for loading the message gradient again.
   int split = 1;
   if (!LIST)
-    while ((long long)a.n_seg * split < 4 * 148 * (16 / S::kWarps) && a.n_edges >= 16LL * split * a.n_seg && split < 16) split *= 2;
+    while ((long long)a.n_seg * split < 4 * kSMs * (16 / S::kWarps) && a.n_edges >= 16LL * split * a.n_seg && split < 16) split *= 2;
   kernel<<<dim3(LIST ? (a.n_seg + kWideListRows - 1) / kWideListRows : a.n_seg, split), S::kWarps * 32, S::kBytes, s>>>(a);
   return cudaGetLastError();
 }
@@ -594,13 +595,13 @@ cudaError_t launch_wide_bwd(const TPArgs<float>& a, cudaStream_t s) {
     // edges while there are fewer than eight warps per SM, because then the walk over a share is all that is waited for
     // (32 targets of 42 edges: 10.5 -> 4.6 us; with 500 targets such shares cost 15 -> 19 us).
     int shares = 1;
-    while (shares < 16 && (((long long)a.n_seg * shares < 3 * 148 * 16 && a.n_edges >= 16LL * shares * a.n_seg) ||
-                           ((long long)a.n_seg * shares < 8 * 148 && a.n_edges >= 4LL * shares * a.n_seg)))
+    while (shares < 16 && (((long long)a.n_seg * shares < 3 * kSMs * 16 && a.n_edges >= 16LL * shares * a.n_seg) ||
+                           ((long long)a.n_seg * shares < 8 * kSMs && a.n_edges >= 4LL * shares * a.n_seg)))
       shares *= 2;
     tp_bwd_scalar_wide_kernel<TP, C, ENV><<<(unsigned)(((long long)a.n_seg * shares + 3) / 4), 128, 0, s>>>(a, shares);
     return cudaGetLastError();
   } else {
-    return a.row_ids ? launch_wide_bwd_k<TP, 1, C, ENV, true>(a, s) : launch_wide_bwd_k<TP, 1, C, ENV, false>(a, s);
+    return a.row_ids ? launch_wide_bwd_k<TP, C, ENV, true>(a, s) : launch_wide_bwd_k<TP, C, ENV, false>(a, s);
   }
 }
 template <typename TP>

@@ -313,8 +313,9 @@ def radial_table(out: Dict[str, np.ndarray], layer: int, plan: "ModelPlan", cuto
 
 
 def radial_table_intervals(knots: np.ndarray) -> np.ndarray:
-    """The device layout of ``radial_table``'s result: [K][paths * channels][4] = the (value, h * slope) pairs of both
-    ends of interval k, so that one 16-byte load feeds the interpolation of one (path, channel) weight."""
+    """What the library is given of ``radial_table``'s result: [K][paths * channels][4] = the (value, h * slope) pairs of both
+    ends of interval k.  ``tace_set_weight`` turns them into the four coefficients of the interval's cubic, one 16-byte load per
+    (path, channel) weight."""
     return np.ascontiguousarray(np.concatenate([knots[:-1], knots[1:]], axis=-1))
 
 
