@@ -9,9 +9,9 @@
 // source components are live together.  NV = 1 (16 warps per SM backward) beat NV = 2 (12 warps, half the shared-memory
 // reads): 1.04 against 1.18 ms for the rank-3 backward pass below.
 //
-// Measured against one channel per thread, on B200 at rank 3, 128 channels, 2 407 targets, 150 400 edges: backward 1.51 -> 1.04 ms
-// (FMA pipe 62 % busy, L1 68 % of its wavefronts), forward 0.80 -> 0.54 ms (L1 81 %: per edge 368 wavefronts of table, 320 of
-// coupling rows, 64 of source rows), scalar source forward 0.11 -> 0.08 ms; rank 2, 64 channels, 131 072 targets,
+// Measured against one channel per thread, on B200 at rank 3, 128 channels, 2 283 targets, 142 222 edges: backward 1.51 -> 1.04 ms
+// (FMA pipe 62 % busy, LSU 66 % of its wavefronts), forward 0.80 -> 0.54 ms (LSU 80 %: of 848 wavefronts per edge 368 are table
+// entries, 320 coupling rows, 64 source rows; 14.4 TB/s out of L2, of 19.6 that all SMs together can read), scalar source forward 0.11 -> 0.08 ms; rank 2, 64 channels, 131 072 targets,
 // 5.5 M edges: 10.4 -> 7.2 and 5.1 -> 3.9 ms; 32 targets of 42 edges: 51 -> 10 and 31 -> 13 us.
 #include <cstdint>
 #include "kernels.h"
@@ -435,7 +435,7 @@ __global__ void __maxnreg__(128) tp_bwd_wide_kernel(const TPArgs<float> a) {
 // builds edge e's coupling row, the next edge's source row is on its way. Shares of a target's edges go to neighbouring warps.
 // With the gradient rows in shared memory, two warps per edge at 128 channels and two exchanges, the LSU was 73 % busy with them;
 // what is left are the table entries.  Rank 2, 64 channels, 5.5 M edges: 2.82 -> 1.94 ms; rank 3, 64 channels, 1 372 targets of 42 edges:
-// 47 -> 36 us; rank 3, 128 channels, 2.8 M edges: 2.56 -> 2.16 ms, 150 400 edges: 148 -> 125 us.
+// 47 -> 36 us; rank 3, 128 channels, 2.8 M edges: 2.56 -> 2.16 ms, 142 222 edges: 148 -> 125 us.
 template <int NV, int D>
 struct WideMsgRegs {
   F2 g[D][NV];
