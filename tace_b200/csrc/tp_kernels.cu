@@ -92,12 +92,14 @@ __device__ __forceinline__ void rt_load<float>(const float* p, RtCubic<float>& q
 }
 
 // RT: path weights interpolated from the table a.rtab instead of read from a.W.
-// Messages of target atom i (output group GRP); Gs, esrc, rts: shared memory of the block.
-template <typename T, typename TP, int GRP, bool ENV, bool RT>
-__device__ __forceinline__ void tp_fwd_row(const TPArgs<T>& a, int i, T* Gs, int* esrc, RtEdge<T>* rts) {
+// Messages of target atom i (output group GRP); Gs, esrc, rts, buf: shared memory of the block.  ES sets of C threads deal the edges of
+// a batch between them; their sums are added in a fixed order.
+constexpr int kShareRows = 8;  // rows of the sums that pass through shared memory at a time
+template <typename T, typename TP, int GRP, bool ENV, bool RT, int ES>
+__device__ __forceinline__ void tp_fwd_row(const TPArgs<T>& a, int i, T* Gs, int* esrc, RtEdge<T>* rts, T* buf) {
   constexpr int NMG = GRP == 0 ? TP::NMG0 : TP::NMG1, NPG = GRP == 0 ? TP::NPG0 : TP::NPG1;
   constexpr int P0 = GRP == 0 ? TP::P00 : TP::P01, M0 = GRP == 0 ? TP::M00 : TP::M01;
-  const int c = threadIdx.x, C = a.C;
+  const int C = a.C, share = ES == 1 ? 0 : threadIdx.x / C, c = threadIdx.x - share * C;
   const int rt_first = blockDim.x > 32 ? 32 : 0;  // the second warp (when there is one) prepares the interpolation
   T acc[NMG];
 #pragma unroll
@@ -111,7 +113,7 @@ __device__ __forceinline__ void tp_fwd_row(const TPArgs<T>& a, int i, T* Gs, int
       rt_prepare<T>(a, a.dlen[e0 + threadIdx.x - rt_first], rts[threadIdx.x - rt_first]);
     build_G_rows<T, TP>(a.Y, e0, nb, 2 * GRP, 2, Gs);
     __syncthreads();
-    for (int e = 0; e < nb; ++e) {
+    for (int e = share; e < nb; e += ES) {
       const long long s = esrc[e];
       T xv[TP::NX], wv[NPG];
 #pragma unroll
@@ -139,13 +141,32 @@ __device__ __forceinline__ void tp_fwd_row(const TPArgs<T>& a, int i, T* Gs, int
       else TP::template fwd1<T>(xv, Gs + e * TP::NG, wv, acc);
     }
   }
+  if constexpr (ES > 1) {  // buf: [ES - 1][kShareRows][C]
+#pragma unroll
+    for (int k0 = 0; k0 < NMG; k0 += kShareRows) {
+      __syncthreads();
+      if (share > 0) {
+#pragma unroll
+        for (int k = k0; k < k0 + kShareRows && k < NMG; ++k) buf[((share - 1) * kShareRows + k - k0) * C + c] = acc[k];
+      }
+      __syncthreads();
+      if (share == 0) {
+#pragma unroll
+        for (int k = k0; k < k0 + kShareRows && k < NMG; ++k)
+#pragma unroll
+          for (int w = 0; w < ES - 1; ++w) acc[k] += buf[(w * kShareRows + k - k0) * C + c];
+      }
+    }
+    if (share > 0) return;
+  }
   T* Mi = a.M + ((long long)i * TP::NM + M0) * C;
 #pragma unroll
   for (int k = 0; k < NMG; ++k) Mi[k * C + c] = acc[k];
 }
 // LIST: block b works on kListRows entries of the row list of a partial pass (tp_row); otherwise block i = target i.
-template <typename T, typename TP, int GRP, bool ENV, bool RT, bool LIST>
+template <typename T, typename TP, int GRP, bool ENV, bool RT, bool LIST, int ES>
 __global__ void __maxnreg__(128) tp_fwd_kernel(const TPArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) T Gs[kEdgeBatch * TP::NG];
   __shared__ int esrc[kEdgeBatch];
   __shared__ RtEdge<T> rts[RT ? kEdgeBatch : 1];
@@ -153,10 +174,10 @@ __global__ void __maxnreg__(128) tp_fwd_kernel(const TPArgs<T> a) {
     for (int it = blockIdx.x * kListRows; it < (blockIdx.x + 1) * kListRows; ++it) {
       const int i = tp_row(a, it);
       if (i < 0) break;
-      tp_fwd_row<T, TP, GRP, ENV, RT>(a, i, Gs, esrc, rts);
+      tp_fwd_row<T, TP, GRP, ENV, RT, 1>(a, i, Gs, esrc, rts, nullptr);
     }
   } else {
-    tp_fwd_row<T, TP, GRP, ENV, RT>(a, blockIdx.x, Gs, esrc, rts);
+    tp_fwd_row<T, TP, GRP, ENV, RT, ES>(a, blockIdx.x, Gs, esrc, rts, reinterpret_cast<T*>(smem_raw));
   }
 }
 
@@ -189,18 +210,25 @@ struct RtBwdWeights {
   }
 };
 
-// The same for path weights held in memory (W[edge][path][channel]): each weight is loaded one path ahead of its use
-// and its gradient stored as soon as it is known.
+// The same for path weights held in memory (W[edge][path][channel]): each weight is loaded kWeightsAhead paths ahead of its use and
+// its gradient stored as soon as it is known (dW may be W: a path's weight is read before its gradient is written, and no other thread
+// touches either).
+constexpr int kWeightsAhead = 4;
 template <typename T, typename TP, bool ENV>
 struct ArrayBwdWeights {
+  static constexpr int Q = TP::NP < kWeightsAhead ? TP::NP : kWeightsAhead;
   const T* W;   // this edge's weights, this thread's channel: path p at W[p * C]
   T* dW;
   int C;
-  T u, next, w_now, du;
-  __device__ __forceinline__ void start() { du = T(0); next = W[0]; }
+  T u, next[Q], w_now, du;
+  __device__ __forceinline__ void start() {
+    du = T(0);
+#pragma unroll
+    for (int p = 0; p < Q; ++p) next[p] = W[p * C];
+  }
   template <int P> __device__ __forceinline__ T get() {
-    w_now = next;
-    if (P + 1 < TP::NP) next = W[(P + 1) * C];
+    w_now = next[P % Q];
+    if (P + Q < TP::NP) next[P % Q] = W[(P + Q) * C];
     return ENV ? w_now * u : w_now;
   }
   template <int P> __device__ __forceinline__ void put(T dwv) {
@@ -239,6 +267,18 @@ __device__ __forceinline__ T warp_sums(const T (&in)[N], int lane, int& k) {
   return v[0];
 }
 
+// Edges [beg, end) of target i that this block works on: all of them, or its share where gridDim.y blocks deal them.  Everything the
+// backward pass produces belongs to one edge.
+template <typename T>
+__device__ __forceinline__ void tp_share(const TPArgs<T>& a, int i, int& beg, int& end) {
+  beg = a.rowptr[i]; end = a.rowptr[i + 1];
+  if (gridDim.y > 1) {
+    const int deg = end - beg, first = beg;
+    beg = first + (int)((long long)deg * blockIdx.y / gridDim.y);
+    end = first + (int)((long long)deg * (blockIdx.y + 1) / gridDim.y);
+  }
+}
+
 // Dynamic shared memory: [NM][C] message gradient of the target | G rows | dY partial sums.
 template <typename T, typename TP, bool ENV, bool RT>
 __device__ __forceinline__ void tp_bwd_row(const TPArgs<T>& a, int i, unsigned char* smem_raw, T* red_u, T* red_r, RtEdge<T>* rts,
@@ -249,7 +289,8 @@ __device__ __forceinline__ void tp_bwd_row(const TPArgs<T>& a, int i, unsigned c
   T* Gs = gMs + TP::NM * C;                          // [kEdgeBatch][NG]
   T* red = Gs + kEdgeBatch * TP::NG;                 // [kEdgeBatch][8 warps][D]
   const int rt_first = blockDim.x > 32 ? 32 : 0;  // the second warp (when there is one) prepares the interpolation
-  const int beg = a.rowptr[i], end = a.rowptr[i + 1];
+  int beg, end;
+  tp_share(a, i, beg, end);
   const T* gMi = a.gM + (long long)i * TP::NM * C;
   if (beg < end)
     for (int k = 0; k < TP::NM; ++k) gMs[k * C + c] = gMi[k * C + c];  // each thread reads and writes only its own column
@@ -380,8 +421,10 @@ __global__ void tp_bwd_scalar_kernel(const TPArgs<T> a) {
   __shared__ T env_s[EB];
   __shared__ RtEdge<T> rts[RT ? EB : 1];
   const T* gMi = a.gM + (long long)i * D * C;
+  int beg, end;
+  tp_share(a, i, beg, end);
+  if (beg >= end) return;
   for (int k = 0; k < D; ++k) gMs[k * C + c] = gMi[k * C + c];
-  const int beg = a.rowptr[i], end = a.rowptr[i + 1];
   for (int e0 = beg; e0 < end; e0 += EB) {
     const int nb = min(EB, end - e0);
     __syncthreads();
@@ -547,15 +590,23 @@ cudaError_t launch_chunk_src_sum(const T* dxe_chunk, const int* keys, const int*
   return cudaGetLastError();
 }
 
+// Few targets: four sets of threads share the edges of one, so that a cell of a few hundred atoms does not walk its edge lists with
+// two warps per SM.  Rank 2, 64 channels, fp64, 256 targets of 42 edges: 60 -> 26 us, first layer 15 -> 12.  Above twelve warps per SM
+// the chip has other targets to work on while one waits.
+template <typename T>
+bool share_fwd_edges(const TPArgs<T>& a) {
+  return a.split_sums && a.C <= 128 && (long long)a.n_seg * (a.C / 32) <= 12LL * kSMs && a.n_edges >= 16LL * a.n_seg;
+}
+template <typename T, typename TP, int GRP, bool ENV, bool RT>
+void launch_fwd_grp(const TPArgs<T>& a, cudaStream_t s) {
+  if (a.row_ids) tp_fwd_kernel<T, TP, GRP, ENV, RT, true, 1><<<(a.n_seg + kListRows - 1) / kListRows, a.C, 0, s>>>(a);
+  else if (share_fwd_edges(a)) tp_fwd_kernel<T, TP, GRP, ENV, RT, false, 4><<<a.n_seg, 4 * a.C, sizeof(T) * 3 * kShareRows * a.C, s>>>(a);
+  else tp_fwd_kernel<T, TP, GRP, ENV, RT, false, 1><<<a.n_seg, a.C, 0, s>>>(a);
+}
 template <typename T, typename TP, bool ENV, bool RT>
 cudaError_t launch_fwd_v(const TPArgs<T>& a, cudaStream_t s) {
-  if (a.row_ids) {
-    tp_fwd_kernel<T, TP, 0, ENV, RT, true><<<(a.n_seg + kListRows - 1) / kListRows, a.C, 0, s>>>(a);
-    if (TP::NGRP > 1) tp_fwd_kernel<T, TP, 1, ENV, RT, true><<<(a.n_seg + kListRows - 1) / kListRows, a.C, 0, s>>>(a);
-  } else {
-    tp_fwd_kernel<T, TP, 0, ENV, RT, false><<<a.n_seg, a.C, 0, s>>>(a);
-    if (TP::NGRP > 1) tp_fwd_kernel<T, TP, 1, ENV, RT, false><<<a.n_seg, a.C, 0, s>>>(a);
-  }
+  launch_fwd_grp<T, TP, 0, ENV, RT>(a, s);
+  if constexpr (TP::NGRP > 1) launch_fwd_grp<T, TP, 1, ENV, RT>(a, s);
   return cudaGetLastError();
 }
 template <typename T, typename TP>
@@ -565,6 +616,15 @@ cudaError_t launch_fwd_t(const TPArgs<T>& a, cudaStream_t s) {
     return a.env ? launch_fwd_v<T, TP, true, true>(a, s) : launch_fwd_v<T, TP, false, true>(a, s);
   }
   return a.env ? launch_fwd_v<T, TP, true, false>(a, s) : launch_fwd_v<T, TP, false, false>(a, s);
+}
+// Blocks per target in the backward pass: up to twelve warps per SM, while a share keeps at least one batch of edges.
+// Rank 2, 64 channels, fp64, 256 targets of 42 edges (four blocks per target): 173 -> 54 us, of which the weights that are on
+// their way four paths ahead; first layer 40 -> 18 us.
+template <typename T>
+int bwd_shares(const TPArgs<T>& a) {
+  int shares = 1;
+  while (shares < 16 && (long long)a.n_seg * (a.C / 32) * shares < 12LL * kSMs && a.n_edges >= 2LL * kEdgeBatch * shares * a.n_seg) shares *= 2;
+  return shares;
 }
 template <typename T, typename TP, bool RT>
 cudaError_t launch_bwd_v(const TPArgs<T>& a, size_t smem, cudaStream_t s) {
@@ -583,8 +643,9 @@ cudaError_t launch_bwd_v(const TPArgs<T>& a, size_t smem, cudaStream_t s) {
     if (a.env) tp_bwd_kernel<T, TP, true, RT, true><<<(a.n_seg + kListRows - 1) / kListRows, a.C, smem, s>>>(a);
     else tp_bwd_kernel<T, TP, false, RT, true><<<(a.n_seg + kListRows - 1) / kListRows, a.C, smem, s>>>(a);
   } else {
-    if (a.env) tp_bwd_kernel<T, TP, true, RT, false><<<a.n_seg, a.C, smem, s>>>(a);
-    else tp_bwd_kernel<T, TP, false, RT, false><<<a.n_seg, a.C, smem, s>>>(a);
+    const dim3 grid(a.n_seg, bwd_shares(a));
+    if (a.env) tp_bwd_kernel<T, TP, true, RT, false><<<grid, a.C, smem, s>>>(a);
+    else tp_bwd_kernel<T, TP, false, RT, false><<<grid, a.C, smem, s>>>(a);
   }
   return cudaGetLastError();
 }
@@ -599,7 +660,7 @@ cudaError_t launch_bwd_scalar(const TPArgs<T>& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     configured[dev] = smem;
   }
-  tp_bwd_scalar_kernel<T, TP, ENV, RT><<<a.n_seg, a.C, smem, s>>>(a);
+  tp_bwd_scalar_kernel<T, TP, ENV, RT><<<dim3(a.n_seg, bwd_shares(a)), a.C, smem, s>>>(a);
   return cudaGetLastError();
 }
 template <typename T, typename TP>
