@@ -781,12 +781,12 @@ struct Model : ModelBase {
 
   // ---- GEMM helpers ----------------------------------------------------------------------------
   static void add_problem(GemmBatch<T>& gb, const T* A, long long a_s1, long long a_s2, int q, int K, const T* Bm, int N,
-                          T* Cm, long long c_s1, long long c_s2, const T* bias, int accumulate, long long b_gs = 0,
+                          T* Cm, long long c_s1, long long c_s2, const T* bias, int accumulate, int join = 0, long long b_gs = 0,
                           long long bias_gs = 0, const int* tile_ptr = nullptr) {
     GemmProblem<T>& p = gb.p[gb.n_problems++];
     p.A = A; p.B = Bm; p.C = Cm; p.bias = bias; p.q = q; p.N = N; p.K = K;
     p.a_s1 = a_s1; p.a_s2 = a_s2; p.c_s1 = c_s1; p.c_s2 = c_s2;
-    p.b_group_stride = b_gs; p.bias_group_stride = bias_gs; p.accumulate = accumulate; p.tile_ptr = tile_ptr;
+    p.b_group_stride = b_gs; p.bias_group_stride = bias_gs; p.accumulate = accumulate; p.join = join; p.tile_ptr = tile_ptr;
   }
   static GemmBatch<T> plain_batch(long long n_atoms) {
     GemmBatch<T> gb;
@@ -807,22 +807,31 @@ struct Model : ModelBase {
   // accumulate = kJoin: the product is added to that of the spec before it (same rows and result), in one pass over both K ranges
   // where the tensor-core path takes them.
   static constexpr int kJoin = 2;
-  // The specs of one call, a run of joined ones at a time: tcgen05 for fp32 models where every shape of the run fits, the other
-  // kernels for the rest, joined products in launches of their own.
+  // The specs of one call, a run of joined ones at a time: tcgen05 for fp32 models where every shape of the run fits and there is
+  // enough work, the kernels of gemm.cuh for the rest.
+  //
+  // kSmallLinear: multiply-adds of a call up to which the CUDA cores are done before a launch of the tensor-core kernel has set up its
+  // tensor memory, barriers and tiles: one evaluation of 32 atoms at rank 2, 64 channels 216 -> 173 us, at rank 3, 128 channels
+  // 356 -> 279; 108 atoms 226 -> 187 and 420 -> 380; a limit of 64 Mi loses at 256 and 1 372 atoms (232 against 227 us, 446 against
+  // 437), one of 16 Mi at 128 channels (518 against 503 at 256 atoms).  Models with the edge block keep one path for every linear: their energies
+  // feel the rounding of the linears most (3e-5 between the two paths), and that is not to show between systems of different size.
+  static constexpr long long kSmallLinear = 32LL << 20;
   template <typename Spec, typename FillTc, typename Add>
   cudaError_t run_specs(const std::vector<Spec>& specs, long long n_atoms, cudaStream_t s, const GemmBatch<T>& empty, FillTc&& fill, Add&& add) {
     TcLinearProblem probs[kMaxLinears];
     int n_tc = 0;
-    std::vector<std::vector<const Spec*>> rest;  // by place in the run
+    GemmBatch<T> gb = empty;
     cudaError_t err = cudaSuccess;
+    long long work = 0;
+    for (const Spec& sp : specs) work += n_atoms * sp.q * sp.K * sp.N;
     for (size_t i = 0, j; i < specs.size() && err == cudaSuccess; i = j) {
-      bool tc = kTensorCore;
+      bool tc = kTensorCore && (tece_mask || work > kSmallLinear);
       for (j = i; j < specs.size() && (j == i || specs[j].accumulate == kJoin); ++j) tc = tc && tc_linear_supported(specs[j].N, specs[j].K);
-      for (size_t k = i; k < j && !tc; ++k) {
-        if (rest.size() <= k - i) rest.resize(k - i + 1);
-        rest[k - i].push_back(&specs[k]);
+      if (!tc) {
+        if (gb.n_problems + (int)(j - i) > kMaxProblems) { err = launch_gemm(gb, n_atoms, s); gb = empty; }
+        for (size_t k = i; k < j; ++k) add(gb, specs[k], specs[k].accumulate == 1, specs[k].accumulate == kJoin);
+        continue;
       }
-      if (!tc) continue;
       if (n_tc + (int)(j - i) > kMaxLinears) { err = launch_tc_linear(probs, n_tc, dev_error, s); n_tc = 0; }
       for (size_t k = i; k < j; ++k) {
         const Spec& sp = specs[k];
@@ -837,12 +846,7 @@ struct Model : ModelBase {
       }
     }
     if (err == cudaSuccess && n_tc > 0) err = launch_tc_linear(probs, n_tc, dev_error, s);
-    for (size_t level = 0; level < rest.size(); ++level)
-      for (size_t i = 0; i < rest[level].size() && err == cudaSuccess; i += kMaxProblems) {
-        GemmBatch<T> gb = empty;
-        for (size_t k = i; k < rest[level].size() && k < i + kMaxProblems; ++k) add(gb, *rest[level][k], level > 0 || rest[level][k]->accumulate == 1);
-        err = launch_gemm(gb, n_atoms, s);
-      }
+    if (err == cudaSuccess && gb.n_problems > 0) err = launch_gemm(gb, n_atoms, s);
     return err;
   }
   // Plain (not per-species) linears.  c_map: row a of the results belongs to atom c_map[a] (nullptr: the same order).
@@ -850,8 +854,8 @@ struct Model : ModelBase {
     GemmBatch<T> gb = plain_batch(n_atoms);
     gb.c_atom_map = c_map;
     return run_specs(specs, n_atoms, s, gb, [&](TcLinearProblem& h, const LinSpec&) { h.atom_map = c_map; },
-                     [&](GemmBatch<T>& g, const LinSpec& sp, int accumulate) {
-                       add_problem(g, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, accumulate);
+                     [&](GemmBatch<T>& g, const LinSpec& sp, int accumulate, int join) {
+                       add_problem(g, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, accumulate, join);
                      });
   }
 
@@ -878,8 +882,8 @@ struct Model : ModelBase {
                        h.b_group_stride = (long long)sp.K * sp.N; h.bias_group_stride = sp.N;
                        h.b_tiled = 1;  // the packed per-species hi / lo parts are K-tile-major (read once per pass, straight from DRAM)
                      },
-                     [&](GemmBatch<T>& g, const SpeciesSpec& sp, int accumulate) {
-                       add_problem(g, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, accumulate,
+                     [&](GemmBatch<T>& g, const SpeciesSpec& sp, int accumulate, int join) {
+                       add_problem(g, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, accumulate, join,
                                    (long long)sp.K * sp.N, sp.N, tiles(b, sp.q / 2));
                      });
   }

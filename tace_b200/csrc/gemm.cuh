@@ -15,7 +15,10 @@
 // all ranks of a linear together: 144 tiles for 148 SMs), and what bound the former 64 x 64 CUDA-core tiles was one block per
 // four SMs walking its K loop with nothing in flight: K = N = 64 on those rows 18 -> 5 us, the 10 944 x 704 x 64 GEMMs of the
 // radial MLP 139 / 255 -> 48 / 45 us.
-// FP32 shapes that the tcgen05 kernel does not take: CUDA cores, 32 x 64 x 16 tiles, 256 threads, 2 x 4 outputs per thread.
+// FP32 runs on the CUDA cores in the same tiles: linears with so little work that a launch of the tcgen05 kernel is nothing but its
+// latency, and shapes which that kernel does not take.
+//
+// Problems can be joined to the one before them: their products are summed in the same accumulators.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -38,12 +41,14 @@ struct GemmProblem {
   long long c_s1, c_s2; // same for C rows
   long long b_group_stride, bias_group_stride;
   int accumulate;       // 0: C = ..., 1: C += ...
+  int join;             // the product is added to that of the problem before (same rows and result)
   const int* tile_ptr;  // grouped launches: [n_groups+1] prefix sum of ceil(atoms_g * q / 32)
 };
 
 template <typename T>
 struct GemmBatch {
   GemmProblem<T> p[kMaxProblems];
+  int first[kMaxProblems + 1];  // first problem of result i (set by launch_gemm)
   int n_problems;
   int n_groups;          // 1 unless per-species
   const int* group_ptr;  // [n_groups+1] atom ranges in `atom_map` order, or nullptr (=> all atoms)
@@ -97,7 +102,8 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool ok) 
 static __global__ void __launch_bounds__(128) gemm_f64_kernel(const GemmBatch<double> batch) {
   constexpr int BM = kGemmBM, BN = 32, BK = 16, ST = 3;
   constexpr int LA = BK + 4, LB = BN + 4;  // leading dimensions: a fragment's rows start four 8-byte banks apart
-  const GemmProblem<double>& P = batch.p[blockIdx.z];
+  const int first = batch.first[blockIdx.z], last = batch.first[blockIdx.z + 1];
+  const GemmProblem<double>& P = batch.p[first];
   int group, row0, M, a_begin;
   const int col0 = blockIdx.y * BN;
   if (col0 >= P.N || !gemm_tile(batch, P, group, row0, M, a_begin)) return;
@@ -111,18 +117,28 @@ static __global__ void __launch_bounds__(128) gemm_f64_kernel(const GemmBatch<do
   gemm_row(batch, P, a_begin, row0 + ar, M, ao, co);
   if (ap == 0) c_off[ar] = co;
   const int bk = tid >> 3, bp = tid & 7;
-  const double* Bg = P.B + group * P.b_group_stride + col0;
-  const int K = P.K, N = P.N, steps = (K + BK - 1) / BK;
+  const double *Ag = P.A, *Bg = P.B + group * P.b_group_stride + col0;
+  const int N = P.N;
+  int steps = 0;
+  for (int i = first; i < last; ++i) steps += (batch.p[i].K + BK - 1) / BK;
+  int cur = first, k0 = 0, K = P.K;  // problem and place in its K range that the next load is for
   auto load = [&](int step) {
-    const int s = step % ST, k0 = step * BK;
+    const int s = step % ST;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int k = k0 + 2 * (ap + 4 * h);
       const bool ok = ao >= 0 && k < K;
-      cp_async16(&As[s][ar * LA + 2 * (ap + 4 * h)], ok ? P.A + ao + k : P.A, ok);
+      cp_async16(&As[s][ar * LA + 2 * (ap + 4 * h)], ok ? Ag + ao + k : Ag, ok);
       const int c = 2 * (bp + 8 * h);
       const bool okb = k0 + bk < K && col0 + c < N;
       cp_async16(&Bs[s][bk * LB + c], okb ? Bg + (long long)(k0 + bk) * N + c : P.B, okb);
+    }
+    k0 += BK;
+    if (k0 >= K && cur + 1 < last) {
+      const GemmProblem<double>& Q = batch.p[++cur];
+      long long unused;
+      gemm_row(batch, Q, a_begin, row0 + ar, M, ao, unused);
+      Ag = Q.A; Bg = Q.B + group * Q.b_group_stride + col0; K = Q.K; k0 = 0;
     }
   };
 #pragma unroll
@@ -172,99 +188,121 @@ static __global__ void __launch_bounds__(128) gemm_f64_kernel(const GemmBatch<do
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) gemm_kernel(const GemmBatch<T> batch) {
-  constexpr int BM = kGemmBM, BN = 64, BK = 16;
-  const GemmProblem<T>& P = batch.p[blockIdx.z];
+// 32 x 32 tiles, K in steps of 32 through a ring of four cp.async stages; four sets of 64 threads with 4 x 4 outputs each take a quarter
+// of every step and their sums are added at the end (with one output row per thread and no such sets, shared-memory reads bounded
+// the longer K loops: 10.6 against 7.2 us for the joined products of 32 atoms, rank 2, 64 channels).  What is left is latency: 2.9 us for
+// 288 rows of K = N = 64, of which a third is the launch; the tensor-core kernel takes 5.5.
+static __global__ void __launch_bounds__(256) gemm_f32_kernel(const GemmBatch<float> batch) {
+  constexpr int BM = kGemmBM, BN = 32, BK = 32, ST = 4, LA = BK + 4;  // rows of A start four banks apart
+  const int first = batch.first[blockIdx.z], last = batch.first[blockIdx.z + 1];
+  const GemmProblem<float>& P = batch.p[first];
   int group, row0, M, a_begin;
   const int col0 = blockIdx.y * BN;
   if (col0 >= P.N || !gemm_tile(batch, P, group, row0, M, a_begin)) return;
-
-  __shared__ T As[BK][BM + 4];
-  __shared__ T Bs[BK][BN + 4];
-  __shared__ long long a_off[BM];
-  __shared__ long long c_off[BM];
-
-  const int tid = threadIdx.x;
-  if (tid < BM) gemm_row(batch, P, a_begin, row0 + tid, M, a_off[tid], c_off[tid]);
+  __shared__ __align__(16) float As[ST][BM * LA];
+  __shared__ __align__(16) float Bs[ST][BK * BN];
+  // this thread's piece of a stage: four values of A (row r, k 4 p ...) and of B (k r, columns 4 p ...)
+  const int r = threadIdx.x >> 3, p = threadIdx.x & 7, N = P.N;
+  long long ao, co;
+  gemm_row(batch, P, a_begin, row0 + r, M, ao, co);
+  const float *Ag = P.A, *Bg = P.B + group * P.b_group_stride + col0;
+  int steps = 0;
+  for (int i = first; i < last; ++i) steps += (batch.p[i].K + BK - 1) / BK;
+  int cur = first, k0 = 0, K = P.K;  // problem and place in its K range that the next load is for
+  auto load = [&](int step) {
+    float* a = &As[step % ST][r * LA + 4 * p];
+    float* b = &Bs[step % ST][r * BN + 4 * p];
+    const int k = k0 + 4 * p, kb = k0 + r, c = col0 + 4 * p;
+    const bool ok = ao >= 0 && k < K, okb = kb < K && c < N;
+    cp_async16(a, ok ? Ag + ao + k : Ag, ok);
+    cp_async16(b, okb ? Bg + (long long)kb * N + 4 * p : P.B, okb);
+    k0 += BK;
+    if (k0 >= K && cur + 1 < last) {
+      const GemmProblem<float>& Q = batch.p[++cur];
+      long long unused;
+      gemm_row(batch, Q, a_begin, row0 + r, M, ao, unused);
+      Ag = Q.A; Bg = Q.B + group * Q.b_group_stride + col0; K = Q.K; k0 = 0;
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < ST - 1; ++i) {
+    if (i < steps) load(i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // outputs of this thread: rows tr + 8 i, columns 4 p .. 4 p + 3, summed over k = 8 set .. 8 set + 7 of every step
+  const int set = threadIdx.x >> 6, tr = (threadIdx.x >> 3) & 7;
+  float acc[4][4] = {};
+  for (int i = 0; i < steps; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+    __syncthreads();  // stage i has landed for everybody, and everybody is done with the stage the next load overwrites
+    if (i + ST - 1 < steps) load(i + ST - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* A = &As[i % ST][tr * LA + 8 * set];
+    const float* B = &Bs[i % ST][8 * set * BN + 4 * p];
+#pragma unroll
+    for (int k = 0; k < 8; k += 4) {
+      float4 a[4], b[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        a[j] = *reinterpret_cast<const float4*>(A + 8 * j * LA + k);
+        b[j] = *reinterpret_cast<const float4*>(B + (k + j) * BN);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          const float x = j == 0 ? a[m].x : j == 1 ? a[m].y : j == 2 ? a[m].z : a[m].w;
+          acc[m][0] = fmaf(x, b[j].x, acc[m][0]); acc[m][1] = fmaf(x, b[j].y, acc[m][1]);
+          acc[m][2] = fmaf(x, b[j].z, acc[m][2]); acc[m][3] = fmaf(x, b[j].w, acc[m][3]);
+        }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-
-  const T* __restrict__ Bg = P.B + group * P.b_group_stride;
-  const int tx = tid % 16, ty = tid / 16;  // 16 x 16 thread grid, 2x4 outputs each
-  T acc[2][4];
+  float* sums = &As[0][0];  // [set][32][32]: the ring is done with
+  static_assert(sizeof(As) >= 4 * BM * BN * sizeof(float), "the sums of the sets reuse the ring");
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int m = 0; m < 4; ++m)
+    *reinterpret_cast<float4*>(sums + (set * BM + tr + 8 * m) * BN + 4 * p) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
+  __syncthreads();
+  const int col = col0 + 4 * p;
+  if (co < 0 || col >= N) return;
+  float4 v = *reinterpret_cast<const float4*>(sums + r * BN + 4 * p);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
-
-  for (int k0 = 0; k0 < P.K; k0 += BK) {
-    // A tile: 32 rows x 16 k  (512 elements, 2 per thread); k fastest for coalescing
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int idx = tid + i * 256;
-      const int r = idx / BK, kk = idx % BK;
-      const long long ao = a_off[r];
-      T v = T(0);
-      if (ao >= 0 && k0 + kk < P.K) v = P.A[ao + k0 + kk];
-      As[kk][r] = v;
-    }
-    // B tile: 16 k x 64 cols
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int idx = tid + i * 256;
-      const int kk = idx / BN, cc = idx % BN;
-      T v = T(0);
-      if (k0 + kk < P.K && col0 + cc < P.N) v = Bg[(long long)(k0 + kk) * P.N + col0 + cc];
-      Bs[kk][cc] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      T a[2], b[4];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) a[i] = As[kk][ty * 2 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * b[j];
-    }
-    __syncthreads();
+  for (int q = 1; q < 4; ++q) {
+    const float4 o = *reinterpret_cast<const float4*>(sums + (q * BM + r) * BN + 4 * p);
+    v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
   }
-
-  const T* bias = P.bias ? P.bias + group * P.bias_group_stride : nullptr;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const long long co = c_off[ty * 2 + i];
-    if (co < 0) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int col = col0 + tx * 4 + j;
-      if (col >= P.N) continue;
-      T v = acc[i][j];
-      if (bias) v += bias[col];
-      if (P.accumulate) v += P.C[co + col];
-      P.C[co + col] = v;
-    }
-  }
+  const float* bias = P.bias ? P.bias + group * P.bias_group_stride + col : nullptr;
+  float* dst = P.C + co + col;
+  if (bias) { v.x += bias[0]; v.y += bias[1]; v.z += bias[2]; v.w += bias[3]; }
+  if (P.accumulate) { const float4 o = *reinterpret_cast<const float4*>(dst); v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
+  *reinterpret_cast<float4*>(dst) = v;
 }
 
 // n_atoms_total: atoms covered by the launch (all groups together); sizes grid.x.
 template <typename T>
-inline cudaError_t launch_gemm(const GemmBatch<T>& b, long long n_atoms_total, cudaStream_t stream) {
-  int maxN = 0, maxq = 0;
+inline cudaError_t launch_gemm(GemmBatch<T>& b, long long n_atoms_total, cudaStream_t stream) {
+  int maxN = 0, maxq = 0, n_results = 0;
+  constexpr int V = 16 / sizeof(T);
   for (int i = 0; i < b.n_problems; ++i) {
-    maxN = b.p[i].N > maxN ? b.p[i].N : maxN;
-    maxq = b.p[i].q > maxq ? b.p[i].q : maxq;
+    const GemmProblem<T>& p = b.p[i];
+    maxN = p.N > maxN ? p.N : maxN;
+    maxq = p.q > maxq ? p.q : maxq;
+    // whole 16-byte pieces everywhere: channels come in multiples of 32, other widths of four, buffers from arenas
+    if (((reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.B) | reinterpret_cast<uintptr_t>(p.C)) & 15) != 0 ||
+        (p.a_s1 | p.a_s2 | p.c_s1 | p.c_s2 | p.b_group_stride | p.K | p.N) % V != 0)
+      return cudaErrorInvalidValue;
+    if (p.join && (i == 0 || p.q != b.p[i - 1].q || p.N != b.p[i - 1].N)) return cudaErrorInvalidValue;
+    if (!p.join) b.first[n_results++] = i;
   }
+  b.first[n_results] = b.n_problems;
   if (n_atoms_total <= 0 || maxN <= 0 || b.n_problems <= 0) return cudaSuccess;
   long long tiles = (n_atoms_total * maxq + kGemmBM - 1) / kGemmBM;
   if (b.group_ptr) tiles += b.n_groups;  // every group may end with a partial tile
-  if constexpr (std::is_same<T, double>::value)
-    gemm_f64_kernel<<<dim3((unsigned)tiles, (maxN + 31) / 32, b.n_problems), 128, 0, stream>>>(b);
-  else
-    gemm_kernel<T><<<dim3((unsigned)tiles, (maxN + 63) / 64, b.n_problems), 256, 0, stream>>>(b);
+  const dim3 grid((unsigned)tiles, (maxN + 31) / 32, n_results);
+  if constexpr (std::is_same<T, double>::value) gemm_f64_kernel<<<grid, 128, 0, stream>>>(b);
+  else gemm_f32_kernel<<<grid, 256, 0, stream>>>(b);
   return cudaGetLastError();
 }
 
