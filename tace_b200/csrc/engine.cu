@@ -802,8 +802,13 @@ struct Model : ModelBase {
     const T* A; long long a_s1, a_s2; int q, K;
     std::string wname, wname_t; int N;
     T* Cm; long long c_s1, c_s2; const T* bias;
-    int accumulate;  // Cm += instead of Cm =
+    int accumulate = 0;          // Cm += instead of Cm =
+    T* act_out = nullptr;        // fused activations of GemmProblem (double precision)
+    const T* act_in = nullptr;
   };
+  // the layers of the radial MLP of fp64 models apply their activations themselves (a LayerNorm in between needs whole rows)
+  bool fused_activations() const { return !kTensorCore && !element2; }
+
   // accumulate = kJoin: the product is added to that of the spec before it (same rows and result), in one pass over both K ranges
   // where the tensor-core path takes them.
   static constexpr int kJoin = 2;
@@ -856,6 +861,7 @@ struct Model : ModelBase {
     return run_specs(specs, n_atoms, s, gb, [&](TcLinearProblem& h, const LinSpec&) { h.atom_map = c_map; },
                      [&](GemmBatch<T>& g, const LinSpec& sp, int accumulate, int join) {
                        add_problem(g, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, accumulate, join);
+                       g.p[g.n_problems - 1].act_out = sp.act_out; g.p[g.n_problems - 1].act_in = sp.act_in;
                      });
   }
 
@@ -910,7 +916,8 @@ struct Model : ModelBase {
     for (size_t i = 0; i < ts.size(); ++i) {
       r.mlp[i] = ea.mlp[ts[i]];
       r.Z1[i] = b.lay[ts[i]].Z1;
-      r.H1[i] = nh == 1 ? b.lay[ts[i]].H3 : b.lay[ts[i]].Hact;  // activation of the first hidden layer
+      // activation of the first hidden layer; the last one's has to end up in H3, and fused layers go back and forth between the two
+      r.H1[i] = nh == 1 || (nh == 3 && fused_activations()) ? b.lay[ts[i]].H3 : b.lay[ts[i]].Hact;
       r.dH1[i] = dh1_buffer(b.lay[ts[i]]);
     }
     return r;
@@ -1044,10 +1051,11 @@ struct Model : ModelBase {
     CKL(launch_edge_mlp_in(er, s));
     const long long n64 = Ec * kHidden;
     const bool ln = element2;  // LayerNorm before every hidden activation
+    const bool fused = fused_activations();
     for (int j = 0; j < nh; ++j) {  // hidden layer j: activation, then (unless it is the last) the next 64 x 64 layer
       const bool last_hidden = (j == nh - 1);
       for (int t : ts) {
-        if (!ln && j == 0) break;  // launch_edge_mlp_in wrote silu(Z1) already
+        if (fused || (!ln && j == 0)) break;  // launch_edge_mlp_in or the layer before wrote the activation already
         const LayerBufs& lb = b.lay[t];
         const T* z = j == 0 ? lb.Z1 : j == 1 ? lb.Z2 : lb.Z3;
         T* h = last_hidden ? lb.H3 : lb.Hact;
@@ -1064,8 +1072,11 @@ struct Model : ModelBase {
         const std::string pre = "t" + std::to_string(t) + ".";
         const std::string an = j == 0 ? "A1" : "A2";
         const LayerBufs& lb = b.lay[t];
-        sp.push_back({lb.Hact, kHidden, 0, 1, kHidden, pre + an, pre + an + "t", kHidden, j == 0 ? lb.Z2 : lb.Z3, kHidden,
-                      0, mlp_bias ? w(pre + (j == 0 ? "b1" : "b2")) : nullptr});
+        T* const in = fused && (nh - 1 - j) % 2 == 0 ? lb.H3 : lb.Hact;
+        LinSpec spec{in, kHidden, 0, 1, kHidden, pre + an, pre + an + "t", kHidden, j == 0 ? lb.Z2 : lb.Z3, kHidden,
+                     0, mlp_bias ? w(pre + (j == 0 ? "b1" : "b2")) : nullptr};
+        if (fused) spec.act_out = in == lb.H3 ? lb.Hact : lb.H3;
+        sp.push_back(spec);
       }
       CKL(run_linear(sp, Ec, s));
     }
@@ -1093,6 +1104,7 @@ struct Model : ModelBase {
       for (int t : ts) {
         const LayerBufs& lb = b.lay[t];
         T* g = (j == nh - 1) ? lb.H3 : lb.Hact;
+        if (fused_activations()) break;  // the product that made g applied the derivative
         if (ln) {
           const std::string pre = "t" + std::to_string(t) + ".ln" + std::to_string(j);
           CKL(launch_ln_silu_bwd(g, j == 1 ? lb.Z2 : lb.Z3, w(pre + "g"), w(pre + "b"), Ec, s));
@@ -1107,7 +1119,9 @@ struct Model : ModelBase {
         const LayerBufs& lb = b.lay[t];
         const T* g = (j == nh - 1) ? lb.H3 : lb.Hact;
         T* dst = (j == nh - 1) ? lb.Hact : lb.Z3;
-        sp.push_back({g, kHidden, 0, 1, kHidden, pre + an + "t", pre + an, kHidden, dst, kHidden, 0, nullptr});
+        LinSpec spec{g, kHidden, 0, 1, kHidden, pre + an + "t", pre + an, kHidden, dst, kHidden, 0, nullptr};
+        if (fused_activations() && j == 2) spec.act_in = lb.Z2;  // (j == 1: launch_edge_mlp_out applies the first layer's)
+        sp.push_back(spec);
       }
       CKL(run_linear(sp, Ec, s));
     }
@@ -1143,6 +1157,7 @@ struct Model : ModelBase {
       if (!backward) add_problem(gb, lb.H3, kHidden, 0, 1, kHidden, w(pre + "W3"), NW, lb.W, (long long)NW, 0,
                                  mlp_bias ? w(pre + "b3") : nullptr, 0);
       else add_problem(gb, lb.W, (long long)NW, 0, 1, NW, w(pre + "W3t"), kHidden, lb.H3, kHidden, 0, nullptr, 0);
+      if (backward && fused_activations() && nh > 1) gb.p[0].act_in = nh == 3 ? lb.Z3 : lb.Z2;
       CKL(launch_gemm(gb, Ec, s));
     }
     return TACE_OK;

@@ -14,7 +14,9 @@
 // 16 through a ring of three cp.async stages.  The tiles are small because the systems are (a 256-atom cell has 2 304 rows in
 // all ranks of a linear together: 144 tiles for 148 SMs), and what bound the former 64 x 64 CUDA-core tiles was one block per
 // four SMs walking its K loop with nothing in flight: K = N = 64 on those rows 18 -> 5 us, the 10 944 x 704 x 64 GEMMs of the
-// radial MLP 139 / 255 -> 48 / 45 us.
+// radial MLP 139 / 255 -> 48 / 45 us (64 x 64 tiles of the tensor instruction 50 / 69: too few blocks).  The layers of the radial MLP
+// have their activation, or the derivative of the one before, in the epilogue (act_out, act_in): eight launches of 5 us less per
+// evaluation of 256 atoms against 1 to 6 us more in the products they leave.
 // FP32 runs on the CUDA cores in the same tiles: linears with so little work that a launch of the tcgen05 kernel is nothing but its
 // latency, and shapes which that kernel does not take.
 //
@@ -42,6 +44,9 @@ struct GemmProblem {
   long long b_group_stride, bias_group_stride;
   int accumulate;       // 0: C = ..., 1: C += ...
   int join;             // the product is added to that of the problem before (same rows and result)
+  // double precision: silu(C) stored as well, or C = result * silu'(act_in), both laid out like C; or nullptr
+  T* act_out;
+  const T* act_in;
   const int* tile_ptr;  // grouped launches: [n_groups+1] prefix sum of ceil(atoms_g * q / 32)
 };
 
@@ -183,7 +188,12 @@ static __global__ void __launch_bounds__(128) gemm_f64_kernel(const GemmBatch<do
       double2* dst = reinterpret_cast<double2*>(P.C + at + col);
       if (bias) { v.x += bias[col]; v.y += bias[col + 1]; }
       if (P.accumulate) { const double2 o = *dst; v.x += o.x; v.y += o.y; }
+      if (P.act_in) {
+        const double2 z = *reinterpret_cast<const double2*>(P.act_in + at + col);
+        v.x *= silu_grad_(z.x); v.y *= silu_grad_(z.y);
+      }
       *dst = v;
+      if (P.act_out) *reinterpret_cast<double2*>(P.act_out + at + col) = make_double2(silu_(v.x), silu_(v.y));
     }
   }
 }
