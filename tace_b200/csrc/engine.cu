@@ -818,19 +818,27 @@ struct Model : ModelBase {
   // kSmallLinear: multiply-adds of a call up to which the CUDA cores are done before a launch of the tensor-core kernel has set up its
   // tensor memory, barriers and tiles: one evaluation of 32 atoms at rank 2, 64 channels 216 -> 173 us, at rank 3, 128 channels
   // 356 -> 279; 108 atoms 226 -> 187 and 420 -> 380; a limit of 64 Mi loses at 256 and 1 372 atoms (232 against 227 us, 446 against
-  // 437), one of 16 Mi at 128 channels (518 against 503 at 256 atoms).  Models with the edge block keep one path for every linear: their energies
-  // feel the rounding of the linears most (3e-5 between the two paths), and that is not to show between systems of different size.
-  static constexpr long long kSmallLinear = 32LL << 20;
+  // 437), one of 16 Mi at 128 channels (518 against 503 at 256 atoms).  Models with the edge block keep one path for the linears of the forward
+  // pass: their energies feel the rounding of the linears most (3e-5 between the two paths), and that is not to show between systems
+  // of different size.
+  // Four times as many where the tensor cores have at most kFewTiles tiles, each walking a long K loop on one SM (128 rows,
+  // K = 4 352: 73 -> 43 us).
+  static constexpr long long kSmallLinear = 32LL << 20, kFewTiles = 8;
+  bool backward_pass = false;  // what forward() is enqueuing
   template <typename Spec, typename FillTc, typename Add>
   cudaError_t run_specs(const std::vector<Spec>& specs, long long n_atoms, cudaStream_t s, const GemmBatch<T>& empty, FillTc&& fill, Add&& add) {
     TcLinearProblem probs[kMaxLinears];
     int n_tc = 0;
     GemmBatch<T> gb = empty;
     cudaError_t err = cudaSuccess;
-    long long work = 0;
-    for (const Spec& sp : specs) work += n_atoms * sp.q * sp.K * sp.N;
+    long long work = 0, tiles = 0;  // tiles of the tensor-core kernel
+    for (const Spec& sp : specs) {
+      work += n_atoms * sp.q * sp.K * sp.N;
+      if (sp.accumulate != kJoin) tiles += (n_atoms * sp.q + 127) / 128 * ((sp.N + 127) / 128);
+    }
+    const bool small = work <= (tiles <= kFewTiles ? 4 : 1) * kSmallLinear;
     for (size_t i = 0, j; i < specs.size() && err == cudaSuccess; i = j) {
-      bool tc = kTensorCore && (tece_mask || work > kSmallLinear);
+      bool tc = kTensorCore && ((tece_mask && !backward_pass) || !small);
       for (j = i; j < specs.size() && (j == i || specs[j].accumulate == kJoin); ++j) tc = tc && tc_linear_supported(specs[j].N, specs[j].K);
       if (!tc) {
         if (gb.n_problems + (int)(j - i) > kMaxProblems) { err = launch_gemm(gb, n_atoms, s); gb = empty; }
@@ -1166,6 +1174,7 @@ struct Model : ModelBase {
 
   int forward(const TaceBatch* bt, const TaceOutputs* o, void* ws, size_t ws_bytes, cudaStream_t s) override {
     if (!bt || !o || !ws) return TACE_ERR_INVALID_ARGUMENT;
+    backward_pass = false;
     if (weights_missing != 0) {
       weights_missing = 0;
       for (const auto& e : weights) weights_missing += e.set ? 0 : 1;
@@ -1474,6 +1483,7 @@ struct Model : ModelBase {
     if (!need_grad) { PH("end"); return TACE_OK; }
 
     // ---- layers, backward
+    backward_pass = true;
     for (int t = NL_ - 1; t >= 0; --t) {
       const LayerPlan& p = layers[t];
       LayerBufs& lb = b.lay[t];
