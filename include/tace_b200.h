@@ -279,7 +279,8 @@ int tace_nl_fill(const double* positions, const double* lattice, const uint8_t* 
                  int64_t* edge_index, int32_t* edge_shifts, void* workspace, size_t workspace_bytes, tace_stream_t stream);
 
 /* The same pair with the row pointers computed on the device and the preparation done once: tace_nl_rows fills counts and
- * row_ptr[n_atoms + 1] (row_ptr[n_atoms] = number of edges) and leaves its bins in the workspace; tace_nl_fill_rows, called
+ * row_ptr[n_atoms + 1] (row_ptr[n_atoms] = number of edges) and leaves its bins in the workspace (with up to 8 192 atoms
+ * also the first sources of every target, where there is room for them); tace_nl_fill_rows, called
  * with the same structures and that workspace untouched, writes the edges.  n_targets >= 0: only the first n_targets atoms
  * get rows (the others, ghost copies, act as sources only).  shift_type: TACE_F32 / TACE_F64 writes the shifts as reals of
  * that type, anything else as int32.  Same edges, same order. */
