@@ -46,13 +46,10 @@ def _checked_species(species, n_atoms: int, n_elements: int) -> np.ndarray:
     return species
 
 
-def build_batch(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cutoff: float, dtype: torch.dtype,
-                device: torch.device) -> Dict[str, torch.Tensor]:
-    """``batch`` as returned by ``tace_b200.synth.collate``: host numpy arrays or (pinned) CPU
-    tensors; an optional ``species`` entry (index into the model's element list) replaces the
-    lookup from ``atomic_numbers``.  Uploads the structure, builds the neighbour list on ``device``
-    and returns the model input dictionary."""
-    n_el = len(model_numbers)
+def _structures_on_device(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cutoff: float, dtype: torch.dtype,
+                          device: torch.device, returned):
+    """Uploads the structures of ``batch`` and builds their neighbour list: the fields named in ``returned`` on the device, the
+    addresses of all, edge list and shifts."""
     positions = np.asarray(batch["positions"])
     pbc_host = np.asarray(batch["pbc"], dtype=np.uint8)
     lattice_host = np.asarray(batch["lattice"], dtype=np.float64)
@@ -63,11 +60,21 @@ def build_batch(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cuto
         cells = np.stack([complete_cell(c, positions[a:b], p, cutoff)
                           for c, p, a, b in zip(lattice_host, pbc_host, ptr_host[:-1], ptr_host[1:])])
     n, b = len(positions), len(lattice_host)
-    species_host = (_checked_species(batch["species"], n, n_el) if "species" in batch
+    species_host = (_checked_species(batch["species"], n, len(model_numbers)) if "species" in batch
                     else z_to_index(np.asarray(batch["atomic_numbers"]), model_numbers))
     up, at = _upload(n, b, np.float64 if dtype == torch.float64 else np.float32,
-                     (positions, cells, ptr_host, batch["batch"], positions, lattice_host, ptr_host, species_host, pbc_host), device)
-    edge_index, shifts = _list_at(device, n, b, (at["pos64"], at["cells"], at["pbc"], at["ptr32"]), cutoff, -1, dtype)
+                     (positions, cells, ptr_host, batch["batch"], positions, lattice_host, ptr_host, species_host, pbc_host), device, returned)
+    return up, at, *_list_at(device, n, b, (at["pos64"], at["cells"], at["pbc"], at["ptr32"]), cutoff, -1, dtype)
+
+
+def build_batch(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cutoff: float, dtype: torch.dtype,
+                device: torch.device) -> Dict[str, torch.Tensor]:
+    """``batch`` as returned by ``tace_b200.synth.collate``: host numpy arrays or (pinned) CPU
+    tensors; an optional ``species`` entry (index into the model's element list) replaces the
+    lookup from ``atomic_numbers``.  Uploads the structure, builds the neighbour list on ``device``
+    and returns the model input dictionary."""
+    up, at, edge_index, shifts = _structures_on_device(batch, model_numbers, cutoff, dtype, device, ("batch", "ptr", "positions", "lattice", "species"))
+    n, n_el = len(up["positions"]), len(model_numbers)
     node_attrs = torch.empty(n, n_el, dtype=dtype, device=device)
     with _lib.on_device(device):
         _lib.check(_lib.load().tace_one_hot(at["species"], n, n_el, _lib.dtype_code(dtype), node_attrs.data_ptr(),
@@ -82,6 +89,15 @@ def build_batch(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cuto
         "batch": up["batch"],
         "ptr": up["ptr"],
     }
+
+
+def model_inputs(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cutoff: float, dtype: torch.dtype,
+                 device: torch.device) -> Dict[str, torch.Tensor]:
+    """What ``TensorModel.forward`` reads of ``build_batch``'s dictionary, in the types that it uses, for callers who hand it on and
+    keep nothing: no one-hot attributes beside the species, and structure offsets that need no conversion."""
+    up, _, edge_index, shifts = _structures_on_device(batch, model_numbers, cutoff, dtype, device, ("ptr32", "positions", "lattice", "species"))
+    return {"positions": up["positions"], "lattice": up["lattice"], "species": up["species"], "edge_index": edge_index, "edge_shifts": shifts,
+            "ptr": up["ptr32"]}
 
 
 _STAGED_BYTES = 1 << 20  # up to here the fields travel as one block; above, the copy into the block costs more than the transfers it saves
@@ -99,14 +115,11 @@ def _layout(n: int, b: int, real):
     return tuple(places), at
 
 
-_RETURNED = ("batch", "ptr", "positions", "lattice", "species")  # fields of the model's input; the others only go to the list kernels
-
-
-def _upload(n: int, b: int, real, values, device: torch.device):
-    """Host values (in the order of ``_layout``) on the device: (tensors, addresses) by name.  A small batch is packed into one
-    pinned block, every field at a multiple of 16 bytes and already in its final type: one transfer instead of one transfer and
-    one conversion kernel per field.  The pinned block comes from torch's caching host allocator, which keeps it until the
-    transfer has finished."""
+def _upload(n: int, b: int, real, values, device: torch.device, returned):
+    """Host values (in the order of ``_layout``) on the device: tensors of the fields in ``returned`` and the addresses of all, by
+    name.  A small batch is packed into one pinned block, every field at a multiple of 16 bytes and already in its final type: one
+    transfer instead of one transfer and one conversion kernel per field.  The pinned block comes from torch's caching host
+    allocator, which keeps it until the transfer has finished."""
     places, size = _layout(n, b, real)
     if size > _STAGED_BYTES:
         up = {name: torch.as_tensor(v).to(device, non_blocking=True).to(_TORCH[kind]).reshape(shape).contiguous()
@@ -119,7 +132,7 @@ def _upload(n: int, b: int, real, values, device: torch.device):
     dev = block.to(device, non_blocking=True)
     base, typed, up = dev.data_ptr(), {}, {}
     for name, kind, shape, lo in places:
-        if name in _RETURNED:
+        if name in returned:
             if kind not in typed:
                 typed[kind] = dev.view(_TORCH[kind])
             up[name] = typed[kind].as_strided(shape, _STRIDES[len(shape)], lo // _BYTES[kind])

@@ -13,7 +13,7 @@ from typing import List, Optional, Union
 import numpy as np
 import torch
 
-from ..graph import build_batch
+from ..graph import model_inputs
 from ..models import TensorModel, create_model
 
 try:  # ASE is optional: without it the class still works with any object exposing the four getters below
@@ -126,7 +126,7 @@ class TACEAseCalc(Calculator):
             "batch": np.zeros(n, dtype=np.int64),
             "ptr": np.array([0, n], dtype=np.int64),
         }
-        data = build_batch(host, self.atomic_numbers, self.cutoff, self.dtype, self.device)
+        data = model_inputs(host, self.atomic_numbers, self.cutoff, self.dtype, self.device)
         outs = self.model(data)
         fetch = _fetch([outs[p] for p in self.target_property if outs.get(p) is not None])
         self.results = {}

@@ -18,7 +18,8 @@ import torch
 
 from ..graph import z_to_index  # noqa: F401  (re-exported for drivers that prepare species themselves)
 from ..models import TensorModel
-from ..neighbour_list import neighbor_list_batch
+from ..lib import TaceError
+from ..neighbour_list import _list_on_device, neighbor_list_batch
 from .ase_calculator import load_tace
 
 try:  # pragma: no cover - torch_sim is not part of the test environment
@@ -144,13 +145,16 @@ class TACETorchSimCalc(_Base):
                 and all(isinstance(p, (bool, int)) for p in pbc) and state.row_vector_cell.numel() == 9 * self.n_systems):
             # this package's own list, without working the systems' offsets out again (they belong to `system_idx`) and
             # without the edges' system indices, which the model does not read
-            edge_index, unit_shifts = neighbor_list_batch(state.positions, state.row_vector_cell,
-                                                          self._periodic_rows(tuple(map(bool, pbc)), state.positions.device),
-                                                          self._ptr32, self.r_max)
+            if state.positions.device.type != "cuda":
+                raise TaceError("tace_b200 neighbour lists run on CUDA devices only")
+            edge_index, unit_shifts = _list_on_device(state.positions.to(torch.float64).contiguous(),
+                                                      state.row_vector_cell.to(torch.float64).reshape(-1, 3, 3).contiguous(),
+                                                      self._periodic_rows(tuple(map(bool, pbc)), state.positions.device),
+                                                      self._ptr32, self.r_max, -1, self._dtype)
         else:
             edge_index, _mapping, unit_shifts = self.neighbor_list_fn(state.positions, state.row_vector_cell, pbc, self.r_max, self.system_idx)
         out = self.model({
-            "ptr": self.ptr, "node_attrs": self.node_attrs, "species": self.species, "batch": self.system_idx, "pbc": state.pbc,
+            "ptr": self._ptr32, "node_attrs": self.node_attrs, "species": self.species, "batch": self.system_idx, "pbc": state.pbc,
             "lattice": state.row_vector_cell, "positions": state.positions, "edge_index": edge_index, "edge_shifts": unit_shifts,
         })
         results: Dict[str, torch.Tensor] = {}
