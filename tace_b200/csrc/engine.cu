@@ -398,9 +398,10 @@ struct Model : ModelBase {
   double t_row_scale[16], t_p_scale[12];
   int m0 = 1;  // 1: every rank gated (gate_m0 = True); 0: e3nn Gate, scalars through SiLU (gate_m0 = False)
   std::vector<LayerPlan> layers;
-  std::vector<WeightEntry> weights;
+  std::vector<WeightEntry> weights;  // the first n_listed are the caller's, n_unset of them not set yet; the others are folded from them
+  int n_listed = 0, n_unset = 0;
+  bool folded = true;
   std::unordered_map<std::string, int> weight_index;
-  int weights_missing = -1;   // entries not set yet (-1: not counted)
   T* arena = nullptr;
   long long arena_numel = 0;
   // perm: the `row` elements of atom i are row perm[i] (nullptr: atom order)
@@ -601,6 +602,14 @@ struct Model : ModelBase {
     add_weight("scale", (long long)n_fid * n_el);
     add_weight("e0", (long long)n_fid * n_el);
     if (zbl) { add_weight("zbl.z", n_el); add_weight("zbl.rcov", n_el); add_weight("zbl.par", 2); }
+    n_listed = n_unset = (int)weights.size();
+    folded = tece_mask == 0;
+    if (folded) add_weight("emb_up", (long long)n_el * C);
+    for (int t = 0; t < NL_ && folded; ++t)
+      for (int l : layers[t].out_ls) {
+        for (int j = 0; j < c.correlation; ++j) add_weight(coef_name(t, j, "f", l), (long long)n_el * coef_rows(t, j, l) * C);
+        if (l == 0) add_weight("t" + std::to_string(t) + ".cf.b", (long long)n_el * C);
+      }
     if (cudaMalloc(&arena, sizeof(T) * (size_t)arena_numel) != cudaSuccess) return TACE_ERR_CUDA;
     if (cudaMemset(arena, 0, sizeof(T) * (size_t)arena_numel) != cudaSuccess) return TACE_ERR_CUDA;
     if (cudaMalloc(&dev_error, sizeof(int)) != cudaSuccess || cudaMemset(dev_error, 0, sizeof(int)) != cudaSuccess)
@@ -608,16 +617,78 @@ struct Model : ModelBase {
     return TACE_OK;
   }
 
-  int weight_count() const override { return (int)weights.size(); }
+  int weight_count() const override { return n_listed; }
   int weight_info(int i, const char** name, int64_t* numel) const override {
-    if (i < 0 || i >= (int)weights.size()) return TACE_ERR_INVALID_ARGUMENT;
+    if (i < 0 || i >= n_listed) return TACE_ERR_INVALID_ARGUMENT;
     if (name) *name = weights[i].name.c_str();
     if (numel) *numel = weights[i].numel;
     return TACE_OK;
   }
+  // ---- folded weights ----------------------------------------------------------------------
+  // Two linears that follow each other without anything in between are one: the final linear of the product goes into the
+  // per-species coefficients before it (every order and rank: c0, c1, c2, and their bias, to which the skip connection's is added),
+  // the first linear_up into the species embedding.  The products are taken here, once, when the weights are set, with sums in
+  // double precision.  Per layer and pass one linear less, and the skip connection joins the sum of the coefficients: two launches
+  // of 3 to 20 us each way and a pass over the rows per linear: 1 372 atoms 588 -> 570 us, 64 crystals 2 681 -> 2 639, 256 atoms in
+  // double precision 749 -> 730.  Models with the edge block keep their linears apart: their energies feel the rounding of a linear
+  // most (2.2e-5 between the two forms, where the others move by 3e-6).
+  //   cJ.lL [n_el][K][C] stays as it was set; cJf.lL is the folded matrix, cJT.lL its transpose, cJ.lL_hi/_lo and cJT.lL_hi/_lo the
+  //   K-tile-major TF32 parts of both (what the caller sets under these names is the same before folding, and is not kept).
+  static std::string coef_name(int t, int order, const char* form, int l) {
+    return "t" + std::to_string(t) + ".c" + std::to_string(order) + form + ".l" + std::to_string(l);
+  }
+  long long coef_rows(int t, int order, int l) const {  // out_ls holds 0..lmax, so l is also the index
+    const LayerPlan& p = layers[t];
+    return (long long)C * (order == 0 ? 1 : order == 1 ? p.pb.k[l] : p.pb3.k[l]);
+  }
+  T* w_mut(const std::string& name) {
+    const auto it = weight_index.find(name);
+    return it == weight_index.end() ? nullptr : arena + weights[it->second].offset;
+  }
+  cudaError_t fold_coefs(int t, int order, int l) {
+    const std::string lin = "t" + std::to_string(t) + ".lin.l" + std::to_string(l), c = coef_name(t, order, "", l), cT = coef_name(t, order, "T", l);
+    return launch_fold_linear(w(c), w(lin), w_mut(coef_name(t, order, "f", l)), w_mut(cT), w_mut(c + "_hi"), w_mut(c + "_lo"), w_mut(cT + "_hi"),
+                              w_mut(cT + "_lo"), n_el, (int)coef_rows(t, order, l), C, cudaStream_t(0));
+  }
+  cudaError_t fold_bias(int t) {
+    const std::string pre = "t" + std::to_string(t) + ".";
+    return launch_fold_rows(w(pre + "c.b"), w(pre + "lin.l0"), w(pre + "lin.b"), w(pre + "res.b"), w_mut(pre + "cf.b"), n_el, C, cudaStream_t(0));
+  }
+  cudaError_t fold_embedding() {
+    return launch_fold_rows(w("emb"), w("t0.up.l0"), w("t0.up.b"), (const T*)nullptr, w_mut("emb_up"), n_el, C, cudaStream_t(0));
+  }
+  // Order and form of a coefficient name "tN.cJ...": J and true where its content is derived, -1 for every other name.
+  static int coef_order(const std::string& name, bool& derived) {
+    const size_t dot = name.find('.');
+    if (name[0] != 't' || dot == std::string::npos || name.size() < dot + 5 || name[dot + 1] != 'c' || name[dot + 2] < '0' || name[dot + 2] > '2') return -1;
+    derived = name[dot + 3] == 'T' || name.back() < '0' || name.back() > '9';
+    return name[dot + 2] - '0';
+  }
+  // Takes the folded weights again that depend on `name`; all of them when the last weight has arrived.
+  cudaError_t fold_after(const std::string& name, bool all) {
+    const size_t dot = name.find('.');
+    const int layer = name[0] == 't' && dot != std::string::npos ? atoi(name.c_str() + 1) : -1;
+    const std::string stem = layer >= 0 ? name.substr(dot + 1) : "";
+    bool derived = false, any = false;
+    const int order = coef_order(name, derived);
+    cudaError_t e = cudaSuccess;
+    if (all || name == "emb" || name == "t0.up.l0" || name == "t0.up.b") { e = fold_embedding(); any = true; }
+    for (int t = 0; t < NL_ && e == cudaSuccess; ++t) {
+      if (!all && t != layer) continue;
+      for (int l : layers[t].out_ls) {
+        const std::string ls = ".l" + std::to_string(l);
+        for (int j = 0; j < cfg.correlation && e == cudaSuccess; ++j)
+          if (all || stem == "lin" + ls || (order == j && stem == "c" + std::to_string(j) + ls)) { e = fold_coefs(t, j, l); any = true; }
+      }
+      if (e == cudaSuccess && (all || stem == "lin.l0" || stem == "lin.b" || stem == "c.b" || stem == "res.b")) { e = fold_bias(t); any = true; }
+    }
+    return e == cudaSuccess && any ? cudaStreamSynchronize(cudaStream_t(0)) : e;  // a later pass may run on any stream
+  }
+
   int set_weight(const char* name, const void* host, int64_t numel) override {
     if (!name || !host) return TACE_ERR_INVALID_ARGUMENT;
-    for (auto& e : weights) {
+    for (int i = 0; i < n_listed; ++i) {
+      WeightEntry& e = weights[i];
       if (e.name == name) {
         if (numel != e.numel) return TACE_ERR_INVALID_ARGUMENT;
         std::vector<T> cubic;
@@ -641,11 +712,16 @@ struct Model : ModelBase {
           }
           host = cubic.data();
         }
-        if (cudaMemcpy(arena + e.offset, host, sizeof(T) * (size_t)numel, cudaMemcpyHostToDevice) != cudaSuccess)
+        bool derived = false;
+        if (!folded || coef_order(e.name, derived) < 0) derived = false;
+        if (!derived && cudaMemcpy(arena + e.offset, host, sizeof(T) * (size_t)numel, cudaMemcpyHostToDevice) != cudaSuccess)
           return TACE_ERR_CUDA;
         if (e.name == "bessel") memcpy(host_bessel, host, sizeof(T) * kNumBessel);
         if (e.name == "bessel_pref") memcpy(host_bessel + kNumBessel, host, sizeof(T));
+        const bool last = !e.set && n_unset == 1;
+        if (!e.set) --n_unset;
         e.set = true;
+        if (folded && n_unset == 0 && (last || !derived) && fold_after(e.name, last) != cudaSuccess) return TACE_ERR_CUDA;
         return TACE_OK;
       }
     }
@@ -708,7 +784,7 @@ struct Model : ModelBase {
       shared_W = ar.take<T>((size_t)Ec * np_max * C);
     }
     b.lay.resize(NL_);
-    T* prev_h = ar.take<T>((size_t)N * C);   // h_0: species embedding, scalar channels
+    T* prev_h = folded ? nullptr : ar.take<T>((size_t)N * C);  // the species embedding, where it is not folded into linear_up
     T* prev_gh = nullptr;
     for (int t = 0; t < NL_; ++t) {
       const LayerPlan& p = layers[t];
@@ -761,7 +837,7 @@ struct Model : ModelBase {
       lb.gAs = ar.take<T>((size_t)NL * D * C);
       lb.gout_s = ar.take<T>((size_t)NL * p.Dout * C);
       lb.hs = p.has_res ? ar.take<T>((size_t)NL * p.Din * C) : nullptr;
-      lb.out = ar.take<T>((size_t)NL * p.Dout * C);
+      lb.out = folded ? nullptr : ar.take<T>((size_t)NL * p.Dout * C);
       lb.h_out = ar.take<T>((size_t)N * p.Dout * C);
       lb.gh_out = ar.take<T>((size_t)N * p.Dout * C);
       prev_h = lb.h_out;
@@ -1175,11 +1251,7 @@ struct Model : ModelBase {
   int forward(const TaceBatch* bt, const TaceOutputs* o, void* ws, size_t ws_bytes, cudaStream_t s) override {
     if (!bt || !o || !ws) return TACE_ERR_INVALID_ARGUMENT;
     backward_pass = false;
-    if (weights_missing != 0) {
-      weights_missing = 0;
-      for (const auto& e : weights) weights_missing += e.set ? 0 : 1;
-      if (weights_missing) return TACE_ERR_WEIGHTS_MISSING;
-    }
+    if (n_unset != 0) return TACE_ERR_WEIGHTS_MISSING;
     const long long N = bt->n_atoms, NL = bt->n_local, E = bt->n_edges;
     const int B = bt->n_graphs;
     if (N < 0 || NL < 0 || NL > N || E < 0 || B <= 0 || !bt->species || !bt->graph_ptr || (E > 0 && !bt->edge_index))
@@ -1298,21 +1370,20 @@ struct Model : ModelBase {
     // ---- layers, forward
     bool wigner_done = false, tece_seen = false;
     PH("embed");
-    CKL(launch_species_gather(w("emb"), b.species, b.lay[0].h_in, (int)N, C, s));
+    CKL(launch_species_gather(w(folded ? "emb_up" : "emb"), b.species, folded ? b.lay[0].x : b.lay[0].h_in, (int)N, C, s));  // ghosts too
     for (int t = 0; t < NL_; ++t) {
       const LayerPlan& p = layers[t];
       LayerBufs& lb = b.lay[t];
       const std::string pre = "t" + std::to_string(t) + ".";
       const std::string ts = std::to_string(t);
-      PH(("t" + ts + ".fwd.linear_up").c_str());
-      const long long n_up = p.scalar_src ? N : NL;  // layer 0 embeds every atom; later layers own only local rows
-      {  // linear_up
+      if (t > 0 || !folded) {  // linear_up (the first layer's is part of the folded embedding)
+        PH(("t" + ts + ".fwd.linear_up").c_str());
         std::vector<LinSpec> sp;
         for (int l : p.in_ls)
           sp.push_back({lb.h_in + (long long)l * l * C, (long long)p.Din * C, C, 2 * l + 1, C, pre + "up.l" + std::to_string(l),
                         pre + "upT.l" + std::to_string(l), C, lb.x + (long long)l * l * C, (long long)p.tp.NX * C, C,
                         l == 0 ? w(pre + "up.b") : nullptr});
-        CKL(run_linear(sp, n_up, s));
+        CKL(run_linear(sp, t == 0 ? N : NL, s));  // layer 0 embeds every atom; later layers own only local rows
       }
       const T* x_src = lb.x;
       const bool split = overlap && lb.xx && !p.tece;
@@ -1404,28 +1475,34 @@ struct Model : ModelBase {
       if (cfg.correlation >= 3) CKL(launch_pb3_fwd(lb.As, lb.B2, lb.B3, (int)NL, L, p.last ? -1 : Ln, C, s));
       {
         std::vector<SpeciesSpec> sp;
-        // the products of all correlation orders add up in one pass per rank
+        // the products of all correlation orders and the skip connection from the layer input add up in one pass per rank
+        const bool res = p.has_res && !res_identity && folded;
+        const std::string f = folded ? "f.l" : ".l";
+        if (res) CKL(launch_gather_rows(lb.h_in, b.species_perm, lb.hs, NL, p.Din * C, s));
         for (size_t i = 0; i < p.out_ls.size(); ++i) {
           const int l = p.out_ls[i];
           const std::string ls = std::to_string(l);
-          T* out = lb.out + (long long)l * l * C;
+          T* out = (folded ? lb.h_out : lb.out) + (long long)l * l * C;
           sp.push_back({bilinear ? lb.XY + (long long)l * l * 2 * C : lb.As + (long long)l * l * C, (long long)D * C * (bilinear ? 2 : 1),
-                        (long long)C * (bilinear ? 2 : 1), 2 * l + 1, C, pre + "c0.l" + ls, pre + "c0T.l" + ls, C, out,
-                        (long long)p.Dout * C, C, l == 0 ? w(pre + "c.b") : nullptr, true, 0});
+                        (long long)C * (bilinear ? 2 : 1), 2 * l + 1, C, pre + "c0" + f + ls, pre + "c0T.l" + ls, C, out,
+                        (long long)p.Dout * C, C, l == 0 ? w(pre + (folded ? "cf.b" : "c.b")) : nullptr, true, 0});
           if (cfg.correlation >= 2) {
             const int K = p.pb.k[i] * C;
-            sp.push_back({lb.B2 + (long long)p.pb.base[i] * C, (long long)p.pb.NB * C, K, 2 * l + 1, K, pre + "c1.l" + ls, pre + "c1T.l" + ls,
+            sp.push_back({lb.B2 + (long long)p.pb.base[i] * C, (long long)p.pb.NB * C, K, 2 * l + 1, K, pre + "c1" + f + ls, pre + "c1T.l" + ls,
                           C, out, (long long)p.Dout * C, C, nullptr, true, kJoin});
           }
           if (cfg.correlation >= 3) {
             const int K = p.pb3.k[i] * C;
-            sp.push_back({lb.B3 + (long long)p.pb3.base[i] * C, (long long)p.pb3.NB * C, K, 2 * l + 1, K, pre + "c2.l" + ls, pre + "c2T.l" + ls,
+            sp.push_back({lb.B3 + (long long)p.pb3.base[i] * C, (long long)p.pb3.NB * C, K, 2 * l + 1, K, pre + "c2" + f + ls, pre + "c2T.l" + ls,
                           C, out, (long long)p.Dout * C, C, nullptr, true, kJoin});
           }
+          if (res)
+            sp.push_back({lb.hs + (long long)l * l * C, (long long)p.Din * C, C, 2 * l + 1, C, pre + "res.l" + ls, pre + "resT.l" + ls, C, out,
+                          (long long)p.Dout * C, C, nullptr, true, kJoin});
         }
         CKL(run_species_linear(sp, b, NL, s));
       }
-      {
+      if (!folded) {
         std::vector<LinSpec> sp;
         for (int l : p.out_ls)
           sp.push_back({lb.out + (long long)l * l * C, (long long)p.Dout * C, C, 2 * l + 1, C, pre + "lin.l" + std::to_string(l),
@@ -1435,7 +1512,7 @@ struct Model : ModelBase {
       }
       if (p.has_res && res_identity) {  // tace/models/_e3nn/residual.py:216-250: the ranks the output keeps, copied over
         CKL(launch_add_rows(lb.h_out, (long long)p.Dout * C, lb.h_in, (long long)p.Din * C, NL, p.Dout * C, s));
-      } else if (p.has_res) {  // per-species skip connection from the layer input
+      } else if (p.has_res && !folded) {  // per-species skip connection from the layer input
         CKL(launch_gather_rows(lb.h_in, b.species_perm, lb.hs, NL, p.Din * C, s));
         std::vector<SpeciesSpec> sp;
         for (int l : p.out_ls)
@@ -1493,7 +1570,9 @@ struct Model : ModelBase {
       if (cfg.use_alllayer && t + 1 < NL_)  // this layer's own linear read-out, on top of what the layer above sent down
         CKL(launch_readout_linear_bwd(lb.gh_out, (long long)p.Dout * C, b.ro_factor, w("ro.lin" + ts), b.atom_graph, bt->fidelity,
                                       (int)NL, C, s));
-      {  // through the final linear
+      if (folded) {  // the final linear is part of the coefficients
+        CKL(launch_gather_rows(lb.gh_out, b.species_perm, lb.gout_s, NL, p.Dout * C, s));
+      } else {  // through the final linear
         std::vector<LinSpec> sp;
         for (int l : p.out_ls)
           sp.push_back({lb.gh_out + (long long)l * l * C, (long long)p.Dout * C, C, 2 * l + 1, C, pre + "linT.l" + std::to_string(l),
@@ -1661,8 +1740,8 @@ struct Model : ModelBase {
         if (p.has_res && res_identity) {
           CKL(launch_add_rows(lb.gh_in, (long long)p.Din * C, lb.gh_out, (long long)p.Dout * C, NL, p.Dout * C, s));
         } else if (p.has_res) {
-          CKL(launch_gather_rows(lb.gh_out, b.species_perm, lb.gout_s, NL, p.Dout * C, s));
-          std::vector<SpeciesSpec> sp2;
+          if (!folded) CKL(launch_gather_rows(lb.gh_out, b.species_perm, lb.gout_s, NL, p.Dout * C, s));
+          std::vector<SpeciesSpec> sp2;  // gout_s: the species-sorted gradient of this layer's output
           for (int l : p.out_ls)
             sp2.push_back({lb.gout_s + (long long)l * l * C, (long long)p.Dout * C, C, 2 * l + 1, C, pre + "resT.l" + std::to_string(l),
                            pre + "res.l" + std::to_string(l), C, lb.gh_in + (long long)l * l * C, (long long)p.Din * C, C, nullptr, true, 1});

@@ -82,6 +82,11 @@ template <typename T> cudaError_t launch_chunk_src_sum(const T* dxe_chunk, const
                                                        long long k1, long long key_base, T* gx, int row_len, cudaStream_t s);
 
 // ---- per-atom element-wise kernels (node_kernels.cu) -----------------------------------------
+// weights set: per-species matrices (rows) times the linear that follows them, in every form the linears read
+template <typename T>
+cudaError_t launch_fold_linear(const T* c, const T* lin, T* f, T* fT, T* hi, T* lo, T* hiT, T* loT, int n_groups, int K, int C, cudaStream_t s);
+template <typename T>
+cudaError_t launch_fold_rows(const T* rows, const T* lin, const T* bias, const T* extra, T* out, int n_groups, int C, cudaStream_t s);
 // x0[n][c] = table[species[n]][c]
 template <typename T> cudaError_t launch_species_gather(const T* table, const int* species, T* out, int n, int C, cudaStream_t s);
 // gate (tace/models/_e3nn/nonlinear.py:125-135): Gt = [(L+1)C gates | D*C gated] per atom.

@@ -102,6 +102,64 @@ cudaError_t launch_species_gather(const T* table, const int* species, T* out, in
   return cudaGetLastError();
 }
 
+// ---- folded weights -------------------------------------------------------------------------------
+// Product of per-species matrices c [n_el][K][C] and a common one, lin [C][C], in the forms that the linears read: f = [K][C], fT = [C][K],
+// and for fp32 the TF32 high part and residual of both, K-tile-major ([C / 32][K][32] and [K / 32][C][32] per species).  Run when weights
+// are set, not per evaluation: a block per eight rows of a species, a thread per column, sums in double precision.
+constexpr int kFoldRows = 8;
+template <typename T>
+__global__ void __launch_bounds__(128) fold_linear_kernel(const T* __restrict__ c, const T* __restrict__ lin, T* f, T* fT, T* hi, T* lo, T* hiT, T* loT,
+                                                          int K, int C) {
+  const int k0 = blockIdx.x * kFoldRows, rows = min(kFoldRows, K - k0);
+  const long long g = (long long)blockIdx.y * K * C;
+  for (int n = threadIdx.x; n < C; n += blockDim.x) {
+    double acc[kFoldRows];
+#pragma unroll
+    for (int r = 0; r < kFoldRows; ++r) acc[r] = 0.0;
+    for (int j = 0; j < C; ++j) {
+      const double b = (double)lin[(long long)j * C + n];
+#pragma unroll
+      for (int r = 0; r < kFoldRows; ++r) acc[r] += (double)c[g + (long long)(k0 + min(r, rows - 1)) * C + j] * b;
+    }
+#pragma unroll
+    for (int r = 0; r < kFoldRows; ++r) {
+      if (r >= rows) break;
+      const int k = k0 + r;
+      const T v = (T)acc[r];
+      f[g + (long long)k * C + n] = v;
+      fT[g + (long long)n * K + k] = v;
+      if constexpr (sizeof(T) == 4) {
+        const float h = __uint_as_float(__float_as_uint(v) & 0xFFFFE000u), d = v - h;
+        const long long at = g + ((long long)(n / 32) * K + k) * 32 + n % 32, atT = g + ((long long)(k / 32) * C + n) * 32 + k % 32;
+        hi[at] = h; lo[at] = d; hiT[atT] = h; loT[atT] = d;
+      }
+    }
+  }
+}
+template <typename T>
+cudaError_t launch_fold_linear(const T* c, const T* lin, T* f, T* fT, T* hi, T* lo, T* hiT, T* loT, int n_groups, int K, int C, cudaStream_t s) {
+  if (!c || !lin || !f || !fT || (sizeof(T) == 4 && (!hi || !lo || !hiT || !loT || K % 32 || C % 32))) return cudaErrorInvalidValue;
+  fold_linear_kernel<T><<<dim3((K + kFoldRows - 1) / kFoldRows, n_groups), 128, 0, s>>>(c, lin, f, fT, hi, lo, hiT, loT, K, C);
+  return cudaGetLastError();
+}
+// out[g] = rows[g] lin + bias (+ extra[g]), a block per row
+template <typename T>
+__global__ void __launch_bounds__(128) fold_rows_kernel(const T* __restrict__ rows, const T* __restrict__ lin, const T* __restrict__ bias,
+                                                        const T* __restrict__ extra, T* out, int C) {
+  const T* row = rows + (long long)blockIdx.x * C;
+  for (int n = threadIdx.x; n < C; n += blockDim.x) {
+    double acc = (double)bias[n] + (extra ? (double)extra[(long long)blockIdx.x * C + n] : 0.0);
+    for (int j = 0; j < C; ++j) acc += (double)row[j] * (double)lin[(long long)j * C + n];
+    out[(long long)blockIdx.x * C + n] = (T)acc;
+  }
+}
+template <typename T>
+cudaError_t launch_fold_rows(const T* rows, const T* lin, const T* bias, const T* extra, T* out, int n_groups, int C, cudaStream_t s) {
+  if (!rows || !lin || !bias || !out) return cudaErrorInvalidValue;
+  fold_rows_kernel<T><<<n_groups, 128, 0, s>>>(rows, lin, bias, extra, out, C);
+  return cudaGetLastError();
+}
+
 // ---- gate --------------------------------------------------------------------------------------
 // Row of Gt per atom, (L + 1 + D) * C long.  m0 != 0 (the reference's gate_m0 = True, nonlinear.py:27-42): [L + 1 gate
 // scalars | all D components], every rank scaled by its gate.  m0 == 0 (gate_m0 = False, the e3nn Gate,
@@ -654,6 +712,8 @@ __global__ void one_hot_kernel(const int* __restrict__ species, long long n, int
   template cudaError_t launch_add_inplace<T>(T*, const T*, long long, cudaStream_t);                          \
   template cudaError_t launch_gather_rows<T>(const T*, const int*, T*, long long, int, cudaStream_t);         \
   template cudaError_t launch_species_gather<T>(const T*, const int*, T*, int, int, cudaStream_t);            \
+  template cudaError_t launch_fold_linear<T>(const T*, const T*, T*, T*, T*, T*, T*, T*, int, int, int, cudaStream_t); \
+  template cudaError_t launch_fold_rows<T>(const T*, const T*, const T*, const T*, T*, int, int, cudaStream_t); \
   template cudaError_t launch_gate_fwd<T>(const T*, T*, int, int, int, int, cudaStream_t);                    \
   template cudaError_t launch_gate_bwd<T>(const T*, const T*, T*, int, int, int, int, cudaStream_t);          \
   template cudaError_t launch_pb_fwd<T>(const T*, T*, int, int, int, int, cudaStream_t);                      \

@@ -1,0 +1,74 @@
+"""Weights that the library multiplies together when they are set (the product's final linear into the per-species coefficients, the first
+linear_up into the species embedding): set in another order, and one at a time on a model that has been evaluated already, they give what a
+model loaded with the same parameters gives, to the last bit; against the oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from tace_b200 import lib as _lib
+from tace_b200 import synth
+from tace_b200.pack import RADIAL_TABLE_INTERVALS, pack_weights
+from helpers import check_parity, make_models, oracle_batch, to_device
+
+pytestmark = pytest.mark.gpu
+
+DEV = torch.device("cuda:0")
+
+
+def _packed(model):
+    rf = model.readout_fn
+    spec = (model.get_cutoff(), int(rf.cfg["radial_basis"]["polynomial_cutoff"]), RADIAL_TABLE_INTERVALS) if model.uses_radial_table else None
+    return pack_weights(rf.plan, rf.state_dict(), float(rf.cfg["avg_num_neighbors"]), radial_table_spec=spec)
+
+
+def _set(model, packed, names, dtype):
+    lib = _lib.load()
+    for name in names:
+        arr = np.ascontiguousarray(packed[name], dtype=np.float64 if dtype is torch.float64 else np.float32).reshape(-1)
+        _lib.check(lib.tace_set_weight(model._handle, name.encode(), arr.ctypes.data_as(ctypes.c_void_p), arr.size), name)
+
+
+def _names(model):
+    lib, name, numel, out = _lib.load(), ctypes.c_char_p(), ctypes.c_int64(), []
+    for i in range(lib.tace_weight_count(model._handle)):
+        _lib.check(lib.tace_weight_info(model._handle, i, ctypes.byref(name), ctypes.byref(numel)), "tace_weight_info")
+        out.append(name.value.decode())
+    return out
+
+
+@pytest.mark.parametrize("correlation,C,dtype,kind", [(1, 32, torch.float32, "aware"), (2, 64, torch.float32, "aware"), (3, 32, torch.float64, "agnostic"),
+                                                      (2, 48, torch.float64, "identity"), (2, 128, torch.float32, "agnostic")])
+def test_weights_set_again(correlation, C, dtype, kind):
+    options = dict(correlation=correlation, resnet_linear_type=kind)
+    structs = [synth.fcc_supercell(2, 3.65, 0.05, seed=3, species=(13, 29), fractions=(0.5, 0.5))]
+    model, _, _ = make_models(2, C, [13, 29], 4.0, 12.0, dtype, seed=1, **options)
+    other, oracle, _ = make_models(2, C, [13, 29], 4.0, 12.0, dtype, seed=5, **options)
+    data = oracle_batch(structs, [13, 29], 4.0, dtype)
+    gpu = to_device(data, DEV)
+    before, want = model(gpu), other(gpu)
+    before = {k: before[k].clone() for k in ("energy", "forces")}
+    want = {k: want[k].clone() for k in ("energy", "forces")}
+    check_parity(other(gpu), oracle(data), data["ptr"], dtype, f"correlation {correlation} {kind}")
+    assert not torch.equal(before["energy"], want["energy"])
+
+    names = _names(model)
+    mine, theirs = _packed(model), _packed(other)
+    for order in (names, names[::-1]):  # the derived forms before and after what they are derived from
+        _set(model, theirs, order, dtype)
+        out = model(gpu)
+        assert torch.equal(out["energy"], want["energy"]) and torch.equal(out["forces"], want["forces"])
+        _set(model, mine, order, dtype)
+        out = model(gpu)
+        assert torch.equal(out["energy"], before["energy"]) and torch.equal(out["forces"], before["forces"])
+
+    # each factor by itself reaches the folded product, and back
+    factors = ["emb", "t0.up.l0", "t0.up.b", "t0.lin.l0", "t0.lin.l2", "t0.lin.b", "t0.c.b", "t1.lin.l0", "t1.c.b", "t0.c0.l1", "t1.c0.l0"]
+    factors += ["t1.res.b"] if kind != "identity" else []
+    factors += [f"t0.c{j}.l2" for j in range(1, correlation)]
+    for name in factors:
+        _set(model, theirs, [name], dtype)
+        assert not torch.equal(model(gpu)["energy"], before["energy"]), name
+        _set(model, mine, [name], dtype)
+        assert torch.equal(model(gpu)["energy"], before["energy"]), name
