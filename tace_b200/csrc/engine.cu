@@ -401,6 +401,7 @@ struct Model : ModelBase {
   std::vector<WeightEntry> weights;  // the first n_listed are the caller's, n_unset of them not set yet; the others are folded from them
   int n_listed = 0, n_unset = 0;
   bool folded = true;
+  int device = 0;  // holds the arena
   std::unordered_map<std::string, int> weight_index;
   T* arena = nullptr;
   long long arena_numel = 0;
@@ -610,6 +611,7 @@ struct Model : ModelBase {
         for (int j = 0; j < c.correlation; ++j) add_weight(coef_name(t, j, "f", l), (long long)n_el * coef_rows(t, j, l) * C);
         if (l == 0) add_weight("t" + std::to_string(t) + ".cf.b", (long long)n_el * C);
       }
+    if (cudaGetDevice(&device) != cudaSuccess) return TACE_ERR_CUDA;
     if (cudaMalloc(&arena, sizeof(T) * (size_t)arena_numel) != cudaSuccess) return TACE_ERR_CUDA;
     if (cudaMemset(arena, 0, sizeof(T) * (size_t)arena_numel) != cudaSuccess) return TACE_ERR_CUDA;
     if (cudaMalloc(&dev_error, sizeof(int)) != cudaSuccess || cudaMemset(dev_error, 0, sizeof(int)) != cudaSuccess)
@@ -671,7 +673,10 @@ struct Model : ModelBase {
     const std::string stem = layer >= 0 ? name.substr(dot + 1) : "";
     bool derived = false, any = false;
     const int order = coef_order(name, derived);
-    cudaError_t e = cudaSuccess;
+    int current = 0;  // the weights may be set with another device current than the one that holds them
+    cudaError_t e = cudaGetDevice(&current);
+    if (e == cudaSuccess && current != device) e = cudaSetDevice(device);
+    if (e != cudaSuccess) return e;
     if (all || name == "emb" || name == "t0.up.l0" || name == "t0.up.b") { e = fold_embedding(); any = true; }
     for (int t = 0; t < NL_ && e == cudaSuccess; ++t) {
       if (!all && t != layer) continue;
@@ -682,7 +687,9 @@ struct Model : ModelBase {
       }
       if (e == cudaSuccess && (all || stem == "lin.l0" || stem == "lin.b" || stem == "c.b" || stem == "res.b")) { e = fold_bias(t); any = true; }
     }
-    return e == cudaSuccess && any ? cudaStreamSynchronize(cudaStream_t(0)) : e;  // a later pass may run on any stream
+    if (e == cudaSuccess && any) e = cudaStreamSynchronize(cudaStream_t(0));  // a later pass may run on any stream
+    const cudaError_t back = current != device ? cudaSetDevice(current) : cudaSuccess;
+    return e != cudaSuccess ? e : back;
   }
 
   int set_weight(const char* name, const void* host, int64_t numel) override {
