@@ -266,7 +266,12 @@ struct WideBwdShape {
   static constexpr int CW = C / (64 * kPairs);       // warps per edge
   static constexpr int kWarps = CW > 1 ? 8 : 4, EW = kWarps / CW;  // edges in flight per block
   static constexpr int NRED = TP::D + 2;          // dY | dE/d(length) | dE/d(envelope)
-  static constexpr int kMsgFloats = TP::NM * C, kGFloats = kWideBatch * TP::GVS, kRedFloats = CW > 1 ? kWideBatch * CW * NRED : 0;
+  static constexpr int kMsgFloats = TP::NM * C, kEdgeFloats = TP::GVS + (CW > 1 ? CW * NRED : 0);
+  // Edges of a batch, which costs the block two barriers: 32, so that a whole warp of lanes builds rows, where the 16 warps that fit
+  // an SM by their registers then still fit its shared memory (rank 3, 128 channels: two blocks of 96 KB).  Against 16: 64 crystals
+  // 2 705 -> 2 692 us, 1 372 atoms 588 -> 583, MD step of 131 072 atoms 23 491 -> 23 342.
+  static constexpr int kBatch = (16 / kWarps) * ((kMsgFloats + 32 * kEdgeFloats) * 4 + 2048) <= 224 * 1024 ? 32 : 16;
+  static constexpr int kGFloats = kBatch * TP::GVS, kRedFloats = CW > 1 ? kBatch * CW * NRED : 0;
   static constexpr int kBytes = (kMsgFloats + kGFloats + kRedFloats) * 4;
 };
 
@@ -335,8 +340,8 @@ __device__ __forceinline__ void wide_bwd_row(const TPArgs<float>& a, int i, unsi
   const float* table = a.rtab + 4 * c0 + 4 * lane;
   WideMsg<kPairs, C> gm;
   gm.g = gMs + c0 + 2 * lane;
-  for (int e0 = beg; e0 < end; e0 += kWideBatch) {
-    const int nb = min(kWideBatch, end - e0);
+  for (int e0 = beg; e0 < end; e0 += S::kBatch) {
+    const int nb = min(S::kBatch, end - e0);
     if (e0 != beg) __syncthreads();
     if (lane < nb) {
       if (warp == 0) {
@@ -419,8 +424,8 @@ __device__ __forceinline__ void wide_bwd_row(const TPArgs<float>& a, int i, unsi
 template <typename TP, int C, bool ENV, bool LIST>
 __global__ void __maxnreg__(128) tp_bwd_wide_kernel(const TPArgs<float> a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int esrc[kWideBatch], ek[kWideBatch];
-  __shared__ float et[kWideBatch], eu[kWideBatch];
+  __shared__ int esrc[32], ek[32];
+  __shared__ float et[32], eu[32];
   if constexpr (LIST) {
     for (int it = blockIdx.x * kWideListRows; it < ((int)blockIdx.x + 1) * kWideListRows; ++it) {
       const int i = wide_row(a, it);
