@@ -133,6 +133,45 @@ struct ModelBase {
   virtual ~ModelBase() {
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
+    if (ev_branch) cudaEventDestroy(ev_branch);
+    if (ev_merge) cudaEventDestroy(ev_merge);
+  }
+  // Branches of a pass that is being captured: `branch` gives the stream for work that depends on what `s` has so far and that
+  // nothing on `s` needs before the next `merge`.  In a pass that is launched kernel by kernel both do nothing and the work
+  // goes to `s`.
+  bool branches = false;  // the running pass is captured and has branch_stream at its disposal
+  bool branch_open = false;
+  cudaStream_t branch_stream = nullptr;
+  cudaEvent_t ev_branch = nullptr, ev_merge = nullptr;
+  int branch(cudaStream_t s, cudaStream_t* side) {
+    *side = s;
+    if (!branches) return TACE_OK;
+    if (cudaEventRecord(ev_branch, s) != cudaSuccess || cudaStreamWaitEvent(branch_stream, ev_branch, 0) != cudaSuccess) return TACE_ERR_CUDA;
+    *side = branch_stream;
+    branch_open = true;
+    return TACE_OK;
+  }
+  int merge(cudaStream_t s) {
+    if (!branch_open) return TACE_OK;
+    branch_open = false;
+    if (cudaEventRecord(ev_merge, branch_stream) != cudaSuccess || cudaStreamWaitEvent(s, ev_merge, 0) != cudaSuccess) return TACE_ERR_CUDA;
+    return TACE_OK;
+  }
+  // Branches end where a pass fills the chip by itself: 8 600 edges of the edge block 3 831 -> 3 671 us for two frames, 524 000 edges
+  // 74.5 -> 75.8 ms; 11 000 edges in double precision 1 456 -> 1 374 us for two frames.
+  static constexpr int64_t kBranchEdges = 1 << 16;
+  // Streams and events of a captured pass.  With the fp64 products of the radial MLPs (thousands of blocks) on a branch, the main line
+  // takes the higher priority, so that its small kernels do not stand in line behind them (1 374 us above, 1 439 without).  The edge
+  // block's main line is large products with small kernels on the branch; there it loses (3 671 us without, 3 745 with).
+  virtual bool main_line_first() const = 0;
+  bool capture_streams() {
+    if (capture_stream) return true;
+    int least = 0, greatest = 0;
+    if (main_line_first() && cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess) return false;
+    if (!ev_branch && cudaEventCreateWithFlags(&ev_branch, cudaEventDisableTiming) != cudaSuccess) return false;
+    if (!ev_merge && cudaEventCreateWithFlags(&ev_merge, cudaEventDisableTiming) != cudaSuccess) return false;
+    if (!branch_stream && cudaStreamCreateWithPriority(&branch_stream, cudaStreamNonBlocking, least) != cudaSuccess) return false;
+    return cudaStreamCreateWithPriority(&capture_stream, cudaStreamNonBlocking, greatest) == cudaSuccess;
   }
   // Runs the exchange callback.  Without an exchange stream: on the stream of the pass (after a host synchronisation when
   // the callback asks for one).  With one: everything enqueued on `s` so far happens before the callback's work, which
@@ -265,6 +304,7 @@ struct ModelBase {
     for (auto& g : graphs) cudaGraphExecDestroy(g.exec);
     graphs.clear(); seen.clear(); rejected.clear();
     if (capture_stream) { cudaStreamDestroy(capture_stream); capture_stream = nullptr; }
+    if (branch_stream) { cudaStreamDestroy(branch_stream); branch_stream = nullptr; }
   }
 
   int forward_entry(const TaceBatch* bt, const TaceOutputs* o, void* ws, size_t ws_bytes, cudaStream_t s) {
@@ -298,8 +338,7 @@ struct ModelBase {
         return forward(bt, o, ws, ws_bytes, s);
       }
       // second call: capture a pass that works on the staged copies
-      if (!capture_stream && cudaStreamCreateWithFlags(&capture_stream, cudaStreamNonBlocking) != cudaSuccess)
-        return forward(bt, o, ws, ws_bytes, s);
+      if (!capture_streams()) return forward(bt, o, ws, ws_bytes, s);
       TaceBatch sbt = *bt;
       sbt.n_edges = Ecap;
       TaceOutputs so;
@@ -324,13 +363,15 @@ struct ModelBase {
       cudaGraphExec_t exec = nullptr;
       bool ok = cudaStreamBeginCapture(capture_stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
       if (ok) {
+        branches = Ecap <= kBranchEdges;
         const int status = forward(&sbt, &so, ws, body_bytes, capture_stream);
+        branches = branch_open = false;
         const cudaError_t ce = cudaStreamEndCapture(capture_stream, &graph);
         ok = status == TACE_OK && ce == cudaSuccess && graph != nullptr;
       }
       const long long per_pass = launches - before;
       launches = before;
-      if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
+      if (ok) ok = cudaGraphInstantiate(&exec, graph, main_line_first() ? cudaGraphInstantiateFlagUseNodePriority : 0) == cudaSuccess;
       if (graph) cudaGraphDestroy(graph);
       if (!ok) {
         cudaGetLastError();  // a failed capture leaves a sticky-free error behind; this sizes runs without a graph
@@ -619,6 +660,7 @@ struct Model : ModelBase {
     return TACE_OK;
   }
 
+  bool main_line_first() const override { return rt_K == 0 && !tece_mask; }
   int weight_count() const override { return n_listed; }
   int weight_info(int i, const char** name, int64_t* numel) const override {
     if (i < 0 || i >= n_listed) return TACE_ERR_INVALID_ARGUMENT;
@@ -995,6 +1037,7 @@ struct Model : ModelBase {
   } while (0)
 
 #define CKL(expr) do { CK(expr); ++launches; } while (0)
+#define CKS(expr) do { const int st__ = (expr); if (st__ != TACE_OK) return st__; } while (0)
 #define PH(name) phase(name, s)
 
   // Arguments of the per-edge MLP kernels for layers `ts` over edges [e0, e0 + Ec); row r of every [.][64] buffer is edge e0 + r.
@@ -1086,38 +1129,46 @@ struct Model : ModelBase {
     CKL(launch_tece(ta, TECE_ROTATE_IN, s));
     so2_specs(sp, pre, {{0, lb.tKs, t_NR, lb.tKp, t_NR}, {1, lb.tQt, t_NR, lb.tQp, t_NR}}, false);
     CKL(run_linear(sp, E, s)); sp.clear();
-    CKL(launch_tece(ta, TECE_LOGIT, s));
-    CKL(launch_tece(ta, TECE_SOFTMAX, s));
+    cudaStream_t side;  // the attention weights, beside the linears and the cluster expansion of the messages
+    CKS(branch(s, &side));
+    CKL(launch_tece(ta, TECE_LOGIT, side));
+    CKL(launch_tece(ta, TECE_SOFTMAX, side));
     so2_specs(sp, pre, {{2, lb.tMw, t_NR, lb.tup, t_G + t_NF}, {3, lb.tMw, t_NR, lb.tglu, t_NF}, {4, lb.tMw, t_NR, lb.tcoef, t_WN}}, false);
     CKL(run_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_MIX, s));
     so2_specs(sp, pre, {{5, lb.tU, t_NF, lb.tdown, t_NR}}, false);
     CKL(run_linear(sp, E, s)); sp.clear();
+    CKS(merge(s));
     CKL(launch_tece(ta, TECE_ROTATE_OUT, s));
     return TACE_OK;
   }
   // backward: lb.M holds dE/d(messages); leaves dE/d(radial weights) in lb.W, the per-edge source rows in dxe, the target part
   // added to lb.gx by the caller's order (source sum first), and this layer's share of dE/d(edge vector) in tgvec / tddlen
   int tece_backward(TeceArgs<T> ta, const Bufs& b, const LayerBufs& lb, const std::string& pre, long long N, long long E, bool first_tece,
-                    cudaStream_t s) {
+                    cudaStream_t s, cudaStream_t* after) {
     std::vector<LinSpec> sp;
+    cudaStream_t side;
     CKL(launch_tece(ta, TECE_ROTATE_OUT_BWD, s));
-    CKL(launch_tece(ta, TECE_ALPHA_BWD, s));
-    CKL(launch_tece(ta, TECE_SOFTMAX_BWD, s));
-    CKL(launch_tece(ta, TECE_LOGIT_BWD, s));
-    CKL(launch_tece(ta, TECE_EDGE_SCALAR_BWD, s));
+    // the attention weights down to the rotated rows, beside the way back through the messages (cluster expansion and linears)
+    CKS(branch(s, &side));
+    CKL(launch_tece(ta, TECE_ALPHA_BWD, side));
+    CKL(launch_tece(ta, TECE_SOFTMAX_BWD, side));
+    CKL(launch_tece(ta, TECE_LOGIT_BWD, side));
+    CKL(launch_tece(ta, TECE_EDGE_SCALAR_BWD, side));
     so2_specs(sp, pre, {{5, lb.tgdown, t_NF, lb.tU, t_NR}}, true);   // gU over U
     CKL(run_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_MIX_BWD, s));                           // gup / gglu / gcoef over their forward buffers
     // gMw over Mw: the three linears that read Mw add up in one pass per order
     so2_specs(sp, pre, {{2, lb.tup, t_NR, lb.tMw, t_G + t_NF}, {3, lb.tglu, t_NR, lb.tMw, t_NF}, {4, lb.tcoef, t_NR, lb.tMw, t_WN}}, true);
     CKL(run_linear(sp, E, s)); sp.clear();
+    CKS(merge(s));
     so2_specs(sp, pre, {{0, lb.tgKp, t_NR, lb.tgKs, t_NR}, {1, lb.tgQp, t_NR, lb.tgQt, t_NR}}, true);
     CKL(run_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_ROTATE_IN_BWD, s));
-    CKL(launch_segment_sum_rows(b.dxe, b.rowptr_src, b.perm_src, lb.gx, 0, (int)N, D * C, s, /*accumulate=*/1));
     ta.accumulate_gvec = first_tece ? 0 : 1;
-    CKL(launch_tece(ta, TECE_WIGNER_BWD, s));
+    CKS(branch(s, after));  // what only the end of the pass needs
+    CKL(launch_tece(ta, TECE_WIGNER_BWD, *after));
+    CKL(launch_segment_sum_rows(b.dxe, b.rowptr_src, b.perm_src, lb.gx, 0, (int)N, D * C, s, /*accumulate=*/1));
     return TACE_OK;
   }
 
@@ -1253,7 +1304,6 @@ struct Model : ModelBase {
     }
     return TACE_OK;
   }
-#define CKS(expr) do { const int st__ = (expr); if (st__ != TACE_OK) return st__; } while (0)
 
   int forward(const TaceBatch* bt, const TaceOutputs* o, void* ws, size_t ws_bytes, cudaStream_t s) override {
     if (!bt || !o || !ws) return TACE_ERR_INVALID_ARGUMENT;
@@ -1318,8 +1368,14 @@ struct Model : ModelBase {
     // for the gradients.  Every target is still summed in one piece, so the numbers do not depend on the schedule.
     const bool overlap = exchange_on_side() && !chunked && NL != N && NL_ > 1;
     gp.split_rows = overlap ? 1 : 0; gp.row_ids = b.row_ids; gp.row_split = b.row_split;
+    gp.defer_src = branches || !need_grad;  // the view by sources is read by the backward pass only
     CK(launch_graph_prep(gp, s));
     launches += graph_prep_launches(gp);
+    if (branches && need_grad) {
+      cudaStream_t side;
+      CKS(branch(s, &side));
+      CKL(launch_edge_order_src(gp, side));
+    }
     std::vector<int> chunk_atom{0, (int)NL}, chunk_edge{0, (int)E};
     if (chunked) {
       const int nc = b.n_chunks;
@@ -1374,6 +1430,15 @@ struct Model : ModelBase {
     debug.push_back({"Y", b.Y, (long long)D * E});
     debug.push_back({"vec", b.vec, 3 * E});
 
+    // The last layers of the radial MLPs of all interactions but the first run beside the first interaction and its products per atom,
+    // which leave most of the chip idle on small systems; the way back (dE/dW of an interaction is not needed before the end of the
+    // pass) in the same way.
+    if (branches && !chunked && !rt_K && NL_ > 1) {
+      cudaStream_t side;
+      CKS(branch(s, &side));
+      for (int t = 1; t < NL_; ++t) CKS(radial_last(layers[t], b.lay[t], "t" + std::to_string(t) + ".", E, false, side));
+    }
+
     // ---- layers, forward
     bool wigner_done = false, tece_seen = false;
     PH("embed");
@@ -1410,7 +1475,8 @@ struct Model : ModelBase {
           CKS(radial_forward(ea, b, std::vector<int>{t}, e0, Ec, s));
         }
         PH(("t" + ts + ".fwd.radial_gemm").c_str());
-        CKS(radial_last(p, lb, pre, Ec, false, s));
+        if (branches && !chunked && t > 0) CKS(merge(s));
+        else CKS(radial_last(p, lb, pre, Ec, false, s));
         PH(("t" + ts + ".fwd.tp").c_str());
         if (p.tece) {  // the edge block instead of the tensor product (whole batch only)
           if (chunked) return TACE_ERR_CAPACITY;
@@ -1678,10 +1744,12 @@ struct Model : ModelBase {
             if (b.denv) CKL(launch_fill_zero(b.denv, E, s));
           }
           const TeceArgs<T> tc = tece_args(ea, b, lb, pre, lb.xx ? lb.xx : lb.x, N, NL, E);
-          CKS(tece_backward(tc, b, lb, pre, N, E, !tece_seen, s));
+          cudaStream_t side = s;
+          CKS(merge(s));  // the Wigner gradients of the edge block above
+          CKS(tece_backward(tc, b, lb, pre, N, E, !tece_seen, s, &side));
           tece_seen = true;
           PH(("t" + ts + ".bwd.radial_gemm").c_str());
-          CKS(radial_last(p, lb, pre, Ec, true, s));
+          CKS(radial_last(p, lb, pre, Ec, true, side));
           continue;
         }
         TPArgs<T> ta;
@@ -1721,7 +1789,9 @@ struct Model : ModelBase {
           }
         }
         PH(("t" + ts + ".bwd.radial_gemm").c_str());
-        CKS(radial_last(p, lb, pre, Ec, true, s));  // back through the last radial-MLP layer: H3 <- dE/dh3
+        cudaStream_t side = s;
+        if (t > 0 && !chunked && !rt_K) CKS(branch(s, &side));
+        CKS(radial_last(p, lb, pre, Ec, true, side));  // back through the last radial-MLP layer: H3 <- dE/dh3
         if (chunked) {
           PH("radial_mlp_bwd");
           CKS(radial_backward(ea, b, std::vector<int>{t}, e0, Ec, t != NL_ - 1, s));
@@ -1759,6 +1829,7 @@ struct Model : ModelBase {
 
     // ---- back to the edge vectors, then forces and virials
     PH("radial_mlp_bwd");
+    CKS(merge(s));
     if (!chunked) CKS(radial_backward(ea, b, all_layers, 0, E, 0, s));  // lay[t].H3 holds dE/dh3 of each layer's radial MLP
     for (int t = 0; t < NL_; ++t)  // the edge blocks' own dependence on the edge lengths (radial projection, cutoff in the softmax)
       if (layers[t].tece) CKL(launch_add_inplace(b.ddlen, b.lay[t].tddlen, E, s));

@@ -355,8 +355,12 @@ size_t graph_prep_temp_bytes(long long E, int n_atoms) {
   return (edge > sorts ? edge : sorts) + 256;
 }
 
+// Sorts that follow the edge sort reuse its scratch, which the view by sources reads.
+static bool src_deferred(const GraphPrepArgs& a) {
+  return a.defer_src && !a.split_rows && a.n_local <= kSpeciesBlockAtoms && a.n_elements <= kSpeciesBlockElements;
+}
 int graph_prep_launches(const GraphPrepArgs& a) {
-  return 6 + (a.n_atoms >= kScanBlock ? 1 : 0) + (a.split_rows && a.n_local > 0 ? 2 : 0) +
+  return 6 - (src_deferred(a) ? 1 : 0) + (a.n_atoms >= kScanBlock ? 1 : 0) + (a.split_rows && a.n_local > 0 ? 2 : 0) +
          (a.n_local > kSpeciesBlockAtoms || a.n_elements > kSpeciesBlockElements ? 4 : 0);
 }
 
@@ -365,17 +369,31 @@ __global__ void invert_kernel(const int* __restrict__ perm, int n, int* __restri
   if (i < n) rank[perm[i]] = i;
 }
 
-cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s) {
+// Arrays of the edge sort, its scratch in a.temp.
+static EdgeSort edge_sort_of(const GraphPrepArgs& a) {
   unsigned char* p = static_cast<unsigned char*>(a.temp);
-  if (a.temp_bytes < graph_prep_temp_bytes(a.E, a.n_atoms)) return cudaErrorInvalidValue;
   auto take = [&p](size_t count) { int* r = reinterpret_cast<int*>(p); p += align_up(sizeof(int) * (count ? count : 1)); return r; };
   EdgeSort es;
   es.src = a.edge_index; es.dst = a.edge_index + a.E; es.E = a.E; es.n = a.n_atoms;
   es.by_dst = take(a.E); es.by_src = take(a.E); es.cur_dst = take((size_t)a.n_atoms + 1); es.cur_src = take((size_t)a.n_atoms + 1);
-  const int scan_blocks = a.n_atoms / kScanBlock + 1;
-  es.block_sums = take(2 * (size_t)scan_blocks);
+  es.block_sums = take(2 * (size_t)(a.n_atoms / kScanBlock + 1));
   es.rowptr_dst = a.rowptr_dst; es.rowptr_src = a.rowptr_src;
   es.e_src = a.e_src; es.e_dst = a.e_dst; es.e_orig = a.e_orig; es.perm_src = a.perm_src;
+  return es;
+}
+static void order_by_source(const GraphPrepArgs& a, cudaStream_t s) {
+  edge_order_src_kernel<<<(unsigned)(((long long)a.n_atoms + 7) / 8), 256, 0, s>>>(edge_sort_of(a));
+}
+cudaError_t launch_edge_order_src(const GraphPrepArgs& a, cudaStream_t s) {
+  if (!src_deferred(a) || a.E <= 0) return cudaSuccess;
+  order_by_source(a, s);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s) {
+  if (a.temp_bytes < graph_prep_temp_bytes(a.E, a.n_atoms)) return cudaErrorInvalidValue;
+  const int scan_blocks = a.n_atoms / kScanBlock + 1;
+  const EdgeSort es = edge_sort_of(a);
   SpeciesSort sp{a.species_safe, a.n_local, a.n_elements, a.species_perm, a.species_rank, a.species_ptr, a.tile_ptr, a.tc_tile_ptr};
   const bool small_species = a.n_local <= kSpeciesBlockAtoms && a.n_elements <= kSpeciesBlockElements;
 
@@ -392,14 +410,15 @@ cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s) {
     edge_scatter_kernel<<<(unsigned)((a.E + 255) / 256), 256, 0, s>>>(es);
     const unsigned wb = (unsigned)(((long long)a.n_atoms + 7) / 8);
     edge_order_dst_kernel<<<wb, 256, 0, s>>>(es);
-    edge_order_src_kernel<<<wb, 256, 0, s>>>(es);
+    if (!src_deferred(a)) order_by_source(a, s);
   }
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
 
   // sorts whose scratch overlays the edge sort's
   const long long n = a.E > a.n_atoms ? a.E : a.n_atoms;
-  p = static_cast<unsigned char*>(a.temp);
+  unsigned char* p = static_cast<unsigned char*>(a.temp);
+  auto take = [&p](size_t count) { int* r = reinterpret_cast<int*>(p); p += align_up(sizeof(int) * (count ? count : 1)); return r; };
   int* keys_in = take(n); int* vals_in = take(n); int* keys_out = take(n);
   void* cub_temp = p;
   size_t cub_bytes = cub_sort_bytes(n);

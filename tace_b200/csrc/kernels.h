@@ -287,10 +287,12 @@ struct GraphPrepArgs {
   int* species_rank;          // [n_local] place of every atom in species_perm
   int* tile_ptr;              // [4][n_elements+1] for q = 1,3,5,7: 32-row tiles per species
   int* tc_tile_ptr;           // [4][n_elements+1]: (128 / q)-atom tiles per species
+  bool defer_src = false;     // perm_src comes from launch_edge_order_src (on any stream behind this one, before `temp` is used again)
   void* temp; size_t temp_bytes;
 };
 size_t graph_prep_temp_bytes(long long E, int n_atoms);
 cudaError_t launch_graph_prep(const GraphPrepArgs& a, cudaStream_t s);
+cudaError_t launch_edge_order_src(const GraphPrepArgs& a, cudaStream_t s);  // nothing where launch_graph_prep did it already
 int graph_prep_launches(const GraphPrepArgs& a);  // kernels of this file it runs
 // Edge chunks for systems whose per-edge tensors do not fit: chunk c = target atoms [atom_ptr[c], atom_ptr[c+1]) with
 // atom_ptr[c] = first atom whose edge offset reaches c * target_edges; edge_ptr[c] = rowptr_dst[atom_ptr[c]].
