@@ -1305,6 +1305,14 @@ struct Model : ModelBase {
     return TACE_OK;
   }
 
+  // Buffers of a layer's backward pass that are added to, or written only where the output has a rank.
+  int zero_gradients(const LayerPlan& p, const LayerBufs& lb, long long NL, cudaStream_t s) {
+    if (bilinear) CKL(launch_fill_zero(lb.gXY, NL * D * 2 * C, s));
+    else if ((int)p.out_ls.size() != L + 1) CKL(launch_fill_zero(lb.gAs, NL * D * C, s));
+    if (cfg.correlation >= 3) CKL(launch_fill_zero(lb.gB2, NL * p.pb.NB * C, s));  // ranks above the output ranks only receive third-order terms
+    return TACE_OK;
+  }
+
   int forward(const TaceBatch* bt, const TaceOutputs* o, void* ws, size_t ws_bytes, cudaStream_t s) override {
     if (!bt || !o || !ws) return TACE_ERR_INVALID_ARGUMENT;
     backward_pass = false;
@@ -1375,6 +1383,7 @@ struct Model : ModelBase {
       cudaStream_t side;
       CKS(branch(s, &side));
       CKL(launch_edge_order_src(gp, side));
+      for (int t = 0; t < NL_; ++t) CKS(zero_gradients(layers[t], b.lay[t], NL, side));
     }
     std::vector<int> chunk_atom{0, (int)NL}, chunk_edge{0, (int)E};
     if (chunked) {
@@ -1634,6 +1643,7 @@ struct Model : ModelBase {
 
     // ---- layers, backward
     backward_pass = true;
+    CKS(merge(s));  // a single interaction has not met the branch yet
     for (int t = NL_ - 1; t >= 0; --t) {
       const LayerPlan& p = layers[t];
       LayerBufs& lb = b.lay[t];
@@ -1653,8 +1663,7 @@ struct Model : ModelBase {
         CKL(run_linear(sp, NL, s, b.species_rank));
       }
       // through the per-species coefficients and the product basis, in species-sorted space
-      if (bilinear) CKL(launch_fill_zero(lb.gXY, NL * D * 2 * C, s));
-      else if ((int)p.out_ls.size() != L + 1) CKL(launch_fill_zero(lb.gAs, NL * D * C, s));
+      if (!branches) CKS(zero_gradients(p, lb, NL, s));
       {
         std::vector<SpeciesSpec> sp;
         for (int l : p.out_ls)
@@ -1667,7 +1676,6 @@ struct Model : ModelBase {
           // gradient of the second-order basis: written over B2 itself, or into gB2 when the third order still needs B2
           T* g2 = cfg.correlation >= 3 ? lb.gB2 : lb.B2;
           if (cfg.correlation >= 3) {
-            CKL(launch_fill_zero(lb.gB2, NL * p.pb.NB * C, s));  // ranks above the output ranks only receive third-order terms
             for (size_t i = 0; i < p.out_ls.size(); ++i) {
               const int l = p.out_ls[i];
               const int K = p.pb3.k[i] * C;

@@ -16,6 +16,7 @@ DEV = torch.device("cuda:0")
     (2, torch.float64, None, ("energy", "forces", "stress")),
     (3, torch.float64, None, ("energy", "forces", "stress")),
     (3, torch.float64, None, ("energy",)),
+    (1, torch.float64, None, ("energy", "forces", "stress")),
     (2, torch.float32, None, ("energy", "forces", "stress")),
     (2, torch.float32, {"num_head": 4, "edge_ace_hidden": 16, "mmax": 2}, ("energy", "forces", "stress")),
     (3, torch.float32, {"num_head": 4, "edge_ace_hidden": 16, "mmax": 1}, ("energy", "forces", "stress")),
@@ -40,3 +41,17 @@ def test_replays_equal_the_direct_pass(layers, dtype, tece, targets, monkeypatch
         for k, v in direct[n % 3].items():
             assert torch.equal(out[k], v), (n, k)
     assert model.graph_replays() >= before + 30
+
+
+@pytest.mark.parametrize("layers,Lmax,correlation", [(1, 2, 2), (2, 1, 2), (2, 2, 3), (3, 2, 3)])
+def test_zeroed_gradients_of_other_products(layers, Lmax, correlation):
+    """Buffers that a branch clears: a product with fewer ranks than the basis, third order, one to three interactions (radial table)."""
+    structs = [synth.fcc_supercell(2, 3.65, 0.05, seed=2, species=(13, 29), fractions=(0.5, 0.5))]
+    model, _, _ = make_models(2, 64, [13, 29], 4.5, 20.0, torch.float32, num_layers=layers, Lmax=Lmax, correlation=correlation)
+    data = to_device(oracle_batch(structs, [13, 29], 4.5, torch.float32), DEV)
+    direct = {k: v.clone() for k, v in model(data).items() if v is not None}
+    for n in range(10):
+        out = model(data)
+        for k, v in direct.items():
+            assert torch.equal(out[k], v), (n, k)
+    assert model.graph_replays() >= 9
