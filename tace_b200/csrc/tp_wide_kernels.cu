@@ -10,7 +10,7 @@
 // reads): 1.04 against 1.18 ms for the rank-3 backward pass below.
 //
 // Measured against one channel per thread, on B200 at rank 3, 128 channels, 2 283 targets, 142 222 edges: backward 1.51 -> 1.04 ms
-// (FMA pipe 62 % busy, LSU 66 % of its wavefronts), forward 0.80 -> 0.54 ms (LSU 80 %: of 848 wavefronts per edge 368 are table
+// (0.98 since; FMA pipe 67 % busy, LSU 71 % of its wavefronts), forward 0.80 -> 0.54 ms (LSU 80 %: of 848 wavefronts per edge 368 are table
 // entries, 320 coupling rows, 64 source rows; 14.4 TB/s out of L2, of 19.6 that all SMs together can read), scalar source forward 0.11 -> 0.08 ms; rank 2, 64 channels, 131 072 targets,
 // 5.5 M edges: 10.4 -> 7.2 and 5.1 -> 3.9 ms; 32 targets of 42 edges: 51 -> 10 and 31 -> 13 us.
 #include <cstdint>
