@@ -950,16 +950,18 @@ struct Model : ModelBase {
   // K = 4 352: 73 -> 43 us).
   static constexpr long long kSmallLinear = 32LL << 20, kFewTiles = 8;
   bool backward_pass = false;  // what forward() is enqueuing
+  // counted: rows for which the kernels are chosen.
   template <typename Spec, typename FillTc, typename Add>
-  cudaError_t run_specs(const std::vector<Spec>& specs, long long n_atoms, cudaStream_t s, const GemmBatch<T>& empty, FillTc&& fill, Add&& add) {
+  cudaError_t run_specs(const std::vector<Spec>& specs, long long n_atoms, long long counted, cudaStream_t s, const GemmBatch<T>& empty, FillTc&& fill,
+                        Add&& add) {
     TcLinearProblem probs[kMaxLinears];
     int n_tc = 0;
     GemmBatch<T> gb = empty;
     cudaError_t err = cudaSuccess;
     long long work = 0, tiles = 0;  // tiles of the tensor-core kernel
     for (const Spec& sp : specs) {
-      work += n_atoms * sp.q * sp.K * sp.N;
-      if (sp.accumulate != kJoin) tiles += (n_atoms * sp.q + 127) / 128 * ((sp.N + 127) / 128);
+      work += counted * sp.q * sp.K * sp.N;
+      if (sp.accumulate != kJoin) tiles += (counted * sp.q + 127) / 128 * ((sp.N + 127) / 128);
     }
     const bool small = work <= (tiles <= kFewTiles ? 4 : 1) * kSmallLinear;
     for (size_t i = 0, j; i < specs.size() && err == cudaSuccess; i = j) {
@@ -989,9 +991,17 @@ struct Model : ModelBase {
   }
   // Plain (not per-species) linears.  c_map: row a of the results belongs to atom c_map[a] (nullptr: the same order).
   cudaError_t run_linear(const std::vector<LinSpec>& specs, long long n_atoms, cudaStream_t s, const int* c_map = nullptr) {
+    return run_linear(specs, n_atoms, n_atoms, s, c_map);
+  }
+  // Linears whose rows are edges: a captured pass has the edges of its capacity where a direct one has those of the list, and both are to
+  // take the same kernels.
+  cudaError_t run_edge_linear(const std::vector<LinSpec>& specs, long long n_edges, cudaStream_t s) {
+    return run_linear(specs, n_edges, round_edges(n_edges), s, nullptr);
+  }
+  cudaError_t run_linear(const std::vector<LinSpec>& specs, long long n_atoms, long long counted, cudaStream_t s, const int* c_map) {
     GemmBatch<T> gb = plain_batch(n_atoms);
     gb.c_atom_map = c_map;
-    return run_specs(specs, n_atoms, s, gb, [&](TcLinearProblem& h, const LinSpec&) { h.atom_map = c_map; },
+    return run_specs(specs, n_atoms, counted, s, gb, [&](TcLinearProblem& h, const LinSpec&) { h.atom_map = c_map; },
                      [&](GemmBatch<T>& g, const LinSpec& sp, int accumulate, int join) {
                        add_problem(g, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, accumulate, join);
                        g.p[g.n_problems - 1].act_out = sp.act_out; g.p[g.n_problems - 1].act_in = sp.act_in;
@@ -1014,7 +1024,7 @@ struct Model : ModelBase {
     gb.c_atom_map = specs[0].mapped ? b.species_perm : nullptr;
     for (const auto& sp : specs)
       if (sp.mapped != specs[0].mapped) return cudaErrorInvalidValue;
-    return run_specs(specs, n_atoms, s, gb,
+    return run_specs(specs, n_atoms, n_atoms, s, gb,
                      [&](TcLinearProblem& h, const SpeciesSpec& sp) {
                        h.n_groups = n_el; h.group_ptr = b.species_ptr; h.tile_ptr = b.tc_tile_ptr + (sp.q / 2) * (n_el + 1);
                        h.atom_map = gb.c_atom_map;
@@ -1128,16 +1138,16 @@ struct Model : ModelBase {
     std::vector<LinSpec> sp;
     CKL(launch_tece(ta, TECE_ROTATE_IN, s));
     so2_specs(sp, pre, {{0, lb.tKs, t_NR, lb.tKp, t_NR}, {1, lb.tQt, t_NR, lb.tQp, t_NR}}, false);
-    CKL(run_linear(sp, E, s)); sp.clear();
+    CKL(run_edge_linear(sp, E, s)); sp.clear();
     cudaStream_t side;  // the attention weights, beside the linears and the cluster expansion of the messages
     CKS(branch(s, &side));
     CKL(launch_tece(ta, TECE_LOGIT, side));
     CKL(launch_tece(ta, TECE_SOFTMAX, side));
     so2_specs(sp, pre, {{2, lb.tMw, t_NR, lb.tup, t_G + t_NF}, {3, lb.tMw, t_NR, lb.tglu, t_NF}, {4, lb.tMw, t_NR, lb.tcoef, t_WN}}, false);
-    CKL(run_linear(sp, E, s)); sp.clear();
+    CKL(run_edge_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_MIX, s));
     so2_specs(sp, pre, {{5, lb.tU, t_NF, lb.tdown, t_NR}}, false);
-    CKL(run_linear(sp, E, s)); sp.clear();
+    CKL(run_edge_linear(sp, E, s)); sp.clear();
     CKS(merge(s));
     CKL(launch_tece(ta, TECE_ROTATE_OUT, s));
     return TACE_OK;
@@ -1156,14 +1166,14 @@ struct Model : ModelBase {
     CKL(launch_tece(ta, TECE_LOGIT_BWD, side));
     CKL(launch_tece(ta, TECE_EDGE_SCALAR_BWD, side));
     so2_specs(sp, pre, {{5, lb.tgdown, t_NF, lb.tU, t_NR}}, true);   // gU over U
-    CKL(run_linear(sp, E, s)); sp.clear();
+    CKL(run_edge_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_MIX_BWD, s));                           // gup / gglu / gcoef over their forward buffers
     // gMw over Mw: the three linears that read Mw add up in one pass per order
     so2_specs(sp, pre, {{2, lb.tup, t_NR, lb.tMw, t_G + t_NF}, {3, lb.tglu, t_NR, lb.tMw, t_NF}, {4, lb.tcoef, t_NR, lb.tMw, t_WN}}, true);
-    CKL(run_linear(sp, E, s)); sp.clear();
+    CKL(run_edge_linear(sp, E, s)); sp.clear();
     CKS(merge(s));
     so2_specs(sp, pre, {{0, lb.tgKp, t_NR, lb.tgKs, t_NR}, {1, lb.tgQp, t_NR, lb.tgQt, t_NR}}, true);
-    CKL(run_linear(sp, E, s)); sp.clear();
+    CKL(run_edge_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_ROTATE_IN_BWD, s));
     ta.accumulate_gvec = first_tece ? 0 : 1;
     CKS(branch(s, after));  // what only the end of the pass needs
@@ -1220,7 +1230,7 @@ struct Model : ModelBase {
         if (fused) spec.act_out = in == lb.H3 ? lb.Hact : lb.H3;
         sp.push_back(spec);
       }
-      CKL(run_linear(sp, Ec, s));
+      CKL(run_edge_linear(sp, Ec, s));
     }
     return TACE_OK;
   }
@@ -1265,7 +1275,7 @@ struct Model : ModelBase {
         if (fused_activations() && j == 2) spec.act_in = lb.Z2;  // (j == 1: launch_edge_mlp_out applies the first layer's)
         sp.push_back(spec);
       }
-      CKL(run_linear(sp, Ec, s));
+      CKL(run_edge_linear(sp, Ec, s));
     }
     EdgeArgs<T> er = edge_range(ea, b, ts, e0, Ec);
     if (ln) {  // through the first hidden layer's LayerNorm and activation; launch_edge_mlp_out then starts from dE/dz1

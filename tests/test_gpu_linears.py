@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from tace_b200 import synth
+from helpers import make_models, oracle_batch, to_device
 from test_gpu_parity import run_case
 
 pytestmark = pytest.mark.gpu
@@ -30,3 +31,39 @@ def test_double_precision_tiles(L, channels):
 @pytest.mark.parametrize("channels", [64, 96, 128])
 def test_products_of_several_orders_in_one_loop(channels, correlation):
     run_case([_cluster((1, 17, 43, 3), (1, 6, 7, 8))], 2, channels, [1, 6, 7, 8], 3.0, torch.float32, correlation=correlation)
+
+
+# Multiply-adds of a call up to which its linears run on the CUDA cores (kSmallLinear in csrc/engine.cu)
+SMALL = 32 << 20
+
+
+def _edge_linear_work(model, calls):
+    """Multiply-adds per edge of the SO(2) linears numbered in `calls` (two rows per order above 0)."""
+    linears = model.readout_fn.plan.so2_linears()
+    return sum((1 if m == 0 else 2) * n_in[m] * ci * n_out[m] * co
+               for _, _, ci, co, n_in, n_out in (linears[k] for k in calls) for m in range(len(n_in)))
+
+
+@pytest.mark.parametrize("calls", [None, (5,), (0, 1)])
+def test_replays_take_the_kernels_of_the_direct_pass(calls, monkeypatch):
+    """A captured pass holds more edges than the list (its capacity), a direct one exactly the list's: with the last edge count below
+    a limit in the work of the linears over edges, and the capacity above it, both run the same kernels and agree bit for bit.  The
+    hidden layers of the radial MLPs of three interactions, and the SO(2) linears of two launches in the edge block's backward pass."""
+    monkeypatch.setenv("TACE_B200_RADIAL_TABLE", "0")
+    tece = {"num_head": 4, "edge_ace_hidden": 64, "mmax": 2} if calls else None
+    model, _, _ = make_models(2, 64, [13, 29], 5.0, 40.0, torch.float32, num_layers=2 if calls else 3, tece=tece,
+                              radial={"apply_cutoff": False} if calls else None)
+    n_edges = SMALL // (_edge_linear_work(model, calls) if calls else 3 * 64 * 64)
+    assert 32 <= n_edges <= 4096 and n_edges % (64 if n_edges <= 2048 else 128) != 0
+    data = to_device(oracle_batch([synth.fcc_supercell(3, 3.65, 0.05, seed=2, species=(13, 29), fractions=(0.5, 0.5))], [13, 29], 5.0, torch.float32),
+                     torch.device("cuda:0"))
+    assert data["edge_index"].shape[1] > n_edges
+    keep = torch.randperm(data["edge_index"].shape[1], generator=torch.Generator().manual_seed(0))[:n_edges].to("cuda:0")
+    data = dict(data, edge_index=data["edge_index"][:, keep].contiguous(), edge_shifts=data["edge_shifts"][keep].contiguous())
+    direct = {k: v.clone() for k, v in model(data).items() if v is not None}
+    assert model.graph_replays() == 0
+    for n in range(3):
+        out = model(data)
+        for k, v in direct.items():
+            assert torch.equal(out[k], v), (n, k)
+    assert model.graph_replays() >= 2
