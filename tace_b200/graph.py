@@ -93,8 +93,9 @@ def build_batch(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cuto
 
 def model_inputs(batch: Dict[str, np.ndarray], model_numbers: Sequence[int], cutoff: float, dtype: torch.dtype,
                  device: torch.device) -> Dict[str, torch.Tensor]:
-    """What ``TensorModel.forward`` reads of ``build_batch``'s dictionary, in the types that it uses, for callers who hand it on and
-    keep nothing: no one-hot attributes beside the species, and structure offsets that need no conversion."""
+    """What ``TensorModel.forward`` reads of ``build_batch``'s dictionary, in the types that it uses, for callers who hand it to that
+    function alone (``models.reads_inputs_only``) and keep nothing: no one-hot attributes beside the species, and structure offsets
+    that need no conversion."""
     up, _, edge_index, shifts = _structures_on_device(batch, model_numbers, cutoff, dtype, device, ("ptr32", "positions", "lattice", "species"))
     return {"positions": up["positions"], "lattice": up["lattice"], "species": up["species"], "edge_index": edge_index, "edge_shifts": shifts,
             "ptr": up["ptr32"]}

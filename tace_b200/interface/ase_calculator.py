@@ -13,8 +13,8 @@ from typing import List, Optional, Union
 import numpy as np
 import torch
 
-from ..graph import model_inputs
-from ..models import TensorModel, create_model
+from ..graph import build_batch, model_inputs
+from ..models import TensorModel, create_model, reads_inputs_only
 
 try:  # ASE is optional: without it the class still works with any object exposing the four getters below
     from ase.calculators.calculator import Calculator, all_changes
@@ -126,7 +126,8 @@ class TACEAseCalc(Calculator):
             "batch": np.zeros(n, dtype=np.int64),
             "ptr": np.array([0, n], dtype=np.int64),
         }
-        data = model_inputs(host, self.atomic_numbers, self.cutoff, self.dtype, self.device)
+        inputs = model_inputs if reads_inputs_only(self.model) else build_batch
+        data = inputs(host, self.atomic_numbers, self.cutoff, self.dtype, self.device)
         outs = self.model(data)
         fetch = _fetch([outs[p] for p in self.target_property if outs.get(p) is not None])
         self.results = {}

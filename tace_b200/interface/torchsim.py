@@ -17,7 +17,7 @@ from typing import Callable, Dict, List, Optional, Union
 import torch
 
 from ..graph import z_to_index  # noqa: F401  (re-exported for drivers that prepare species themselves)
-from ..models import TensorModel
+from ..models import TensorModel, reads_inputs_only
 from ..lib import TaceError
 from ..neighbour_list import _list_on_device, neighbor_list_batch
 from .ase_calculator import load_tace
@@ -141,6 +141,7 @@ class TACETorchSimCalc(_Base):
                 self._setup_ptr(sidx)
                 self.system_idx = sidx
         pbc = state.pbc
+        own = reads_inputs_only(self.model)  # offsets and shifts in the types that it uses instead of the contract's
         if (self.neighbor_list_fn is tace_b200_nl and isinstance(pbc, (tuple, list)) and len(pbc) == 3
                 and all(isinstance(p, (bool, int)) for p in pbc) and state.row_vector_cell.numel() == 9 * self.n_systems):
             # this package's own list, without working the systems' offsets out again (they belong to `system_idx`) and
@@ -150,11 +151,11 @@ class TACETorchSimCalc(_Base):
             edge_index, unit_shifts = _list_on_device(state.positions.to(torch.float64).contiguous(),
                                                       state.row_vector_cell.to(torch.float64).reshape(-1, 3, 3).contiguous(),
                                                       self._periodic_rows(tuple(map(bool, pbc)), state.positions.device),
-                                                      self._ptr32, self.r_max, -1, self._dtype)
+                                                      self._ptr32, self.r_max, -1, self._dtype if own else torch.int32)
         else:
             edge_index, _mapping, unit_shifts = self.neighbor_list_fn(state.positions, state.row_vector_cell, pbc, self.r_max, self.system_idx)
         out = self.model({
-            "ptr": self._ptr32, "node_attrs": self.node_attrs, "species": self.species, "batch": self.system_idx, "pbc": state.pbc,
+            "ptr": self._ptr32 if own else self.ptr, "node_attrs": self.node_attrs, "species": self.species, "batch": self.system_idx, "pbc": state.pbc,
             "lattice": state.row_vector_cell, "positions": state.positions, "edge_index": edge_index, "edge_shifts": unit_shifts,
         })
         results: Dict[str, torch.Tensor] = {}

@@ -730,6 +730,18 @@ class TensorModel(torch.nn.Module):
         return buf[:n]
 
 
+_FORWARD = TensorModel.forward
+
+
+def reads_inputs_only(model) -> bool:
+    """Whether calling ``model`` runs ``TensorModel.forward`` of this module and nothing else that sees its input: then the input may
+    hold what that function reads, in the types that it uses.  Everything else (another object, a subclass, hooks, a replaced or
+    compiled forward) is promised the fields of the reference's ``forward(data)`` contract."""
+    hooks = torch.nn.modules.module
+    return (type(model) is TensorModel and getattr(model.forward, "__func__", None) is _FORWARD and model._compiled_call_impl is None
+            and not (model._forward_pre_hooks or model._forward_hooks or hooks._global_forward_pre_hooks or hooks._global_forward_hooks))
+
+
 def create_model(model_config: Dict, statistics=None, target_property=None, **_) -> TensorModel:
     """``TensorModel(e3nnTACE(**model_config))`` as tace/lightning/torch_model.py:54-114 builds it."""
     cfg = dict(model_config)

@@ -65,6 +65,69 @@ def test_ase_calculator_calls_the_model_as_a_module():
     assert np.abs(calc.results["forces"] - 0.5 * (singles[0]["forces"] + singles[1]["forces"])).max() < 1e-12
 
 
+def _contract(model, seen):
+    """An object in a model's place that works from the fields of the reference's ``forward(data)`` contract alone."""
+    def call(data):
+        fields = {k: data[k] for k in ("positions", "lattice", "node_attrs", "edge_index", "edge_shifts", "batch", "ptr")}
+        n = fields["positions"].shape[0]
+        assert fields["node_attrs"].dtype == fields["positions"].dtype and (fields["node_attrs"].sum(1) == 1).all()
+        assert fields["batch"].dtype == fields["ptr"].dtype == torch.int64 and fields["batch"].shape == (n,)
+        assert fields["edge_shifts"].dtype in (torch.int32, torch.float64)
+        assert torch.equal(fields["ptr"], torch.cat([fields["ptr"][:1] * 0, torch.bincount(fields["batch"]).cumsum(0)]))
+        assert torch.equal(fields["node_attrs"].argmax(1), data["species"].long())
+        seen.append(set(data))
+        return model(fields)
+    return call
+
+
+def test_ase_calculator_hands_others_the_whole_contract():
+    """Whatever is called in the place of this package's own forward, or looks on, gets every field of the contract in its types: an
+    object put there, a subclass, hooks of the model and of all modules, a forward set on the object."""
+    from tace_b200 import TensorModel
+
+    s = synth.fcc_supercell(2, 3.61, 0.05, seed=0, species=(13, 29), fractions=(0.5, 0.5))
+    model = make_models(2, 32, [13, 29], 4.0, 20.0, torch.float64)[0]
+    calc = TACEAseCalc(model, device="cuda:0")
+    atoms, seen = FakeAtoms(s), []
+    calc.calculate(atoms)
+    want = calc.results
+    inner = make_models(2, 32, [13, 29], 4.0, 20.0, torch.float64)[0]
+    look = _contract(inner, seen)
+
+    def check(count):
+        calc.calculate(atoms)
+        assert len(seen) == count
+        assert calc.results["energy"] == want["energy"] and np.array_equal(calc.results["forces"], want["forces"])
+
+    calc.model = look
+    check(1)
+    calc.model = model
+    for n, register in enumerate((model.register_forward_pre_hook, model.register_forward_hook,
+                                  torch.nn.modules.module.register_module_forward_pre_hook)):
+        busy = []
+
+        def hook(module, args, *_):
+            if module is model and not busy:  # `look` calls a model itself
+                busy.append(1)
+                look(args[0])
+
+        handle = register(hook)
+        check(2 + n)
+        handle.remove()
+
+    class Sub(TensorModel):
+        def forward(self, data):
+            return look(data)
+
+    model.__class__ = Sub
+    check(5)
+    model.__class__ = TensorModel
+    model.forward = look
+    check(6)
+    del model.forward
+    check(6)
+
+
 class FakeLammpsData:
     """Single-rank stand-in for the Kokkos ML-IAP data object: local atoms plus periodic ghost copies."""
 
@@ -184,6 +247,29 @@ def test_torchsim_model_matches_oracle_and_reuses_cached_setup():
     state.atomic_numbers[0] = 7
     with pytest.raises(ValueError):
         calc(state)
+
+
+def test_torchsim_model_hands_others_the_whole_contract():
+    """The same for the TorchSim model, with this package's own list and with the systems' flags as a tensor."""
+    from tace_b200.interface import TACETorchSimCalc
+
+    structs = synth.random_crystals(3, seed=12, nmin=4, nmax=10, zmax=3)
+    dev = torch.device("cuda:0")
+    calc = TACETorchSimCalc(make_models(2, 32, [1, 2, 3], 4.5, 20.0, torch.float64)[0], device=dev, dtype=torch.float64)
+    inner = make_models(2, 32, [1, 2, 3], 4.5, 20.0, torch.float64)[0]
+    seen, state = [], FakeSimState(structs, dev)
+    look = _contract(inner, seen)
+    for pbc in ((True, True, True), state.pbc):
+        state.pbc = pbc
+        want = {k: v.clone() for k, v in calc(state).items()}
+        shifts = []
+        handle = calc.model.register_forward_pre_hook(lambda _, args: (look(args[0]), shifts.append(args[0]["edge_shifts"].dtype)) and None)
+        out = calc(state)
+        handle.remove()
+        assert shifts == [torch.int32]  # what neighbour-list functions return
+        for k, v in want.items():
+            assert torch.equal(out[k], v), k
+    assert len(seen) == 2
 
 
 def test_lammps_mliap_with_the_tece_edge_block():
