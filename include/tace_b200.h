@@ -159,7 +159,12 @@ void tace_destroy(TaceModel* model);
  * (tace/lightning/lit_model.py:587-609,664-677): the host side repacks the reference's
  * parameters (normalisation constants folded in) into the named arrays listed here and
  * uploads each one (HOST pointer, model dtype).  tace_forward refuses to run until every
- * array has been set. */
+ * array has been set; an array may be set again at any time between two evaluations.
+ * Derived arrays: in models without the edge block (TaceConfig.tece_layers == 0) the library takes the
+ * transposes and the TF32 parts of the product's per-species coefficients ("tN.cJT.lL" and every
+ * "tN.cJ.lL_hi", "tN.cJ.lL_lo", "tN.cJT.lL_hi", "tN.cJT.lL_lo") from "tN.cJ.lL" and "tN.lin.lL", which it
+ * multiplies.  They are listed and have to be set once, with the listed size, but their content is not
+ * read: to change coefficients set "tN.cJ.lL". */
 int tace_weight_count(const TaceModel* model);
 int tace_weight_info(const TaceModel* model, int index, const char** name, int64_t* numel);
 int tace_set_weight(TaceModel* model, const char* name, const void* host_data, int64_t numel);

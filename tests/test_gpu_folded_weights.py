@@ -72,3 +72,22 @@ def test_weights_set_again(correlation, C, dtype, kind):
         assert not torch.equal(model(gpu)["energy"], before["energy"]), name
         _set(model, mine, [name], dtype)
         assert torch.equal(model(gpu)["energy"], before["energy"]), name
+
+
+@pytest.mark.parametrize("dtype,tece", [(torch.float32, None), (torch.float64, None), (torch.float64, {"num_head": 4, "edge_ace_hidden": 8, "mmax": 2})])
+def test_derived_coefficients_are_taken_from_what_they_derive_from(dtype, tece):
+    """include/tace_b200.h: the content of the derived arrays is not read, of the right size they are accepted, of another refused; models
+    with the edge block use them as they are set."""
+    model, _, _ = make_models(2, 64, [13, 29], 4.0, 12.0, dtype, seed=1, tece=tece, radial={"apply_cutoff": False} if tece else None)
+    gpu = to_device(oracle_batch([synth.fcc_supercell(2, 3.65, 0.05, seed=3, species=(13, 29), fractions=(0.5, 0.5))], [13, 29], 4.0, dtype), DEV)
+    before = {k: v.clone() for k, v in model(gpu).items() if v is not None}
+    derived = [n for n in _names(model) if n[3:4] == "c" and n[4:5] in "012" and (n[5] == "T" or n.endswith(("_hi", "_lo")))]
+    assert len(derived) == 4 * 2 * (5 if dtype is torch.float32 else 1)  # two orders of three ranks and one of the scalar layer above
+    packed = _packed(model)
+    noise = {n: np.full(np.shape(packed[n]), 3.0) for n in derived}
+    _set(model, noise, derived, dtype)
+    out = model(gpu)
+    for k, v in before.items():
+        assert torch.equal(out[k], v) == (tece is None or k in ("energy", "node_energy")), k
+    with pytest.raises(_lib.TaceError):
+        _set(model, {derived[0]: np.zeros(7)}, derived[:1], dtype)
