@@ -660,10 +660,12 @@ int bwd_shares(const TPArgs<T>& a) {
 }
 template <typename T, typename TP, bool RT>
 cudaError_t launch_bwd_v(const TPArgs<T>& a, size_t smem, cudaStream_t s) {
-  static size_t configured[64] = {};  // the attribute belongs to a device: one slot per device ordinal
+  // The attribute belongs to a device: one slot per device ordinal.  It is raised for every size: the kernels have static shared memory
+  // besides, so that sizes up to the default 48 KB do not fit without it either.
+  static size_t configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidValue;
-  if (smem > 48 * 1024 && smem > configured[dev]) {
+  if (smem > configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(tp_bwd_kernel<T, TP, false, RT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(tp_bwd_kernel<T, TP, true, RT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(tp_bwd_kernel<T, TP, false, RT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -687,7 +689,7 @@ cudaError_t launch_bwd_scalar(const TPArgs<T>& a, cudaStream_t s) {
   static size_t configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidValue;
-  if (smem > 48 * 1024 && smem > configured[dev]) {
+  if (smem > configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(tp_bwd_scalar_kernel<T, TP, ENV, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     configured[dev] = smem;

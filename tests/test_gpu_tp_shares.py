@@ -33,3 +33,13 @@ def test_few_and_many_targets_agree(C, dtype):
     few, many = (model(build_batch(synth.collate([synth.fcc_supercell(n, 3.61, 0.0, seed=1)]), [29], 5.0, dtype, DEV))["energy"].item() / (4 * n ** 3)
                  for n in (3, 10))
     assert abs(many - few) <= (1e-5 if dtype is torch.float32 else 1e-8)
+
+
+@pytest.mark.parametrize("C,dtype", [(96, torch.float64), (192, torch.float32)])
+def test_first_interaction_with_48_kb_of_dynamic_shared_memory(C, dtype):
+    """Rank 3 at these widths: (16 + 8 (4 + 2)) C values are 48 KB to the byte, and the kernel has static shared memory besides."""
+    structs = [_ring(9)]
+    model, oracle, _ = make_models(3, C, [13, 29], 4.0, 12.0, dtype)
+    model.set_radial_table(False)
+    data = oracle_batch(structs, [13, 29], 4.0, dtype)
+    check_parity(model(to_device(data, DEV)), oracle(data), data["ptr"], dtype, f"C{C}")
