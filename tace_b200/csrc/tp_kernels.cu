@@ -623,16 +623,22 @@ cudaError_t launch_chunk_src_sum(const T* dxe_chunk, const int* keys, const int*
 }
 
 // Few targets: four sets of threads share the edges of one, so that a cell of a few hundred atoms does not walk its edge lists with
-// two warps per SM.  Rank 2, 64 channels, fp64, 256 targets of 42 edges: 60 -> 26 us, first layer 15 -> 12.  Above twelve warps per SM
-// the chip has other targets to work on while one waits.
-template <typename T>
+// two warps per SM.  Rank 2, 64 channels, fp64, 256 targets of 42 edges: 60 -> 26 us, first layer 15 -> 12.  The line is at six warps per
+// SM (888; warps = targets x channels / 32), from there on the chip has other targets to work on while one waits.  Passes without -> with
+// shares, in us, 42 edges per target: fp64, rank 2, 64 channels, 864 warps 755 -> 725, 1 296: 999 -> 1 009; rank 3, 128 channels, 864:
+// 1 660 -> 1 593, 1 296: 2 189 -> 2 238; rank 1, 96 channels, 648: 401 -> 401, 972: 468 -> 482.  fp32 with weights in memory, rank 3,
+// 64 channels (where the shares spill 164 bytes), 432: 578 -> 525, 864: 807 -> 801, 1 296: 966 -> 1 019; 96 channels, 648: 821 -> 825, 972:
+// 1 110 -> 1 168.  fp32 with the table, rank 3, 32 channels, 756: 455 -> 441, 1 404: 668 -> 672.  Only fp64 at rank 3 over sources of rank 2
+// gains up to twice the line (64 channels, 1 296: 1 608 -> 1 500, 1 728: 1 881 -> 1 784).
+template <typename T, typename TP>
 bool share_fwd_edges(const TPArgs<T>& a) {
-  return a.split_sums && a.C <= 128 && (long long)a.n_seg * (a.C / 32) <= 12LL * kSMs && a.n_edges >= 16LL * a.n_seg;
+  constexpr int kWarps = std::is_same<T, double>::value && std::is_same<TP, TPX_L3_N2>::value ? 12 : 6;
+  return a.split_sums && a.C <= 128 && (long long)a.n_seg * (a.C / 32) <= (long long)kWarps * kSMs && a.n_edges >= 16LL * a.n_seg;
 }
 template <typename T, typename TP, int GRP, bool ENV, bool RT>
 void launch_fwd_grp(const TPArgs<T>& a, cudaStream_t s) {
   if (a.row_ids) tp_fwd_kernel<T, TP, GRP, ENV, RT, true, 1><<<(a.n_seg + kListRows - 1) / kListRows, a.C, 0, s>>>(a);
-  else if (share_fwd_edges(a)) tp_fwd_kernel<T, TP, GRP, ENV, RT, false, 4><<<a.n_seg, 4 * a.C, sizeof(T) * 3 * kShareRows * a.C, s>>>(a);
+  else if (share_fwd_edges<T, TP>(a)) tp_fwd_kernel<T, TP, GRP, ENV, RT, false, 4><<<a.n_seg, 4 * a.C, sizeof(T) * 3 * kShareRows * a.C, s>>>(a);
   else tp_fwd_kernel<T, TP, GRP, ENV, RT, false, 1><<<a.n_seg, a.C, 0, s>>>(a);
 }
 template <typename T, typename TP, bool ENV, bool RT>
