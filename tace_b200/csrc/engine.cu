@@ -947,8 +947,11 @@ struct Model : ModelBase {
   // pass: their energies feel the rounding of the linears most (3e-5 between the two paths), and that is not to show between systems
   // of different size.
   // Four times as many where the tensor cores have at most kFewTiles tiles, each walking a long K loop on one SM (128 rows,
-  // K = 4 352: 73 -> 43 us).
-  static constexpr long long kSmallLinear = 32LL << 20, kFewTiles = 8;
+  // K = 4 352: 73 -> 43 us).  A per-species launch has tiles for every element present, which the host does not know, and that keeps
+  // the tensor cores ahead from some number of elements on: evaluations of 24 and 48 atoms at rank 3, 128 channels, with the limit as it
+  // is -> fourfold, 8 elements in the model 301 -> 292 us and 323 -> 316, 16 elements 305 -> 300 and even, 32 elements 318 -> 321 and
+  // 345 -> 350, 89 elements 340 -> 346 and 389 -> 385 (40 atoms 373 -> 377).  So it ends at kFewElements.
+  static constexpr long long kSmallLinear = 32LL << 20, kFewTiles = 8, kFewElements = 16;
   bool backward_pass = false;  // what forward() is enqueuing
   // counted: rows for which the kernels are chosen.
   template <typename Spec, typename FillTc, typename Add>
@@ -958,12 +961,13 @@ struct Model : ModelBase {
     int n_tc = 0;
     GemmBatch<T> gb = empty;
     cudaError_t err = cudaSuccess;
-    long long work = 0, tiles = 0;  // tiles of the tensor-core kernel
+    long long work = 0, tiles = 0;  // tiles: of the tensor-core kernel, all elements taken together
     for (const Spec& sp : specs) {
       work += counted * sp.q * sp.K * sp.N;
       if (sp.accumulate != kJoin) tiles += (counted * sp.q + 127) / 128 * ((sp.N + 127) / 128);
     }
-    const bool small = work <= (tiles <= kFewTiles ? 4 : 1) * kSmallLinear;
+    const bool few = tiles <= kFewTiles && empty.n_groups <= kFewElements;
+    const bool small = work <= (few ? 4 : 1) * kSmallLinear;
     for (size_t i = 0, j; i < specs.size() && err == cudaSuccess; i = j) {
       bool tc = kTensorCore && ((tece_mask && !backward_pass) || !small);
       for (j = i; j < specs.size() && (j == i || specs[j].accumulate == kJoin); ++j) tc = tc && tc_linear_supported(specs[j].N, specs[j].K);

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from tace_b200 import synth
-from helpers import make_models, oracle_batch, to_device
+from helpers import check_parity, make_models, oracle_batch, to_device
 from test_gpu_parity import run_case
 
 pytestmark = pytest.mark.gpu
@@ -67,3 +67,18 @@ def test_replays_take_the_kernels_of_the_direct_pass(calls, monkeypatch):
         for k, v in direct.items():
             assert torch.equal(out[k], v), (n, k)
     assert model.graph_replays() >= 2
+
+
+@pytest.mark.parametrize("n_el", [16, 17])
+@pytest.mark.parametrize("n_atoms", [24, 40])
+def test_per_species_linears_of_few_tiles(n_el, n_atoms):
+    """Per-species linears of little more than the limit in work, for a model with the largest number of elements for which they stay on the
+    CUDA cores and for one with an element more."""
+    elements = list(range(1, n_el + 1))
+    structs = synth.random_crystals(1, seed=5, nmin=n_atoms, nmax=n_atoms, zmax=n_el)
+    model, oracle, _ = make_models(3, 128, elements, 4.0, 20.0, torch.float32)
+    plan = model.readout_fn.plan.layers[0]
+    rows = [n_atoms * (2 * l + 1) for l in plan.out_ls]
+    assert SMALL < sum(r * (1 + k) for r, k in zip(rows, plan.kp)) * 128 * 128 <= 4 * SMALL and sum((r + 127) // 128 for r in rows) <= 8
+    data = oracle_batch(structs, elements, 4.0, torch.float32)
+    check_parity(model(to_device(data, torch.device("cuda:0"))), oracle(data), data["ptr"], torch.float32, f"{n_el} elements {n_atoms} atoms")
