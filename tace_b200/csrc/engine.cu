@@ -157,12 +157,16 @@ struct ModelBase {
     if (cudaEventRecord(ev_merge, branch_stream) != cudaSuccess || cudaStreamWaitEvent(s, ev_merge, 0) != cudaSuccess) return TACE_ERR_CUDA;
     return TACE_OK;
   }
-  // Branches end where a pass fills the chip by itself: 8 600 edges of the edge block 3 831 -> 3 671 us for two frames, 524 000 edges
-  // 74.5 -> 75.8 ms; 11 000 edges in double precision 1 456 -> 1 374 us for two frames.
+  // Branches end where a pass fills the chip by itself; the line is the last size at which no kind of model loses by them.  One pass
+  // without -> with them, in us.  Edge block (rank 3, 128 channels): 8 200 edges 1 760 -> 1 646, 28 000: 4 457 -> 4 412, 66 000: 10 018 ->
+  // 9 927, 94 000: 13 663 -> 13 685, 128 000: 18 634 -> 18 824, 526 000: 74 207 -> 75 390.  Radial table: rank 2, 64 channels, 11 000: 205 ->
+  // 201, 59 000: 409 -> 407, 88 000: 525 -> 523, 469 000: 1 972 -> 1 975; rank 3, 128 channels, 21 000: 643 -> 641, even above.  fp32 with
+  // weights in memory (rank 3, 128 channels): 21 000: 1 375 -> 1 356, 59 000: 2 818 -> 2 808, even above.  Double precision (rank 2, 64
+  // channels) gains above the line too: 11 000: 535 -> 497, 59 000: 1 961 -> 1 888, 88 000: 2 609 -> 2 542, 171 000: 4 877 -> 4 762.
   static constexpr int64_t kBranchEdges = 1 << 16;
   // Streams and events of a captured pass.  With the fp64 products of the radial MLPs (thousands of blocks) on a branch, the main line
-  // takes the higher priority, so that its small kernels do not stand in line behind them (1 374 us above, 1 439 without).  The edge
-  // block's main line is large products with small kernels on the branch; there it loses (3 671 us without, 3 745 with).
+  // takes the higher priority, so that its small kernels do not stand in line behind them (two frames of 256 atoms 1 439 -> 1 374 us).  The edge
+  // block's main line is large products with small kernels on the branch; there it loses (two frames of 128 atoms 3 671 us without, 3 745 with).
   virtual bool main_line_first() const = 0;
   bool capture_streams() {
     if (capture_stream) return true;
@@ -1319,7 +1323,9 @@ struct Model : ModelBase {
     return TACE_OK;
   }
 
-  // Buffers of a layer's backward pass that are added to, or written only where the output has a rank.
+  // Buffers of a layer's backward pass that are added to, or written only where the output has a rank.  Captured passes clear them on the
+  // branch: rank 3 with features of rank 2, 64 channels, 32 atoms 175.7 -> 173.6 us, 256: 253.4 -> 251.3, 1 372: 567.0 -> 565.1; rank 2,
+  // 108 atoms 166.3 -> 165.1 (runs of one side within 0.2 to 1.2 us); edge block, 54 atoms 1 037 -> 1 035, nothing beyond the spread above.
   int zero_gradients(const LayerPlan& p, const LayerBufs& lb, long long NL, cudaStream_t s) {
     if (bilinear) CKL(launch_fill_zero(lb.gXY, NL * D * 2 * C, s));
     else if ((int)p.out_ls.size() != L + 1) CKL(launch_fill_zero(lb.gAs, NL * D * C, s));

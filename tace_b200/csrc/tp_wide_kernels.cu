@@ -268,8 +268,9 @@ struct WideBwdShape {
   static constexpr int NRED = TP::D + 2;          // dY | dE/d(length) | dE/d(envelope)
   static constexpr int kMsgFloats = TP::NM * C, kEdgeFloats = TP::GVS + (CW > 1 ? CW * NRED : 0);
   // Edges of a batch, which costs the block two barriers: 32, so that a whole warp of lanes builds rows, where the 16 warps that fit
-  // an SM by their registers then still fit its shared memory (rank 3, 128 channels: two blocks of 96 KB).  Against 16: 64 crystals
-  // 2 705 -> 2 692 us, 1 372 atoms 588 -> 583, MD step of 131 072 atoms 23 491 -> 23 342.
+  // an SM by their registers then still fit its shared memory (rank 3, 128 channels: two blocks of 96 KB).  Against 16 (runs of one side
+  // within 0.2 %): 64 crystals 2 641 -> 2 632 us, 1 372 atoms 563 -> 558, water box of 32 400 atoms 44 932 -> 44 610, eight of 192 atoms
+  // 2 451 -> 2 439, MD step of 131 072 atoms 22 981 -> 22 928.
   static constexpr int kBatch = (16 / kWarps) * ((kMsgFloats + 32 * kEdgeFloats) * 4 + 2048) <= 224 * 1024 ? 32 : 16;
   static constexpr int kGFloats = kBatch * TP::GVS, kRedFloats = CW > 1 ? kBatch * CW * NRED : 0;
   static constexpr int kBytes = (kMsgFloats + kGFloats + kRedFloats) * 4;
