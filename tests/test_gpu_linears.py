@@ -1,6 +1,7 @@
 """The linears at the sizes where their tiles end: the double-precision kernel (32 x 32 tiles, K steps of 16) with species that own
-one atom, one tile less a row, exactly one tile and one row more; the tensor-core kernel where the products of several
-correlation orders share one accumulator loop, mixed with widths it does not take.  Against the oracle."""
+one atom, one tile less a row, exactly one tile and one row more; the products of several correlation orders in one accumulator loop, on
+the CUDA cores and, with more work, on the tensor cores, mixed with widths that those do not take.  The limit in work between the two: sizes on
+both sides, and all linears of a pass above it.  Against the oracle."""
 import numpy as np
 import pytest
 import torch
@@ -35,6 +36,69 @@ def test_products_of_several_orders_in_one_loop(channels, correlation):
 
 # Multiply-adds of a call up to which its linears run on the CUDA cores (kSmallLinear in csrc/engine.cu)
 SMALL = 32 << 20
+
+
+def _atom_linear_work(plan):
+    """Multiply-adds per atom of the calls of a pass whose rows are atoms, by name (fp32, gated scalars, skip connections aware)."""
+    C2, L, out = plan.C * plan.C, plan.L, {}
+    for t, lp in enumerate(plan.layers):
+        out[f"t{t}.down"] = sum((2 * l + 1) * lp.k[l] * (L + 2 if l == 0 else 1) for l in range(L + 1)) * C2
+        out[f"t{t}.nl"] = (L + 1) ** 2 * C2
+        orders = [1 + a + b + (1 if lp.has_res else 0) for a, b in zip(lp.kp if plan.correlation > 1 else [0] * len(lp.out_ls), lp.kp3)]
+        out[f"t{t}.coef"] = sum((2 * l + 1) * k for l, k in zip(lp.out_ls, orders)) * C2
+        if not lp.scalar_src:
+            out[f"t{t}.up"] = sum(2 * l + 1 for l in lp.in_ls) * C2
+    return out
+
+
+@pytest.mark.parametrize("correlation", [1, 2, 3])
+@pytest.mark.parametrize("channels", [64, 96, 128])
+def test_products_of_several_orders_on_the_tensor_cores(channels, correlation):
+    """The same on so many atoms that the coefficients of the lower interaction are above the limit (channels that are no multiple of 64
+    leave all but the widest results to the CUDA cores)."""
+    counts = (8, 136, 344, 536 if channels == 64 else 24)
+    model, oracle, _ = make_models(2, channels, [1, 6, 7, 8], 3.0, 20.0, torch.float32, correlation=correlation)
+    work = _atom_linear_work(model.readout_fn.plan)
+    assert sum(counts) * min(work["t0.coef"], work["t0.down"]) > SMALL
+    data = oracle_batch([_cluster(counts, (1, 6, 7, 8))], [1, 6, 7, 8], 3.0, torch.float32)
+    check_parity(model(to_device(data, torch.device("cuda:0"))), oracle(data), data["ptr"], torch.float32, f"C{channels} correlation {correlation}")
+
+
+@pytest.mark.parametrize("L,channels,cells", [(2, 64, 10), (3, 128, 6)])
+def test_all_linears_on_the_tensor_cores(L, channels, cells):
+    """Every linear of the lower interactions and of the radial MLP above the limit: FCC copper and aluminium with twelve neighbours per atom,
+    path weights in memory."""
+    struct = synth.fcc_supercell(cells, 3.61, 0.05, seed=9, species=(13, 29), fractions=(0.5, 0.5))
+    n = len(struct["positions"])
+    keep = np.arange(n) < (1024 if L == 2 else 512)  # a block with surfaces
+    struct = synth.Structure(positions=struct["positions"][keep], atomic_numbers=struct["atomic_numbers"][keep], cell=struct["cell"] * 2.0, pbc=struct["pbc"])
+    model, oracle, _ = make_models(L, channels, [13, 29], 3.0, 12.0, torch.float32)
+    model.set_radial_table(False)
+    data = oracle_batch([struct], [13, 29], 3.0, torch.float32)
+    n, work = int(keep.sum()), _atom_linear_work(model.readout_fn.plan)
+    assert n * min(work[k] for k in ("t0.down", "t0.nl", "t0.coef", "t1.up", "t1.down", "t1.nl")) > SMALL
+    assert data["edge_index"].shape[1] * 2 * 64 * 64 > SMALL  # two interactions' hidden layers in one call
+    check_parity(model(to_device(data, torch.device("cuda:0"))), oracle(data), data["ptr"], torch.float32, f"L{L} C{channels}")
+
+
+@pytest.mark.parametrize("call,L,channels", [("t0.nl", 2, 64), ("t0.down", 3, 128), ("t0.nl", 3, 128)])
+def test_both_sides_of_the_work_limit(call, L, channels):
+    """The largest number of atoms with which a call is within the limit and one atom more: every four-atom crystal of the batch has the
+    energy and the forces that it has alone, on both sides, and they are the oracle's."""
+    model, oracle, _ = make_models(L, channels, [13, 29], 3.0, 12.0, torch.float32)
+    n = SMALL // _atom_linear_work(model.readout_fn.plan)[call]
+    crystal = synth.fcc_supercell(1, 3.61, 0.05, seed=4, species=(13, 29), fractions=(0.5, 0.5))
+    lone = synth.Structure(positions=np.zeros((1, 3)), atomic_numbers=np.array([29]), cell=np.eye(3) * 30.0, pbc=(True, True, True))
+    one = oracle_batch([crystal], [13, 29], 3.0, torch.float32)
+    ref = oracle(one)
+    for atoms in (n, n + 1):
+        structs = [crystal] * (atoms // 4) + [lone] * (atoms % 4)
+        data = oracle_batch(structs, [13, 29], 3.0, torch.float32)
+        out = model(to_device(data, torch.device("cuda:0")))
+        for g in (0, atoms // 4 - 1):
+            part = {"energy": out["energy"][g:g + 1], "forces": out["forces"][4 * g:4 * g + 4], "stress": out["stress"][g:g + 1],
+                    "virials": out["virials"][g:g + 1], "node_energy": out["node_energy"][4 * g:4 * g + 4]}
+            check_parity(part, ref, one["ptr"], torch.float32, f"{call} {atoms} atoms")
 
 
 def _edge_linear_work(model, calls):

@@ -177,7 +177,8 @@ def test_energy_of_large_graphs_is_the_sum_of_their_node_energies():
 
 @pytest.mark.parametrize("L,C", [(2, 64), (3, 128)])
 def test_fp32_tensor_core_channel_widths(L, C):
-    """Channel counts for which fp32 models run the radial GEMMs and the per-rank linears on tcgen05."""
+    """Channel counts whose per-rank linears tcgen05 can take, on systems so small that only the largest of them go there; systems
+    whose linears all do are in test_gpu_linears.py."""
     structs = synth.random_crystals(2, seed=9, nmin=6, nmax=12, zmax=2)
     model_out, ref = run_case(structs, L, C, [1, 2], 4.5, torch.float32)
 
