@@ -1082,12 +1082,12 @@ struct Model : ModelBase {
   // Whether FP16 parts pay for the tensor-core call (tc_fp16_pays): the largest elements are not looked for in vain.
   template <typename Spec>
   static bool long_loops(const std::vector<Spec>& specs) {
-    long long steps = 0, tiles = 0;
+    long long steps = 0, results = 0;
     for (const Spec& sp : specs) {
       steps += (long long)sp.q * sp.N * (sp.K / 32);
-      if (sp.accumulate != kJoin) tiles += (long long)sp.q * sp.N;
+      if (sp.accumulate != kJoin) results += (long long)sp.q * sp.N;
     }
-    return tc_fp16_pays(tiles, steps);
+    return tc_fp16_pays(results, steps);
   }
   // Which linears of the nodes take FP16 parts.  Those of models with the edge block do not: their energies move by 4e-5 with the rounding.  Nor do
   // those of the forward pass with few elements: the weights come out of L2 there, and the errors of the TF32 linears cancel in part in the

@@ -366,8 +366,8 @@ struct TcLinearProblem {
   int b_tiled;           // B, Bhi / Blo are stored K-tile-major, [groups][K/32][N][32] (b_group_stride must be N*K)
 };
 bool tc_linear_supported(int N, int K);
-// whether a launch that could takes FP16 parts: its tiles (in any unit) and their K steps of 32 in all
-bool tc_fp16_pays(long long tiles, long long steps);
+// whether a launch that could takes FP16 parts: its results per atom (or edge) and their K steps of 32 in all; no count of rows enters
+bool tc_fp16_pays(long long results, long long steps);
 cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* error_flag, cudaStream_t s);
 cudaError_t launch_tc_gemm(const float* A, long long lda, const float* Bhi, const float* Blo, float* C, long long ldc, int M,
                            int N, int K, int* error_flag, cudaStream_t s, const float* bias = nullptr);

@@ -671,9 +671,9 @@ cudaError_t launch_tc_fp16(const TcBatch& b, int dev, int sms, cudaStream_t s) {
 static uint32_t g_test_spin_limit = 0, g_test_extra_tx = 0;
 void tc_gemm_set_test_mode(uint32_t spin_limit, uint32_t extra_tx) { g_test_spin_limit = spin_limit; g_test_extra_tx = extra_tx; }
 
-// FP16 from four K steps a tile on, on the average of the launch: 75 776 x 512 rows with K = 96 take 48.0 us as TF32 and 49.4 as FP16, 526 336 x
+// FP16 where the results of a launch take more than three K steps on average: 75 776 x 512 rows with K = 96 take 48.0 us as TF32 and 49.4 as FP16, 526 336 x
 // 128 with K = 128 100 and 89.
-bool tc_fp16_pays(long long tiles, long long steps) { return steps > 3 * tiles; }
+bool tc_fp16_pays(long long results, long long steps) { return steps > 3 * results; }
 bool tc_linear_supported(int N, int K) { return N % 64 == 0 && K % kBK == 0; }
 
 cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* error_flag, cudaStream_t s) {
@@ -705,14 +705,15 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
   }
   first[n_results] = n_problems;
   for (int i = 0; i < n_results; ++i) one = one && steps_of[i] <= kChunk;
-  long long all_tiles = 0, all_steps = 0;
+  // From the shapes alone: with a count of tiles, the last of them rounded up, one row more could change the kernel, and a replayed pass, whose
+  // rows are those of its capacity, could take another one than the direct pass.
+  long long results = 0, all_steps = 0;
   for (int i = 0; i < n_results; ++i) {
-    const TcLinearProblem& h = probs[first[i]];
-    const long long t = (h.n_atoms * h.q + kBM - 1) / kBM * (h.N / 64);
-    all_tiles += t;
-    all_steps += t * steps_of[i];
+    const long long per_atom = (long long)probs[first[i]].q * probs[first[i]].N;
+    results += per_atom;
+    all_steps += per_atom * steps_of[i];
   }
-  fp16 = fp16 && tc_fp16_pays(all_tiles, all_steps);
+  fp16 = fp16 && tc_fp16_pays(results, all_steps);
   const int bn = all128 ? 128 : 64;
   TcBatch b;
   memset(&b, 0, sizeof(b));

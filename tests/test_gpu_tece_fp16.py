@@ -43,3 +43,44 @@ def test_powers_of_two_leave_no_trace(power):
     assert torch.isfinite(before["forces"]).all()
     for k, v in before.items():
         assert torch.equal(after[k], v), k
+
+
+def _rank_one(n_edges):
+    """Edge block of rank 1 and order 1 at 64 channels: its key and query linears take exactly three K steps per result on average (K = 128 for
+    order 0, two rows of K = 64 for order 1), the line between the two kernels."""
+    model, _, _ = make_models(1, 64, [13, 29], 5.0, 40.0, torch.float32, radial={"apply_cutoff": False}, tece={"num_head": 4, "edge_ace_hidden": 64, "mmax": 1})
+    data = to_device(oracle_batch([synth.fcc_supercell(3, 3.65, 0.05, seed=2, species=(13, 29), fractions=(0.5, 0.5))], [13, 29], 5.0, torch.float32), DEV)
+    assert data["edge_index"].shape[1] > n_edges
+    keep = torch.randperm(data["edge_index"].shape[1], generator=torch.Generator().manual_seed(0))[:n_edges].to(DEV)
+    return model, dict(data, edge_index=data["edge_index"][:, keep].contiguous(), edge_shifts=data["edge_shifts"][keep].contiguous())
+
+
+@pytest.mark.parametrize("n_edges", [1985, 2049])
+def test_replays_take_the_kernels_of_the_direct_pass_on_the_line(n_edges):
+    """2 049 edges fill 17 tiles of 128 and their pairs 33, the 2 176 of the capacity 17 and 34: a count of tiles puts the two on
+    different sides of the line."""
+    model, data = _rank_one(n_edges)
+    direct = {k: v.clone() for k, v in model(data).items() if v is not None}
+    assert model.graph_replays() == 0
+    for n in range(3):
+        out = model(data)
+        for k, v in direct.items():
+            assert torch.equal(out[k], v), (n, k)
+    assert model.graph_replays() >= 2
+
+
+def _launched(model, data, kernel):
+    """Launches of kernels whose name holds `kernel` in one evaluation, kernel by kernel."""
+    model.set_graph_mode(False)
+    model(data)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        model(data)
+        torch.cuda.synchronize()
+    assert any("tc_gemm" in e.name for e in prof.events())
+    return sum(kernel in e.name for e in prof.events())
+
+
+def test_the_number_of_edges_does_not_choose_the_kernel():
+    """The same shapes run the same kernels whatever the last tile holds (128 edges and none, one, half of them, ...)."""
+    seen = {n: _launched(*_rank_one(n), "tc_gemm_fp16_kernel") for n in (2048, 2049, 2112, 2113, 2175)}
+    assert len(set(seen.values())) == 1, seen
