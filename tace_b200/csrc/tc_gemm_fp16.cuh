@@ -76,11 +76,6 @@ __device__ __forceinline__ uint32_t split_fp16(float& x0, float& x1, float scale
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// Arrival that orders no memory: the epilogue's, after loads whose values it holds.  An ordinary arrival waits until the warp's stores to
-// the result rows have been acknowledged, some 1 000 cycles.
-__device__ __forceinline__ void mbar_arrive_relaxed(uint32_t bar) {
-  asm volatile("mbarrier.arrive.relaxed.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 // Two neighbouring 8-column blocks of one row, as tmem_ld_rows left them: lanes exchange pairs so that each holds four consecutive columns, and
 // four lanes write 64 consecutive bytes of the row, eight rows per store.  (Through shared memory, in rows of 128 bytes, a tile took 3 700
 // cycles; stored straight from a row per lane every store touched 32 rows.)
@@ -425,10 +420,16 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive_relaxed(acc_empty(a));  // the issuer may overwrite this accumulator
+        if (lane == 0) mbar_arrive(acc_empty(a));  // the issuer may overwrite this accumulator
       }
       if (!ok) break;
-      float* const* rows = row_addr + slot * kBM + r0;
+      // What the stores need of the slot goes to registers first: the arrival that hands the slot back then comes after every load from
+      // it, and before this tile's stores (an arrival after them waits until they have been acknowledged, some 1 000 cycles).
+      float* rows[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) rows[k] = row_addr[slot * kBM + r0 + 8 * k];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(info_empty(slot));
 #pragma unroll
       for (int c = 0; c < HN / 32; ++c) {
 #pragma unroll
@@ -443,7 +444,7 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
             for (int k = 0; k < 2; ++k) {
               const float4 v = gather_columns(&sum[h][c][8 * pair + 2 * k], odd);
               o[k] = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
-              dst[k] = rows[16 * h + 8 * k];
+              dst[k] = rows[2 * h + k];
             }
             if (accumulate) {  // both loads before the first store
               float4 p[2];
@@ -458,8 +459,6 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
           }
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive_relaxed(info_empty(slot));
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -39,3 +39,14 @@ def test_no_cached_function_hands_out_device_tensors():
         module = importlib.import_module(info.name)
         cached |= {f"{f.__module__}.{f.__name__}" for f in vars(module).values() if hasattr(f, "cache_info")}
     assert cached == {"tace_b200.graph._element_table", "tace_b200.graph._layout", "tace_b200.neighbour_list._workspace_bytes"}
+
+
+def test_arrivals_of_the_tensor_core_gemms_order_memory():
+    """What a role has read of a ring slot, a tile's description or an accumulator is overwritten by another role after the arrival that hands it
+    back, so every such arrival has to order the reads before it; and nothing of the slot is read after it."""
+    for name in ("tc_gemm.cu", "tc_gemm_fp16.cuh"):
+        src = open(os.path.join(ROOT, "tace_b200", "csrc", name)).read()
+        assert not re.search(r"mbarrier\.arrive[\w.]*\.relaxed", src), name
+    epilogue = src[src.index("// -- epilogue"):src.index("tcgen05.dealloc")]
+    after = epilogue[epilogue.index("mbar_arrive(info_empty(slot))"):]
+    assert not re.search(r"\b(row_addr|row_top|info)\[", after)
