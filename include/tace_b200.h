@@ -248,9 +248,21 @@ int tace_profile_read(TaceModel* model, int index, const char** name, float* ms)
  * non-zero code if a bounded wait inside the kernel expired (results are then undefined). */
 int tace_tc_gemm_f32(const float* A, int64_t lda, const float* B_hi, const float* B_lo, float* C, int64_t ldc, int32_t M,
                      int32_t N, int32_t K, int32_t* error_flag, tace_stream_t stream);
-/* Test mode of that kernel's bounded waits: every wait gives up after `spin_limit` polls (0: the normal 2^22), and every
+/* The same product on FP16 parts of operands scaled by powers of two, which tace_forward takes for the linears of the edge block and, of the
+ * larger fp32 models, of the nodes: C = bias + sum over the operands i of A_i[n_atoms][q][K_i] @ B_i[N][K_i]^T (C[n_atoms][q][N], added to what
+ * it holds with `accumulate`).  A_top holds the bits of the largest |element| of every atom's q rows; joined operands have the same.  B_packed
+ * (N * K + N floats per group) receives the parts of B_hi + B_lo.  n_groups > 0: atoms [group_ptr[g], group_ptr[g + 1]) take the matrix g,
+ * whose parts are K-tile-major [K / 32][N][32], and bias[g][N]; tile_ptr counts the groups' tiles of 128 / q atoms (device arrays of
+ * n_groups + 1).  Rows and pointers as above; `error_flag` also receives 6, a wait for the description of a tile. */
+typedef struct {
+  const float* A; const uint32_t* A_top; const float* B_hi; const float* B_lo; float* B_packed; int32_t K;
+} TaceTcOperands;
+int tace_tc_gemm_fp16_f32(const TaceTcOperands* operands, int32_t n_operands, int32_t n_atoms, int32_t q, int32_t N, int32_t n_groups,
+                          const int32_t* group_ptr, const int32_t* tile_ptr, float* C, const float* bias, int32_t accumulate,
+                          int32_t* error_flag, tace_stream_t stream);
+/* Test mode of the bounded waits of both kernels: every wait gives up after `spin_limit` polls (0: the normal 2^22), and every
  * load barrier expects `extra_expected_bytes` more than its loads deliver (0: normal), so that with a non-zero value it
- * never completes.  With both set, the next tace_tc_gemm_f32 records the code of the wait that ran out in `error_flag`
+ * never completes.  With both set, the next of these two calls records the code of the wait that ran out in `error_flag`
  * (1 ring slot free, 2 operands ready, 3 load landed, 4 accumulator free, 5 accumulator full), waits for the loads it has
  * issued, frees its tensor memory and returns without a result; no fault is involved.  Process-wide; reset with (0, 0). */
 int tace_tc_gemm_set_test_mode(uint32_t spin_limit, uint32_t extra_expected_bytes);

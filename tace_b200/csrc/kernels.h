@@ -368,7 +368,8 @@ struct TcLinearProblem {
 bool tc_linear_supported(int N, int K);
 // whether a launch that could takes FP16 parts: its results per atom (or edge) and their K steps of 32 in all; no count of rows enters
 bool tc_fp16_pays(long long results, long long steps);
-cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* error_flag, cudaStream_t s);
+// any_length: FP16 parts wherever the problems bring what they need, whether they pay or not
+cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* error_flag, cudaStream_t s, bool any_length = false);
 cudaError_t launch_tc_gemm(const float* A, long long lda, const float* Bhi, const float* Blo, float* C, long long ldc, int M,
                            int N, int K, int* error_flag, cudaStream_t s, const float* bias = nullptr);
 // packed [n] and scale [2] (its second entry is what b_inv points to) of the weights hi + lo, n a multiple of 32

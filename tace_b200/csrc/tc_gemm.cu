@@ -676,7 +676,7 @@ void tc_gemm_set_test_mode(uint32_t spin_limit, uint32_t extra_tx) { g_test_spin
 bool tc_fp16_pays(long long results, long long steps) { return steps > 3 * results; }
 bool tc_linear_supported(int N, int K) { return N % 64 == 0 && K % kBK == 0; }
 
-cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* error_flag, cudaStream_t s) {
+cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* error_flag, cudaStream_t s, bool any_length) {
   if (n_problems <= 0) return cudaSuccess;
   if (n_problems > kTcMaxProblems || !error_flag) return cudaErrorInvalidValue;
   static int sms_of[kMaxDevices] = {};
@@ -713,7 +713,7 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
     results += per_atom;
     all_steps += per_atom * steps_of[i];
   }
-  fp16 = fp16 && tc_fp16_pays(results, all_steps);
+  fp16 = fp16 && (any_length || tc_fp16_pays(results, all_steps));
   const int bn = all128 ? 128 : 64;
   TcBatch b;
   memset(&b, 0, sizeof(b));
@@ -811,4 +811,32 @@ extern "C" int tace_tc_gemm_f32(const float* A, int64_t lda, const float* B_hi, 
 extern "C" int tace_tc_gemm_set_test_mode(uint32_t spin_limit, uint32_t extra_expected_bytes) {
   tace::tc_gemm_set_test_mode(spin_limit, extra_expected_bytes);
   return TACE_OK;
+}
+
+extern "C" int tace_tc_gemm_fp16_f32(const TaceTcOperands* operands, int32_t n_operands, int32_t n_atoms, int32_t q, int32_t N, int32_t n_groups,
+                                     const int32_t* group_ptr, const int32_t* tile_ptr, float* C, const float* bias, int32_t accumulate,
+                                     int32_t* error_flag, tace_stream_t stream) {
+  constexpr int kMost = 4;
+  if (!operands || n_operands < 1 || n_operands > kMost || n_atoms < 0 || q < 1 || q > 128 || N < 64 || n_groups < 0 || !C || !error_flag ||
+      (n_groups > 0 && (!group_ptr || !tile_ptr)))
+    return TACE_ERR_INVALID_ARGUMENT;
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  tace::TcLinearProblem probs[kMost];
+  memset(probs, 0, sizeof(probs));
+  for (int i = 0; i < n_operands; ++i) {
+    const TaceTcOperands& o = operands[i];
+    if (!o.A || !o.A_top || !o.B_hi || !o.B_lo || !o.B_packed || o.K < 32 || !tace::tc_linear_supported(N, o.K)) return TACE_ERR_INVALID_ARGUMENT;
+    const long long n = (long long)(n_groups > 0 ? n_groups : 1) * N * o.K;
+    const cudaError_t e = tace::launch_tc_pack(o.B_hi, o.B_lo, n, o.B_packed, o.B_packed + n, s);
+    if (e != cudaSuccess) return TACE_ERR_CUDA;
+    tace::TcLinearProblem& h = probs[i];
+    h.A = o.A; h.a_atom_stride = (long long)q * o.K; h.a_comp_stride = o.K; h.q = q; h.n_atoms = n_atoms; h.K = o.K; h.N = N;
+    h.Bhi = o.B_hi; h.Blo = o.B_lo; h.B = o.B_packed; h.b_inv = o.B_packed + n + 1; h.a_top = o.A_top;
+    h.C = C; h.c_s1 = (long long)q * N; h.c_s2 = N; h.bias = bias;
+    h.n_groups = n_groups; h.group_ptr = group_ptr; h.tile_ptr = tile_ptr; h.b_group_stride = (long long)N * o.K; h.bias_group_stride = N;
+    h.b_tiled = n_groups > 0; h.accumulate = accumulate != 0; h.join = i > 0;
+  }
+  const cudaError_t e = tace::launch_tc_linear(probs, n_operands, error_flag, s, true);
+  if (e == cudaErrorInvalidValue) return TACE_ERR_INVALID_ARGUMENT;
+  return e == cudaSuccess ? TACE_OK : TACE_ERR_CUDA;
 }

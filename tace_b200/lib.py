@@ -19,11 +19,15 @@ TACE_F32, TACE_F64 = 0, 1
 EXPORTS = [
     "tace_status_string", "tace_create", "tace_destroy", "tace_weight_count", "tace_weight_info", "tace_set_weight",
     "tace_workspace_bytes", "tace_forward", "tace_debug_read", "tace_nl_count", "tace_nl_fill", "tace_nl_workspace_bytes",
-    "tace_launch_count", "tace_profile_enable", "tace_profile_count", "tace_profile_read", "tace_tc_gemm_f32", "tace_tc_gemm_set_test_mode",
+    "tace_launch_count", "tace_profile_enable", "tace_profile_count", "tace_profile_read", "tace_tc_gemm_f32", "tace_tc_gemm_fp16_f32", "tace_tc_gemm_set_test_mode",
     "tace_device_error", "tace_set_exchange", "tace_nl_build_noalloc", "tace_md_kick_drift", "tace_md_kinetic_energy",
     "tace_edge_vectors", "tace_edges_within", "tace_edges_scan_workspace_bytes", "tace_edges_scan", "tace_edges_compact", "tace_rows_gather", "tace_rows_scatter_add", "tace_rows_segment_add", "tace_set_graph_mode", "tace_graph_replays", "tace_set_exchange_sync", "tace_set_exchange_stream",
     "tace_set_chunk_edges", "tace_md_langevin", "tace_nl_rows", "tace_nl_fill_rows", "tace_one_hot",
 ]
+
+
+class TaceTcOperands(ctypes.Structure):
+    _fields_ = [(name, ctypes.c_void_p) for name in ("A", "A_top", "B_hi", "B_lo", "B_packed")] + [("K", ctypes.c_int32)]
 
 
 class TaceConfig(ctypes.Structure):
@@ -94,6 +98,8 @@ def load() -> ctypes.CDLL:
     lib.tace_profile_read.argtypes = [c_void_p, c_int, POINTER(c_char_p), POINTER(ctypes.c_float)]
     lib.tace_tc_gemm_f32.argtypes = [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_int32, c_int32,
                                      c_void_p, c_void_p]
+    lib.tace_tc_gemm_fp16_f32.argtypes = [POINTER(TaceTcOperands), c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p,
+                                          c_int32, c_void_p, c_void_p]
     lib.tace_device_error.argtypes = [c_void_p, POINTER(c_int32)]
     lib.tace_nl_build_noalloc.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int64, c_double, c_int64, c_void_p,
                                           c_void_p, c_void_p, c_void_p]
