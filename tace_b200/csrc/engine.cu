@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <string>
 #include <type_traits>
 #include <unordered_map>
@@ -472,23 +473,34 @@ struct Model : ModelBase {
     add_weight(name, numel);
     if (kTensorCore) { add_weight(name + "_hi", numel); add_weight(name + "_lo", numel); }
   }
-  // What the tensor cores read of them: "X_pk", FP16 parts of X_hi + X_lo times a power of two, and that scale behind them.
+  // The same for a [K][N] matrix per group, X, and its transpose, which linears on FP16 parts may read (each that of the other direction)
+  void add_packed_weight(const std::string& name, const std::string& nameT, int groups, long long K, long long N, bool tiled) {
+    add_linear_weight(name, groups * K * N);
+    add_linear_weight(nameT, groups * K * N);
+    if (kTensorCore && tc_linear_supported((int)K, (int)N)) pack_shapes[name] = {groups, (int)K, (int)N, tiled};
+    if (kTensorCore && tc_linear_supported((int)N, (int)K)) pack_shapes[nameT] = {groups, (int)N, (int)K, tiled};
+  }
+  // What the tensor cores read of them: "X_pk", FP16 parts of X_hi + X_lo with every column of the result scaled by a power of two, and behind
+  // them the inverse scales.
   struct Packed { const float* B; const float* inv; };
+  struct PackShape { int groups, N, K; bool tiled; };
+  std::map<std::string, PackShape> pack_shapes;  // by the name of the array, X
   Packed packed(const std::string& name) const {
     const auto it = weight_index.find(name + "_pk");
     if (it == weight_index.end()) return {nullptr, nullptr};
     const WeightEntry& e = weights[it->second];
     const float* B = reinterpret_cast<const float*>(arena + e.offset);
-    return {B, B + e.numel - kPackTail + 1};
+    const PackShape& sh = pack_shapes.at(name);
+    return {B, B + (long long)sh.groups * sh.N * sh.K};
   }
-  static constexpr int kPackTail = 64;
   cudaError_t pack_weight(const std::string& name) {
     const auto it = weight_index.find(name + "_pk");
     if (it == weight_index.end()) return cudaSuccess;
     const WeightEntry& e = weights[it->second];
     float* B = reinterpret_cast<float*>(arena + e.offset);
-    return launch_tc_pack(reinterpret_cast<const float*>(w(name + "_hi")), reinterpret_cast<const float*>(w(name + "_lo")), e.numel - kPackTail, B,
-                          B + e.numel - kPackTail, cudaStream_t(0));
+    const PackShape& sh = pack_shapes.at(name);
+    return launch_tc_pack(reinterpret_cast<const float*>(w(name + "_hi")), reinterpret_cast<const float*>(w(name + "_lo")), sh.groups, sh.N, sh.K, sh.tiled,
+                          B, B + (long long)sh.groups * sh.N * sh.K, cudaStream_t(0));
   }
   const T* w(const std::string& name) const {
     const auto it = weight_index.find(name);
@@ -588,9 +600,8 @@ struct Model : ModelBase {
         for (int i = 0; i < 6; ++i) {
           const So2Shape sh = so2_shape(i);
           for (int m = 0; m <= sh.mm; ++m) {
-            const long long numel = (long long)sh.n_in[m] * sh.c_in * sh.n_out[m] * sh.c_out;
-            add_linear_weight(pre + "so2." + sh.name + ".m" + std::to_string(m), numel);
-            add_linear_weight(pre + "so2." + sh.name + "T.m" + std::to_string(m), numel);
+            add_packed_weight(pre + "so2." + sh.name + ".m" + std::to_string(m), pre + "so2." + sh.name + "T.m" + std::to_string(m), 1,
+                              (long long)sh.n_in[m] * sh.c_in, (long long)sh.n_out[m] * sh.c_out, false);
           }
           add_weight(pre + "so2." + sh.name + ".b", (long long)sh.n_out[0] * sh.c_out);
         }
@@ -618,8 +629,7 @@ struct Model : ModelBase {
       }
       for (int l = 0; l <= L; ++l) {
         const long long outl = (l == 0) ? (long long)(L + 1 + m0) * C : C;
-        add_linear_weight(pre + "down.l" + std::to_string(l), (long long)p.tp.k[l] * C * outl);
-        add_linear_weight(pre + "downT.l" + std::to_string(l), (long long)p.tp.k[l] * C * outl);
+        add_packed_weight(pre + "down.l" + std::to_string(l), pre + "downT.l" + std::to_string(l), 1, (long long)p.tp.k[l] * C, outl, false);
         add_linear_weight(pre + "nl.l" + std::to_string(l), (long long)C * C);
         add_linear_weight(pre + "nlT.l" + std::to_string(l), (long long)C * C);
       }
@@ -628,12 +638,8 @@ struct Model : ModelBase {
       for (size_t i = 0; i < p.out_ls.size(); ++i) {
         const int l = p.out_ls[i];
         const std::string ls = std::to_string(l);
-        add_linear_weight(pre + "c0.l" + ls, (long long)n_el * C * C);
-        add_linear_weight(pre + "c0T.l" + ls, (long long)n_el * C * C);
-        if (cfg.correlation >= 2) {
-          add_linear_weight(pre + "c1.l" + ls, (long long)n_el * p.pb.k[i] * C * C);
-          add_linear_weight(pre + "c1T.l" + ls, (long long)n_el * p.pb.k[i] * C * C);
-        }
+        add_packed_weight(pre + "c0.l" + ls, pre + "c0T.l" + ls, n_el, C, C, true);
+        if (cfg.correlation >= 2) add_packed_weight(pre + "c1.l" + ls, pre + "c1T.l" + ls, n_el, (long long)p.pb.k[i] * C, C, true);
         if (cfg.correlation >= 3) {
           add_linear_weight(pre + "c2.l" + ls, (long long)n_el * p.pb3.k[i] * C * C);
           add_linear_weight(pre + "c2T.l" + ls, (long long)n_el * p.pb3.k[i] * C * C);
@@ -641,8 +647,7 @@ struct Model : ModelBase {
         add_linear_weight(pre + "lin.l" + ls, (long long)C * C);
         add_linear_weight(pre + "linT.l" + ls, (long long)C * C);
         if (p.has_res && !res_identity) {
-          add_linear_weight(pre + "res.l" + ls, (long long)n_el * C * C);
-          add_linear_weight(pre + "resT.l" + ls, (long long)n_el * C * C);
+          add_packed_weight(pre + "res.l" + ls, pre + "resT.l" + ls, n_el, C, C, true);
         }
       }
       if (bilinear) {  // linear_up of the product: every rank to both factors, the scalars also to the gates
@@ -667,11 +672,7 @@ struct Model : ModelBase {
     add_weight("e0", (long long)n_fid * n_el);
     if (zbl) { add_weight("zbl.z", n_el); add_weight("zbl.rcov", n_el); add_weight("zbl.par", 2); }
     n_listed = n_unset = (int)weights.size();
-    for (int i = 0; i < n_listed && kTensorCore; ++i) {
-      const std::string nm = weights[i].name;
-      if (nm.size() > 3 && nm.compare(nm.size() - 3, 3, "_hi") == 0 && weights[i].numel % 32 == 0)
-        add_weight(nm.substr(0, nm.size() - 3) + "_pk", weights[i].numel + kPackTail);
-    }
+    for (const auto& e : pack_shapes) add_weight(e.first + "_pk", (long long)e.second.groups * e.second.N * (e.second.K + 1));
     folded = tece_mask == 0;
     if (folded) add_weight("emb_up", (long long)n_el * C);
     for (int t = 0; t < NL_ && folded; ++t)
@@ -821,8 +822,9 @@ struct Model : ModelBase {
     T *h_in, *x, *xx, *gxx, *W, *H3, *Z1, *Z2, *Z3, *Hact, *M, *Gt, *gGt, *a, *B2, *out, *h_out;
     T *gh_out, *ga, *gx, *gh_in;
     T *As, *gAs, *gout_s, *hs;  // species-sorted copies used by the per-species linears
-    unsigned *top, *gtop;       // largest elements of their rows, forward and backward; nullptr: not taken
-    unsigned *mtop, *dtop;      // of the rows that linear_down reads, forward (M) and backward (gGt)
+    // largest elements per rank; nullptr: not taken
+    unsigned *top, *gtop;       // of those rows, forward [NL][3][L + 1] (As, B2, hs) and backward [NL][L + 1] (gout_s)
+    unsigned *mtop, *dtop;      // of the rows that linear_down reads, forward (M) and backward (gGt), [NL][L + 1]
     T *B3, *gB2;                // third-order basis (reused for its gradient) and the gradient of the second-order one
     T *inv_density, *gdens;     // learned edge density: 1 / density_i and dE / d density_i
     T *XY, *gXY, *Zg, *gZg;     // gated bilinear product: both factors per (atom, component), gate pre-activations, gradients
@@ -928,11 +930,11 @@ struct Model : ModelBase {
       lb.gAs = ar.take<T>((size_t)NL * D * C);
       lb.gout_s = ar.take<T>((size_t)NL * p.Dout * C);
       const bool tops = kTensorCore && folded && !bilinear && cfg.correlation == 2 && pb_tops(C);
-      lb.top = tops ? ar.take<unsigned>((size_t)NL) : nullptr;
-      lb.gtop = tops ? ar.take<unsigned>((size_t)NL) : nullptr;
+      lb.top = tops ? ar.take<unsigned>((size_t)NL * 3 * (L + 1)) : nullptr;
+      lb.gtop = tops ? ar.take<unsigned>((size_t)NL * (L + 1)) : nullptr;
       const bool down_tops = kTensorCore && folded && rt_K && !density && pb_tops(C);
-      lb.mtop = down_tops && tp_wide_channels(C) ? ar.take<unsigned>((size_t)NL) : nullptr;
-      lb.dtop = down_tops ? ar.take<unsigned>((size_t)NL) : nullptr;
+      lb.mtop = down_tops && tp_wide_channels(C) ? ar.take<unsigned>((size_t)NL * (L + 1)) : nullptr;
+      lb.dtop = down_tops ? ar.take<unsigned>((size_t)NL * (L + 1)) : nullptr;
       lb.hs = p.has_res ? ar.take<T>((size_t)NL * p.Din * C) : nullptr;
       lb.out = folded ? nullptr : ar.take<T>((size_t)NL * p.Dout * C);
       lb.h_out = ar.take<T>((size_t)N * p.Dout * C);
@@ -978,7 +980,7 @@ struct Model : ModelBase {
     int accumulate = 0;          // Cm += instead of Cm =
     T* act_out = nullptr;        // fused activations of GemmProblem (double precision)
     const T* act_in = nullptr;
-    const unsigned* a_top = nullptr;  // TcLinearProblem::a_top
+    const unsigned* a_top = nullptr; int a_top_stride = 0;  // those of TcLinearProblem
   };
   // the layers of the radial MLP of fp64 models apply their activations themselves (a LayerNorm in between needs whole rows)
   bool fused_activations() const { return !kTensorCore && !element2; }
@@ -1062,7 +1064,7 @@ struct Model : ModelBase {
                        h.atom_map = c_map;
                        if (!sp.a_top) return;
                        const Packed pk = packed(sp.wname_t);
-                       h.a_top = sp.a_top; h.B = pk.B; h.b_inv = pk.inv;
+                       h.a_top = sp.a_top; h.a_top_stride = sp.a_top_stride; h.B = pk.B; h.b_inv = pk.inv;
                      },
                      [&](GemmBatch<T>& g, const LinSpec& sp, int accumulate, int join) {
                        add_problem(g, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, accumulate, join);
@@ -1077,7 +1079,8 @@ struct Model : ModelBase {
     const T* A; long long a_s1, a_s2; int q, K;
     std::string wname, wname_t; int N;
     T* Cm; long long c_s1, c_s2; const T* bias; bool mapped; int accumulate;
-    const unsigned* a_top = nullptr;  // TcLinearProblem::a_top, in species-sorted order
+    int rank = 0, operand = 0;  // of A: l, and 0..2 for As, B2, hs (species_tops)
+    const unsigned* a_top = nullptr; int a_top_stride = 0;  // those of TcLinearProblem, in species-sorted order
   };
   // Whether FP16 parts pay for the tensor-core call (tc_fp16_pays): the largest elements are not looked for in vain.
   template <typename Spec>
@@ -1115,7 +1118,7 @@ struct Model : ModelBase {
   // us, energies of 33 729 -> 722; backward only, 32 400 water atoms, both together 45 190 -> 44 800.
   unsigned* down_tops(std::vector<LinSpec>& sp, unsigned* top, long long n_atoms, bool backward) const {
     if (!top || !fp16_nodes(backward) || small_call(sp, n_atoms, 1) || !long_loops(sp)) return nullptr;
-    for (auto& q : sp) q.a_top = top;
+    for (int l = 0; l <= L; ++l) { sp[l].a_top = top + l; sp[l].a_top_stride = L + 1; }
     return top;
   }
   // Largest elements of the atoms' rows for the per-species linears (`top`, or nullptr where they are not wanted): those read their weights
@@ -1124,14 +1127,18 @@ struct Model : ModelBase {
   // 2 426.
   unsigned* species_tops(std::vector<SpeciesSpec>& sp, unsigned* top, long long n_atoms, bool backward) const {
     if (!top || !fp16_nodes(backward) || small_call(sp, n_atoms, n_el) || !long_loops(sp)) return nullptr;
-    for (auto& q : sp) q.a_top = top;
+    set_tops(sp, top, backward ? 1 : 3);
     return top;
   }
-  static cudaError_t gather_rows(const T* src, const int* perm, T* dst, long long n, int row_len, unsigned* top, bool more, cudaStream_t s) {
+  void set_tops(std::vector<SpeciesSpec>& sp, const unsigned* top, int operands) const {
+    for (auto& q : sp) { q.a_top = top ? top + q.operand * (L + 1) + q.rank : nullptr; q.a_top_stride = operands * (L + 1); }
+  }
+  // Rows of D ranks
+  cudaError_t gather_rows(const T* src, const int* perm, T* dst, long long n, int rows, unsigned* top, int top_stride, cudaStream_t s) const {
     if constexpr (kTensorCore) {
-      if (top) return launch_gather_rows_top(src, perm, dst, n, row_len, top, more, s);
+      if (top) return launch_gather_rows_top(src, perm, dst, n, rows == 1 ? 0 : Ln, C, top, top_stride, s);
     }
-    return launch_gather_rows(src, perm, dst, n, row_len, s);
+    return launch_gather_rows(src, perm, dst, n, rows * C, s);
   }
   cudaError_t run_species_linear(const std::vector<SpeciesSpec>& specs, const Bufs& b, long long n_atoms, cudaStream_t s) {
     if (specs.empty()) return cudaSuccess;
@@ -1149,7 +1156,7 @@ struct Model : ModelBase {
                        h.b_tiled = 1;  // the packed per-species hi / lo parts are K-tile-major (read once per pass, straight from DRAM)
                        if (!sp.a_top) return;
                        const Packed pk = packed(sp.wname_t);
-                       h.a_top = sp.a_top; h.B = pk.B; h.b_inv = pk.inv;
+                       h.a_top = sp.a_top; h.a_top_stride = sp.a_top_stride; h.B = pk.B; h.b_inv = pk.inv;
                      },
                      [&](GemmBatch<T>& g, const SpeciesSpec& sp, int accumulate, int join) {
                        add_problem(g, sp.A, sp.a_s1, sp.a_s2, sp.q, sp.K, w(sp.wname), sp.N, sp.Cm, sp.c_s1, sp.c_s2, sp.bias, accumulate, join,
@@ -1211,9 +1218,10 @@ struct Model : ModelBase {
   // GEMM problems of SO(2) linears over the E edges: `in` [E][in_rows][c_in] -> `out` [E][out_rows][c_out] (forward), or the
   // gradient of the output back to the gradient of the input (backward; `out` is then the input gradient, and linears of the
   // call with the same input gradient add up)
-  struct So2Run { int which; const T* in; int in_rows; T* out; int out_rows; };
-  // top: largest elements per edge of what the linears of the call read
-  void so2_specs(std::vector<LinSpec>& sp, const std::string& pre, const std::vector<So2Run>& runs, bool backward, const unsigned* top) const {
+  struct So2Run { int which; const T* in; int in_rows; T* out; int out_rows; int top = 0; };  // top: first of its largest elements of an edge
+  // Where the largest elements of what the linears of the call read are, per edge and order
+  struct Tops { const unsigned* first; int stride; };
+  void so2_specs(std::vector<LinSpec>& sp, const std::string& pre, const std::vector<So2Run>& runs, bool backward, Tops tops) const {
     std::vector<int> off_in(runs.size(), 0), off_out(runs.size(), 0);
     for (int m = 0; m <= mmax; ++m) {
       for (size_t i = 0; i < runs.size(); ++i) {
@@ -1229,7 +1237,7 @@ struct Model : ModelBase {
           sp.push_back({r.in + (long long)off_out[i] * sh.c_out, (long long)r.out_rows * sh.c_out, Nn, m ? 2 : 1, Nn, nmT, nm, K,
                         r.out + (long long)off_in[i] * sh.c_in, (long long)r.in_rows * sh.c_in, K, nullptr,
                         i > 0 && r.out == runs[i - 1].out ? kJoin : 0});
-        sp.back().a_top = top;
+        if (tops.first) { sp.back().a_top = tops.first + r.top + m; sp.back().a_top_stride = tops.stride; }
         // the order-0 block of the input always spans L + 1 rows (oam_2026_07_05.py:211)
         off_in[i] += (m == 0) ? (L + 1) : 2 * sh.n_in[m];
         off_out[i] += (m == 0) ? sh.n_out[0] : 2 * sh.n_out[m];
@@ -1259,10 +1267,10 @@ struct Model : ModelBase {
   // forward of the block for one layer: lb.W holds the radial weights, the result lands in lb.M
   int tece_forward(const TeceArgs<T>& ta, const LayerBufs& lb, const std::string& pre, long long E, cudaStream_t s) {
     std::vector<LinSpec> sp;
-    auto top = [&](TeceTop k) { return lb.ttop ? lb.ttop + k * E : nullptr; };
+    auto top = [&](TeceTop k) { return Tops{lb.ttop ? lb.ttop + k * E : nullptr, tece_top_width(k)}; };
     if (lb.ttop && E > 0) CK(cudaMemsetAsync(lb.ttop, 0, sizeof(unsigned) * (size_t)(kTeceTops * E), s));
     CKL(launch_tece(ta, TECE_ROTATE_IN, s));
-    so2_specs(sp, pre, {{0, lb.tKs, t_NR, lb.tKp, t_NR}, {1, lb.tQt, t_NR, lb.tQp, t_NR}}, false, top(TECE_TOP_IN));
+    so2_specs(sp, pre, {{0, lb.tKs, t_NR, lb.tKp, t_NR}, {1, lb.tQt, t_NR, lb.tQp, t_NR, 3}}, false, top(TECE_TOP_IN));
     CKL(run_edge_linear(sp, E, s)); sp.clear();
     cudaStream_t side;  // the attention weights, beside the linears and the cluster expansion of the messages
     CKS(branch(s, &side));
@@ -1282,7 +1290,7 @@ struct Model : ModelBase {
   int tece_backward(TeceArgs<T> ta, const Bufs& b, const LayerBufs& lb, const std::string& pre, long long N, long long E, bool first_tece,
                     cudaStream_t s, cudaStream_t* after) {
     std::vector<LinSpec> sp;
-    auto top = [&](TeceTop k) { return lb.ttop ? lb.ttop + k * E : nullptr; };
+    auto top = [&](TeceTop k) { return Tops{lb.ttop ? lb.ttop + k * E : nullptr, tece_top_width(k)}; };
     cudaStream_t side;
     CKL(launch_tece(ta, TECE_ROTATE_OUT_BWD, s));
     // the attention weights down to the rotated rows, beside the way back through the messages (cluster expansion and linears)
@@ -1295,10 +1303,10 @@ struct Model : ModelBase {
     CKL(run_edge_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_MIX_BWD, s));                           // gup / gglu / gcoef over their forward buffers
     // gMw over Mw: the three linears that read Mw add up in one pass per order
-    so2_specs(sp, pre, {{2, lb.tup, t_NR, lb.tMw, t_G + t_NF}, {3, lb.tglu, t_NR, lb.tMw, t_NF}, {4, lb.tcoef, t_NR, lb.tMw, t_WN}}, true, top(TECE_TOP_GMIX));
+    so2_specs(sp, pre, {{2, lb.tup, t_NR, lb.tMw, t_G + t_NF}, {3, lb.tglu, t_NR, lb.tMw, t_NF, 3}, {4, lb.tcoef, t_NR, lb.tMw, t_WN, 6}}, true, top(TECE_TOP_GMIX));
     CKL(run_edge_linear(sp, E, s)); sp.clear();
     CKS(merge(s));
-    so2_specs(sp, pre, {{0, lb.tgKp, t_NR, lb.tgKs, t_NR}, {1, lb.tgQp, t_NR, lb.tgQt, t_NR}}, true, top(TECE_TOP_GPROJ));
+    so2_specs(sp, pre, {{0, lb.tgKp, t_NR, lb.tgKs, t_NR}, {1, lb.tgQp, t_NR, lb.tgQt, t_NR, 3}}, true, top(TECE_TOP_GPROJ));
     CKL(run_edge_linear(sp, E, s)); sp.clear();
     CKL(launch_tece(ta, TECE_ROTATE_IN_BWD, s));
     ta.accumulate_gvec = first_tece ? 0 : 1;
@@ -1616,7 +1624,7 @@ struct Model : ModelBase {
       }
       std::vector<LinSpec> down = down_specs(p, lb, pre, false);
       unsigned* mtop = p.tece ? nullptr : down_tops(down, lb.mtop, NL, false);
-      if (mtop) CK(cudaMemsetAsync(mtop, 0, sizeof(unsigned) * (size_t)NL, s));
+      if (mtop) CK(cudaMemsetAsync(mtop, 0, sizeof(unsigned) * (size_t)NL * (L + 1), s));
       for (int c = 0; c < n_chunks; ++c) {
         const long long e0 = chunk_edge[c], Ec = chunk_edge[c + 1] - e0;
         const int a0 = chunk_atom[c], na = chunk_atom[c + 1] - a0;
@@ -1640,7 +1648,7 @@ struct Model : ModelBase {
         ta.L = L; ta.scalar_src = p.scalar_src; ta.Lin = Ln; ta.C = C; ta.n_seg = na; ta.rowptr = b.rowptr_dst + a0;
         ta.e_src = b.e_src; ta.Y = b.Y; ta.W = lb.W; ta.x = x_src; ta.M = lb.M + (long long)a0 * p.tp.NM * C; ta.e_base = e0; ta.n_edges = round_edges(Ec);
         ta.split_sums = lb.xx == nullptr; ta.env = b.env;
-        if (mtop) ta.top = mtop + a0;
+        if (mtop) ta.top = mtop + (long long)a0 * (L + 1);
         if (rt_K) { ta.rtab = w(pre + "rtab"); ta.rt_K = rt_K; ta.rt_inv_h = T(rt_K) / T(cfg.cutoff); ta.dlen = b.dlen; }
         if (split) {  // targets that read owned rows only (final in x itself); the others once the ghost rows have arrived
           ta.x = lb.x; ta.row_ids = b.row_ids; ta.row_split = b.row_split + 1; ta.row_part = 0;
@@ -1694,11 +1702,11 @@ struct Model : ModelBase {
           T* out = (folded ? lb.h_out : lb.out) + (long long)l * l * C;
           sp.push_back({bilinear ? lb.XY + (long long)l * l * 2 * C : lb.As + (long long)l * l * C, (long long)D * C * (bilinear ? 2 : 1),
                         (long long)C * (bilinear ? 2 : 1), 2 * l + 1, C, pre + "c0" + f + ls, pre + "c0T.l" + ls, C, out,
-                        (long long)p.Dout * C, C, l == 0 ? w(pre + (folded ? "cf.b" : "c.b")) : nullptr, true, 0});
+                        (long long)p.Dout * C, C, l == 0 ? w(pre + (folded ? "cf.b" : "c.b")) : nullptr, true, 0, l});
           if (cfg.correlation >= 2) {
             const int K = p.pb.k[i] * C;
             sp.push_back({lb.B2 + (long long)p.pb.base[i] * C, (long long)p.pb.NB * C, K, 2 * l + 1, K, pre + "c1" + f + ls, pre + "c1T.l" + ls,
-                          C, out, (long long)p.Dout * C, C, nullptr, true, kJoin});
+                          C, out, (long long)p.Dout * C, C, nullptr, true, kJoin, l, 1});
           }
           if (cfg.correlation >= 3) {
             const int K = p.pb3.k[i] * C;
@@ -1707,12 +1715,12 @@ struct Model : ModelBase {
           }
           if (res)
             sp.push_back({lb.hs + (long long)l * l * C, (long long)p.Din * C, C, 2 * l + 1, C, pre + "res.l" + ls, pre + "resT.l" + ls, C, out,
-                          (long long)p.Dout * C, C, nullptr, true, kJoin});
+                          (long long)p.Dout * C, C, nullptr, true, kJoin, l, 2});
         }
         unsigned* top = species_tops(sp, lb.top, NL, false);
-        if (!bilinear && cfg.correlation >= 2) CKL(launch_pb_fwd(lb.As, lb.B2, (int)NL, L, p.pb_lout, C, s, top));
+        if (!bilinear && cfg.correlation >= 2) CKL(launch_pb_fwd(lb.As, lb.B2, (int)NL, L, p.pb_lout, C, s, top, 3 * (L + 1)));
         if (cfg.correlation >= 3) CKL(launch_pb3_fwd(lb.As, lb.B2, lb.B3, (int)NL, L, p.last ? -1 : Ln, C, s));
-        if (res) CKL(gather_rows(lb.h_in, b.species_perm, lb.hs, NL, p.Din * C, top, true, s));
+        if (res) CKL(gather_rows(lb.h_in, b.species_perm, lb.hs, NL, p.Din, top ? top + 2 * (L + 1) : nullptr, 3 * (L + 1), s));
         CKL(run_species_linear(sp, b, NL, s));
       }
       if (!folded) {
@@ -1799,7 +1807,7 @@ struct Model : ModelBase {
         for (int l : p.out_ls)
           sp.push_back({lb.gout_s + (long long)l * l * C, (long long)p.Dout * C, C, 2 * l + 1, C, pre + "c0T.l" + std::to_string(l),
                         pre + "c0.l" + std::to_string(l), C, bilinear ? lb.gXY + (long long)l * l * 2 * C : lb.gAs + (long long)l * l * C,
-                        (long long)D * C * (bilinear ? 2 : 1), (long long)C * (bilinear ? 2 : 1), nullptr, false, 0});
+                        (long long)D * C * (bilinear ? 2 : 1), (long long)C * (bilinear ? 2 : 1), nullptr, false, 0, l});
         if (cfg.correlation < 2) {
           if (folded) CKL(launch_gather_rows(lb.gh_out, b.species_perm, lb.gout_s, NL, p.Dout * C, s));
           CKL(run_species_linear(sp, b, NL, s));
@@ -1812,7 +1820,7 @@ struct Model : ModelBase {
               const int K = p.pb3.k[i] * C;
               sp.push_back({lb.gout_s + (long long)l * l * C, (long long)p.Dout * C, C, 2 * l + 1, C, pre + "c2T.l" + std::to_string(l),
                             pre + "c2.l" + std::to_string(l), K, lb.B3 + (long long)p.pb3.base[i] * C, (long long)p.pb3.NB * C, K,
-                            nullptr, false, 0});
+                            nullptr, false, 0, l});
             }
           }
           for (size_t i = 0; i < p.out_ls.size(); ++i) {
@@ -1820,10 +1828,10 @@ struct Model : ModelBase {
             const int K = p.pb.k[i] * C;
             sp.push_back({lb.gout_s + (long long)l * l * C, (long long)p.Dout * C, C, 2 * l + 1, C, pre + "c1T.l" + std::to_string(l),
                           pre + "c1.l" + std::to_string(l), K, g2 + (long long)p.pb.base[i] * C, (long long)p.pb.NB * C, K, nullptr,
-                          false, 0});
+                          false, 0, l});
           }
           gtop = species_tops(sp, lb.gtop, NL, true);
-          if (folded) CKL(gather_rows(lb.gh_out, b.species_perm, lb.gout_s, NL, p.Dout * C, gtop, false, s));
+          if (folded) CKL(gather_rows(lb.gh_out, b.species_perm, lb.gout_s, NL, p.Dout, gtop, L + 1, s));
           CKL(run_species_linear(sp, b, NL, s));  // B2 (gB2) and B3 now hold their gradients
           if (cfg.correlation >= 3) {
             CKL(launch_pb3_bwd(lb.As, lb.B2, lb.B3, lb.gB2, lb.gAs, (int)NL, L, p.last ? -1 : Ln, C, s));
@@ -1953,8 +1961,8 @@ struct Model : ModelBase {
           std::vector<SpeciesSpec> sp2;  // gout_s: the species-sorted gradient of this layer's output
           for (int l : p.out_ls)
             sp2.push_back({lb.gout_s + (long long)l * l * C, (long long)p.Dout * C, C, 2 * l + 1, C, pre + "resT.l" + std::to_string(l),
-                           pre + "res.l" + std::to_string(l), C, lb.gh_in + (long long)l * l * C, (long long)p.Din * C, C, nullptr, true, 1});
-          for (auto& q : sp2) q.a_top = gtop;
+                           pre + "res.l" + std::to_string(l), C, lb.gh_in + (long long)l * l * C, (long long)p.Din * C, C, nullptr, true, 1, l});
+          set_tops(sp2, gtop, 1);
           CKL(run_species_linear(sp2, b, NL, s));
         }
       }

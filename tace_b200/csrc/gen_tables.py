@@ -85,6 +85,12 @@ def tp_paths(L, in1_ls, in2_ls, out_ls):
     return paths
 
 
+def rank_of_row(lay, outs) -> str:
+    """C++ function: rank that row r of the layout belongs to."""
+    expr = " + ".join(f"(r >= {lay.base[l]})" for l in outs if l > 0)
+    return f"static TACE_HD constexpr int rank_of(int r) {{ return {expr}; }}" if expr else "static TACE_HD constexpr int rank_of(int) { return 0; }"
+
+
 class Layout:
     """Message layout [l3][m3][p_local]: index = base[l3] + m3 * k[l3] + p_local."""
 
@@ -175,6 +181,7 @@ def gen_interaction(L, Lin, out):
     o(f"static const int tp_{tag}_base[{L + 1}] = {{{', '.join(str(lay.base[l]) for l in outs)}}};")
     o(f"struct TPX_{tag} {{")
     o(f"  static constexpr int L = {L}, NP = {P}, NX = {nx}, NM = {lay.nm}, NG = {ng}, D = {D}, NGRP = {ngrp};")
+    o(f"  {rank_of_row(lay, outs)}")
     for name, arr in [("GOFF", grp_goff), ("GCNT", [((c + 3) // 4) * 4 for c in grp_gcnt]), ("P0", grp_p0), ("NPG", grp_np),
                       ("M0", grp_m0), ("NMG", grp_nm)]:
         o(f"  static constexpr int {name}0 = {arr[0]}, {name}1 = {arr[-1]};")
@@ -487,7 +494,7 @@ def gen_product(L, Lout, out):
     nnz = sum(int(np.count_nonzero(w3j(*p))) for p in paths)
     o(f"// ---- product basis (A x A), L={L}, {'scalar outputs' if last else f'output ranks <= {Lout}'}: {P} paths, "
       f"{lay.nm} components, {nnz} coupling non-zeros")
-    o(f"struct PB_{tag} {{ static constexpr int L = {L}, NP = {P}, NB = {lay.nm}, D = {D}; }};")
+    o(f"struct PB_{tag} {{ static constexpr int L = {L}, NP = {P}, NB = {lay.nm}, D = {D}; {rank_of_row(lay, outs)} }};")
     o(f"static const int pb_{tag}_k[{len(outs)}] = {{{', '.join(str(lay.k[l]) for l in outs)}}};")
     o(f"static const int pb_{tag}_base[{len(outs)}] = {{{', '.join(str(lay.base[l]) for l in outs)}}};")
     o("template <typename T>")

@@ -36,7 +36,7 @@ struct TPArgs {
   const T* W;         // [E][NP*C] per-edge path weights
   const T* x;         // [N][NX][C] source features
   T* M;               // forward output [n_seg][NM][C]
-  unsigned* top;      // wide kernels: [n_seg], raised to the bits of the largest |element| of a target's rows of M (zeroed before), or nullptr
+  unsigned* top;      // wide kernels: [n_seg][L + 1], raised to the bits of the largest |element| of a target's rows of M, rank by rank (zeroed before), or nullptr
   const T* gM;        // [n_seg][NM][C] gradient of the messages
   T* dW;              // backward output [E][NP*C] (may alias W)
   T* dY;              // backward output [E][D]
@@ -98,12 +98,12 @@ template <typename T> cudaError_t launch_pb3_bwd(const T* A, const T* B2, const 
                                                  cudaStream_t s);
 // m0: 1 = every rank (l = 0 included) scaled by a sigmoid gate; 0 = scalars through the normalised SiLU, ranks >= 1 gated
 template <typename T> cudaError_t launch_gate_fwd(const T* Gt, T* a, int n, int L, int C, int m0, cudaStream_t s);
-// top (fp32, pb_tops(C)): receives the bits of the largest |element| of every atom's row of gGt
+// top (fp32, pb_tops(C)): [n][L + 1], receives the bits of the largest |element| of every atom's row of gGt, rank by rank (0: gates and scalars)
 template <typename T> cudaError_t launch_gate_bwd(const T* Gt, const T* ga, T* gGt, int n, int L, int C, int m0, cudaStream_t s, unsigned* top = nullptr);
 // product basis A (x) A (tace/models/_e3nn/prod.py:242-256, fused.py:90-95)
 // L: rank of A; Lout: highest output rank, or < 0 for scalar outputs only (the last layer)
-// top (fp32, pb_tops(C)): receives the bits of the largest |element| of every atom's rows of A and B2
-template <typename T> cudaError_t launch_pb_fwd(const T* A, T* B2, int n, int L, int Lout, int C, cudaStream_t s, unsigned* top = nullptr);
+// top (fp32, pb_tops(C)): rows of top_stride, receives the bits of the largest |element| of every atom's rows of A, rank by rank, and of B2, those from L + 1 on
+template <typename T> cudaError_t launch_pb_fwd(const T* A, T* B2, int n, int L, int Lout, int C, cudaStream_t s, unsigned* top = nullptr, int top_stride = 0);
 inline bool pb_tops(int C) { return C == 32 || C == 64 || C == 128; }
 template <typename T> cudaError_t launch_pb_bwd(const T* A, const T* gB2, T* gA, int n, int L, int Lout, int C, cudaStream_t s);
 // gated bilinear product (product_basis.nonlinear = silu_bilineargate): XY [n][D][2C] holds both factors (channels [0, C) /
@@ -199,8 +199,8 @@ struct CopySegments {
 cudaError_t launch_copy_segments(const CopySegments& c, cudaStream_t s);
 // dst[i] = src[perm[i]] (gather) / dst[perm[i]] = src[i] (scatter), rows of row_len elements
 template <typename T> cudaError_t launch_gather_rows(const T* src, const int* perm, T* dst, long long n, int row_len, cudaStream_t s);
-// the same for rows of a multiple of four floats, and top[i] = bits of the largest |element| of row i of dst (more: not below what it held)
-cudaError_t launch_gather_rows_top(const float* src, const int* perm, float* dst, long long n, int row_len, unsigned* top, bool more, cudaStream_t s);
+// the same for rows of the ranks 0..L of C channels, a multiple of four, and top[i * top_stride + l] = bits of the largest |element| of rank l in row i
+cudaError_t launch_gather_rows_top(const float* src, const int* perm, float* dst, long long n, int L, int C, unsigned* top, int top_stride, cudaStream_t s);
 template <typename T> cudaError_t launch_add_inplace(T* dst, const T* src, long long n, cudaStream_t s);
 // dst[i, :width] += src[i, :width], rows dst_stride / src_stride elements apart
 template <typename T> cudaError_t launch_add_rows(T* dst, long long dst_stride, const T* src, long long src_stride, long long n, int width,
@@ -336,10 +336,23 @@ struct TeceArgs {
   T* up; T* glu; T* coefZ; T* U; T* down; T* M;
   const T* gM; T* gdown; T* galpha; T* glogit; T* gcut; T* gproj; T* proj; T* gQp; T* gKp; T* gKs; T* gQt; T* gMw;
   const T* gU; T* gup; T* gglu; T* gcoefZ; T* gWg; T* gvec; T* dxe; T* gx; T* ddlen_extra;
-  unsigned* top;                                                     // [kTeceTops][E], zeroed: bits of the largest |element| a stage wrote for an edge
+  unsigned* top;                                                     // kTeceTops * E, zeroed: TeceTop
 };
-// Where a stage notes the largest element of the rows that the SO(2) linears then read (nullptr: not wanted)
-enum TeceTop { TECE_TOP_IN, TECE_TOP_MW, TECE_TOP_MIX, TECE_TOP_DOWN, TECE_TOP_GMIX, TECE_TOP_GPROJ, kTeceTops };
+// Where a stage notes the bits of the largest |element| of the rows that the SO(2) linears then read, for every edge, operand and order: at
+// top + offset * E, [E][width of the stage], the orders 0..2 of an operand next to one another.
+enum TeceTop {
+  TECE_TOP_IN = 0,       // Ks, Qt
+  TECE_TOP_MW = 6,       // Mw
+  TECE_TOP_MIX = 9,      // U
+  TECE_TOP_DOWN = 12,    // gdown
+  TECE_TOP_GMIX = 15,    // gup (its gates are rows of order 0), gglu, gcoefZ (order 0 only)
+  TECE_TOP_GPROJ = 22,   // gKp, gQp
+  kTeceTops = 28
+};
+constexpr int tece_top_width(int stage) {
+  return stage == TECE_TOP_IN || stage == TECE_TOP_GPROJ ? 6 : stage == TECE_TOP_GMIX ? 7 : 3;
+}
+template <int STAGE> constexpr int kTeceTopWidth = tece_top_width(STAGE);
 int tece_wigner_stride(int L, int mmax);  // entries of one edge's packed Wigner rows (tece_kernels.cu)
 template <typename T> cudaError_t launch_tece(const TeceArgs<T>& a, int stage, cudaStream_t s);
 
@@ -350,7 +363,7 @@ struct TcLinearProblem {
   long long n_atoms;
   int K, N;
   const float* Bhi; const float* Blo;  // [N][K]
-  const float* B; const float* b_inv;  // for a_top: [N][K], packed by launch_tc_pack, and the inverse of its scale (device memory)
+  const float* B; const float* b_inv;  // for a_top: [N][K], packed by launch_tc_pack, and the inverse scales of its columns [N] (per group; device memory)
   float* C; long long c_s1, c_s2;
   const float* bias;     // [N] or nullptr
   // per-species form: atoms of A are sorted by species; group g owns atoms [group_ptr[g], group_ptr[g+1]) and tiles
@@ -359,12 +372,13 @@ struct TcLinearProblem {
   int n_groups;          // 0: a single group (plain linear)
   const int* group_ptr; const int* tile_ptr; const int* atom_map;
   long long b_group_stride, bias_group_stride;
-  const unsigned* a_top; // bits of the largest |element| among every atom's rows of A, or nullptr.  A launch whose problems all have it (joined ones
-                         // the same) multiplies FP16 parts of scaled operands instead of TF32 ones
+  const unsigned* a_top; // bits of the largest |element| among the rows of A of atom i at [i * a_top_stride], or nullptr.  A launch whose problems all
+  int a_top_stride;      // have it (at most kTcJoined to a result) multiplies FP16 parts of scaled operands instead of TF32 ones
   int accumulate;        // C += instead of C =
   int join;              // the product is added to the problem before (same rows, N and groups), in one pass over both K ranges
   int b_tiled;           // B, Bhi / Blo are stored K-tile-major, [groups][K/32][N][32] (b_group_stride must be N*K)
 };
+constexpr int kTcJoined = 3;
 bool tc_linear_supported(int N, int K);
 // whether a launch that could takes FP16 parts: its results per atom (or edge) and their K steps of 32 in all; no count of rows enters
 bool tc_fp16_pays(long long results, long long steps);
@@ -372,6 +386,6 @@ bool tc_fp16_pays(long long results, long long steps);
 cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* error_flag, cudaStream_t s, bool any_length = false);
 cudaError_t launch_tc_gemm(const float* A, long long lda, const float* Bhi, const float* Blo, float* C, long long ldc, int M,
                            int N, int K, int* error_flag, cudaStream_t s, const float* bias = nullptr);
-// packed [n] and scale [2] (its second entry is what b_inv points to) of the weights hi + lo, n a multiple of 32
-cudaError_t launch_tc_pack(const float* hi, const float* lo, long long n, float* packed, float* scale, cudaStream_t s);
+// FP16 parts of the weights hi + lo [groups][N][K] (K-tile-major with `tiled`), and the inverse scale of every column of the result, inv [groups][N]
+cudaError_t launch_tc_pack(const float* hi, const float* lo, int groups, int N, int K, bool tiled, float* packed, float* inv, cudaStream_t s);
 }  // namespace tace

@@ -87,36 +87,41 @@ cudaError_t launch_gather_rows(const T* src, const int* perm, T* dst, long long 
   return cudaGetLastError();
 }
 
-// Row gather that also finds the largest |element| of every row, by which the tensor-core GEMM scales its FP16 parts: a block per row.
+// Row gather that also finds the largest |element| of every rank of a row, by which the tensor-core GEMM scales its FP16 parts: a block per row.
 __device__ __forceinline__ unsigned top_bits(uint4 v) {
   const unsigned m = 0x7FFFFFFFu;
   return max(max(v.x & m, v.y & m), max(v.z & m, v.w & m));
 }
 __global__ void __launch_bounds__(128) gather_rows_top_kernel(const uint4* __restrict__ src, const int* __restrict__ perm, uint4* __restrict__ dst,
-                                                              int len, unsigned* __restrict__ top, bool more) {
-  __shared__ unsigned part[4];
+                                                              int D, int C4, unsigned* __restrict__ top, int top_stride) {
+  __shared__ unsigned part[4][4];
   const long long i = blockIdx.x;
+  const int len = D * C4, lane = threadIdx.x & 31;
   const uint4* from = src + (long long)perm[i] * len;
   uint4* to = dst + i * len;
-  unsigned m = 0;
+  unsigned m[4] = {0u, 0u, 0u, 0u};
 #pragma unroll 4
   for (int k = threadIdx.x; k < len; k += 128) {
     const uint4 v = from[k];
     to[k] = v;
-    m = max(m, top_bits(v));
+    const unsigned t = top_bits(v);
+    const int row = k / C4, l = (row >= 1) + (row >= 4) + (row >= 9);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) m[j] = max(m[j], l == j ? t : 0u);
   }
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    m[j] = __reduce_max_sync(0xffffffffu, m[j]);
+    if (lane == j) part[threadIdx.x >> 5][j] = m[j];
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    m = max(max(part[0], part[1]), max(part[2], part[3]));
-    top[i] = more ? max(top[i], m) : m;
-  }
+  const int l = threadIdx.x;
+  if (l < 4 && l * l < D) top[i * top_stride + l] = max(max(part[0][l], part[1][l]), max(part[2][l], part[3][l]));
 }
-cudaError_t launch_gather_rows_top(const float* src, const int* perm, float* dst, long long n, int row_len, unsigned* top, bool more, cudaStream_t s) {
+cudaError_t launch_gather_rows_top(const float* src, const int* perm, float* dst, long long n, int L, int C, unsigned* top, int top_stride, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  if (row_len % 4 || ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15)) return cudaErrorInvalidValue;
-  gather_rows_top_kernel<<<(unsigned)n, 128, 0, s>>>(reinterpret_cast<const uint4*>(src), perm, reinterpret_cast<uint4*>(dst), row_len / 4, top, more);
+  if (L < 0 || L > 3 || C % 4 || ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15)) return cudaErrorInvalidValue;
+  gather_rows_top_kernel<<<(unsigned)n, 128, 0, s>>>(reinterpret_cast<const uint4*>(src), perm, reinterpret_cast<uint4*>(dst), (L + 1) * (L + 1), C / 4, top, top_stride);
   return cudaGetLastError();
 }
 
@@ -234,17 +239,22 @@ __global__ void gate_fwd_kernel(const T* __restrict__ Gt, T* __restrict__ a, int
     for (int m = 0; m < 2 * l + 1; ++m) out[(l * l + m) * C + c] = v[l * l + m] * gate;
   }
 }
-// The largest of an atom's threads (its C / 32 warps are in one block of 128, pb_tops) to top[i].  All threads of the block that work call it.
-__device__ __forceinline__ void block_top(unsigned* top, int i, int c, int C, float m) {
-  __shared__ unsigned part[4];
-  const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-  const int warp = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) part[warp] = w;
+// The R largest elements of an atom's threads (its C / 32 warps are in one block of 128, pb_tops) to top[0..R).  All threads of the block that work
+// call it.
+template <int R>
+__device__ __forceinline__ void block_tops(unsigned* top, int c, int C, const float (&m)[R]) {
+  __shared__ unsigned part[4][R];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(m[r]));
+    if (lane == r) part[warp][r] = w;
+  }
   __syncthreads();
-  if (c == 0) {
-    unsigned t = w;
-    for (int k = 1; k < C / 32; ++k) t = max(t, part[warp + k]);
-    top[i] = t;
+  if (c < R) {  // (R <= 8: lanes of the atom's first warp)
+    unsigned t = part[warp][c];
+    for (int k = 1; k < C / 32; ++k) t = max(t, part[warp + k][c]);
+    top[c] = t;
   }
 }
 template <typename T, int L>
@@ -257,13 +267,15 @@ __global__ void gate_bwd_kernel(const T* __restrict__ Gt, const T* __restrict__ 
   const T* g = ga + (long long)i * D * C;
   T* out = gGt + (long long)i * (L + 1 + D) * C;
   T gs[L + 1], v[D], gk[D];
-  T most = T(0);
-  auto put = [&](int k, T x) {
+  T most[L + 1];  // per rank of the rows
+#pragma unroll
+  for (int l = 0; l <= L; ++l) most[l] = T(0);
+  auto put = [&](int l, int k, T x) {
     out[k * C + c] = x;
-    if constexpr (sizeof(T) == 4) most = fmaxf(most, fabsf(x));
+    if constexpr (sizeof(T) == 4) most[l] = fmaxf(most[l], fabsf(x));
   };
   auto note = [&]() {
-    if constexpr (sizeof(T) == 4) { if (top) block_top(top, i, c, C, most); }
+    if constexpr (sizeof(T) == 4) { if (top) block_tops<L + 1>(top + (long long)i * (L + 1), c, C, most); }
   };
 #pragma unroll
   for (int l = 0; l <= L; ++l) gs[l] = row[l * C + c];
@@ -272,7 +284,7 @@ __global__ void gate_bwd_kernel(const T* __restrict__ Gt, const T* __restrict__ 
   if (!m0) {
 #pragma unroll
     for (int k = 1; k < D; ++k) v[k] = row[(L + k) * C + c];
-    put(0, gk[0] * T(kSiluCst) * silu_grad_(gs[0]));
+    put(0, 0, gk[0] * T(kSiluCst) * silu_grad_(gs[0]));
 #pragma unroll
     for (int l = 1; l <= L; ++l) {
       const T sg = sigmoid_(gs[l]);
@@ -282,9 +294,9 @@ __global__ void gate_bwd_kernel(const T* __restrict__ Gt, const T* __restrict__ 
       for (int m = 0; m < 2 * l + 1; ++m) {
         const int k = l * l + m;
         acc += gk[k] * v[k];
-        put(L + k, gk[k] * gate);
+        put(l, L + k, gk[k] * gate);
       }
-      put(l, acc * T(kSigmoidCst) * sg * (T(1) - sg));
+      put(0, l, acc * T(kSigmoidCst) * sg * (T(1) - sg));
     }
     note();
     return;
@@ -300,9 +312,9 @@ __global__ void gate_bwd_kernel(const T* __restrict__ Gt, const T* __restrict__ 
     for (int m = 0; m < 2 * l + 1; ++m) {
       const int k = l * l + m;
       acc += gk[k] * v[k];
-      put(L + 1 + k, gk[k] * gate);
+      put(l, L + 1 + k, gk[k] * gate);
     }
-    put(l, acc * T(kSigmoidCst) * sg * (T(1) - sg));
+    put(0, l, acc * T(kSigmoidCst) * sg * (T(1) - sg));
   }
   note();
 }
@@ -331,7 +343,7 @@ cudaError_t launch_gate_bwd(const T* Gt, const T* ga, T* gGt, int n, int L, int 
 // ---- product basis -----------------------------------------------------------------------------
 // top: see launch_pb_fwd; the C / 32 warps of an atom are in one block
 template <typename T, typename PB>
-__global__ void __launch_bounds__(128) pb_fwd_kernel(const T* __restrict__ A, T* __restrict__ B2, int n, int C, unsigned* __restrict__ top) {
+__global__ void __launch_bounds__(128) pb_fwd_kernel(const T* __restrict__ A, T* __restrict__ B2, int n, int C, unsigned* __restrict__ top, int top_stride) {
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= (long long)n * C) return;
   const int i = idx / C, c = idx - (long long)i * C;
@@ -345,12 +357,15 @@ __global__ void __launch_bounds__(128) pb_fwd_kernel(const T* __restrict__ A, T*
   for (int k = 0; k < PB::NB; ++k) Bi[k * C + c] = b[k];
   if constexpr (sizeof(T) == 4) {
     if (!top) return;
-    float m = 0.f;
+    constexpr int R = PB::L + 1;
+    float m[2 * R];
 #pragma unroll
-    for (int k = 0; k < PB::D; ++k) m = fmaxf(m, fabsf(a[k]));
+    for (int r = 0; r < 2 * R; ++r) m[r] = 0.f;
 #pragma unroll
-    for (int k = 0; k < PB::NB; ++k) m = fmaxf(m, fabsf(b[k]));
-    block_top(top, i, c, C, m);
+    for (int k = 0; k < PB::D; ++k) { const int l = (k >= 1) + (k >= 4) + (k >= 9); m[l] = fmaxf(m[l], fabsf(a[k])); }
+#pragma unroll
+    for (int k = 0; k < PB::NB; ++k) { const int l = R + PB::rank_of(k); m[l] = fmaxf(m[l], fabsf(b[k])); }
+    block_tops<2 * R>(top + (long long)i * top_stride, c, C, m);
   }
 }
 // gA += d(B2)/dA^T gB2
@@ -388,9 +403,9 @@ __global__ void __launch_bounds__(128) pb_bwd_kernel(const T* __restrict__ A, co
   return cudaGetLastError();
 
 template <typename T>
-cudaError_t launch_pb_fwd(const T* A, T* B2, int n, int L, int Lout, int C, cudaStream_t s, unsigned* top) {
+cudaError_t launch_pb_fwd(const T* A, T* B2, int n, int L, int Lout, int C, cudaStream_t s, unsigned* top, int top_stride) {
   if (top && !pb_tops(C)) return cudaErrorInvalidValue;
-  TACE_PB_DISPATCH(pb_fwd_kernel, A, B2, n, C, top)
+  TACE_PB_DISPATCH(pb_fwd_kernel, A, B2, n, C, top, top_stride)
 }
 template <typename T>
 cudaError_t launch_pb_bwd(const T* A, const T* gB2, T* gA, int n, int L, int Lout, int C, cudaStream_t s) {
@@ -784,7 +799,7 @@ __global__ void one_hot_kernel(const int* __restrict__ species, long long n, int
   template cudaError_t launch_fold_rows<T>(const T*, const T*, const T*, const T*, T*, int, int, cudaStream_t); \
   template cudaError_t launch_gate_fwd<T>(const T*, T*, int, int, int, int, cudaStream_t);                    \
   template cudaError_t launch_gate_bwd<T>(const T*, const T*, T*, int, int, int, int, cudaStream_t, unsigned*); \
-  template cudaError_t launch_pb_fwd<T>(const T*, T*, int, int, int, int, cudaStream_t, unsigned*);           \
+  template cudaError_t launch_pb_fwd<T>(const T*, T*, int, int, int, int, cudaStream_t, unsigned*, int);      \
   template cudaError_t launch_pbl_fwd<T>(const T*, const T*, T*, int, int, int, int, cudaStream_t);           \
   template cudaError_t launch_pbl_bwd<T>(const T*, const T*, const T*, T*, T*, int, int, int, int, cudaStream_t); \
   template cudaError_t launch_pb_bwd<T>(const T*, const T*, T*, int, int, int, int, cudaStream_t);            \

@@ -129,7 +129,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 // Several products can share a result: their K ranges are walked one after the other in the same accumulators.
 struct TcSegment {
   CUtensorMap tmA, tmBhi, tmBlo;  // B maps are 3-D {K, N, groups}; FP16: A {32, q, atoms, K/32}, tmBhi {32, N, K/32, groups} over packed weights
-  const float* b_inv;    // FP16: inverse of the weights' scale (device memory)
+  const float* b_inv;    // FP16: inverse scales of the weights' columns, [groups][N]
+  const unsigned* a_top; // FP16: bits of the largest |element| of the rows of atom i at [i * a_top_stride]
+  int a_top_stride;
   int num_k;             // 32-wide K steps
   int b_tiled;           // B maps are 4-D {32, N, K/32, groups} over K-tile-major weights
 };
@@ -139,14 +141,13 @@ struct TcProblem {
   long long c_s1, c_s2;  // atom stride / component stride of C rows (elements)
   long long bias_group_stride;
   int q, R, n_atoms, N;
-  int seg0, num_k;       // first of its segments, K steps of all of them
+  int seg0, n_seg, num_k;  // first of its segments, their number, K steps of all of them
   int row_tiles;         // of a plain problem
   // per-species problems: atoms are sorted by species, group g owns atoms [group_ptr[g], group_ptr[g+1]) and
   // R-atom tiles [tile_ptr[g], tile_ptr[g+1]); both arrays live in device memory.  n_groups == 0: one group.
   int n_groups;
   const int* group_ptr;
   const int* tile_ptr;
-  const unsigned* a_top; // FP16: bits of the largest |element| of every atom's rows of A
   const int* atom_map;   // row of C for sorted atom a is atom_map[a]; nullptr: identity
   int accumulate;        // C += instead of C =
   int table;             // offset of its row pointers in the kernel's shared-memory tables, -1: read from global memory
@@ -692,7 +693,7 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
     if (!tc_linear_supported(h.N, h.K) || h.q < 1 || h.q > 128 || (h.a_atom_stride & 3) || (h.a_comp_stride & 3) || (h.c_s1 & 3) ||
         (h.c_s2 & 3))
       return cudaErrorInvalidValue;
-    fp16 = fp16 && h.a_top && h.B && h.b_inv && (!h.join || (i > 0 && h.a_top == probs[i - 1].a_top));
+    fp16 = fp16 && h.a_top && h.B && h.b_inv;
     if (h.join) {
       if (i == 0 || h.q != probs[i - 1].q || h.N != probs[i - 1].N || h.n_atoms != probs[i - 1].n_atoms || h.n_groups != probs[i - 1].n_groups)
         return cudaErrorInvalidValue;
@@ -704,7 +705,7 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
     all128 = all128 && (h.N % 128 == 0);
   }
   first[n_results] = n_problems;
-  for (int i = 0; i < n_results; ++i) one = one && steps_of[i] <= kChunk;
+  for (int i = 0; i < n_results; ++i) { one = one && steps_of[i] <= kChunk; fp16 = fp16 && first[i + 1] - first[i] <= kTcJoined; }
   // From the shapes alone: with a count of tiles, the last of them rounded up, one row more could change the kernel, and a replayed pass, whose
   // rows are those of its capacity, could take another one than the direct pass.
   long long results = 0, all_steps = 0;
@@ -735,7 +736,7 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
     TcProblem& P = b.p[b.n_problems];
     P.q = h.q; P.R = kBM / h.q; P.n_atoms = (int)h.n_atoms; P.N = h.N;
     P.C = h.C; P.bias = h.bias; P.c_s1 = h.c_s1; P.c_s2 = h.c_s2; P.bias_group_stride = h.bias_group_stride;
-    P.n_groups = h.n_groups; P.group_ptr = h.group_ptr; P.tile_ptr = h.tile_ptr; P.atom_map = h.atom_map; P.a_top = h.a_top;
+    P.n_groups = h.n_groups; P.group_ptr = h.group_ptr; P.tile_ptr = h.tile_ptr; P.atom_map = h.atom_map;
     P.accumulate = h.accumulate;
     P.table = -1;
     for (int k = 0; k < b.n_problems && h.n_groups > 0; ++k)  // the tables of an earlier problem
@@ -743,7 +744,7 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
     if (h.n_groups > 0 && P.table < 0 && table + 2 * (h.n_groups + 1) <= TcSmem<128>::kTableInts) { P.table = table; P.copy_table = 1; table += 2 * (h.n_groups + 1); }
     const int groups = h.n_groups > 0 ? h.n_groups : 1;
     if (h.n_groups > 0 && (!h.group_ptr || !h.tile_ptr)) return cudaErrorInvalidValue;
-    P.seg0 = segs;
+    P.seg0 = segs; P.n_seg = first[order[i] + 1] - first[order[i]];
     for (int k = first[order[i]]; k < first[order[i] + 1]; ++k) {
       const TcLinearProblem& g = probs[k];
       TcSegment& G = b.seg[segs++];
@@ -752,7 +753,7 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
       P.num_k += G.num_k;
       if (g.b_tiled && groups > 1 && g.b_group_stride != (long long)g.N * g.K) return cudaErrorInvalidValue;
       if (fp16) {
-        G.b_inv = g.b_inv;
+        G.b_inv = g.b_inv; G.a_top = g.a_top; G.a_top_stride = g.a_top_stride;
         if (!make_map_a_pairs(&G.tmA, g.A, g.n_atoms, g.q, g.K, g.a_atom_stride, g.a_comp_stride, P.R) ||
             !make_map_b_pairs(&G.tmBhi, g.B, groups, g.N, g.K, g.b_group_stride, g.b_tiled != 0, bn))
           return cudaErrorInvalidValue;
@@ -787,14 +788,10 @@ cudaError_t launch_tc_gemm(const float* A, long long lda, const float* Bhi, cons
   return launch_tc_linear(&h, 1, error_flag, s);
 }
 
-cudaError_t launch_tc_pack(const float* hi, const float* lo, long long n, float* packed, float* scale, cudaStream_t s) {
-  if (!hi || !lo || !packed || !scale || n <= 0 || n % kBK) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(scale, 0, 2 * sizeof(float), s);
-  if (e != cudaSuccess) return e;
-  const long long blocks = (n + 1023) / 1024;
-  const unsigned grid = (unsigned)(blocks < 2048 ? blocks : 2048);
-  tc_pack_top_kernel<<<grid, 256, 0, s>>>(hi, lo, n, reinterpret_cast<unsigned*>(scale));
-  tc_pack_kernel<<<grid, 256, 0, s>>>(hi, lo, n, scale, reinterpret_cast<__half*>(packed));
+cudaError_t launch_tc_pack(const float* hi, const float* lo, int groups, int N, int K, bool tiled, float* packed, float* inv, cudaStream_t s) {
+  if (!hi || !lo || !packed || !inv || groups <= 0 || N <= 0 || K <= 0 || K % kBK) return cudaErrorInvalidValue;
+  const long long columns = (long long)groups * N;
+  tc_pack_kernel<<<(unsigned)((columns + 7) / 8), 256, 0, s>>>(hi, lo, columns, N, K / kBK, tiled, reinterpret_cast<__half*>(packed), inv);
   return cudaGetLastError();
 }
 
@@ -816,7 +813,7 @@ extern "C" int tace_tc_gemm_set_test_mode(uint32_t spin_limit, uint32_t extra_ex
 extern "C" int tace_tc_gemm_fp16_f32(const TaceTcOperands* operands, int32_t n_operands, int32_t n_atoms, int32_t q, int32_t N, int32_t n_groups,
                                      const int32_t* group_ptr, const int32_t* tile_ptr, float* C, const float* bias, int32_t accumulate,
                                      int32_t* error_flag, tace_stream_t stream) {
-  constexpr int kMost = 4;
+  constexpr int kMost = tace::kTcJoined;
   if (!operands || n_operands < 1 || n_operands > kMost || n_atoms < 0 || q < 1 || q > 128 || N < 64 || n_groups < 0 || !C || !error_flag ||
       (n_groups > 0 && (!group_ptr || !tile_ptr)))
     return TACE_ERR_INVALID_ARGUMENT;
@@ -827,11 +824,11 @@ extern "C" int tace_tc_gemm_fp16_f32(const TaceTcOperands* operands, int32_t n_o
     const TaceTcOperands& o = operands[i];
     if (!o.A || !o.A_top || !o.B_hi || !o.B_lo || !o.B_packed || o.K < 32 || !tace::tc_linear_supported(N, o.K)) return TACE_ERR_INVALID_ARGUMENT;
     const long long n = (long long)(n_groups > 0 ? n_groups : 1) * N * o.K;
-    const cudaError_t e = tace::launch_tc_pack(o.B_hi, o.B_lo, n, o.B_packed, o.B_packed + n, s);
+    const cudaError_t e = tace::launch_tc_pack(o.B_hi, o.B_lo, n_groups > 0 ? n_groups : 1, N, o.K, n_groups > 0, o.B_packed, o.B_packed + n, s);
     if (e != cudaSuccess) return TACE_ERR_CUDA;
     tace::TcLinearProblem& h = probs[i];
     h.A = o.A; h.a_atom_stride = (long long)q * o.K; h.a_comp_stride = o.K; h.q = q; h.n_atoms = n_atoms; h.K = o.K; h.N = N;
-    h.Bhi = o.B_hi; h.Blo = o.B_lo; h.B = o.B_packed; h.b_inv = o.B_packed + n + 1; h.a_top = o.A_top;
+    h.Bhi = o.B_hi; h.Blo = o.B_lo; h.B = o.B_packed; h.b_inv = o.B_packed + n; h.a_top = o.A_top; h.a_top_stride = 1;
     h.C = C; h.c_s1 = (long long)q * N; h.c_s2 = N; h.bias = bias;
     h.n_groups = n_groups; h.group_ptr = group_ptr; h.tile_ptr = tile_ptr; h.b_group_stride = (long long)N * o.K; h.bias_group_stride = N;
     h.b_tiled = n_groups > 0; h.accumulate = accumulate != 0; h.join = i > 0;

@@ -2,10 +2,11 @@
 // (TcLinearProblem::a_top: the SO(2) linears over edges).  Included by tc_gemm.cu, whose barriers, tile search and tensor maps it uses.
 //
 // FP16 has the eleven mantissa bits of TF32 at twice its rate and half its bytes, and five exponent bits instead of eight; what those
-// lack is given back by powers of two: the rows of an atom are scaled so that their largest element lies in [2^13, 2^14), the weights
-// likewise, all of an array by one power.  x = hi + lo with both parts rounded to nearest, and hi*hi + hi*lo + lo*hi is accumulated as
-// in TF32: an element keeps its 22 bits down to 2^-16 of the largest one, and the error of a smaller one is 2^-39 of it.  The epilogue takes
-// the scales out of the sums, which is exact.  Relative error (2-norm) of 75 776 x 512 x 1 024 normal numbers 1.9e-6, 2.3e-6 as TF32; with K = 128
+// lack is given back by powers of two: the rows that an operand has of an atom (edge) are scaled so that their largest element lies in [2^13,
+// 2^14), the weights likewise, every column of the result (of every element) by a power of its own; what shares a scale is the components of
+// one rank or order.  x = hi + lo with both parts rounded to nearest, and hi*hi + hi*lo + lo*hi is accumulated as in TF32: an element keeps its 22 bits
+// down to 2^-16 of the largest one of its row or column, and the error of a smaller one is 2^-39 of that.  The epilogue takes the scales out of
+// the sums, which is exact.  Relative error (2-norm) of 75 776 x 512 x 1 024 normal numbers 1.9e-6, 2.3e-6 as TF32; with K = 128
 // 5.4e-7 and 1.4e-6.
 //
 // What it had to solve besides: the TF32 kernel takes .72 us per K step of a CTA with the tensor pipe busy 69 % of it, and with FP16 parts in the
@@ -88,7 +89,7 @@ __device__ __forceinline__ float4 gather_columns(const float* v, int odd) {  // 
 // What the scheduler tells the other roles about a tile; num_k = 0 ends the list.
 struct alignas(64) TileSlot {
   const float* bias;
-  int num_k, seg0, atom0, n0, group, rows, accumulate;
+  int num_k, seg0, atom0, n0, group, rows, accumulate, column;  // column: first one among those of all groups
 };
 template <int BN>
 struct Fp16Smem {
@@ -101,7 +102,7 @@ struct Fp16Smem {
   static constexpr int kTmemA = 2 * BN, kTmemStage = 64, kTmemStep = kTmemStage / kSteps;
   static constexpr int kBarrierBytes = 576;              // and the tile counts of the problems
   static constexpr int kInfoBytes = kInfo * (64 + kBM * 8);  // tile descriptions and the addresses of their rows
-  static constexpr int kTopBytes = kInfo * kBM * 4;          // largest elements of the tiles' rows
+  static constexpr int kTopBytes = kInfo * kTcJoined * kBM * 4;  // largest elements of the tiles' rows
   static constexpr int kTotal = kStages * kStageBytes + kInfoBytes + kBarrierBytes + 4 * kTableInts + kTopBytes + 1024;  // + alignment slack
   static_assert(kTmemA + kTmemStage * kStages <= kTmemCols && kTotal <= 232448, "on-chip memory");
 };
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
   TileSlot* info = reinterpret_cast<TileSlot*>(after + kInfo * kBM * 8);                 // [kInfo]
   const uint32_t bars = base + kStages * S::kStageBytes + S::kInfoBytes;
   int* tables = reinterpret_cast<int*>(after + S::kInfoBytes + S::kBarrierBytes);
-  unsigned* row_top = reinterpret_cast<unsigned*>(tables + kTableInts);  // [kInfo][kBM], FP16: largest element of a row
+  unsigned* row_top = reinterpret_cast<unsigned*>(tables + kTableInts);  // [kInfo][kTcJoined][kBM]: largest element of a row of every segment
   // barriers: ready[s] operands split | empty[s] MMAs done reading | raw[s] operands landed | acc_full[a] | acc_empty[a] | info_full[i] | info_empty[i] |
   // rows_full[i] addresses and scales of a tile's rows known
   constexpr int kRing = 3 * kStages, kBars = kRing + 5 + 3 * kInfo;
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
         if (lane == 0) {
           d.bias = P.bias ? P.bias + t.group * P.bias_group_stride + t.n0 : nullptr;
           d.num_k = P.num_k; d.seg0 = P.seg0; d.atom0 = t.atom0; d.n0 = t.n0; d.group = t.group;
-          d.rows = rows; d.accumulate = P.accumulate;
+          d.rows = rows; d.accumulate = P.accumulate; d.column = t.group * P.N + t.n0;
           mbar_arrive(info_full(slot));  // the producer and the issuer can begin
         }
         // The largest elements come in asynchronously and count as arrivals of their own: waited for here, they were the longest step of a tile
@@ -217,9 +218,10 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
           const int r = k * 32 + lane, al = r / P.q, m = r - al * P.q;
           const bool valid = r < rows && t.atom0 + al < t.atom_end;
           long long atom = t.atom0 + al;
-          {
-            unsigned* top = row_top + slot * kBM + r;
-            if (valid) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(top)), "l"(P.a_top + atom) : "memory");
+          for (int g = 0; g < P.n_seg; ++g) {
+            const TcSegment& G = batch.seg[P.seg0 + g];
+            unsigned* top = row_top + (slot * kTcJoined + g) * kBM + r;
+            if (valid) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(top)), "l"(G.a_top + atom * G.a_top_stride) : "memory");
             else *top = 0u;
           }
           if (valid && P.atom_map) atom = P.atom_map[atom];
@@ -336,14 +338,24 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
       if (!warp_wait(rows_full(slot), phase_of(i), abort_flag, batch.error, 6, batch.spin_limit)) break;
       const int num_k = info[slot].num_k, seg0 = num_k ? info[slot].seg0 : 0;
       const int at = set * info[slot].rows + row;  // row of the stage: the steps follow each other without a gap
-      float inv;
-      const float scale = fp16_scale(__uint_as_float(row_top[slot * kBM + row]), inv);
+      unsigned tops[kTcJoined];  // (those of segments that the tile does not have are not used)
+#pragma unroll
+      for (int g = 0; g < kTcJoined; ++g) tops[g] = row_top[(slot * kTcJoined + g) * kBM + row];
       __syncwarp();
       if (lane == 0) mbar_arrive(info_empty(slot));
       if (num_k == 0) break;
-      int stages = 0;  // of the tile: the steps of a segment in pairs
-      for (int seg = seg0, left = num_k; left > 0; ++seg) { left -= batch.seg[seg].num_k; stages += (batch.seg[seg].num_k + 1) / kSteps; }
-      for (; stages > 0; --stages) {
+      int seg = seg0, left = num_k, stages = 0;  // stages: left of the segment, its steps in pairs
+      float scale = 0.f;
+      while (left > 0 || stages > 0) {
+        if (stages == 0) {
+          const int steps = batch.seg[seg].num_k, g = seg - seg0;
+          stages = (steps + 1) / kSteps;
+          left -= steps;
+          ++seg;
+          float inv;
+          scale = fp16_scale(__uint_as_float(g == 0 ? tops[0] : g == 1 ? tops[1] : tops[2]), inv);
+        }
+        --stages;
         if (!warp_wait(raw_bar(s), ph, abort_flag, batch.error, 3, batch.spin_limit)) { ok = false; break; }
         // the row's eight 16-byte pieces sit at positions j ^ (at & 7) of its 128 bytes (the swizzle the TMA unit wrote); the columns of the
         // residuals follow those of the high parts
@@ -387,10 +399,11 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
       const float* bias = info[slot].bias;
       const bool accumulate = info[slot].accumulate != 0;
       const TcSegment* G = &batch.seg[info[slot].seg0];
+      const unsigned* tops = row_top + slot * kTcJoined * kBM + r0;
       int left = G->num_k;
-      float w_inv = *G->b_inv;
+      const int column = info[slot].column + half * HN + 2 * (lane & 3);  // this lane's first one, as tmem_ld_rows leaves them
       for (int ks = 0; ks < num_k; ++chunk) {
-        if (left == 0) { left = (++G)->num_k; w_inv = *G->b_inv; }
+        if (left == 0) { left = (++G)->num_k; tops += kBM; }
         const int n = left < kSteps * kFp16Chunk ? left : kSteps * kFp16Chunk;
         const bool first = ks == 0;
         ks += n; left -= n;
@@ -398,25 +411,25 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
         if (!warp_wait(acc_full(a), (chunk >> 1) & 1, abort_flag, batch.error, 5, batch.spin_limit)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem_base + ((uint32_t)(ew * 32) << 16) + a * BN + half * HN;
+        float f[4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          float f[2];
+        for (int k = 0; k < 4; ++k) fp16_scale(__uint_as_float(tops[8 * k]), f[k]);
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            fp16_scale(__uint_as_float(row_top[slot * kBM + r0 + 16 * h + 8 * k]), f[k]);
-            f[k] *= w_inv;
-          }
-          float v[HN / 32][16];
+        for (int c = 0; c < HN / 32; ++c) {
+          float2 w_inv[4];
 #pragma unroll
-          for (int c = 0; c < HN / 32; ++c) tmem_ld_rows(acc + ((uint32_t)(16 * h) << 16) + 32 * c, v[c]);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          for (int k = 0; k < 4; ++k) w_inv[k] = __ldg(reinterpret_cast<const float2*>(G->b_inv + column + 32 * c + 8 * k));
 #pragma unroll
-          for (int c = 0; c < HN / 32; ++c)
+          for (int h = 0; h < 2; ++h) {
+            float v[16];
+            tmem_ld_rows(acc + ((uint32_t)(16 * h) << 16) + 32 * c, v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
-              const float x = v[c][q] * f[q >> 1 & 1];  // exact: a power of two
-              sum[h][c][q] = (first ? 0.f : sum[h][c][q]) + x;
+              const float x = v[q] * f[2 * h + (q >> 1 & 1)];  // exact, as the other product: powers of two
+              sum[h][c][q] = fmaf(x, q & 1 ? w_inv[q >> 2].y : w_inv[q >> 2].x, first ? 0.f : sum[h][c][q]);
             }
+          }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -469,25 +482,27 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
 // ---- packed weights: run when weights are set ------------------------------------------------------------------
 // Every run of 32 weights (128 bytes) becomes 32 FP16 high parts and 32 residuals of the scaled weights, in place of the 32 floats: strides
 // and tensor maps are those of an fp32 array, and one load brings both parts of a K step.
-__global__ void __launch_bounds__(256) tc_pack_top_kernel(const float* __restrict__ hi, const float* __restrict__ lo, long long n, unsigned* top) {
+// A warp per column of the result; blocks of the array: [column][K / 32], or [group][K / 32][column of the group].
+__global__ void __launch_bounds__(256) tc_pack_kernel(const float* __restrict__ hi, const float* __restrict__ lo, long long columns, int N, int steps, bool tiled,
+                                                      __half* out, float* inv) {
+  const long long col = blockIdx.x * 8LL + (threadIdx.x >> 5);
+  if (col >= columns) return;
+  const int lane = threadIdx.x & 31;
+  const long long g = col / N, first = tiled ? g * steps * N + (col - g * N) : col * steps, stride = tiled ? N : 1;
   unsigned m = 0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+  for (int k = 0; k < steps; ++k) {
+    const long long i = (first + k * stride) * 32 + lane;
     const unsigned b = __float_as_uint(hi[i] + lo[i]) & 0x7FFFFFFFu;
     if (b < 0x7F800000u && b > m) m = b;  // infinities and NaN keep what they are under any scale
   }
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(top, m);
-}
-// scale[0]: bits of the largest weight (in), scale[1]: inverse of the scale (out)
-__global__ void __launch_bounds__(256) tc_pack_kernel(const float* __restrict__ hi, const float* __restrict__ lo, long long n, float* scale, __half* out) {
-  float inv;
-  const float sc = fp16_scale(scale[0], inv);
-  if (blockIdx.x == 0 && threadIdx.x == 0) scale[1] = inv;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+  float back;
+  const float sc = fp16_scale(__uint_as_float(__reduce_max_sync(0xffffffffu, m)), back);
+  if (lane == 0) inv[col] = back;
+  for (int k = 0; k < steps; ++k) {
+    const long long run = first + k * stride, i = run * 32 + lane;
     const float v = (hi[i] + lo[i]) * sc;
     const __half h = __float2half_rn(v);
-    __half* row = out + (i >> 5) * 64 + (i & 31);
-    row[0] = h;
-    row[32] = __float2half_rn(v - __half2float(h));
+    out[run * 64 + lane] = h;
+    out[run * 64 + 32 + lane] = __float2half_rn(v - __half2float(h));
   }
 }

@@ -358,15 +358,26 @@ struct WigRows {
       if (i * 32 + lane < Q) reinterpret_cast<uint4*>(buf)[i * 32 + lane] = q[i];
   }
 };
-// Largest |element| of the rows that the linears read next, per edge: the tensor-core GEMM scales its FP16 parts by it.  One warp
-// instruction and an atomic per (edge, 32 channels), beside some 56 stores per lane.
+// Largest |element| of the rows that the linears read next, per edge, operand and order (TeceTop): the tensor-core GEMM scales its FP16
+// parts by it.  A warp instruction each and one atomic of neighbouring lanes per (edge, 32 channels), beside some 56 stores per lane.
 TACE_D TACE_INLINE float larger(float m, float v) { return fmaxf(m, fabsf(v)); }
 TACE_D TACE_INLINE double larger(double m, double) { return m; }  // double precision has no use for it
-TACE_D TACE_INLINE void note_top(unsigned* top, float m) {  // all lanes of a warp, one edge
-  const unsigned b = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-  if ((threadIdx.x & 31) == 0) atomicMax(top, b);
+TACE_HD constexpr int row_order(int L, int r) { return r < L + 1 ? 0 : r < L + 1 + 2 * L ? 1 : 2; }
+// Where the stage's largest elements of edge e begin
+template <int STAGE, typename T>
+TACE_D TACE_INLINE unsigned* tops_of(const TeceArgs<T>& a, long long e) { return a.top + STAGE * a.E + e * kTeceTopWidth<STAGE>; }
+template <int N>
+TACE_D TACE_INLINE void note_tops(unsigned* top, const float (&m)[N]) {  // all lanes of a warp, one edge
+  unsigned mine = 0u;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const unsigned b = __reduce_max_sync(0xffffffffu, __float_as_uint(m[j]));
+    if ((threadIdx.x & 31) == j) mine = b;
+  }
+  if ((threadIdx.x & 31) < N) atomicMax(top + (threadIdx.x & 31), mine);
 }
-TACE_D TACE_INLINE void note_top(unsigned*, double) {}
+template <int N>
+TACE_D TACE_INLINE void note_tops(unsigned*, const double (&)[N]) {}
 TACE_D TACE_INLINE void note_top_lane(unsigned* top, float m) { atomicMax(top, __float_as_uint(m)); }
 TACE_D TACE_INLINE void note_top_lane(unsigned*, double) {}
 // where a block of the kernels below works (channel counts are multiples of 32)
@@ -450,7 +461,7 @@ __global__ void __launch_bounds__(kRotWarps * 32) tece_rotate_in_kernel(const Te
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < D; ++j) vs[j] = st[(2 * NC + j) * 32];
-    T top = T(0), top_w = T(0);
+    T top[6] = {T(0), T(0), T(0), T(0), T(0), T(0)}, top_w[3] = {T(0), T(0), T(0)};
     for_rows<L, MM>([&](int r, int l, int comp, int k) {
       T ks = T(0), qt = T(0);
 #pragma unroll
@@ -464,12 +475,14 @@ __global__ void __launch_bounds__(kRotWarps * 32) tece_rotate_in_kernel(const Te
       a.Qt[at * C + c] = qt;
       a.Mw[at * 2 * C + c] = ws * ks;
       a.Mw[at * 2 * C + C + c] = wt * qt;
-      top = larger(larger(top, ks), qt);
-      top_w = larger(larger(top_w, ws * ks), wt * qt);
+      const int m = row_order(L, r);
+      top[m] = larger(top[m], ks);
+      top[3 + m] = larger(top[3 + m], qt);
+      top_w[m] = larger(larger(top_w[m], ws * ks), wt * qt);
     });
     if (a.top) {
-      note_top(a.top + TECE_TOP_IN * a.E + e, top);
-      note_top(a.top + TECE_TOP_MW * a.E + e, top_w);
+      note_tops(tops_of<TECE_TOP_IN>(a, e), top);
+      note_tops(tops_of<TECE_TOP_MW>(a, e), top_w);
     }
   }
 }
@@ -659,17 +672,17 @@ __global__ void __launch_bounds__(kRotWarps * 32) tece_rotate_out_bwd_kernel(con
     for (int r = 0; r < NR; ++r) v[r] = dn[(long long)r * C];
     __syncwarp();
     if (e + kRotWarps < e1) wq.fetch(a.Wg, e + kRotWarps, s.lane);
-    T part = T(0), top = T(0);
+    T part = T(0), top[3] = {T(0), T(0), T(0)};
     for_rows<L, MM>([&](int r, int l, int, int k) {
       T t = T(0);
 #pragma unroll
       for (int j = 0; j < 2 * l + 1; ++j) t += w[k + j] * vg[l * l + j];
       t *= a.row_scale[r];
       a.gdown[((long long)e * NR + r) * C + c] = al * t;
-      top = larger(top, al * t);
+      top[row_order(L, r)] = larger(top[row_order(L, r)], al * t);
       part += v[r] * t;
     });
-    if (a.top) note_top(a.top + TECE_TOP_DOWN * a.E + e, top);
+    if (a.top) note_tops(tops_of<TECE_TOP_DOWN>(a, e), top);
     if (FUSE) {
       for (int o = Ch >> 1; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
       if (s.lane % Ch == 0) a.galpha[(long long)e * a.H + h] = part;
@@ -749,10 +762,16 @@ __global__ void tece_logit_bwd_kernel(const TeceArgs<T> a) {
   for (int r = 0; r < n0; ++r)
     for (int u = 0; u < Ch; ++u) { gq[r * C + u] = gs * k[r * C + u]; gk[r * C + u] = gs * q[r * C + u]; }
   int off = n0;
-  T gphase = T(0), top = T(0);
-  if (a.top)
-    for (int r = 0; r < n0; ++r)
-      for (int u = 0; u < Ch; ++u) top = larger(larger(top, gq[r * C + u]), gk[r * C + u]);
+  T gphase = T(0), top_q = T(0), top_k = T(0);
+  auto note = [&](int m) {
+    if (!a.top) return;
+    note_top_lane(tops_of<TECE_TOP_GPROJ>(a, e) + m, top_k);
+    note_top_lane(tops_of<TECE_TOP_GPROJ>(a, e) + 3 + m, top_q);
+    top_q = top_k = T(0);
+  };
+  for (int r = 0; r < n0; ++r)
+    for (int u = 0; u < Ch; ++u) { top_q = larger(top_q, gq[r * C + u]); top_k = larger(top_k, gk[r * C + u]); }
+  note(0);
   for (int m = 1; m <= a.mmax; ++m) {
     const int n = a.L + 1 - m;
     const T cs = cos(T(m) * phase), sn = sin(T(m) * phase);
@@ -764,13 +783,14 @@ __global__ void tece_logit_bwd_kernel(const TeceArgs<T> a) {
         gq[ii] = gs * (sn * kr + cs * ki);
         gk[ir] = gs * (cs * qr + sn * qi);
         gk[ii] = gs * (-sn * qr + cs * qi);
-        top = larger(larger(larger(larger(top, gq[ir]), gq[ii]), gk[ir]), gk[ii]);
+        top_q = larger(larger(top_q, gq[ir]), gq[ii]);
+        top_k = larger(larger(top_k, gk[ir]), gk[ii]);
         // d score / d (m phase) = qr (-sn kr - cs ki) + qi (cs kr - sn ki)
         gphase += gs * T(m) * (qr * (-sn * kr - cs * ki) + qi * (cs * kr - sn * ki));
       }
+    note(m);
     off += 2 * n;
   }
-  if (a.top) note_top_lane(a.top + TECE_TOP_GPROJ * a.E + e, top);
   a.gproj[e * 2 * a.H + h] = gl;
   a.gproj[e * 2 * a.H + a.H + h] = gphase * T(3.141592653589793) * (T(1) - th * th);
 }
@@ -815,11 +835,12 @@ __global__ void __launch_bounds__(128) tece_logit_lane_kernel(const TeceArgs<T> 
   T gs = T(0);
   T* gq = nullptr; T* gk = nullptr;
   if (BWD) { gs = a.glogit[e * a.H + h] * a.temp[h]; gq = a.gQp + e * NR * C + c; gk = a.gKp + e * NR * C + c; }
-  T part = T(0), top = T(0);  // forward: the channel's share of the score; backward: of d score / d phase
+  T top[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+  T part = T(0);  // forward: the channel's share of the score; backward: of d score / d phase
 #pragma unroll
   for (int r = 0; r < N0; ++r) {
     if (!BWD) part += qv[r] * kv[r];
-    else { gq[r * C] = gs * kv[r]; gk[r * C] = gs * qv[r]; top = larger(larger(top, gs * kv[r]), gs * qv[r]); }
+    else { gq[r * C] = gs * kv[r]; gk[r * C] = gs * qv[r]; top[3] = larger(top[3], gs * kv[r]); top[0] = larger(top[0], gs * qv[r]); }
   }
 #pragma unroll
   for (int m = 1; m <= MM; ++m) {
@@ -836,12 +857,13 @@ __global__ void __launch_bounds__(128) tece_logit_lane_kernel(const TeceArgs<T> 
         gq[ii * C] = g1;
         gk[ir * C] = g2;
         gk[ii * C] = g3;
-        top = larger(larger(larger(larger(top, g0), g1), g2), g3);
+        top[3 + m] = larger(larger(top[3 + m], g0), g1);
+        top[m] = larger(larger(top[m], g2), g3);
         part += gs * T(m) * (qr * (-sn[m] * kr - cs[m] * ki) + qi * (cs[m] * kr - sn[m] * ki));
       }
     }
   }
-  if (BWD && a.top) note_top(a.top + TECE_TOP_GPROJ * a.E + e, top);
+  if (BWD && a.top) note_tops(tops_of<TECE_TOP_GPROJ>(a, e), top);
   for (int o = Ch >> 1; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
   if (c % Ch == 0) {
     if (!BWD) a.logit[e * a.H + h] = part * a.temp[h] + a.proj[e * 2 * a.H + h];
@@ -957,7 +979,10 @@ __global__ void __launch_bounds__(128) tece_mix_kernel(const TeceArgs<T> a) {
   const long long up = e * (G + NF) * Ca + (long long)i * Ca + ca, full = e * NF * Ca + (long long)i * Ca + ca,
                   path = e * NPATH * N * Ca + (long long)i * Ca + ca;
   const int row = N * Ca;
-  T top = T(0);
+  constexpr int STAGE = BWD ? TECE_TOP_GMIX : TECE_TOP_MIX, NTOP = kTeceTopWidth<STAGE>;
+  T top[NTOP];
+#pragma unroll
+  for (int j = 0; j < NTOP; ++j) top[j] = T(0);
   // every input is in registers before the first store: the gradients overwrite their forward buffers
 #pragma unroll
   for (int q = 0; q < NG; ++q) gz[q] = a.up[up + q * row];
@@ -986,7 +1011,7 @@ __global__ void __launch_bounds__(128) tece_mix_kernel(const TeceArgs<T> a) {
       if (BWD) {
         const T g = gg * act_grad<T>(a.act, gz[m - START]);
         a.gup[up + (m - START) * row] = g;
-        top = larger(top, g);
+        top[0] = larger(top[0], g);
       }
     }
   }
@@ -1013,7 +1038,7 @@ __global__ void __launch_bounds__(128) tece_mix_kernel(const TeceArgs<T> a) {
             const T gr = go[oq], gi = m3 ? go[oi_] : T(0);
             const T g = (gr * zr + gi * zi) * sc * act_grad<T>(a.act, cz[p]);
             a.gcoefZ[path + p * row] = g;
-            top = larger(top, g);
+            top[NTOP - 1] = larger(top[NTOP - 1], g);
             const T ar = w * gr, ai = w * gi;
             gx[xq] += ar * yr + sg * ai * yi;
             if (m1) gx[xi_] += -sg * ar * yi + ai * yr;
@@ -1023,13 +1048,23 @@ __global__ void __launch_bounds__(128) tece_mix_kernel(const TeceArgs<T> a) {
         }
 #pragma unroll
   for (int q = 0; q < M; ++q) {
-    if (BWD) { a.gup[up + G * Ca + q * row] = gx[q]; a.gglu[full + q * row] = gy[q]; top = larger(larger(top, gx[q]), gy[q]); }
-    else { a.U[full + q * row] = out[q]; top = larger(top, out[q]); }
+    const int m = (q + 1) / 2;
+    if constexpr (BWD) {
+      a.gup[up + G * Ca + q * row] = gx[q];
+      a.gglu[full + q * row] = gy[q];
+      top[m] = larger(top[m], gx[q]);
+      top[3 + m] = larger(top[3 + m], gy[q]);
+    } else {
+      a.U[full + q * row] = out[q];
+      top[m] = larger(top[m], out[q]);
+    }
   }
   if (a.top) {
-    unsigned* at = a.top + (BWD ? TECE_TOP_GMIX : TECE_TOP_MIX) * a.E + e;
-    if (Ca % 32 == 0) note_top(at, top);  // the lanes of a warp share their edge
-    else note_top_lane(at, top);
+    unsigned* at = tops_of<STAGE>(a, e);
+    if (Ca % 32 == 0) note_tops(at, top);  // the lanes of a warp share their edge
+    else
+#pragma unroll
+      for (int j = 0; j < NTOP; ++j) note_top_lane(at + j, top[j]);
   }
 }
 

@@ -4,7 +4,9 @@ tiles, with and without a skip connection, and the backward pass alone (two elem
 import pytest
 import torch
 
+from helpers import make_models, oracle_batch, to_device
 from tace_b200 import synth
+from tace_b200.pack import LayerPlan
 from test_gpu_parity import run_case
 
 pytestmark = pytest.mark.gpu
@@ -20,3 +22,37 @@ MANY = list(range(1, 21))
 @pytest.mark.parametrize("skip", ["aware", "identity"])
 def test_species_linears(L, Lmax, channels, structs, zs, cutoff, skip):
     run_case(structs(), L, channels, zs, cutoff, torch.float32, Lmax=Lmax, resnet_linear_type=skip)
+
+
+def _blocks(sd, key, ls, power):
+    """Multiplies the blocks of the ranks `ls` of a linear of ranks 0..3 (equal blocks, one after the other) by 2^power."""
+    w = sd[key]
+    n = w.shape[-1] // 4
+    for l in ls:
+        w[..., l * n:(l + 1) * n] *= 2.0 ** power
+
+
+@pytest.mark.parametrize("power", [-24, 20])
+@pytest.mark.parametrize("where", ["gated", "output"])
+def test_ranks_of_every_magnitude(power, where):
+    """Rank 2 times 2^p between two linears is the same function: of the gated features, and of the features that a layer hands to the next one and to
+    its skip connection.  Every scale is a power of two and belongs to one rank, so not a bit of the results may move."""
+    structs = synth.random_crystals(4, seed=31, nmin=9, nmax=23, zmax=20)
+    model, _, _ = make_models(3, 128, MANY, 4.5, 20.0, torch.float32, seed=4)
+    gpu = to_device(oracle_batch(structs, MANY, 4.5, torch.float32), torch.device("cuda:0"))
+    before = {k: v.clone() for k, v in model(gpu).items() if v is not None}
+    sd = {k: v.clone() for k, v in model.state_dict().items()}
+    pre = "readout_fn.representation."
+    if where == "gated":
+        down = sd[pre + "interactions.1.linear_down.weight"]
+        n2, n3 = (LayerPlan(1, 2, 3).k[l] * 128 * 128 for l in (2, 3))
+        down[down.numel() - n3 - n2:down.numel() - n3] *= 2.0 ** power
+        _blocks(sd, pre + "interactions.1.linear_nonlinearity.weight", [2], -power)
+    else:
+        _blocks(sd, pre + "products.0.linear.weight", [2], power)
+        _blocks(sd, pre + "interactions.1.linear_up.weight", [2], -power)
+    model.load_state_dict(sd)
+    after = model(gpu)
+    assert torch.isfinite(before["forces"]).all()
+    for k, v in before.items():
+        assert torch.equal(after[k], v), k

@@ -146,3 +146,28 @@ def test_every_instance_returns_from_an_expired_wait(N, K):
     got = call()
     assert int(call.err.item()) == 0
     assert error(got[:512], exact([(operands[0][0][:512], operands[0][1])])) < tolerance(K)
+
+
+@pytest.mark.parametrize("sizes", [None, [5, 200, 0, 140]])
+def test_columns_of_every_magnitude(sizes):
+    """Weights of results, and of groups, 2^-24 .. 1 apart: every column is as exact as the others."""
+    n, K = 1 if sizes is None else len(sizes), 128
+    W = normal(n, 128, K, seed=17) * torch.exp2(torch.linspace(-24, 0, n * 128).reshape(n, 128, 1))
+    operands = [(normal(300 if sizes is None else sum(sizes), 1, K, seed=18), W)]
+    call = Call(operands, sizes=sizes)
+    got, want, first = call(), exact(operands, sizes=sizes), 0
+    assert int(call.err.item()) == 0
+    for size in sizes or [300]:
+        if size:
+            assert error(got[first:first + size], want[first:first + size], dim=(0, 1)) < tolerance(K)
+        first += size
+
+
+@pytest.mark.parametrize("N,q", [(128, 1), (64, 7)])
+def test_joined_operands_of_every_magnitude(N, q):
+    """Operands 2^-24 .. 2^24 apart whose weights bring their products to one magnitude."""
+    operands = [(normal(70, q, K, seed=19) * 2. ** p, normal(1, N, K, seed=20) * 2. ** -p) for K, p in ((96, 24), (64, 0), (32, -24))]
+    call = Call(operands)
+    got = call()
+    assert int(call.err.item()) == 0
+    assert error(got, exact(operands)) < tolerance(192)
