@@ -693,7 +693,7 @@ cudaError_t launch_tc_linear(const TcLinearProblem* probs, int n_problems, int* 
     if (!tc_linear_supported(h.N, h.K) || h.q < 1 || h.q > 128 || (h.a_atom_stride & 3) || (h.a_comp_stride & 3) || (h.c_s1 & 3) ||
         (h.c_s2 & 3))
       return cudaErrorInvalidValue;
-    fp16 = fp16 && h.a_top && h.B && h.b_inv;
+    fp16 = fp16 && h.a_top && h.B && h.b_inv && !(reinterpret_cast<uintptr_t>(h.b_inv) & 15);
     if (h.join) {
       if (i == 0 || h.q != probs[i - 1].q || h.N != probs[i - 1].N || h.n_atoms != probs[i - 1].n_atoms || h.n_groups != probs[i - 1].n_groups)
         return cudaErrorInvalidValue;

@@ -19,14 +19,13 @@
 // prefetch of A eight steps ahead (228 -> 239), weights as one linear copy per step (no change) and pairs of SMs
 // with half of the weights each (cta_group::2, 223 -> 285) were tried.
 //
-// One persistent CTA per SM.  Warp roles (640 threads, five warpgroups): warp 0 = TMA producer, warp 1 = MMA issuer, warp 2 = tile scheduler, warp 3
-// idle; warps 4..7 and 8..11 = operand splitters, warps 12..15 and 16..19 = epilogue (warp w works on the TMEM lanes 32 * (w % 4) .. + 31; the
+// One persistent CTA per SM.  Warp roles (640 threads, five warpgroups): warp 0 = TMA producer, warp 1 = MMA issuer, warps 2, 3 = tile schedulers; warps 4..7 and 8..11 = operand splitters, warps 12..15 and 16..19 = epilogue (warp w works on the TMEM lanes 32 * (w % 4) .. + 31; the
 // second four of the epilogue take the right half of the columns, so that 64 running sums per thread fit its registers).  Registers move from
 // the first warpgroup to the others: 40 + 2 * 104 + 2 * 112 of the 5 * 96 of the launch.  Every wait is bounded, as in tc_gemm.cu.
 #pragma once
 
 constexpr int kFp16Chunk = 8;  // stages accumulated inside TMEM before draining into FP32 registers: 96 instructions, as in TF32
-constexpr int kInfo = 8;       // tiles the scheduler is ahead
+constexpr int kInfo = 6;       // tiles the scheduler is ahead
 constexpr int kTableInts = TcSmem<128>::kTableInts;
 
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
@@ -89,7 +88,7 @@ __device__ __forceinline__ float4 gather_columns(const float* v, int odd) {  // 
 // What the scheduler tells the other roles about a tile; num_k = 0 ends the list.
 struct alignas(64) TileSlot {
   const float* bias;
-  int num_k, seg0, atom0, n0, group, rows, accumulate, column;  // column: first one among those of all groups
+  int num_k, seg0, atom0, n0, group, rows, accumulate;
 };
 template <int BN>
 struct Fp16Smem {
@@ -102,7 +101,7 @@ struct Fp16Smem {
   static constexpr int kTmemA = 2 * BN, kTmemStage = 64, kTmemStep = kTmemStage / kSteps;
   static constexpr int kBarrierBytes = 576;              // and the tile counts of the problems
   static constexpr int kInfoBytes = kInfo * (64 + kBM * 8);  // tile descriptions and the addresses of their rows
-  static constexpr int kTopBytes = kInfo * kTcJoined * kBM * 4;  // largest elements of the tiles' rows
+  static constexpr int kTopBytes = kInfo * kTcJoined * (kBM + BN) * 4;  // largest elements of the tiles' rows, inverse scales of their columns
   static constexpr int kTotal = kStages * kStageBytes + kInfoBytes + kBarrierBytes + 4 * kTableInts + kTopBytes + 1024;  // + alignment slack
   static_assert(kTmemA + kTmemStage * kStages <= kTmemCols && kTotal <= 232448, "on-chip memory");
 };
@@ -121,9 +120,10 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
   const uint32_t bars = base + kStages * S::kStageBytes + S::kInfoBytes;
   int* tables = reinterpret_cast<int*>(after + S::kInfoBytes + S::kBarrierBytes);
   unsigned* row_top = reinterpret_cast<unsigned*>(tables + kTableInts);  // [kInfo][kTcJoined][kBM]: largest element of a row of every segment
+  float* col_inv = reinterpret_cast<float*>(row_top + kInfo * kTcJoined * kBM);  // [kInfo][kTcJoined][BN]: inverse scale of a column
   // barriers: ready[s] operands split | empty[s] MMAs done reading | raw[s] operands landed | acc_full[a] | acc_empty[a] | info_full[i] | info_empty[i] |
-  // rows_full[i] addresses and scales of a tile's rows known
-  constexpr int kRing = 3 * kStages, kBars = kRing + 5 + 3 * kInfo;
+  // rows_full[i] addresses and scales of a tile's rows known | cols_full[i] scales of its columns
+  constexpr int kRing = 3 * kStages, kBars = kRing + 5 + 4 * kInfo;
   auto ready_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (kStages + s); };
   auto raw_bar = [&](int s) { return bars + 8u * (2 * kStages + s); };
@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
   auto info_full = [&](int i) { return bars + 8u * (kRing + 5 + i); };
   auto info_empty = [&](int i) { return bars + 8u * (kRing + 5 + kInfo + i); };
   auto rows_full = [&](int i) { return bars + 8u * (kRing + 5 + 2 * kInfo + i); };
+  auto cols_full = [&](int i) { return bars + 8u * (kRing + 5 + 3 * kInfo + i); };
   unsigned char* misc = after + S::kInfoBytes + 8 * kBars;
   static_assert(8 * kBars + 16 + 4 * (kTcMaxProblems + 1) <= S::kBarrierBytes, "barriers");
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(misc);
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
     for (int s = 0; s < kStages; ++s) { mbar_init(raw_bar(s), 1); mbar_init(ready_bar(s), kSteps * S::kSplitWarps); mbar_init(empty_bar(s), 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), S::kEpilogueThreads / 32); }
     mbar_init(drain_bar, 1);
-    for (int i = 0; i < kInfo; ++i) { mbar_init(info_full(i), 1); mbar_init(rows_full(i), 33); mbar_init(info_empty(i), 2 + 2 * S::kSplitWarps + S::kEpilogueThreads / 32); }
+    for (int i = 0; i < kInfo; ++i) { mbar_init(info_full(i), 1); mbar_init(rows_full(i), 33); mbar_init(cols_full(i), 32); mbar_init(info_empty(i), 2 + 2 * S::kSplitWarps + S::kEpilogueThreads / 32); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -194,10 +195,10 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
   }
-  if (warp == 2) {
-    // -- tile scheduler
+  if (warp == 2 || warp == 3) {
+    // -- tile schedulers, every other tile each
     bool ok = true;
-    for (int i = 0, tile = blockIdx.x; ok; ++i, tile += gridDim.x) {
+    for (int i = warp - 2, tile = blockIdx.x + i * gridDim.x; ok; i += 2, tile += 2 * gridDim.x) {
       const int slot = slot_of(i);
       if (!warp_wait(info_empty(slot), phase_of(i) ^ 1u, abort_flag, batch.error, 6, batch.spin_limit)) break;
       TileSlot& d = info[slot];
@@ -208,33 +209,52 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
         if (lane == 0) {
           d.bias = P.bias ? P.bias + t.group * P.bias_group_stride + t.n0 : nullptr;
           d.num_k = P.num_k; d.seg0 = P.seg0; d.atom0 = t.atom0; d.n0 = t.n0; d.group = t.group;
-          d.rows = rows; d.accumulate = P.accumulate; d.column = t.group * P.N + t.n0;
+          d.rows = rows; d.accumulate = P.accumulate;
           mbar_arrive(info_full(slot));  // the producer and the issuer can begin
         }
-        // The largest elements come in asynchronously and count as arrivals of their own: waited for here, they were the longest step of a tile
-        // (8 000 cycles under load, against 6 000 for the products of K = 512).
+        // A tile's description is the longest step of tiles with few rows and K steps, so two warps work on it in turn, and nothing here waits
+        // for memory before all of it has been asked for: the map of the result rows, the largest elements of the rows, the scales of the columns.
+        // The last two come in asynchronously and count as arrivals of their own; the splitters do not wait for the scales of the columns, which may
+        // come from DRAM.  89 elements, way back through the coefficients, K = 128 (1 480 atoms): 85 us with one warp, 63 with two.
+        int atom[kBM / 32], comp[kBM / 32], to[kBM / 32];
+        bool valid[kBM / 32];
 #pragma unroll
         for (int k = 0; k < kBM / 32; ++k) {
-          const int r = k * 32 + lane, al = r / P.q, m = r - al * P.q;
-          const bool valid = r < rows && t.atom0 + al < t.atom_end;
-          long long atom = t.atom0 + al;
-          for (int g = 0; g < P.n_seg; ++g) {
-            const TcSegment& G = batch.seg[P.seg0 + g];
-            unsigned* top = row_top + (slot * kTcJoined + g) * kBM + r;
-            if (valid) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(top)), "l"(G.a_top + atom * G.a_top_stride) : "memory");
-            else *top = 0u;
-          }
-          if (valid && P.atom_map) atom = P.atom_map[atom];
-          row_addr[slot * kBM + r] = valid ? P.C + atom * P.c_s1 + (long long)m * P.c_s2 + t.n0 : nullptr;
+          const int r = k * 32 + lane, al = r / P.q;
+          comp[k] = r - al * P.q;
+          atom[k] = to[k] = t.atom0 + al;
+          valid[k] = r < rows && atom[k] < t.atom_end;
+          if (valid[k] && P.atom_map) to[k] = P.atom_map[atom[k]];
         }
+        for (int g = 0; g < P.n_seg; ++g) {
+          const unsigned* from = batch.seg[P.seg0 + g].a_top;
+          const int stride = batch.seg[P.seg0 + g].a_top_stride;
+          unsigned* top = row_top + (slot * kTcJoined + g) * kBM + lane;
+#pragma unroll
+          for (int k = 0; k < kBM / 32; ++k) {
+            if (valid[k]) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(top + 32 * k)), "l"(from + (long long)atom[k] * stride) : "memory");
+            else top[32 * k] = 0u;
+          }
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(rows_full(slot)) : "memory");
+        if (lane < BN / 4) {
+          const long long column = (long long)t.group * P.N + t.n0 + 4 * lane;
+          for (int g = 0; g < P.n_seg; ++g)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(col_inv + (slot * kTcJoined + g) * BN + 4 * lane)),
+                         "l"(batch.seg[P.seg0 + g].b_inv + column) : "memory");
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(cols_full(slot)) : "memory");
+#pragma unroll
+        for (int k = 0; k < kBM / 32; ++k)
+          row_addr[slot * kBM + k * 32 + lane] = valid[k] ? P.C + (long long)to[k] * P.c_s1 + (long long)comp[k] * P.c_s2 + t.n0 : nullptr;
       } else {
         if (lane == 0) {
           d.num_k = 0;
           mbar_arrive(info_full(slot));
         }
         ok = false;
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(rows_full(slot)) : "memory");
       }
-      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(rows_full(slot)) : "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(rows_full(slot));
     }
@@ -396,14 +416,15 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
       if (!warp_wait(rows_full(slot), phase_of(i), abort_flag, batch.error, 6, batch.spin_limit)) break;
       const int num_k = info[slot].num_k;
       if (num_k == 0) break;
+      if (!warp_wait(cols_full(slot), phase_of(i), abort_flag, batch.error, 6, batch.spin_limit)) break;
       const float* bias = info[slot].bias;
       const bool accumulate = info[slot].accumulate != 0;
       const TcSegment* G = &batch.seg[info[slot].seg0];
       const unsigned* tops = row_top + slot * kTcJoined * kBM + r0;
       int left = G->num_k;
-      const int column = info[slot].column + half * HN + 2 * (lane & 3);  // this lane's first one, as tmem_ld_rows leaves them
+      const float* w_inv = col_inv + slot * kTcJoined * BN + half * HN + 2 * (lane & 3);  // from this lane's first column on, as tmem_ld_rows leaves them
       for (int ks = 0; ks < num_k; ++chunk) {
-        if (left == 0) { left = (++G)->num_k; tops += kBM; }
+        if (left == 0) { left = (++G)->num_k; tops += kBM; w_inv += BN; }
         const int n = left < kSteps * kFp16Chunk ? left : kSteps * kFp16Chunk;
         const bool first = ks == 0;
         ks += n; left -= n;
@@ -416,20 +437,20 @@ __global__ void __launch_bounds__(Fp16Smem<BN>::kThreads, 1) tc_gemm_fp16_kernel
         for (int k = 0; k < 4; ++k) fp16_scale(__uint_as_float(tops[8 * k]), f[k]);
 #pragma unroll
         for (int c = 0; c < HN / 32; ++c) {
-          float2 w_inv[4];
+          float v[2][16];
+          float2 w[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) w_inv[k] = __ldg(reinterpret_cast<const float2*>(G->b_inv + column + 32 * c + 8 * k));
+          for (int h = 0; h < 2; ++h) tmem_ld_rows(acc + ((uint32_t)(16 * h) << 16) + 32 * c, v[h]);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            float v[16];
-            tmem_ld_rows(acc + ((uint32_t)(16 * h) << 16) + 32 * c, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          for (int k = 0; k < 4; ++k) w[k] = *reinterpret_cast<const float2*>(w_inv + 32 * c + 8 * k);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
-              const float x = v[q] * f[2 * h + (q >> 1 & 1)];  // exact, as the other product: powers of two
-              sum[h][c][q] = fmaf(x, q & 1 ? w_inv[q >> 2].y : w_inv[q >> 2].x, first ? 0.f : sum[h][c][q]);
+              const float x = v[h][q] * f[2 * h + (q >> 1 & 1)];  // exact, as the other product: powers of two
+              sum[h][c][q] = fmaf(x, q & 1 ? w[q >> 2].y : w[q >> 2].x, first ? 0.f : sum[h][c][q]);
             }
-          }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
