@@ -929,12 +929,10 @@ struct Model : ModelBase {
       lb.As = ar.take<T>((size_t)NL * D * C);
       lb.gAs = ar.take<T>((size_t)NL * D * C);
       lb.gout_s = ar.take<T>((size_t)NL * p.Dout * C);
-      const bool tops = kTensorCore && folded && !bilinear && cfg.correlation == 2 && pb_tops(C);
-      lb.top = tops ? ar.take<unsigned>((size_t)NL * 3 * (L + 1)) : nullptr;
-      lb.gtop = tops ? ar.take<unsigned>((size_t)NL * (L + 1)) : nullptr;
-      const bool down_tops = kTensorCore && folded && rt_K && !density && pb_tops(C);
-      lb.mtop = down_tops && tp_wide_channels(C) ? ar.take<unsigned>((size_t)NL * (L + 1)) : nullptr;
-      lb.dtop = down_tops ? ar.take<unsigned>((size_t)NL * (L + 1)) : nullptr;
+      lb.top = fp16_species(false) ? ar.take<unsigned>((size_t)NL * 3 * (L + 1)) : nullptr;
+      lb.gtop = fp16_species(true) ? ar.take<unsigned>((size_t)NL * (L + 1)) : nullptr;
+      lb.mtop = fp16_down(false) ? ar.take<unsigned>((size_t)NL * (L + 1)) : nullptr;
+      lb.dtop = fp16_down(true) ? ar.take<unsigned>((size_t)NL * (L + 1)) : nullptr;
       lb.hs = p.has_res ? ar.take<T>((size_t)NL * p.Din * C) : nullptr;
       lb.out = folded ? nullptr : ar.take<T>((size_t)NL * p.Dout * C);
       lb.h_out = ar.take<T>((size_t)N * p.Dout * C);
@@ -1097,6 +1095,12 @@ struct Model : ModelBase {
   // energy of an alloy (rank 3, 128 channels, 2 048 atoms: 3.6e-5 off double precision; 1.6e-5 with FP16 for the coefficients, 4.2e-5 for
   // linear_down, 2.1e-5 for both).  With 64 channels and fewer most K loops of the backward pass are too short.
   bool fp16_nodes(bool backward) const { return folded && (backward ? C >= 128 : n_el > kFewElements); }
+  // What can reach the two kinds of them: the kernels that note the largest elements are those of the second-order product and of the tables of
+  // radial weights.
+  bool fp16_species(bool backward) const { return kTensorCore && fp16_nodes(backward) && !bilinear && cfg.correlation == 2 && pb_tops(C); }
+  bool fp16_down(bool backward) const {
+    return kTensorCore && fp16_nodes(backward) && rt_K && !density && pb_tops(C) && (backward || tp_wide_channels(C));
+  }
   // linear_down of a layer (1/avg_num_neighbors folded into the weights) and the way back through it, where the gradient of the messages
   // overwrites the messages
   std::vector<LinSpec> down_specs(const LayerPlan& p, const LayerBufs& lb, const std::string& pre, bool backward) const {
@@ -1117,7 +1121,7 @@ struct Model : ModelBase {
   // Their rows' largest elements where these linears take FP16 parts (after the per-species linears): rank 3, 128 channels, 64 crystals 2 566 -> 2 483
   // us, energies of 33 729 -> 722; backward only, 32 400 water atoms, both together 45 190 -> 44 800.
   unsigned* down_tops(std::vector<LinSpec>& sp, unsigned* top, long long n_atoms, bool backward) const {
-    if (!top || !fp16_nodes(backward) || small_call(sp, n_atoms, 1) || !long_loops(sp)) return nullptr;
+    if (!top || !fp16_down(backward) || small_call(sp, n_atoms, 1) || !long_loops(sp)) return nullptr;
     for (int l = 0; l <= L; ++l) { sp[l].a_top = top + l; sp[l].a_top_stride = L + 1; }
     return top;
   }
@@ -1126,7 +1130,7 @@ struct Model : ModelBase {
   // parts): 64 of them 2 662 -> 2 566 us, 16 1 118 -> 1 057, energies of 33 769 -> 729; backward with two elements, and linear_down: 1 536 atoms 2 461 ->
   // 2 426.
   unsigned* species_tops(std::vector<SpeciesSpec>& sp, unsigned* top, long long n_atoms, bool backward) const {
-    if (!top || !fp16_nodes(backward) || small_call(sp, n_atoms, n_el) || !long_loops(sp)) return nullptr;
+    if (!top || !fp16_species(backward) || small_call(sp, n_atoms, n_el) || !long_loops(sp)) return nullptr;
     set_tops(sp, top, backward ? 1 : 3);
     return top;
   }

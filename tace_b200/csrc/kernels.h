@@ -104,7 +104,8 @@ template <typename T> cudaError_t launch_gate_bwd(const T* Gt, const T* ga, T* g
 // L: rank of A; Lout: highest output rank, or < 0 for scalar outputs only (the last layer)
 // top (fp32, pb_tops(C)): rows of top_stride, receives the bits of the largest |element| of every atom's rows of A, rank by rank, and of B2, those from L + 1 on
 template <typename T> cudaError_t launch_pb_fwd(const T* A, T* B2, int n, int L, int Lout, int C, cudaStream_t s, unsigned* top = nullptr, int top_stride = 0);
-inline bool pb_tops(int C) { return C == 32 || C == 64 || C == 128; }
+// (an atom's threads share a block of 128, and the linears that read the result have widths of 64 and more)
+inline bool pb_tops(int C) { return C == 64 || C == 128; }
 template <typename T> cudaError_t launch_pb_bwd(const T* A, const T* gB2, T* gA, int n, int L, int Lout, int C, cudaStream_t s);
 // gated bilinear product (product_basis.nonlinear = silu_bilineargate): XY [n][D][2C] holds both factors (channels [0, C) /
 // [C, 2C)), Zg [n][NP][C] the gate pre-activations; B2 = silu(Zg) * (x (x) [y, 1]).  bwd: gXY[.., :C] += , gXY[.., C:] = ,

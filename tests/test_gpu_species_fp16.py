@@ -56,3 +56,32 @@ def test_ranks_of_every_magnitude(power, where):
     assert torch.isfinite(before["forces"]).all()
     for k, v in before.items():
         assert torch.equal(after[k], v), k
+
+
+def _launched(model, data):
+    """Names of the kernels of one evaluation."""
+    model.set_graph_mode(False)
+    model(data)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        model(data)
+        torch.cuda.synchronize()
+    return [e.name for e in prof.events()]
+
+
+@pytest.mark.parametrize("channels,structs,cutoff,zs,forward,backward", [
+    (128, lambda: synth.random_crystals(4, seed=31, nmin=9, nmax=23, zmax=20), 4.5, MANY, True, True),
+    (64, lambda: synth.random_crystals(5, seed=32, nmin=20, nmax=40, zmax=20), 4.0, MANY, True, False),
+    (32, lambda: synth.random_crystals(9, seed=33, nmin=38, nmax=44, zmax=20), 3.5, MANY, False, False),
+    (128, lambda: [synth.fcc_supercell(4, 3.65, 0.05, seed=5, species=(13, 29), fractions=(0.02, 0.98))], 4.0, [13, 29], False, True),
+])
+def test_largest_elements_are_noted_where_a_linear_reads_them(channels, structs, cutoff, zs, forward, backward):
+    """The kernel on FP16 parts runs in both directions with 128 channels and many elements, forward only with 64 channels, backward only with two
+    elements, and not with 32 channels (whose linears are too narrow); without it no row gather looks for largest elements."""
+    model, _, _ = make_models(3, channels, zs, cutoff, 20.0, torch.float32, num_layers=3)  # (the second of three has all ranks and a skip connection)
+    names = _launched(model, to_device(oracle_batch(structs(), zs, cutoff, torch.float32), torch.device("cuda:0")))
+    middle = next(i for i, n in enumerate(names) if "tp_bwd" in n)  # (the readout and the last products lie before it in both directions)
+    first = next(i for i, n in enumerate(names) if "readout_kernel" in n)
+    assert first < middle
+    assert any("tc_gemm_fp16_kernel" in n for n in names[:first]) == forward
+    assert any("tc_gemm_fp16_kernel" in n for n in names[first:]) == backward
+    assert any("gather_rows_top_kernel" in n for n in names[:first]) <= forward and any("gather_rows_top_kernel" in n for n in names[first:]) == backward
