@@ -473,12 +473,13 @@ struct Model : ModelBase {
     add_weight(name, numel);
     if (kTensorCore) { add_weight(name + "_hi", numel); add_weight(name + "_lo", numel); }
   }
-  // The same for a [K][N] matrix per group, X, and its transpose, which linears on FP16 parts may read (each that of the other direction)
-  void add_packed_weight(const std::string& name, const std::string& nameT, int groups, long long K, long long N, bool tiled) {
+  // The same for a [K][N] matrix per group, X, which the linears of the backward pass read, and its transpose, which those of the forward pass do;
+  // backward, forward: whether they may take FP16 parts.  Every other array would be packed for nothing.
+  void add_packed_weight(const std::string& name, const std::string& nameT, int groups, long long K, long long N, bool tiled, bool backward, bool forward) {
     add_linear_weight(name, groups * K * N);
     add_linear_weight(nameT, groups * K * N);
-    if (kTensorCore && tc_linear_supported((int)K, (int)N)) pack_shapes[name] = {groups, (int)K, (int)N, tiled};
-    if (kTensorCore && tc_linear_supported((int)N, (int)K)) pack_shapes[nameT] = {groups, (int)N, (int)K, tiled};
+    if (kTensorCore && backward && tc_linear_supported((int)K, (int)N)) pack_shapes[name] = {groups, (int)K, (int)N, tiled};
+    if (kTensorCore && forward && tc_linear_supported((int)N, (int)K)) pack_shapes[nameT] = {groups, (int)N, (int)K, tiled};
   }
   // What the tensor cores read of them: "X_pk", FP16 parts of X_hi + X_lo with every column of the result scaled by a power of two, and behind
   // them the inverse scales.
@@ -519,7 +520,7 @@ struct Model : ModelBase {
     density = c.scatter_norm_density;
     res_identity = c.resnet_identity != 0;
     bilinear = c.product_bilinear != 0;
-    tece_mask = c.tece_layers; mmax = c.mmax; heads = c.num_head > 0 ? c.num_head : 1;
+    tece_mask = c.tece_layers; folded = tece_mask == 0; mmax = c.mmax; heads = c.num_head > 0 ? c.num_head : 1;
     rt_K = c.radial_table;
     if (rt_K < 0 || (rt_K > 0 && (!std::is_same<T, float>::value || element2 || tece_mask || rt_K > (1 << 16))))
       return TACE_ERR_UNSUPPORTED_CONFIG;
@@ -601,7 +602,7 @@ struct Model : ModelBase {
           const So2Shape sh = so2_shape(i);
           for (int m = 0; m <= sh.mm; ++m) {
             add_packed_weight(pre + "so2." + sh.name + ".m" + std::to_string(m), pre + "so2." + sh.name + "T.m" + std::to_string(m), 1,
-                              (long long)sh.n_in[m] * sh.c_in, (long long)sh.n_out[m] * sh.c_out, false);
+                              (long long)sh.n_in[m] * sh.c_in, (long long)sh.n_out[m] * sh.c_out, false, true, true);
           }
           add_weight(pre + "so2." + sh.name + ".b", (long long)sh.n_out[0] * sh.c_out);
         }
@@ -629,7 +630,8 @@ struct Model : ModelBase {
       }
       for (int l = 0; l <= L; ++l) {
         const long long outl = (l == 0) ? (long long)(L + 1 + m0) * C : C;
-        add_packed_weight(pre + "down.l" + std::to_string(l), pre + "downT.l" + std::to_string(l), 1, (long long)p.tp.k[l] * C, outl, false);
+        add_packed_weight(pre + "down.l" + std::to_string(l), pre + "downT.l" + std::to_string(l), 1, (long long)p.tp.k[l] * C, outl, false,
+                          fp16_down(true), fp16_down(false));
         add_linear_weight(pre + "nl.l" + std::to_string(l), (long long)C * C);
         add_linear_weight(pre + "nlT.l" + std::to_string(l), (long long)C * C);
       }
@@ -638,8 +640,9 @@ struct Model : ModelBase {
       for (size_t i = 0; i < p.out_ls.size(); ++i) {
         const int l = p.out_ls[i];
         const std::string ls = std::to_string(l);
-        add_packed_weight(pre + "c0.l" + ls, pre + "c0T.l" + ls, n_el, C, C, true);
-        if (cfg.correlation >= 2) add_packed_weight(pre + "c1.l" + ls, pre + "c1T.l" + ls, n_el, (long long)p.pb.k[i] * C, C, true);
+        add_packed_weight(pre + "c0.l" + ls, pre + "c0T.l" + ls, n_el, C, C, true, fp16_species(true), fp16_species(false));
+        if (cfg.correlation >= 2)
+          add_packed_weight(pre + "c1.l" + ls, pre + "c1T.l" + ls, n_el, (long long)p.pb.k[i] * C, C, true, fp16_species(true), fp16_species(false));
         if (cfg.correlation >= 3) {
           add_linear_weight(pre + "c2.l" + ls, (long long)n_el * p.pb3.k[i] * C * C);
           add_linear_weight(pre + "c2T.l" + ls, (long long)n_el * p.pb3.k[i] * C * C);
@@ -647,7 +650,7 @@ struct Model : ModelBase {
         add_linear_weight(pre + "lin.l" + ls, (long long)C * C);
         add_linear_weight(pre + "linT.l" + ls, (long long)C * C);
         if (p.has_res && !res_identity) {
-          add_packed_weight(pre + "res.l" + ls, pre + "resT.l" + ls, n_el, C, C, true);
+          add_packed_weight(pre + "res.l" + ls, pre + "resT.l" + ls, n_el, C, C, true, fp16_species(true), fp16_species(false));
         }
       }
       if (bilinear) {  // linear_up of the product: every rank to both factors, the scalars also to the gates
@@ -673,7 +676,6 @@ struct Model : ModelBase {
     if (zbl) { add_weight("zbl.z", n_el); add_weight("zbl.rcov", n_el); add_weight("zbl.par", 2); }
     n_listed = n_unset = (int)weights.size();
     for (const auto& e : pack_shapes) add_weight(e.first + "_pk", (long long)e.second.groups * e.second.N * (e.second.K + 1));
-    folded = tece_mask == 0;
     if (folded) add_weight("emb_up", (long long)n_el * C);
     for (int t = 0; t < NL_ && folded; ++t)
       for (int l : layers[t].out_ls) {

@@ -85,3 +85,18 @@ def test_largest_elements_are_noted_where_a_linear_reads_them(channels, structs,
     assert any("tc_gemm_fp16_kernel" in n for n in names[:first]) == forward
     assert any("tc_gemm_fp16_kernel" in n for n in names[first:]) == backward
     assert any("gather_rows_top_kernel" in n for n in names[:first]) <= forward and any("gather_rows_top_kernel" in n for n in names[first:]) == backward
+
+
+@pytest.mark.parametrize("channels,zs,tece,packed", [
+    (64, [13, 29], None, 0),     # no linear takes FP16 parts
+    (128, [13, 29], None, 19),   # those of the backward pass: 4 + 4 of linear_down; 4 + 1 of either order of the coefficients, which are folded; 1 skip connection
+    (64, [13, 29], {"num_head": 4, "edge_ace_hidden": 64, "mmax": 1}, 22),  # the edge block: key, query, up, glu and down of two orders, the coefficients of one, both ways
+])
+def test_packed_copies_are_made_of_what_can_be_read(channels, zs, tece, packed):
+    kw = dict(radial={"apply_cutoff": False}, tece=tece) if tece else {}
+    model, _, _ = make_models(3, channels, zs, 4.0, 20.0, torch.float32, **kw)
+    data = to_device(oracle_batch([synth.fcc_supercell(2, 3.65, 0.05, seed=5, species=(13, 29), fractions=(0.5, 0.5))], zs, 4.0, torch.float32), torch.device("cuda:0"))
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        model(data)  # the weights are set with the first evaluation
+        torch.cuda.synchronize()
+    assert sum("tc_pack_kernel" in e.name for e in prof.events()) == packed
