@@ -1,11 +1,13 @@
 """The node linears on FP16 parts of scaled operands (fp32 models without the edge block): calls beyond the limit of the CUDA cores, one to four
 warps per atom in the kernels that note the largest elements, ranks whose tiles are 126 rows, species with one row, a few and several
 tiles, with and without a skip connection, and the backward pass alone (two elements)."""
+import numpy as np
 import pytest
 import torch
 
 from helpers import make_models, oracle_batch, to_device
 from tace_b200 import synth
+from tace_b200.md import DomainMD
 from tace_b200.pack import LayerPlan
 from test_gpu_parity import run_case
 
@@ -100,3 +102,38 @@ def test_packed_copies_are_made_of_what_can_be_read(channels, zs, tece, packed):
         model(data)  # the weights are set with the first evaluation
         torch.cuda.synchronize()
     assert sum("tc_pack_kernel" in e.name for e in prof.events()) == packed
+
+
+def test_linear_down_over_chunks_of_edges():
+    """The largest elements of the messages are noted chunk by chunk; the linear then reads them for all atoms."""
+    structs = synth.random_crystals(5, seed=32, nmin=20, nmax=40, zmax=20)
+    model, _, _ = make_models(3, 128, MANY, 4.5, 20.0, torch.float32)
+    data = to_device(oracle_batch(structs, MANY, 4.5, torch.float32), torch.device("cuda:0"))
+    count = lambda names: sum("tc_gemm_fp16_kernel" in n for n in names)
+    launches = count(_launched(model, data))
+    whole = {k: v.clone() for k, v in model(data).items() if v is not None}
+    assert data["edge_index"].shape[1] > 3 * 1024
+    model.set_chunk_edges(1024)
+    assert count(_launched(model, data)) == launches > 4
+    out = model(data)
+    for k, v in whole.items():
+        assert (out[k] - v).abs().max().item() <= 2e-5 * max(1.0, v.abs().max().item()), k
+    assert model.device_error() == 0
+
+
+def test_linear_down_with_the_targets_in_two_parts():
+    """With the exchange on its own stream the forward contraction runs over the targets without a ghost neighbour first and over the others
+    afterwards, and both parts note their rows: the energy is that of the serial exchange, bit for bit."""
+    s = synth.fcc_supercell(4, 3.61, 0.05, seed=21, species=tuple(MANY), fractions=(0.05,) * 20)
+    model, oracle, _ = make_models(3, 128, MANY, 4.0, 20.0, torch.float32, targets=("energy", "forces"))
+    ref = oracle(oracle_batch([s], MANY, 4.0, torch.float32))
+    model, energy = model.to(torch.device("cuda:0")), []
+    for overlap in (False, True):
+        model.set_exchange_overlap(overlap)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            md = DomainMD(model, s["cell"], s["positions"], s["atomic_numbers"], masses=np.ones(len(s["positions"])), skin=0.4, device=torch.device("cuda:0"))
+            energy.append(md.potential())
+        assert md.domain.n_ghost > 0 and any("tc_gemm_fp16_kernel" in e.name for e in prof.events())
+        assert abs(energy[-1] - float(ref["energy"][0])) / len(s["positions"]) < 1e-5
+        assert (torch.as_tensor(md.gather()["forces"]) - ref["forces"].detach().double().cpu()).abs().max().item() < 1e-4
+    assert energy[0] == energy[1] and model.device_error() == 0
