@@ -164,8 +164,8 @@ void tace_destroy(TaceModel* model);
  * transposes and the TF32 parts of the product's per-species coefficients ("tN.cJT.lL" and every
  * "tN.cJ.lL_hi", "tN.cJ.lL_lo", "tN.cJT.lL_hi", "tN.cJT.lL_lo") from "tN.cJ.lL" and "tN.lin.lL", which it
  * multiplies.  They are listed and have to be set once, with the listed size, but their content is not
- * read: to change coefficients set "tN.cJ.lL".  Besides, the library keeps FP16 parts of every array that comes as
- * "X_hi" and "X_lo" (fp32 models), taken again whenever one of the two is set. */
+ * read: to change coefficients set "tN.cJ.lL".  Besides, the library keeps FP16 parts of those arrays that come as
+ * "X_hi" and "X_lo" (fp32 models) and that some linear may read in this form, taken again whenever one of the two is set. */
 int tace_weight_count(const TaceModel* model);
 int tace_weight_info(const TaceModel* model, int index, const char** name, int64_t* numel);
 int tace_set_weight(TaceModel* model, const char* name, const void* host_data, int64_t numel);
@@ -250,7 +250,7 @@ int tace_tc_gemm_f32(const float* A, int64_t lda, const float* B_hi, const float
                      int32_t N, int32_t K, int32_t* error_flag, tace_stream_t stream);
 /* The same product on FP16 parts of operands scaled by powers of two, which tace_forward takes for the linears of the edge block and, of the
  * larger fp32 models, of the nodes: C = bias + sum over the operands i of A_i[n_atoms][q][K_i] @ B_i[N][K_i]^T (C[n_atoms][q][N], added to what
- * it holds with `accumulate`).  A_top holds the bits of the largest |element| of every atom's q rows; joined operands have the same.  B_packed
+ * it holds with `accumulate`).  A_top holds the bits of the largest |element| of every atom's q rows; up to three operands.  B_packed
  * (N * K + N floats per group) receives the parts of B_hi + B_lo.  n_groups > 0: atoms [group_ptr[g], group_ptr[g + 1]) take the matrix g,
  * whose parts are K-tile-major [K / 32][N][32], and bias[g][N]; tile_ptr counts the groups' tiles of 128 / q atoms (device arrays of
  * n_groups + 1).  Rows and pointers as above; `error_flag` also receives 6, a wait for the description of a tile. */

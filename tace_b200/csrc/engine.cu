@@ -707,7 +707,7 @@ struct Model : ModelBase {
   // double precision 749 -> 730.  Models with the edge block keep their linears apart: their energies feel the rounding of a linear
   // most (2.2e-5 between the two forms, where the others move by 3e-6).
   //   cJ.lL [n_el][K][C] stays as it was set; cJf.lL is the folded matrix, cJT.lL its transpose, cJ.lL_hi/_lo and cJT.lL_hi/_lo the
-  //   K-tile-major TF32 parts of both (packed for the tensor cores like every other) (what the caller sets under these names is the same before folding, and is not kept).
+  //   K-tile-major TF32 parts of both, from which the packed ones are taken (what the caller sets under these names is the same before folding, and is not kept).
   static std::string coef_name(int t, int order, const char* form, int l) {
     return "t" + std::to_string(t) + ".c" + std::to_string(order) + form + ".l" + std::to_string(l);
   }
@@ -1093,9 +1093,12 @@ struct Model : ModelBase {
     return tc_fp16_pays(results, steps);
   }
   // Which linears of the nodes take FP16 parts.  Those of models with the edge block do not: their energies move by 4e-5 with the rounding.  Nor do
-  // those of the forward pass with few elements: the weights come out of L2 there, and the errors of the TF32 linears cancel in part in the
-  // energy of an alloy (rank 3, 128 channels, 2 048 atoms: 3.6e-5 off double precision; 1.6e-5 with FP16 for the coefficients, 4.2e-5 for
-  // linear_down, 2.1e-5 for both).  With 64 channels and fewer most K loops of the backward pass are too short.
+  // those of the forward pass with few elements: that line is drawn to keep the results, not for time or exactness.  Energies of such models move by
+  // more with the kernel (rank 3, 128 channels, alloy of 2 048 atoms: 3.6e-5 off double precision, 2.1e-5 with FP16 for both kinds of linears) than
+  // from one build to the next.  On the other side of it FP16 would be a little faster and closer to double precision: 64 random crystals with
+  // 2, 5, 8, 16 elements 2 340, 2 343, 2 349, 2 366 us as it is and 2 299, 2 302, 2 308, 2 319 with FP16, energies off by 8e-9, 2e-9, 1e-9, 1e-9 eV an atom
+  // and 3e-9, 9e-10, 6e-10, 5e-10.  With 64 channels most K loops of the backward pass are too short; above 128 the kernels that note largest
+  // elements do not apply (pb_tops).
   bool fp16_nodes(bool backward) const { return folded && (backward ? C >= 128 : n_el > kFewElements); }
   // What can reach the two kinds of them: the kernels that note the largest elements are those of the second-order product and of the tables of
   // radial weights.
@@ -1120,17 +1123,16 @@ struct Model : ModelBase {
     }
     return sp;
   }
-  // Their rows' largest elements where these linears take FP16 parts (after the per-species linears): rank 3, 128 channels, 64 crystals 2 566 -> 2 483
-  // us, energies of 33 729 -> 722; backward only, 32 400 water atoms, both together 45 190 -> 44 800.
+  // Their rows' largest elements where these linears take FP16 parts, rank by rank (figures: species_tops).
   unsigned* down_tops(std::vector<LinSpec>& sp, unsigned* top, long long n_atoms, bool backward) const {
     if (!top || !fp16_down(backward) || small_call(sp, n_atoms, 1) || !long_loops(sp)) return nullptr;
     for (int l = 0; l <= L; ++l) { sp[l].a_top = top + l; sp[l].a_top_stride = L + 1; }
     return top;
   }
-  // Largest elements of the atoms' rows for the per-species linears (`top`, or nullptr where they are not wanted): those read their weights
-  // from DRAM, and FP16 parts are half the bytes of TF32 parts.  Random crystals of 89 elements at rank 3, 128 channels (395 MB of weights as TF32
-  // parts): 64 of them 2 662 -> 2 566 us, 16 1 118 -> 1 057, energies of 33 769 -> 729; backward with two elements, and linear_down: 1 536 atoms 2 461 ->
-  // 2 426.
+  // Largest elements of the atoms' rows for the per-species linears, by operand and rank (`top`, or nullptr where they are not wanted): those read
+  // their weights from DRAM, and FP16 parts are half the bytes of TF32 parts.  These linears and linear_down together, random crystals of 89 elements at
+  // rank 3, 128 channels (395 MB of weights as TF32 parts): 64 of them 2 641 -> 2 500 us, 16 1 121 -> 1 032, energies of 33 772 -> 722; backward only, two
+  // elements: 1 536 atoms 2 447 -> 2 407, 32 400 45.1 -> 44.6 ms.
   unsigned* species_tops(std::vector<SpeciesSpec>& sp, unsigned* top, long long n_atoms, bool backward) const {
     if (!top || !fp16_species(backward) || small_call(sp, n_atoms, n_el) || !long_loops(sp)) return nullptr;
     set_tops(sp, top, backward ? 1 : 3);

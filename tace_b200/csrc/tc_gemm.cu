@@ -7,7 +7,7 @@
 // Plain TF32 (10-bit mantissa) is too coarse for the 1e-5 eV/atom parity target, so every
 // operand is split into a TF32-exact high part and a residual, x = hi + lo, and the product is
 // accumulated as hi*hi + hi*lo + lo*hi in the FP32 TMEM accumulator (the dropped lo*lo term is
-// ~2^-22 relative).  Linears over edges, whose callers know the largest element of every row, take FP16 parts of scaled operands
+// ~2^-22 relative).  Linears whose callers know the largest element of every row take FP16 parts of scaled operands
 // instead (tc_gemm_fp16.cuh).  The weight operand B is split once on the host.  The activation operand A is split by the kernel
 // right after its TMA load: one thread per row reads the row's 128 bytes (in the swizzled order the TMA engine wrote)
 // and stores the high parts and the residuals to tensor memory, from where the tensor core takes its A operand
@@ -672,8 +672,8 @@ cudaError_t launch_tc_fp16(const TcBatch& b, int dev, int sms, cudaStream_t s) {
 static uint32_t g_test_spin_limit = 0, g_test_extra_tx = 0;
 void tc_gemm_set_test_mode(uint32_t spin_limit, uint32_t extra_tx) { g_test_spin_limit = spin_limit; g_test_extra_tx = extra_tx; }
 
-// FP16 where the results of a launch take more than three K steps on average: 75 776 x 512 rows with K = 96 take 48.0 us as TF32 and 49.4 as FP16, 526 336 x
-// 128 with K = 128 100 and 89.
+// FP16 where the results of a launch take more than three K steps on average: 75 776 x 512 rows with K = 96 take 48.0 us as TF32 and 47.9 as FP16, with
+// K = 128 55.5 and 48.1, 526 336 x 128 with K = 128 98.6 and 85.2.
 bool tc_fp16_pays(long long results, long long steps) { return steps > 3 * results; }
 bool tc_linear_supported(int N, int K) { return N % 64 == 0 && K % kBK == 0; }
 

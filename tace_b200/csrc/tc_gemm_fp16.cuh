@@ -1,31 +1,35 @@
-// The GEMM of tc_gemm.cu on FP16 operands, for linears whose caller knows the largest element of every atom's rows
-// (TcLinearProblem::a_top: the SO(2) linears over edges).  Included by tc_gemm.cu, whose barriers, tile search and tensor maps it uses.
+// The GEMM of tc_gemm.cu on FP16 operands, for linears whose caller knows the largest element of an operand's rows of every atom or edge
+// (TcLinearProblem::a_top): the SO(2) linears over edges and, of larger models without the edge block, the per-species linears and linear_down.
+// Included by tc_gemm.cu, whose barriers, tile search and tensor maps it uses.
 //
 // FP16 has the eleven mantissa bits of TF32 at twice its rate and half its bytes, and five exponent bits instead of eight; what those
 // lack is given back by powers of two: the rows that an operand has of an atom (edge) are scaled so that their largest element lies in [2^13,
 // 2^14), the weights likewise, every column of the result (of every element) by a power of its own; what shares a scale is the components of
 // one rank or order.  x = hi + lo with both parts rounded to nearest, and hi*hi + hi*lo + lo*hi is accumulated as in TF32: an element keeps its 22 bits
 // down to 2^-16 of the largest one of its row or column, and the error of a smaller one is 2^-39 of that.  The epilogue takes the scales out of
-// the sums, which is exact.  Relative error (2-norm) of 75 776 x 512 x 1 024 normal numbers 1.9e-6, 2.3e-6 as TF32; with K = 128
-// 5.4e-7 and 1.4e-6.
+// the sums, which is exact.  Relative error (2-norm) of normal numbers 5.4e-7 with K = 128, 1.9e-6 with K = 512 and more; as TF32 1.4e-6 and 2.3e-6.
 //
 // What it had to solve besides: the TF32 kernel takes .72 us per K step of a CTA with the tensor pipe busy 69 % of it, and with FP16 parts in the
 // same arrangement it still took .76.  Counted with clock64 per role: an epilogue of some 6 000 cycles a tile (each role decoding its
 // tiles, results stored through shared memory), 680 cycles per step in the splitters, some 550 in the issuer around 94 of instructions.
-// Hence a scheduler that decodes tiles ahead, two sets of splitters, results that go from registers to their rows, and two K steps per
-// stage (one wait, one commit, two loads).  Times against the TF32 kernel (us): 75 776 x 512 x 1 024 371 -> 223, x 512 177 -> 122, x 256 91 -> 73;
-// 526 336 x 128 x 128 105 -> 91; 2 048 x 128 x 384 13.3 -> 10.1.  What bounds it now: at K >= 512 the ring (192 KB in flight against some 4 000 cycles from a
-// freed stage to its next products; the pipe is busy 49 to 56 % of it), at K <= 128 the memory (5.9 TB/s).  Separate rings for A and B (228 -> 284 us at K = 1 024), L2
-// prefetch of A eight steps ahead (228 -> 239), weights as one linear copy per step (no change) and pairs of SMs
+// Hence schedulers that describe tiles ahead, two sets of splitters, results that go from registers to their rows, and two K steps per
+// stage (one wait, one commit, two loads).  Times beside the TF32 kernel's (us): 75 776 x 512 x 1 024 362 and 215, x 512 192 and 119, x 256 92 and 76, x 128
+// 56 and 48; 526 336 x 128 x 128 99 and 85; 2 048 x 128 x 384 13.3 and 9.6.  What bounds it now: at K >= 512 the ring (192 KB in flight against some
+// 4 000 cycles from a freed stage to its next products; the pipe is busy 47 to 54 % of it), at K <= 128 the memory (5.9 TB/s).  Separate rings for A and
+// B (228 -> 284 us at K = 1 024), L2 prefetch of A eight steps ahead (228 -> 239), weights as one linear copy per step (no change) and pairs of SMs
 // with half of the weights each (cta_group::2, 223 -> 285) were tried.
 //
-// One persistent CTA per SM.  Warp roles (640 threads, five warpgroups): warp 0 = TMA producer, warp 1 = MMA issuer, warps 2, 3 = tile schedulers; warps 4..7 and 8..11 = operand splitters, warps 12..15 and 16..19 = epilogue (warp w works on the TMEM lanes 32 * (w % 4) .. + 31; the
+// One persistent CTA per SM.  Warp roles (640 threads, five warpgroups): warp 0 = TMA producer, warp 1 = MMA issuer, warps 2, 3 = tile schedulers;
+// warps 4..7 and 8..11 = operand splitters, warps 12..15 and 16..19 = epilogue (warp w works on the TMEM lanes 32 * (w % 4) .. + 31; the
 // second four of the epilogue take the right half of the columns, so that 64 running sums per thread fit its registers).  Registers move from
 // the first warpgroup to the others: 40 + 2 * 104 + 2 * 112 of the 5 * 96 of the launch.  Every wait is bounded, as in tc_gemm.cu.
 #pragma once
 
-constexpr int kFp16Chunk = 8;  // stages accumulated inside TMEM before draining into FP32 registers: 96 instructions, as in TF32
-constexpr int kInfo = 6;       // tiles the scheduler is ahead
+// Stages accumulated inside TMEM before draining into FP32 registers: 96 instructions, as in TF32, which are 512 elements of K here and 256 there.
+// With four stages the error at K >= 512 is 9.8e-7 instead of 1.9e-6 (2.3e-6 as TF32), and 75 776 x 512 x 1 024 take 226.5 us instead of 220.5, the
+// linears of the edge block (526 k edges) 27.5 ms instead of 27.0.
+constexpr int kFp16Chunk = 8;
+constexpr int kInfo = 6;       // tiles the schedulers are ahead
 constexpr int kTableInts = TcSmem<128>::kTableInts;
 
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {

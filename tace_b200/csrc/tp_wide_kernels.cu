@@ -231,18 +231,21 @@ __device__ __forceinline__ void wide_fwd_group(const TPArgs<float>& a, int i, in
   }
   if (i < 0) return;
   float* Mi = a.M + (long long)i * TP::NM * C + c0 + 2 * lane;
-  float most[TP::L + 1];  // per rank
-#pragma unroll
-  for (int l = 0; l <= TP::L; ++l) most[l] = 0.0f;
 #pragma unroll
   for (int k = 0; k < NOUT; ++k)
 #pragma unroll
-    for (int v = 0; v < kPairs; ++v) {
-      st_pair(Mi + TP::template vmap<GRP>(k) * C + 64 * v, acc[k][v]);
-      const int l = TP::rank_of(TP::template vmap<GRP>(k));
-      most[l] = fmaxf(most[l], fmaxf(fabsf(acc[k][v].x), fabsf(acc[k][v].y)));
-    }
+    for (int v = 0; v < kPairs; ++v) st_pair(Mi + TP::template vmap<GRP>(k) * C + 64 * v, acc[k][v]);
   if (a.top) {  // (a uniform branch: all lanes of the warp are here)
+    float most[TP::L + 1];  // per rank
+#pragma unroll
+    for (int l = 0; l <= TP::L; ++l) most[l] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NOUT; ++k)
+#pragma unroll
+      for (int v = 0; v < kPairs; ++v) {
+        const int l = TP::rank_of(TP::template vmap<GRP>(k));
+        most[l] = fmaxf(most[l], fmaxf(fabsf(acc[k][v].x), fabsf(acc[k][v].y)));
+      }
     unsigned mine = 0u;
 #pragma unroll
     for (int l = 0; l <= TP::L; ++l) {
