@@ -86,6 +86,23 @@ def test_against_double_precision(N, atoms, q, K):
     assert error(got, exact(operands, bias)) < tolerance(K)
 
 
+@pytest.mark.parametrize("N", [64, 128])
+@pytest.mark.parametrize("tiles,extra", [(1, -128), (1, 1), (2, 0), (5, 1), (6, 0), (6, 1), (7, 0), (13, 1)])
+def test_tiles_of_a_block(N, tiles, extra):
+    """Two warps describe every other tile of a block, six of them ahead: blocks with no tile, one to seven and thirteen, and blocks with one more
+    than others."""
+    sms = torch.cuda.get_device_properties(DEV).multi_processor_count
+    rows = 128 * sms * tiles + extra
+    A, W = normal(rows, 1, 32, seed=21), normal(1, N, 32, seed=22)
+    call = Call([(A, W)])
+    got = call()
+    assert int(call.err.item()) == 0
+    want = (A.to(DEV).double() @ W[0].to(DEV).double().T).cpu()
+    for first in range(0, rows, 128 * sms):  # every row is looked at, and a wrong tile is not lost among the others
+        part = slice(first, first + 128 * sms)
+        assert error(got[part], want[part], dim=(1, 2)) < 2 * tolerance(32)
+
+
 def test_the_kernel_is_the_one_on_fp16_parts():
     call = Call([(normal(300, 1, 128), normal(1, 128, 128, seed=1))])
     call()
